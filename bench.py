@@ -368,7 +368,7 @@ def step_timeline(args) -> dict:
         trace = json.load(open(tf.name))
     ks = sorted((e for e in trace["traceEvents"] if e.get("cat") == "kernel"), key=lambda e: e["ts"])
     short = lambda n: re.sub(r"capsb::(\(anonymous namespace\)::)?", "", re.sub(r"^void ", "", n)).split("(")[0]
-    starts = [e["ts"] for e in ks if "k_nhc_begin" in e["name"]]
+    starts = [e["ts"] for e in ks if "k_move" in e["name"]]
     rows: dict = {}
     for e in ks:
         i = bisect.bisect_right(starts, e["ts"]) - 1

@@ -36,6 +36,8 @@ enum ErrorBits : unsigned {
   kErrRattle = 1u << 11,          // RATTLE (the velocity constraints) did not converge
   kErrLincs = 1u << 12,           // LINCS's rotational corrections did not converge
   kErrConsOverlap = 1u << 13,     // two constrained atoms on each other (LINCS takes their direction)
+  kErrListWait = 1u << 14,        // a wait inside the list kernel gave up
+  kErrListBad = kErrListOverflow | kErrMaskOverflow | kErrScOverflow | kErrColumnTooBig | kErrExclOverflow | kErrListWait,   // no list to use
 };
 
 // What the first failure of a kind leaves for the host's message (the engine's error-detail array, doubles): the

@@ -28,7 +28,7 @@ void Engine::time_pair_kernel(const double* x, const double* cell, int launches,
     if (flush_bytes > 0) cudaMemsetAsync(d_flush_.p, k & 255, size_t(flush_bytes), stream_);
     if (mixed_) cudaMemsetAsync(d_Fs_.p, 0, d_Fs_.n * sizeof(long long), stream_);
     else cudaMemsetAsync(d_Fsd_.p, 0, d_Fsd_.n * sizeof(double), stream_);
-    cudaMemsetAsync(d_counters_.p + kCntPairNext, 0, sizeof(int), stream_);   // the pack kernel resets it in a force evaluation
+    cudaMemsetAsync(d_counters_.p + kCntPairNext, 0, sizeof(int), stream_);   // the list kernel resets it in a force evaluation
     cudaEventRecord(ev[size_t(2 * k)], stream_);
     pair_forces(false, false);
     cudaEventRecord(ev[size_t(2 * k + 1)], stream_);
@@ -47,7 +47,7 @@ void Engine::time_pair_kernel(const double* x, const double* cell, int launches,
 
 // The force evaluation's branches timed one at a time, then together (force-only, as on a plain MD step; the list is
 // built once first and kept): ms[0] the bonded branch (bonded terms, 1-4 pairs, excluded-pair corrections), ms[1] PME,
-// ms[2] the short-range evaluation (displacement check, pack, prune check, pair kernel, and its 1-4 branch), ms[3] the
+// ms[2] the short-range evaluation (displacement check, list kernel, pair kernel, and its 1-4 branch), ms[3] the
 // whole evaluation. Each is the mean over `launches` repetitions, CUDA events on the engine's stream, an L2 flush of
 // flush_bytes before each.
 void Engine::time_phases(const double* x, const double* cell, int launches, int64_t flush_bytes, double* ms) {

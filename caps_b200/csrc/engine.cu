@@ -123,15 +123,15 @@ Engine::Engine(const caps_gpu_ff* ff, const caps_gpu_opts* o) {
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&dev_sms_, cudaDevAttrMultiProcessorCount, dev));
   CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
-  // the main stream (integrator, list, pack, prune, pair kernel) runs at the highest priority, PME's chain of dependent
-  // launches one level below and the bonded terms at the lowest: the chain that leads to the pair kernel takes SM
-  // slots first, then PME's, and the bonded blocks fill what they leave
+  // PME's chain of dependent launches runs at the highest priority: its kernels are short and bound by latency, and one
+  // that waits for the pair kernel's persistent blocks to end holds up the whole chain. The main stream (integrator, list,
+  // pair kernel) is one level below, and the bonded blocks fill what the two leave
   int prio_lo = 0, prio_hi = 0;
   CK(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi));
   CK(cudaStreamDestroy(stream_));
-  CK(cudaStreamCreateWithPriority(&stream_, cudaStreamNonBlocking, prio_hi));
+  CK(cudaStreamCreateWithPriority(&stream_, cudaStreamNonBlocking, prio_hi < prio_lo ? prio_hi + 1 : prio_lo));
   CK(cudaStreamCreateWithPriority(&side_[0], cudaStreamNonBlocking, prio_lo));
-  CK(cudaStreamCreateWithPriority(&side_[1], cudaStreamNonBlocking, prio_hi < prio_lo ? prio_hi + 1 : prio_lo));
+  CK(cudaStreamCreateWithPriority(&side_[1], cudaStreamNonBlocking, prio_hi));
   CK(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
   for (auto& ev : ev_join_) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   CK(cudaMallocHost(&h_counters_, sizeof(int) * kCntNum));
@@ -523,7 +523,7 @@ std::string Engine::capture_state() const {
   const unsigned long long epoch = g_buffer_epoch.load(std::memory_order_relaxed);
   put(&epoch, sizeof epoch);
   put(&opt_, sizeof opt_);
-  const int flags[] = {mixed_ ? 1 : 0, energies_ ? 1 : 0, list_valid_ ? 1 : 0, green_valid_ ? 1 : 0, frozen_ ? 1 : 0, batch_tuned_ ? 1 : 0,
+  const int flags[] = {mixed_ ? 1 : 0, energies_ ? 1 : 0, list_valid_ ? 1 : 0, green_valid_ ? 1 : 0, frozen_ ? 1 : 0, shapes_tuned_ ? 1 : 0,
                        batch_, pme_lines()[0], pme_lines()[1], pme_lines()[2], nsc_cap_, pk_[0], pk_[1], pk_[2], n_, pair_cut_, pme_cap_, bonded_cap_};
   put(flags, sizeof flags);
   put(cell_h_, sizeof cell_h_);
@@ -564,6 +564,7 @@ void Engine::set_cell(const double* cell) {
   g.rv = int(std::floor(g.rlist * g.nv / g.w[1])) + 1;
   g.rq = int(std::ceil(g.rlist / g.w[2])) + 1;
   g.dw = g.rlist / g.w[2];
+  if (!tuning_pinned_ && !frozen_) batch_ = list_depth(g);
   g.batch = batch_;
   // periodic images in range along each axis: 2 ceil(r_list / w) + 1 for the perpendicular width w (the reference counts
   // the images its bins reach the same way and refuses more than 65536 in all, field.cpp:966-972); the device list also
@@ -604,6 +605,21 @@ void Engine::set_cell(const double* cell) {
   }
 }
 
+// Entries per work item of the pair list, from the size of the system alone (so that equal systems get equal work items
+// and the mixed path's sums repeat). A work item is one warp's serial work, and the pair kernel has about 20 warps per SM:
+// a small system needs shallow items to occupy them at all, a large one deep items, which share the staging and the
+// force sums of the super-cluster's 64 atoms. Measured pair kernel, us, at 2 / 8 / 16 / 24 entries: 3,900 entries in all
+// 13 / 20 / 29 / 37, 19,400 entries 22 / 22 / 33 / 42, 36,600 entries 33 / 29 / 36 / 47, 246,000 entries 169 / 111 / 108 /
+// 110, 1,800,000 entries 1242 / 686 / 608 / 587. The entries are estimated from the density: half the clusters whose boxes
+// can come within the list radius of a super-cluster's, times 1.5 for the boxes' real shapes and the columns' ends.
+int Engine::list_depth(const ListGeom& g) const {
+  const double rho = double(n_) / dcell_.vol, R = g.rlist, s = 1.5 * std::cbrt(64.0 / rho);
+  const double reach = s * s * s + 6 * s * s * R + 3 * kPi * s * R * R + 4.0 / 3.0 * kPi * R * R * R;
+  const double entries = 1.5 * (n_ / 64.0 + 0.5 * g.ncol) * 0.5 * reach * rho / 8.0;
+  const double per_warp = entries / (20.0 * dev_sms_);
+  return per_warp < 3 ? 2 : per_warp < 5 ? 4 : per_warp < 20 ? 8 : per_warp < 200 ? 16 : 24;
+}
+
 void Engine::ensure_list_capacity() {
   const int ncol = geom_.ncol;
   const int nsc = n_ / kScAtoms + ncol + 16;
@@ -628,9 +644,10 @@ void Engine::ensure_list_capacity() {
     const size_t ecap = std::max(ent, d_ent_.n);
     d_ent_.alloc(ecap);
     d_ent_shift_.alloc(ecap);
-    d_work_.alloc(ecap / 4 + size_t(nsc_cap_) * 2 + 64);
     d_masks_.alloc(size_t(8) * 96 * nsc_cap_ + 8 * 256);   // 8 rows per (j cluster, image) with exclusions, per super-cluster
   }
+  // work items: full ones, and up to one part-filled item per search warp of a super-cluster
+  d_work_.alloc(d_ent_.n / size_t(std::min(batch_, 4)) + size_t(nsc_cap_) * 8 + 64);
   if (!mixed_) {   // the FP64 path's packed positions and slot sums, also after a switch of precision
     const size_t ns = size_t(nsc_cap_) * kScAtoms;
     d_xqd_.alloc(ns);
@@ -716,6 +733,7 @@ void Engine::check_errors() {
   if (e & kErrNonFinite)   // the reference's text (dynamics.cpp:757), with the step whose positions were not finite
     throw ModelError(CAPS_GPU_EFIELD, "the simulation became unstable at step " + std::to_string((long long)info[kInfoNonFiniteStep]) +
                                           "; lower the time step or relax first");
+  if (e & kErrListWait) throw ModelError(CAPS_GPU_ECUDA, "the pair-list kernel gave up waiting for one of its stages");
   throw ModelError(CAPS_GPU_EINVAL, "device error word " + std::to_string(e));
 }
 
@@ -803,8 +821,6 @@ void Engine::grow_list(size_t ent, size_t mk) {
     d_ent_shift_.release();
     d_ent_.alloc(ent);
     d_ent_shift_.alloc(ent);
-    d_work_.release();
-    d_work_.alloc(ent / 4 + size_t(nsc_cap_) * 2 + 64);
   }
   if (mk > d_masks_.n) {
     d_masks_.release();

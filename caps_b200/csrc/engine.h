@@ -196,8 +196,7 @@ class Engine {
   void join(int k);
   cudaStream_t side_[2] = {nullptr, nullptr};
   int counter(int slot);   // a device counter (synchronises the stream)
-  // Autotuning (timed on this system and GPU, once): the j-tile depth of the pair kernels' work items, and the PME
-  // line-transform block shapes per grid.
+  // The j-tile depth of the pair kernels' work items (list_depth), and launch shapes timed on this system and GPU, once.
   int batch_ = kBatch;
   int pair_cut_ = 0;   // the pair kernel's persistent grid leaves this many block slots per SM to the other branches
   int pme_cap_ = 0;    // at most this many blocks per PME line-transform launch (0: one per line group)
@@ -205,24 +204,24 @@ class Engine {
   bool tuning_pinned_ = false;
   int pinned_lines_[3] = {1, 1, 1};
   bool sums_cleared_ = false;   // the atom-order force sums were cleared by the integrator's kick (the next forces() skips it)
-  bool batch_tuned_ = false;
-  void tune_batch(const double* d_x);
+  bool shapes_tuned_ = false;
+  void tune_shapes(const double* d_x);
+  int list_depth(const ListGeom& g) const;
   template <class R> void fft_passes(PmePath<R>& P, bool ener, bool vir);
   template <class R> void pme_tune(PmePath<R>& P);
   cudaEvent_t ev_fork_ = nullptr, ev_join_[2] = {nullptr, nullptr};
   void read_terms(caps_gpu_terms* out, bool ener, bool vir);
   void check_errors();
-  void launch_build(const double* d_x);
-  // the displacement check's arguments (SHAKE's launch: with the atoms in no constraint cluster), and whether a step may
-  // fold the check into its own kernels: a non-bonded evaluation with a valid list that is not frozen
-  ListCheck list_check(int nfree, const int* free_atoms) const;
+  void launch_list(const double* d_x, bool build);
+  // the displacement check's arguments, and whether a step may fold the check into its own kernels: a non-bonded
+  // evaluation with a valid list that is not frozen
+  ListCheck list_check() const;
   bool list_check_fusable() const;
   void pme_forces(const double* d_x, bool ener, bool vir);
   template <class R> void pme_setup(PmePath<R>& P);
   template <class R> void pme_run(PmePath<R>& P, const double* d_x, bool ener, bool vir);
   void pair_forces(bool ener, bool vir);
   PairArgs pair_args();
-  void prune(const double* d_x);
   void bonded_forces(const double* d_x, bool ener, bool vir, int parts);
   void host_constants(caps_gpu_terms* t, bool ener, bool vir) const;
 
@@ -320,6 +319,7 @@ class Engine {
   PmePath<float> pf_;               // FP32 transforms: the mixed path
   double green_cell_[12] = {0};
   bool green_valid_ = false;        // the active path's influence function matches cell_h_
+  void ensure_grid();
   void ensure_pme();                // the active path's plans, buffers and block shapes for the current grid
   const int* pme_lines() const { return mixed_ ? pf_.lines : pd_.lines; }
 

@@ -100,11 +100,11 @@ struct HostRng {
 };
 
 // --- kernels --------------------------------------------------------------------------------------------------
-// Kick then drift, per atom: v = s v + (hk f + hk2 f2) kAcc / m (s = sc[kScFactor] when `scale`, the thermostat's
-// pending velocity factor, else 1; f2 may be null), x0 = x (the constraint reference), x += hd v. Non-finite positions
-// raise the error word. With `zero_cw` the constraint-virial sums of this step start at zero. With fq (FP32 path) or fd
-// (FP64 path) set, the atom's rows of the force evaluation's atom-order sums are cleared for the evaluation that follows
-// (its own clearing is then skipped).
+// Kick then drift, per atom: v = s v + (hk f + hk2 f2) kAcc / m (s: the thermostat's pending velocity factors; f2 may be
+// null), x0 = x (the constraint reference), x += hd v. Non-finite positions raise the error word. With fq (FP32 path) or
+// fd (FP64 path) set, the force evaluation's atom-order sums are cleared for the evaluation that follows (its own clearing
+// is then skipped).
+struct Chain;
 struct KickArgs {
   int n;
   double* x;
@@ -117,45 +117,50 @@ struct KickArgs {
   double hk2;
   double hd;
   double* sc;
-  int scale, zero_cw;
+  int pending;    // the step before left its velocity factor in sc[kScFactor]: applied first
+  int zero_cw;    // the constraint-virial sums of this step start at zero
   int* counters;
   long long* fq;
   double* fd;
   double* info;   // the engine's error details (the step of the first non-finite position)
-  int step_ahead; // 1 when this step's counter is advanced after this kick (the Langevin step's first kick)
+  int step_ahead; // 1 when this step's counter is advanced after this kick
+  // the first half step of the Nose-Hoover chain, on the kinetic energy the step before left (null: none); its state goes
+  // to chain_half, where the step's last kernel takes it up
+  const Chain* chain;
+  Chain* chain_half;
+  double t0, t1, ndof, t_freq, dt;
+  long long steps;
+  // BAOAB Langevin without constraints: the whole first part of the step per atom, kick, half drift, the O step
+  // v = c1 v + c2 sqrt(kB T kAcc / m) N(0, 1) and the second half drift
+  int lang;
+  double c1, c2;
+  uint64_t seed;
 };
-__device__ __forceinline__ void kick_drift_atom(const KickArgs& K, int i, double s) {
-  const double a = K.hk * kAcc * K.invm[i], a2 = K.hk2 * kAcc * K.invm[i];
-  bool bad = false;
+// One atom's new velocity and position from its old position.
+__device__ __forceinline__ void kick_drift_regs(const KickArgs& K, int i, double s1, double s2, double vr[3], double xn[3], double xo[3]) {
+  const double a = K.hk * kAcc * K.invm[i], a2 = K.f2 ? K.hk2 * kAcc * K.invm[i] : 0.0;
   for (int r = 0; r < 3; ++r) {
-    double vr = K.v[3 * i + r];
-    if (K.scale) vr *= s;
-    vr += a * K.f[3 * i + r];
-    if (K.f2) vr += a2 * K.f2[3 * i + r];   // r-RESPA: the slow and the fast forces in one kick
-    K.v[3 * i + r] = vr;
-    const double xo = K.x[3 * i + r];
-    K.x0[3 * i + r] = xo;
-    const double xn = xo + K.hd * vr;
-    K.x[3 * i + r] = xn;
-    bad |= !isfinite(xn);
-    if (K.fq) K.fq[size_t(r) * K.n + i] = 0;
-    if (K.fd) K.fd[size_t(r) * K.n + i] = 0;
-  }
-  if (bad) {
-    atomicOr(reinterpret_cast<unsigned*>(K.counters + kCntErr), kErrNonFinite);
-    if (K.info && atomicCAS(K.counters + kCntNanClaim, 0, 1) == 0) K.info[kInfoNonFiniteStep] = K.sc[kScStep] + K.step_ahead;
+    double w = K.v[3 * i + r];
+    if (K.pending) w *= s1;
+    if (K.chain) w *= s2;
+    w += a * K.f[3 * i + r];
+    if (K.f2) w += a2 * K.f2[3 * i + r];   // r-RESPA: the slow and the fast forces in one kick
+    vr[r] = w;
+    xo[r] = K.x[3 * i + r];
+    xn[r] = xo[r] + K.hd * w;
   }
 }
-// With L.xb set (a run without constraints), the displacement check of the drifted positions.
-__global__ void k_kick_drift(KickArgs K, ListCheck L) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (K.zero_cw && i < 6) K.sc[kScCW0 + i] = 0;
-  bool mb = false, mp = false;
-  if (i < K.n) {
-    kick_drift_atom(K, i, K.scale ? K.sc[kScFactor] : 1.0);
-    if (L.xb) list_check_atom(L, i, K.x, mb, mp);
-  }
-  if (L.xb) list_check_flags(L, mb, mp);
+__device__ __forceinline__ void flag_non_finite(const KickArgs& K, bool bad) {
+  if (!bad) return;
+  atomicOr(reinterpret_cast<unsigned*>(K.counters + kCntErr), kErrNonFinite);
+  if (K.info && atomicCAS(K.counters + kCntNanClaim, 0, 1) == 0) K.info[kInfoNonFiniteStep] = K.sc[kScStep] + K.step_ahead;
+}
+__device__ __forceinline__ bool non_finite(const double p[3]) { return !isfinite(p[0]) || !isfinite(p[1]) || !isfinite(p[2]); }
+__device__ __forceinline__ void kick_drift_atom(const KickArgs& K, int i, double s1, double s2) {
+  double vr[3], xn[3], xo[3];
+  kick_drift_regs(K, i, s1, s2, vr, xn, xo);
+  for (int r = 0; r < 3; ++r) K.v[3 * i + r] = vr[r], K.x0[3 * i + r] = xo[r], K.x[3 * i + r] = xn[r];
+  flag_non_finite(K, non_finite(xn));
 }
 
 // Constraint clusters. Star clusters (one centre bonded to 1-3 atoms, every constraint through the centre: CH, CH2, CH3)
@@ -187,22 +192,11 @@ struct ConsArgs {
 };
 constexpr int kMaxCouple = 56;   // couplings of a cluster of 8 constraints
 
-// SHAKE on a star cluster with NK constraints, in registers. The same Gauss-Seidel sweep as the general kernel, with each
-// constraint taken as (centre, partner).
+// SHAKE on a star cluster with NK constraints, in registers: p the positions (solved in place), o the old ones. The same
+// Gauss-Seidel sweep as the general kernel, with each constraint taken as (centre, partner). False: p is not to be used.
 template <int NK>
-__device__ void shake_star(const ConsArgs& C, int s, double* __restrict__ x, const double* __restrict__ x0, double* __restrict__ v, double h,
-                           int* counters) {
-  const int4 at = C.star[s];
-  const double4 d4 = C.star_d2[s];
-  const int ids[4] = {at.x, at.y, at.z, at.w};
-  const double dd[3] = {d4.x, d4.y, d4.z};
-  double p[NK + 1][3], o[NK + 1][3], im[NK + 1];
-#pragma unroll
-  for (int a = 0; a <= NK; ++a) {
-    const int g = ids[a];
-    for (int r = 0; r < 3; ++r) p[a][r] = x[3 * g + r], o[a][r] = x0[3 * g + r];
-    im[a] = C.invm[g];
-  }
+__device__ __forceinline__ bool shake_star_solve(const ConsArgs& C, const double dd[3], double p[NK + 1][3], const double o[NK + 1][3],
+                                                 const double im[NK + 1], int* counters) {
   double ref[NK][3];
 #pragma unroll
   for (int k = 0; k < NK; ++k) {
@@ -223,7 +217,7 @@ __device__ void shake_star(const ConsArgs& C, int s, double* __restrict__ x, con
       const double sr = sv[0] * ref[k][0] + sv[1] * ref[k][1] + sv[2] * ref[k][2];
       if (sr < 1e-6 * dd[k]) {
         atomicOr(reinterpret_cast<unsigned*>(counters + kCntErr), kErrShakeTurn);
-        return;
+        return false;
       }
       const double g = diff / (2 * (im[0] + im[k + 1]) * sr);
       for (int r = 0; r < 3; ++r) {
@@ -233,6 +227,24 @@ __device__ void shake_star(const ConsArgs& C, int s, double* __restrict__ x, con
     }
   }
   if (!done) atomicOr(reinterpret_cast<unsigned*>(counters + kCntErr), kErrShake);
+  return true;
+}
+
+template <int NK>
+__device__ void shake_star(const ConsArgs& C, int s, double* __restrict__ x, const double* __restrict__ x0, double* __restrict__ v, double h,
+                           int* counters) {
+  const int4 at = C.star[s];
+  const double4 d4 = C.star_d2[s];
+  const int ids[4] = {at.x, at.y, at.z, at.w};
+  const double dd[3] = {d4.x, d4.y, d4.z};
+  double p[NK + 1][3], o[NK + 1][3], im[NK + 1];
+#pragma unroll
+  for (int a = 0; a <= NK; ++a) {
+    const int g = ids[a];
+    for (int r = 0; r < 3; ++r) p[a][r] = x[3 * g + r], o[a][r] = x0[3 * g + r];
+    im[a] = C.invm[g];
+  }
+  if (!shake_star_solve<NK>(C, dd, p, o, im, counters)) return;
 #pragma unroll
   for (int a = 0; a <= NK; ++a) {
     const int g = ids[a];
@@ -262,12 +274,10 @@ __device__ __forceinline__ void unit3d(double a[3]) {
 // mass) is rotated by the angles phi, psi, theta the paper derives, in a frame with z normal to the previous plane and x
 // normal to the new O direction. The reference solves waters with SHAKE (constraints.cpp:196-230); SETTLE meets the
 // same distances exactly instead of to SHAKE's 1e-8 tolerance. Displacements are added to each atom's own image.
-__device__ void settle_water(const ConsArgs& C, int w, double* __restrict__ x, const double* __restrict__ x0, double* __restrict__ v, double h,
-                             int* counters) {
-  const int4 at = C.water[w];
-  const int ia = at.x, ib = at.y, ic = at.z;
-  const double2 geo = C.water_geo[w];
-  const double mo = 1.0 / C.invm[ia], mh = 1.0 / C.invm[ib];
+// p: the positions of O, H1, H2 now; o: the previous ones; imo, imh: inverse masses; d: the displacements. False: none.
+__device__ __forceinline__ bool settle_solve(const ConsArgs& C, const double2 geo, double imo, double imh, const double p[3][3], const double o[3][3],
+                                             double d[3][3], int* counters) {
+  const double mo = 1.0 / imo, mh = 1.0 / imh;
   const double mt = mo + 2 * mh;
   const double rc = 0.5 * geo.y;
   const double hgt = sqrt(geo.x * geo.x - rc * rc);
@@ -275,8 +285,8 @@ __device__ void settle_water(const ConsArgs& C, int w, double* __restrict__ x, c
   // previous and present positions of the hydrogens relative to their oxygen (nearest images)
   double b0[3], c0[3], b1[3], c1[3];
   for (int r = 0; r < 3; ++r) {
-    b0[r] = x0[3 * ib + r] - x0[3 * ia + r], c0[r] = x0[3 * ic + r] - x0[3 * ia + r];
-    b1[r] = x[3 * ib + r] - x[3 * ia + r], c1[r] = x[3 * ic + r] - x[3 * ia + r];
+    b0[r] = o[1][r] - o[0][r], c0[r] = o[2][r] - o[0][r];
+    b1[r] = p[1][r] - p[0][r], c1[r] = p[2][r] - p[0][r];
   }
   min_image(C.cell, b0[0], b0[1], b0[2]);
   min_image(C.cell, c0[0], c0[1], c0[2]);
@@ -315,7 +325,7 @@ __device__ void settle_water(const ConsArgs& C, int w, double* __restrict__ x, c
   const double disc = ab2 - gamma * gamma;
   if (!(cphi2 > 0) || !(cpsi2 >= 0) || !(disc >= 0) || !(ab2 > 0)) {   // moved too far in one step for a rigid water
     atomicOr(reinterpret_cast<unsigned*>(counters + kCntErr), kErrShake);
-    return;
+    return false;
   }
   const double sinth = (alpha * gamma - beta * sqrt(disc)) / ab2;
   const double costh = sqrt(fmax(1 - sinth * sinth, 0.0));
@@ -323,12 +333,25 @@ __device__ void settle_water(const ConsArgs& C, int w, double* __restrict__ x, c
   const double b3[3] = {xb2 * costh - yb2 * sinth, xb2 * sinth + yb2 * costh, zb1};
   const double c3[3] = {-xb2 * costh - yc2 * sinth, -xb2 * sinth + yc2 * costh, zc1};
   for (int r = 0; r < 3; ++r) {
-    const double da = a3[0] * ex[r] + a3[1] * ey[r] + a3[2] * ez[r] - A1[r];
-    const double db = b3[0] * ex[r] + b3[1] * ey[r] + b3[2] * ez[r] - B1[r];
-    const double dc = c3[0] * ex[r] + c3[1] * ey[r] + c3[2] * ez[r] - C1[r];
-    x[3 * ia + r] += da, x[3 * ib + r] += db, x[3 * ic + r] += dc;
-    if (h > 0) v[3 * ia + r] += da / h, v[3 * ib + r] += db / h, v[3 * ic + r] += dc / h;
+    d[0][r] = a3[0] * ex[r] + a3[1] * ey[r] + a3[2] * ez[r] - A1[r];
+    d[1][r] = b3[0] * ex[r] + b3[1] * ey[r] + b3[2] * ez[r] - B1[r];
+    d[2][r] = c3[0] * ex[r] + c3[1] * ey[r] + c3[2] * ez[r] - C1[r];
   }
+  return true;
+}
+__device__ void settle_water(const ConsArgs& C, int w, double* __restrict__ x, const double* __restrict__ x0, double* __restrict__ v, double h,
+                             int* counters) {
+  const int4 at = C.water[w];
+  const int ids[3] = {at.x, at.y, at.z};
+  double p[3][3], o[3][3], d[3][3];
+  for (int a = 0; a < 3; ++a)
+    for (int r = 0; r < 3; ++r) p[a][r] = x[3 * ids[a] + r], o[a][r] = x0[3 * ids[a] + r];
+  if (!settle_solve(C, C.water_geo[w], C.invm[ids[0]], C.invm[ids[1]], p, o, d, counters)) return;
+  for (int a = 0; a < 3; ++a)
+    for (int r = 0; r < 3; ++r) {
+      x[3 * ids[a] + r] += d[a][r];
+      if (h > 0) v[3 * ids[a] + r] += d[a][r] / h;
+    }
 }
 
 // LINCS on general cluster c (core/src/constraints.cpp:125-185, Hess 1997, order 4): from the old directions B_k, one
@@ -502,33 +525,14 @@ __device__ void check_cluster(const ConsArgs& C, const ListCheck& L, int cc, con
   }
 }
 
-// LINCS, a thread per cluster (every cluster in the general layout), with the displacement check as k_shake has it.
-__global__ void k_lincs(ConsArgs C, double* __restrict__ x, const double* __restrict__ x0, double* __restrict__ v, double h, int* counters,
-                        ListCheck L) {
+// The constraints alone, a thread per cluster (LINCS: every cluster in the general layout).
+__global__ void k_lincs(ConsArgs C, double* __restrict__ x, const double* __restrict__ x0, double* __restrict__ v, double h, int* counters) {
   const int cc = blockIdx.x * blockDim.x + threadIdx.x;
-  bool mb = false, mp = false;
-  if (cc < C.ncl) {
-    lincs_cluster(C, cc, x, x0, v, h, counters);
-    if (L.xb) check_cluster(C, L, cc, x, mb, mp);
-  } else if (L.xb && cc < C.ncl + L.nfree) {
-    list_check_atom(L, L.free_atoms[cc - C.ncl], x, mb, mp);
-  }
-  if (L.xb) list_check_flags(L, mb, mp);
+  if (cc < C.ncl) lincs_cluster(C, cc, x, x0, v, h, counters);
 }
-
-// SHAKE, a thread per cluster; with L.xb set, the displacement check of the step's final positions on the clusters'
-// atoms and, after the clusters, on the L.nfree atoms in none.
-__global__ void k_shake(ConsArgs C, double* __restrict__ x, const double* __restrict__ x0, double* __restrict__ v, double h, int* counters,
-                        ListCheck L) {
+__global__ void k_shake(ConsArgs C, double* __restrict__ x, const double* __restrict__ x0, double* __restrict__ v, double h, int* counters) {
   const int cc = blockIdx.x * blockDim.x + threadIdx.x;
-  bool mb = false, mp = false;
-  if (cc < C.ncl) {
-    shake_cluster(C, cc, x, x0, v, h, counters);
-    if (L.xb) check_cluster(C, L, cc, x, mb, mp);
-  } else if (L.xb && cc < C.ncl + L.nfree) {
-    list_check_atom(L, L.free_atoms[cc - C.ncl], x, mb, mp);
-  }
-  if (L.xb) list_check_flags(L, mb, mp);
+  if (cc < C.ncl) shake_cluster(C, cc, x, x0, v, h, counters);
 }
 
 // The velocity update of one atom before RATTLE: a kick (v += hk kAcc f / m) or the Langevin O step
@@ -589,15 +593,6 @@ __device__ __forceinline__ void vel_op(const VelOp& op, int g, double* vv, const
     const double sd = sqrt(kB * sc[kScTnow] * kAcc * invm[g]);
     for (int r = 0; r < 3; ++r) vv[r] = op.c1 * vv[r] + op.c2 * sd * z[r];
   }
-}
-
-// The velocity update alone, one thread per atom (runs without constraints).
-__global__ void k_vel(int n, double* __restrict__ v, const double* __restrict__ invm, const double* sc, VelOp op) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double vv[3] = {v[3 * i], v[3 * i + 1], v[3 * i + 2]};
-  vel_op(op, i, vv, invm, sc);
-  for (int r = 0; r < 3; ++r) v[3 * i + r] = vv[r];
 }
 
 // RATTLE on a star cluster with NK constraints, in registers (the general kernel's sweep, constraints as (centre, partner)).
@@ -736,11 +731,15 @@ __global__ void k_remap(int n, double* __restrict__ x, double c0x, double c0y, d
   x[3 * i + 2] = c0z + mu * (x[3 * i + 2] - c0z);
 }
 
-// The step counter and the thermostat target: T ramps linearly from t0 to t1 over `steps` when t1 >= 0.
+// The thermostat target of a step: T ramps linearly from t0 to t1 over `steps` when t1 >= 0.
+__device__ __forceinline__ double target_at(double step, double t0, double t1, long long steps) {
+  return (t1 >= 0 && steps > 0) ? t0 + (t1 - t0) * step / double(steps) : t0;
+}
+// The step counter and the thermostat target.
 __device__ void step_begin_body(double* sc, double t0, double t1, long long steps, double ndof) {
   const double step = sc[kScStep] + 1;
   sc[kScStep] = step;
-  const double t = (t1 >= 0 && steps > 0) ? t0 + (t1 - t0) * step / double(steps) : t0;
+  const double t = target_at(step, t0, t1, steps);
   sc[kScTnow] = t;
   sc[kScKtarget] = 0.5 * ndof * kB * t;
 }
@@ -748,15 +747,14 @@ __global__ void k_step_begin(double* sc, double t0, double t1, long long steps, 
   step_begin_body(sc, t0, t1, steps, ndof);
 }
 
-// Nose-Hoover chain over half a step (LAMMPS FixNH::nhc_temp_integrate, as dynamics.cpp:479-508): sets the velocity
-// factor in sc[kScFactor]; the caller scales v by it.
-__device__ void nhc_body(Chain* ch, double* sc, double ndof, double t_freq, double dt) {
+// Nose-Hoover chain over half a step (LAMMPS FixNH::nhc_temp_integrate, as dynamics.cpp:479-508) on chain c at target
+// temperature tt: returns the velocity factor and scales the kinetic energy ke by its square; the caller scales v.
+__device__ double nhc_half(Chain& c, double& ke, double tt, double ndof, double t_freq, double dt) {
   const double dthalf = 0.5 * dt, dt4 = 0.25 * dt, dt8 = 0.125 * dt;
-  const double tt = sc[kScTnow], kt = kB * tt, ke_target = ndof * kt;
-  Chain& c = *ch;
+  const double kt = kB * tt, ke_target = ndof * kt;
   c.eta_mass[0] = ndof * kt / (t_freq * t_freq);
   for (int q = 1; q < 3; ++q) c.eta_mass[q] = kt / (t_freq * t_freq);
-  double kecur = 2 * sc[kScKE];
+  double kecur = 2 * ke;
   c.eta_dotdot[0] = (kecur - ke_target) / c.eta_mass[0];
   for (int q = 2; q > 0; --q) {
     const double ex = exp(-dt8 * c.eta_dot[q + 1]);
@@ -775,8 +773,8 @@ __device__ void nhc_body(Chain* ch, double* sc, double ndof, double t_freq, doub
     c.eta_dotdot[q] = (c.eta_mass[q - 1] * c.eta_dot[q - 1] * c.eta_dot[q - 1] - kt) / c.eta_mass[q];
     c.eta_dot[q] = (c.eta_dot[q] + c.eta_dotdot[q] * dt4) * ex;
   }
-  sc[kScFactor] = factor;
-  sc[kScKE] = 0.5 * kecur;
+  ke = 0.5 * kecur;
+  return factor;
 }
 
 // Bussi velocity rescaling (Bussi, Donadio & Parrinello 2007, appendix; dynamics.cpp:466-477) from this step's draws
@@ -797,7 +795,7 @@ __device__ void bussi_body(double* sc, const double2* __restrict__ draws, long l
 }
 
 // What the last block of k_ke does with the fresh kinetic energy.
-enum KeThen { kThenNone = 0, kThenNhc, kThenBussi, kThenBath };
+enum KeThen { kThenNone = 0, kThenNhc, kThenBussi, kThenBath, kThenLang };
 struct KeArgs {
   int n;
   const double* v;
@@ -806,23 +804,29 @@ struct KeArgs {
   unsigned* done;        // blocks finished; the last block resets it
   double* sc;
   int slot;              // sc slot receiving 0.5 sum m v^2 / kAcc
-  int tensor;            // also the kinetic tensor into kScKin0..
+  int extra;             // further sums: 6 the kinetic tensor into kScKin0.., 1 the energy before the O step into kScKE0
   int begin;             // run the step-begin update first
   int then;              // KeThen
   double t0, t1, ndof;
   long long steps;
   Chain* chain;
+  const Chain* chain_half;   // the chain after the step's first half (kThenNhc)
   double t_freq, dt;
   const double2* draws;
   long long draws_first;
   double tau;
 };
 
-// One atom's share: m v^2, and the tensor terms on request.
+// The share of one atom with velocity v: m v^2, and the tensor terms on request.
+__device__ __forceinline__ void ke_share(const KeArgs& A, double mi, const double v[3], double& e, double t[6]) {
+  e += mi * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+  if (A.extra == 6)
+    t[0] += mi * v[0] * v[0], t[1] += mi * v[1] * v[1], t[2] += mi * v[2] * v[2], t[3] += mi * v[0] * v[1], t[4] += mi * v[0] * v[2],
+        t[5] += mi * v[1] * v[2];
+}
 __device__ __forceinline__ void ke_atom(const KeArgs& A, int i, double& e, double t[6]) {
-  const double vx = A.v[3 * i], vy = A.v[3 * i + 1], vz = A.v[3 * i + 2], mi = A.m[i];
-  e += mi * (vx * vx + vy * vy + vz * vz);
-  if (A.tensor) t[0] += mi * vx * vx, t[1] += mi * vy * vy, t[2] += mi * vz * vz, t[3] += mi * vx * vy, t[4] += mi * vx * vz, t[5] += mi * vy * vz;
+  const double v[3] = {A.v[3 * i], A.v[3 * i + 1], A.v[3 * i + 2]};
+  ke_share(A, A.m[i], v, e, t);
 }
 
 // The block sums of every thread's share into A.part (7 per block), then in the last block to finish: the partials in
@@ -832,11 +836,10 @@ __device__ void ke_blocks(const KeArgs& A, double e, double t[6]) {
   __shared__ bool last;
   const double s = block_sum(e, scratch);
   if (threadIdx.x == 0) A.part[blockIdx.x * 7] = s;
-  if (A.tensor)
-    for (int q = 0; q < 6; ++q) {
-      const double st = block_sum(t[q], scratch);
-      if (threadIdx.x == 0) A.part[blockIdx.x * 7 + 1 + q] = st;
-    }
+  for (int q = 0; q < A.extra; ++q) {
+    const double st = block_sum(t[q], scratch);
+    if (threadIdx.x == 0) A.part[blockIdx.x * 7 + 1 + q] = st;
+  }
   if (threadIdx.x == 0) {
     __threadfence();
     last = atomicAdd(A.done, 1u) == gridDim.x - 1;
@@ -848,30 +851,160 @@ __device__ void ke_blocks(const KeArgs& A, double e, double t[6]) {
   for (int q = 0; q < 6; ++q) t[q] = 0;
   for (int b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
     e += __ldcg(A.part + 7 * b);
-    if (A.tensor)
-      for (int q = 0; q < 6; ++q) t[q] += __ldcg(A.part + 7 * b + 1 + q);
+    for (int q = 0; q < A.extra; ++q) t[q] += __ldcg(A.part + 7 * b + 1 + q);
   }
   const double tot = block_sum(e, scratch);
   double tt[6];
-  if (A.tensor)
-    for (int q = 0; q < 6; ++q) tt[q] = block_sum(t[q], scratch);
+  for (int q = 0; q < A.extra; ++q) tt[q] = block_sum(t[q], scratch);
   if (threadIdx.x != 0) return;
   *A.done = 0;
   double* sc = A.sc;
-  sc[A.slot] = 0.5 * tot / kAcc;
-  if (A.tensor)
+  double ke = 0.5 * tot / kAcc;
+  if (A.extra == 6)
     for (int q = 0; q < 6; ++q) sc[kScKin0 + q] = tt[q] / kAcc;
   if (A.begin) step_begin_body(sc, A.t0, A.t1, A.steps, A.ndof);
-  if (A.then == kThenNhc) nhc_body(A.chain, sc, A.ndof, A.t_freq, A.dt);
-  else if (A.then == kThenBussi) bussi_body(sc, A.draws, A.draws_first, A.dt, A.tau, A.ndof);
-  else if (A.then == kThenBath) sc[kScBath] -= sc[kScKE] - sc[kScKE0];
+  if (A.then == kThenNhc) {   // the second half of the chain, after the first that the step's first kernel left
+    Chain c = *A.chain_half;
+    sc[kScFactor] = nhc_half(c, ke, sc[kScTnow], A.ndof, A.t_freq, A.dt);
+    *A.chain = c;
+  }
+  sc[A.slot] = ke;
+  if (A.then == kThenBussi) bussi_body(sc, A.draws, A.draws_first, A.dt, A.tau, A.ndof);
+  else if (A.then == kThenLang) sc[kScKE0] = 0.5 * tt[0] / kAcc;
+  if (A.then == kThenBath || A.then == kThenLang) sc[kScBath] -= sc[kScKE] - sc[kScKE0];
 }
 
-// The first Nose-Hoover half step of a step, on the kinetic energy the previous step left in sc[kScKE]: its second half
-// set it to the scaled velocities' value, and the velocities have not changed since.
-__global__ void k_nhc_begin(Chain* ch, double* sc, double t0, double t1, long long steps, double ndof, double t_freq, double dt) {
-  step_begin_body(sc, t0, t1, steps, ndof);
-  nhc_body(ch, sc, ndof, t_freq, dt);
+// Thread c's share: the atoms of its constraint cluster, or its free atom.
+__device__ __forceinline__ void cluster_ke(const KeArgs& A, const ConsArgs& C, int c, int nfree, const int* __restrict__ free_atoms, double& e,
+                                           double t[6]) {
+  if (c >= C.ncl) {
+    if (c < C.ncl + nfree) ke_atom(A, free_atoms ? free_atoms[c - C.ncl] : c - C.ncl, e, t);
+  } else if (c < C.e3) {
+    const int4 at = C.star[c];
+    const int ids[4] = {at.x, at.y, at.z, at.w};
+    for (int a = 0; a < 4; ++a)
+      if (ids[a] >= 0) ke_atom(A, ids[a], e, t);
+  } else if (c < C.e4) {
+    const int4 at = C.water[c - C.e3];
+    ke_atom(A, at.x, e, t);
+    ke_atom(A, at.y, e, t);
+    ke_atom(A, at.z, e, t);
+  } else {
+    const int cg = c - C.e4;
+    for (int a = C.cl_atom0[cg]; a < C.cl_atom0[cg + 1]; ++a) ke_atom(A, C.cl_atoms[a], e, t);
+  }
+}
+
+// The first kernel of a step: kick, drift and the constraints of the new positions, a thread per constraint cluster and
+// one per free atom (free_atoms null: every atom), then on request the list's displacement check of the step's final
+// positions (L.xb) and a kinetic energy (A.n > 0). Star clusters and rigid waters stay in registers from the kick to the
+// solved positions. With K.chain the Nose-Hoover chain's first half runs here too, in every block for itself.
+//
+// Bound by latency: one wave of threads, a chain of dependent FP64 operations each. As separate launches the kick (2.9 us),
+// SHAKE (10.7 us) and the thermostat's begin (2.2 us) each paid their own start and loads; 32,000 atoms, 16,000 C-H bonds.
+template <int NK>
+__device__ __forceinline__ void move_star(const KickArgs& K, const ConsArgs& C, const ListCheck& L, int s, double s1, double s2, bool& mb, bool& mp) {
+  const int4 at = C.star[s];
+  const double4 d4 = C.star_d2[s];
+  const int ids[4] = {at.x, at.y, at.z, at.w};
+  const double dd[3] = {d4.x, d4.y, d4.z};
+  double p[NK + 1][3], o[NK + 1][3], vv[NK + 1][3], im[NK + 1];
+  bool bad = false;
+#pragma unroll
+  for (int a = 0; a <= NK; ++a) {
+    kick_drift_regs(K, ids[a], s1, s2, vv[a], p[a], o[a]);
+    im[a] = C.invm[ids[a]];
+    bad |= non_finite(p[a]);
+  }
+  flag_non_finite(K, bad);
+  const bool ok = shake_star_solve<NK>(C, dd, p, o, im, K.counters);
+#pragma unroll
+  for (int a = 0; a <= NK; ++a) {
+    for (int r = 0; r < 3; ++r) {
+      const double xb = o[a][r] + K.hd * vv[a][r];   // the drifted position the solve started from
+      K.x[3 * ids[a] + r] = p[a][r];
+      K.v[3 * ids[a] + r] = ok && K.hd > 0 ? vv[a][r] + (p[a][r] - xb) / K.hd : vv[a][r];
+    }
+    if (L.xb) list_check_at(L, ids[a], p[a], mb, mp);
+  }
+}
+__device__ __forceinline__ void move_water(const KickArgs& K, const ConsArgs& C, const ListCheck& L, int w, double s1, double s2, bool& mb, bool& mp) {
+  const int4 at = C.water[w];
+  const int ids[3] = {at.x, at.y, at.z};
+  double p[3][3], o[3][3], vv[3][3], d[3][3] = {};
+  bool bad = false;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    kick_drift_regs(K, ids[a], s1, s2, vv[a], p[a], o[a]);
+    bad |= non_finite(p[a]);
+  }
+  flag_non_finite(K, bad);
+  const bool ok = settle_solve(C, C.water_geo[w], C.invm[ids[0]], C.invm[ids[1]], p, o, d, K.counters);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    for (int r = 0; r < 3; ++r) {
+      if (ok) p[a][r] += d[a][r];
+      K.x[3 * ids[a] + r] = p[a][r];
+      K.v[3 * ids[a] + r] = ok && K.hd > 0 ? vv[a][r] + d[a][r] / K.hd : vv[a][r];
+    }
+    if (L.xb) list_check_at(L, ids[a], p[a], mb, mp);
+  }
+}
+__global__ void __launch_bounds__(128) k_move(KickArgs K, ConsArgs C, ListCheck L, int nfree, const int* __restrict__ free_atoms, KeArgs A) {
+  __shared__ double s_half;
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int stride = gridDim.x * blockDim.x;
+  for (int i = c; i < 3 * K.n; i += stride) {
+    if (K.fq) K.fq[i] = 0;
+    if (K.fd) K.fd[i] = 0;
+  }
+  if (K.zero_cw && c < 6) K.sc[kScCW0 + c] = 0;
+  if (K.chain) {
+    if (threadIdx.x == 0) {
+      Chain ch = *K.chain;
+      double ke = K.sc[kScKE];
+      s_half = nhc_half(ch, ke, target_at(K.sc[kScStep] + 1, K.t0, K.t1, K.steps), K.ndof, K.t_freq, K.dt);
+      if (blockIdx.x == 0) *K.chain_half = ch;
+    }
+    __syncthreads();
+  }
+  const double s1 = K.pending ? K.sc[kScFactor] : 1.0, s2 = K.chain ? s_half : 1.0;
+  bool mb = false, mp = false;
+  double e = 0, t[6] = {0, 0, 0, 0, 0, 0};
+  if (c < C.e1) move_star<1>(K, C, L, c, s1, s2, mb, mp);
+  else if (c < C.e2) move_star<2>(K, C, L, c, s1, s2, mb, mp);
+  else if (c < C.e3) move_star<3>(K, C, L, c, s1, s2, mb, mp);
+  else if (c < C.e4) move_water(K, C, L, c - C.e3, s1, s2, mb, mp);
+  else if (c < C.ncl) {
+    const int cg = c - C.e4;
+    for (int a = C.cl_atom0[cg]; a < C.cl_atom0[cg + 1]; ++a) kick_drift_atom(K, C.cl_atoms[a], s1, s2);
+    if (C.lincs) lincs_cluster(C, cg, K.x, K.x0, K.v, K.hd, K.counters);
+    else shake_cluster(C, c, K.x, K.x0, K.v, K.hd, K.counters);
+    if (L.xb) check_cluster(C, L, c, K.x, mb, mp);
+  } else if (c < C.ncl + nfree) {
+    const int g = free_atoms ? free_atoms[c - C.ncl] : c - C.ncl;
+    double vr[3], xn[3], xo[3];
+    kick_drift_regs(K, g, s1, s2, vr, xn, xo);
+    flag_non_finite(K, non_finite(xn));
+    if (K.lang) {
+      ke_share(A, A.m[g], vr, t[0], t);
+      const double step = K.sc[kScStep] + 1;
+      double z[4];
+      normals4(K.seed, (uint64_t)step, uint32_t(g), 0x4C414E47u, z);
+      const double sd = sqrt(kB * target_at(step, K.t0, K.t1, K.steps) * kAcc * K.invm[g]);
+      for (int r = 0; r < 3; ++r) vr[r] = K.c1 * vr[r] + K.c2 * sd * z[r];
+      ke_share(A, A.m[g], vr, e, t);
+      for (int r = 0; r < 3; ++r) xn[r] = xn[r] + K.hd * vr[r];
+      flag_non_finite(K, non_finite(xn));
+    }
+    for (int r = 0; r < 3; ++r) K.v[3 * g + r] = vr[r], K.x[3 * g + r] = xn[r];
+    if (L.xb) list_check_at(L, g, xn, mb, mp);
+  }
+  if (L.xb) list_check_flags(L, mb, mp);
+  if (A.n > 0) {
+    if (!K.lang) cluster_ke(A, C, c, nfree, free_atoms, e, t);
+    ke_blocks(A, e, t);
+  }
 }
 
 // Velocity update then RATTLE in one launch: threads [0, ncl) take one constraint cluster each (its atoms' update, then
@@ -884,7 +1017,7 @@ __global__ void k_vel_rattle(ConsArgs C, int nfree, const int* __restrict__ free
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   double w[6] = {0, 0, 0, 0, 0, 0};
   if (c >= C.ncl && c < C.ncl + nfree) {
-    const int g = free_atoms[c - C.ncl];
+    const int g = free_atoms ? free_atoms[c - C.ncl] : c - C.ncl;
     double vv[3] = {v[3 * g], v[3 * g + 1], v[3 * g + 2]};
     vel_op(op, g, vv, C.invm, sc);
     for (int r = 0; r < 3; ++r) v[3 * g + r] = vv[r];
@@ -957,23 +1090,10 @@ __global__ void k_vel_rattle(ConsArgs C, int nfree, const int* __restrict__ free
   // the kinetic energy of the updated velocities (this thread's atoms, read back) and the thermostat update, as k_ke
   if (K.n > 0) {
     double e = 0, t[6] = {0, 0, 0, 0, 0, 0};
-    if (c >= C.ncl && c < C.ncl + nfree) {
-      ke_atom(K, free_atoms[c - C.ncl], e, t);
-    } else if (c < C.e3) {
-      const int4 at = C.star[c];
-      const int ids[4] = {at.x, at.y, at.z, at.w};
-      for (int a = 0; a < 4; ++a)
-        if (ids[a] >= 0) ke_atom(K, ids[a], e, t);
-    } else if (c < C.e4) {
-      const int4 at = C.water[c - C.e3];
-      ke_atom(K, at.x, e, t);
-      ke_atom(K, at.y, e, t);
-      ke_atom(K, at.z, e, t);
-    } else if (c < C.ncl) {
-      const int cg = c - C.e4;
-      for (int a = C.cl_atom0[cg]; a < C.cl_atom0[cg + 1]; ++a) ke_atom(K, C.cl_atoms[a], e, t);
-    }
+    cluster_ke(K, C, c, nfree, free_atoms, e, t);
     ke_blocks(K, e, t);
+  } else if (K.begin && blockIdx.x == 0 && threadIdx.x == 0) {   // no thermostat: the step's scalars alone
+    step_begin_body(sc, K.t0, K.t1, K.steps, K.ndof);
   }
 }
 
@@ -1001,7 +1121,7 @@ struct Stepper {
   DevBuf<unsigned> done;       // k_ke's finished-block counter
   DevBuf<int> free_atoms;      // atoms in no constraint cluster
   int nfree = 0;
-  DevBuf<Chain> chain;
+  DevBuf<Chain> chain, chain_half;   // the Nose-Hoover chain, and its state in the middle of a step
   DevBuf<int> cl_start, cl_atom0, cl_atoms;
   DevBuf<int4> cons, star, water;
   DevBuf<double4> star_d2;
@@ -1106,10 +1226,14 @@ struct Stepper {
       min_image_host(d);
       return std::sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
     };
+    // the bonds of each atom and the angles about each atom, in their order
+    std::vector<std::vector<int>> bonds_of(static_cast<size_t>(n)), angles_about(static_cast<size_t>(n));
+    for (size_t k = 0; k < bonds.size(); ++k) bonds_of[bonds[k][0]].push_back(int(k)), bonds_of[bonds[k][1]].push_back(int(k));
+    for (size_t k = 0; k < E.ha_.size(); ++k) angles_about[E.ha_[k][1]].push_back(int(k));
     auto length = [&](int i, int j) {
-      for (size_t k = 0; k < bonds.size(); ++k)
-        if ((int(bonds[k][0]) == i && int(bonds[k][1]) == j) || (int(bonds[k][0]) == j && int(bonds[k][1]) == i))
-          if (r0[k] > 0.3) return r0[k];
+      for (int k : bonds_of[size_t(i)])
+        if (int(bonds[size_t(k)][0]) == j || int(bonds[size_t(k)][1]) == j)
+          if (r0[size_t(k)] > 0.3) return r0[size_t(k)];
       return dist(i, j);
     };
     struct Cn { int i, j; double d; };
@@ -1125,9 +1249,9 @@ struct Stepper {
       if (!is_h(a) || !is_h(b)) continue;
       const double da = length(ox, a), db = length(ox, b);
       double th = -1;
-      for (size_t k = 0; k < E.ha_.size(); ++k) {
-        const auto& t = E.ha_[k];
-        if (int(t[1]) == ox && ((int(t[0]) == a && int(t[2]) == b) || (int(t[0]) == b && int(t[2]) == a))) th = E.hth0_[k];
+      for (int k : angles_about[size_t(ox)]) {
+        const auto& t = E.ha_[size_t(k)];
+        if ((int(t[0]) == a && int(t[2]) == b) || (int(t[0]) == b && int(t[2]) == a)) th = E.hth0_[size_t(k)];
       }
       if (th < 0) {
         cons_from_positions = true;
@@ -1354,7 +1478,7 @@ struct Stepper {
                             ncons, nfree, nparts, respa, slow_parts, fast_parts, thermo ? 1 : 0};
     put(iv, sizeof iv);
     put(&C, sizeof C);
-    const void* ptrs[] = {x.p, v.p, x0.p, invm.p, m.p, sc.p, part.p, done.p, chain.p, draws.p, free_atoms.p, f_slow.p, f_fast.p};
+    const void* ptrs[] = {x.p, v.p, x0.p, invm.p, m.p, sc.p, part.p, done.p, chain.p, chain_half.p, draws.p, free_atoms.p, f_slow.p, f_fast.p};
     put(ptrs, sizeof ptrs);
     return k;
   }
@@ -1384,7 +1508,8 @@ struct Stepper {
       cudaGraph_t g;
       CK(cudaStreamBeginCapture(E.stream_, cudaStreamCaptureModeThreadLocal));
       try {
-        for (int i = 0; i < (block ? kBlockSteps : 1); ++i) step(thermo, thermo);
+        const int steps = block ? kBlockSteps : 1;
+        for (int i = 0; i < steps; ++i) step(thermo, thermo, i > 0, i + 1 < steps);
       } catch (...) {   // leave no capture open behind an error
         cudaGraph_t junk = nullptr;
         (void)cudaStreamEndCapture(E.stream_, &junk);
@@ -1428,12 +1553,13 @@ struct Stepper {
     A.done = done.p;
     A.sc = sc.p;
     A.slot = slot;
-    A.tensor = tensor ? 1 : 0;
+    A.extra = tensor ? 6 : 0;
     A.t0 = o.temperature;
     A.t1 = o.temperature_end;
     A.steps = (long long)o.steps;
     A.ndof = ndof;
     A.chain = chain.p;
+    A.chain_half = chain_half.p;
     A.t_freq = t_freq;
     A.dt = o.dt;
     A.draws = draws.p;
@@ -1443,32 +1569,45 @@ struct Stepper {
   }
   void ke_launch(const KeArgs& A) { launch_k(k_ke, nparts, 256, 0, E.stream_, A); }
   void ke(int slot, bool tensor) { ke_launch(ke_args(slot, tensor)); }
-  // half kick, then drift with SHAKE; `scale` applies the thermostat's pending factor first
-  // kick + drift, then SHAKE; the kick also clears the force evaluation's atom-order sums for the evaluation that
-  // follows (Engine::forces then skips its own clearing)
-  // check: the list's displacement check runs in the drift (no constraints) or in SHAKE, and the force evaluation that
-  // follows skips its own
-  void kick_drift(double hk, double hd, bool scale, bool zero_cw, const double* f = nullptr, const double* f2 = nullptr, double hk2 = 0,
-                  int step_ahead = 0, bool check = false) {
-    KickArgs K{n, x.p, v.p, x0.p, f ? f : E.d_f_.p, invm.p, hk, f2, hk2, hd, sc.p, scale ? 1 : 0, zero_cw ? 1 : 0, E.d_counters_.p,
-               E.mixed_ ? E.d_F_.p : nullptr, E.mixed_ ? nullptr : E.d_Fd_.p, E.d_errinfo_.p, step_ahead};
-    const ListCheck L = check ? E.list_check(nfree, free_atoms.p) : ListCheck{};
-    launch_k(k_kick_drift, blocks(size_t(n), 256), 256, 0, E.stream_, K, ncons ? ListCheck{} : L);
-    if (ncons) launch_k(C.lincs ? k_lincs : k_shake, blocks(size_t(C.ncl) + (check ? size_t(nfree) : 0), 128), 128, 0, E.stream_, C, x.p, x0.p, v.p, hd, E.d_counters_.p, L);
+  // threads of the per-atom kernels: one per constraint cluster and one per atom in none
+  int movers() const { return ncons ? C.ncl + nfree : n; }
+  // a step's first kernel (k_move): half kick, drift, constraints. pending: the step before left its velocity factor to
+  // apply. The kick also clears the force evaluation's atom-order sums for the evaluation that follows (Engine::forces then
+  // skips its own clearing). check: the list's displacement check runs here too, and the evaluation skips its own.
+  KickArgs kick_args(double hk, double hd, bool pending, bool zero_cw) const {
+    KickArgs K{};
+    K.n = n;
+    K.x = x.p, K.v = v.p, K.x0 = x0.p;
+    K.f = E.d_f_.p;
+    K.invm = invm.p;
+    K.hk = hk, K.hd = hd;
+    K.sc = sc.p;
+    K.pending = pending ? 1 : 0;
+    K.zero_cw = zero_cw ? 1 : 0;
+    K.counters = E.d_counters_.p;
+    K.fq = E.mixed_ ? E.d_F_.p : nullptr;
+    K.fd = E.mixed_ ? nullptr : E.d_Fd_.p;
+    K.info = E.d_errinfo_.p;
+    K.t0 = o.temperature, K.t1 = o.temperature_end, K.steps = (long long)o.steps;
+    K.ndof = ndof, K.t_freq = t_freq, K.dt = o.dt;
+    return K;
+  }
+  void move(const KickArgs& K, bool check = false, const KeArgs* ke = nullptr) {
+    KeArgs A{};
+    if (ke) A = *ke;
+    launch_k(k_move, blocks(size_t(movers()), 128), 128, 0, E.stream_, K, C, check ? E.list_check() : ListCheck{}, ncons ? nfree : n,
+             ncons ? free_atoms.p : nullptr, A);
     E.sums_cleared_ = true;
   }
   // whether this step's drift may take the list's displacement check (a plain step: not r-RESPA)
   bool fuse_check() const { return respa <= 1 && E.list_check_fusable(); }
   // a velocity update, then RATTLE (constraint virial summed when h > 0); with ke, also the kinetic energy and ke's
-  // thermostat update (constraints only: the caller launches k_ke otherwise)
+  // thermostat update
   void vel_rattle(const VelOp& op, double h, const KeArgs* ke = nullptr) {
-    if (!ncons) {
-      if (op.kind != 0) launch_k(k_vel, blocks(size_t(n), 256), 256, 0, E.stream_, n, v.p, invm.p, sc.p, op);
-      return;
-    }
     KeArgs K{};
     if (ke) K = *ke;
-    launch_k(k_vel_rattle, blocks(size_t(C.ncl + nfree), 128), 128, 0, E.stream_, C, nfree, free_atoms.p, x.p, v.p, op, h, sc.p, E.d_counters_.p, K);
+    launch_k(k_vel_rattle, blocks(size_t(movers()), 128), 128, 0, E.stream_, C, ncons ? nfree : n, ncons ? free_atoms.p : nullptr, x.p, v.p, op,
+             ncons ? h : 0.0, sc.p, E.d_counters_.p, K);
   }
   VelOp kick_op(double hk) const { return VelOp{1, E.d_f_.p, hk, 0, 0, 0, nullptr, 0}; }
   // the kick from the force evaluation's sums (its reduction skipped), storing the forces to E.d_f_
@@ -1484,8 +1623,6 @@ struct Stepper {
     op.fout = E.d_f_.p;
     return op;
   }
-  // the kick + RATTLE + kinetic energy + thermostat tail in one launch (constraints, no r-RESPA)
-  bool fused_tail() const { return ncons > 0 && respa == 1; }
   void rattle(double h) {   // RATTLE alone (initial velocities)
     if (ncons) vel_rattle(VelOp{0, nullptr, 0, 0, 0, 0, nullptr, 0}, h);
   }
@@ -1507,12 +1644,14 @@ struct Stepper {
   }
   void fast_forces() { E.forces(x.p, false, false, true, fast_parts, f_fast.p, true); }
 
-  // One MD step (dynamics.cpp:606-666), energies and virial on request. Kernel sequence per step: NVT Nose-Hoover
-  // chain (on the kinetic energy the last step left), kick+drift, SHAKE, forces, kick+RATTLE+KE+chain (with constraints
-  // the kick reads the force sums and the kinetic energy and chain update run in the RATTLE launch's last block), scale;
-  // Bussi step-begin, kick+drift, SHAKE, forces, kick+RATTLE+KE+Bussi, scale; Langevin (BAOAB) kick+drift, SHAKE, KE,
-  // O+RATTLE, KE+bath, drift, SHAKE, forces, kick+RATTLE.
-  void step(bool ener, bool vir) {
+  // One MD step (dynamics.cpp:606-666), energies and virial on request, in four kernels besides the bonded and PME
+  // branches: k_move (the Nose-Hoover chain's first half on the kinetic energy the last step left, kick, drift,
+  // constraints, displacement check), the list kernel, the pair kernel, and k_vel_rattle (kick from the force sums, RATTLE,
+  // kinetic energy, thermostat update in its last block). Langevin (BAOAB) takes kick, half drift, O step and half drift in
+  // k_move, or with constraints k_move, O + RATTLE, k_move.
+  // A thermostat's velocity factor is left pending for the next step's kick (pend_out) where that step follows in the same
+  // graph, or applied at once. pend_in: the step before left one.
+  void step(bool ener, bool vir, bool pend_in = false, bool pend_out = false) {
     const double dt = o.dt;
     const double hw = vir ? dt : 0.0;   // the constraint virial only on steps that report it
     if (respa > 1) {
@@ -1520,66 +1659,57 @@ struct Stepper {
       // with the fast ones; outer half kick. Adjacent kicks with the same forces are merged.
       const double h = dt / respa;
       launch_k(k_step_begin, 1, 1, 0, E.stream_, sc.p, o.temperature, o.temperature_end, (long long)o.steps, ndof);
-      kick_drift(0.5 * dt, h, false, true, f_slow.p, f_fast.p, 0.5 * h);
+      KickArgs K = kick_args(0.5 * dt, h, pend_in, true);
+      K.f = f_slow.p, K.f2 = f_fast.p, K.hk2 = 0.5 * h;
+      move(K);
       for (int j = 0; j + 1 < respa; ++j) {
         fast_forces();
-        kick_drift(h, h, false, false, f_fast.p);
+        K = kick_args(h, h, false, false);
+        K.f = f_fast.p;
+        move(K);
       }
       forces(ener, vir);
-      vel_rattle(VelOp{1, f_fast.p, 0.5 * h, 0, 0, 0, f_slow.p, 0.5 * dt}, hw);
-      if (bussi) {
-        KeArgs A = ke_args(kScKE, false);
-        A.then = kThenBussi;
-        ke_launch(A);
-        scale_v();
-      }
-      return;
-    }
-    if (langevin) {
-      const double c1 = std::exp(-dt / std::max(o.tau_t, 1e-9)), c2 = std::sqrt(1 - c1 * c1);
-      kick_drift(0.5 * dt, 0.5 * dt, false, true, nullptr, nullptr, 0, 1);
-      KeArgs A = ke_args(kScKE0, false);
-      A.begin = 1;
-      ke_launch(A);
-      vel_rattle(VelOp{2, nullptr, 0, c1, c2, o.seed, nullptr, 0}, 0);
-      A = ke_args(kScKE, false);
-      A.then = kThenBath;
-      ke_launch(A);
-      const bool chk = fuse_check();
-      kick_drift(0, 0.5 * dt, false, false, nullptr, nullptr, 0, 0, chk);
-      forces(ener, vir, true, chk);
-      vel_rattle(kick_op(0.5 * dt), hw);
-    } else if (nhc) {
-      launch_k(k_nhc_begin, 1, 1, 0, E.stream_, chain.p, sc.p, o.temperature, o.temperature_end, (long long)o.steps, ndof, t_freq, dt);
-      const bool chk = fuse_check();
-      kick_drift(0.5 * dt, dt, true, true, nullptr, nullptr, 0, 0, chk);
-      KeArgs A = ke_args(kScKE, false);
-      A.then = kThenNhc;
-      if (fused_tail()) {
-        forces(ener, vir, false, chk);
-        vel_rattle(kick_op_sums(0.5 * dt), hw, &A);
-      } else {
-        forces(ener, vir, true, chk);
-        vel_rattle(kick_op(0.5 * dt), hw);
-        ke_launch(A);
-      }
-      scale_v();
-    } else {
-      launch_k(k_step_begin, 1, 1, 0, E.stream_, sc.p, o.temperature, o.temperature_end, (long long)o.steps, ndof);
-      const bool chk = fuse_check();
-      kick_drift(0.5 * dt, dt, false, true, nullptr, nullptr, 0, 0, chk);
       KeArgs A = ke_args(kScKE, false);
       A.then = kThenBussi;
-      if (fused_tail()) {
-        forces(ener, vir, false, chk);
-        vel_rattle(kick_op_sums(0.5 * dt), hw, bussi ? &A : nullptr);
-      } else {
-        forces(ener, vir, true, chk);
-        vel_rattle(kick_op(0.5 * dt), hw);
-        if (bussi) ke_launch(A);
-      }
-      if (bussi) scale_v();
+      vel_rattle(VelOp{1, f_fast.p, 0.5 * h, 0, 0, 0, f_slow.p, 0.5 * dt}, hw, bussi ? &A : nullptr);
+      if (bussi && !pend_out) scale_v();
+      return;
     }
+    const bool chk = fuse_check();
+    if (langevin) {
+      const double c1 = std::exp(-dt / std::max(o.tau_t, 1e-9)), c2 = std::sqrt(1 - c1 * c1);
+      KickArgs K = kick_args(0.5 * dt, 0.5 * dt, false, true);
+      K.step_ahead = 1;
+      KeArgs A = ke_args(ncons ? kScKE0 : kScKE, false);
+      A.begin = 1;
+      if (ncons) {
+        move(K, false, &A);
+        A = ke_args(kScKE, false);
+        A.then = kThenBath;
+        vel_rattle(VelOp{2, nullptr, 0, c1, c2, o.seed, nullptr, 0}, 0, &A);
+        move(kick_args(0, 0.5 * dt, false, false), chk);
+      } else {
+        K.lang = 1;
+        K.c1 = c1, K.c2 = c2, K.seed = o.seed;
+        A.extra = 1;
+        A.then = kThenLang;
+        move(K, chk, &A);
+      }
+      forces(ener, vir, false, chk);
+      vel_rattle(kick_op_sums(0.5 * dt), hw);
+      return;
+    }
+    KickArgs K = kick_args(0.5 * dt, dt, pend_in, true);
+    K.step_ahead = 1;
+    if (nhc) K.chain = chain.p, K.chain_half = chain_half.p;
+    move(K, chk);
+    KeArgs A = ke_args(kScKE, false);
+    A.begin = 1;
+    A.then = nhc ? kThenNhc : kThenBussi;
+    if (!nhc && !bussi) A.n = 0;   // no thermostat: the step's scalars alone
+    forces(ener, vir, false, chk);
+    vel_rattle(kick_op_sums(0.5 * dt), hw, &A);
+    if ((nhc || bussi) && !pend_out) scale_v();
   }
 
   // Bussi draws for steps [first, first + count): r1 = gauss, then the chi-squared of ndof - 1 by a fresh Gamma
@@ -1943,6 +2073,7 @@ void MdRun::start() {
   S.sc.alloc(kScNum);
   S.sc.zero(stream_);
   S.chain.alloc(1);
+  S.chain_half.alloc(1);
   CK(cudaMemsetAsync(S.chain.p, 0, sizeof(Chain), stream_));
   S.nparts = blocks(size_t(n_), 256);
   S.part.alloc(size_t(7) * std::max(S.nparts, blocks(size_t(n_), 128)));   // k_ke's blocks, or k_vel_rattle's
@@ -1973,7 +2104,7 @@ void MdRun::start() {
   S.rng = std::make_unique<HostRng>(o.seed);
   if (S.ncons) {   // the constrained lengths hold from the start (dynamics.cpp:198-203)
     CK(cudaMemcpyAsync(S.x0.p, S.x.p, n3 * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
-    launch_k(S.C.lincs ? k_lincs : k_shake, blocks(size_t(S.C.ncl), 128), 128, 0, stream_, S.C, S.x.p, S.x0.p, S.v.p, 0.0, E.d_counters_.p, ListCheck{});
+    launch_k(S.C.lincs ? k_lincs : k_shake, blocks(size_t(S.C.ncl), 128), 128, 0, stream_, S.C, S.x.p, S.x0.p, S.v.p, 0.0, E.d_counters_.p);
   }
 
   // velocities: given, or Maxwell-Boltzmann from the reference's stream, no centre-of-mass motion, rescaled to T
@@ -2027,7 +2158,7 @@ void MdRun::start() {
     vs.alloc(n3);
     CK(cudaMemcpyAsync(xs.p, S.x.p, n3 * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
     CK(cudaMemcpyAsync(vs.p, S.v.p, n3 * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
-    S.kick_drift(0.5 * o.dt, o.dt, false, true);
+    S.move(S.kick_args(0.5 * o.dt, o.dt, false, true));
     S.vel_rattle(S.kick_op(0.5 * o.dt), o.dt);
     CK(cudaMemcpyAsync(S.x.p, xs.p, n3 * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
     CK(cudaMemcpyAsync(S.v.p, vs.p, n3 * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
@@ -2184,7 +2315,7 @@ void MdRun::mtk_step(long long s) {
   scale_by(std::exp(-dthalf * (omega_dot + mtk_term2)));
   S.vel_rattle(S.kick_op(0.5 * dt), 0);
   mtk_remap();
-  S.kick_drift(0.0, dt, false, true);
+  S.move(S.kick_args(0.0, dt, false, true));
   mtk_remap();
   S.forces(true, true);
   read_virial();
@@ -2261,7 +2392,7 @@ void MdRun::baro_step(long long s) {
   S.C.cell = E.dcell_;
   if (S.ncons) {
     CK(cudaMemcpyAsync(S.x0.p, S.x.p, n3 * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
-    launch_k(S.C.lincs ? k_lincs : k_shake, blocks(size_t(S.C.ncl), 128), 128, 0, stream_, S.C, S.x.p, S.x0.p, S.v.p, 0.0, E.d_counters_.p, ListCheck{});
+    launch_k(S.C.lincs ? k_lincs : k_shake, blocks(size_t(S.C.ncl), 128), 128, 0, stream_, S.C, S.x.p, S.x0.p, S.v.p, 0.0, E.d_counters_.p);
     S.rattle(0);
   }
   S.forces(true, true);

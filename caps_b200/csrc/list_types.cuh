@@ -17,7 +17,7 @@ struct ListGeom {
   double w[3];        // perpendicular widths of the cell
   double rlist, rlist2;
   double dw;          // rlist / w[2]
-  int batch;          // entries per work item (the pair kernels' j-tile depth), at most kBatch; chosen by timing
+  int batch;          // entries per work item (the pair kernels' j-tile depth), at most kBatch (Engine::list_depth)
 };
 
 struct ListBufs {
@@ -56,7 +56,9 @@ struct ListBufs {
 
 // Device counters: list sizes, the error word, the rebuild and prune flags, and running counts of builds and prunes.
 enum Counter { kCntEnt = 0, kCntWork, kCntMask, kCntErr, kCntRebuild, kCntNsc, kCntMaxCol, kCntPrune, kCntBuilds, kCntPrunes, kCntPairNext,
-               kCntFeneClaim, kCntNanClaim, kCntBinDone, kCntNum = 14 };   // *Claim: 1 once the first failure of that kind left its details
+               kCntFeneClaim, kCntNanClaim,   // *Claim: 1 once the first failure of that kind left its details
+               // k_list: the next unit of work, the blocks that left, and the finished units of each stage
+               kCntTicket, kCntLeft, kCntStage, kCntNum = kCntStage + 6 };
 
 __device__ __forceinline__ void raise_error(int* counters, unsigned bit) { atomicOr(reinterpret_cast<unsigned*>(counters + kCntErr), bit); }
 
@@ -70,27 +72,26 @@ __host__ __device__ __forceinline__ void unpack_image(unsigned p, int& qa, int& 
   qc = int((p >> 14) & 127u) - 64;
 }
 
-// Gate for the build kernels in a captured step: they all return at once unless the rebuild flag is set.
-__device__ __forceinline__ bool build_off(const int* counters) { return *(volatile const int*)(counters + kCntRebuild) == 0; }
-
 // The displacement check (core/src/field.cpp:800-838, the constant-cell branch): has an atom moved more than half the
 // skin since the last build (x against xb, lim_b2), or half the prune margin since the last prune (x against xp,
-// lim_p2)? Sets the rebuild and prune flags. It runs in the kernel that writes a step's final positions (the drift, or
-// SHAKE and the atoms in no constraint cluster), or as a kernel of its own; xb null: no check.
+// lim_p2)? Sets the rebuild and prune flags. It runs in the kernel that writes a step's final positions (k_move),
+// or as a kernel of its own; xb null: no check.
 struct ListCheck {
   const double* xb;
   const double* xp;
   double lim_b2, lim_p2;
   int* counters;
-  int nfree;              // SHAKE's launch: the atoms in no cluster, after the clusters
-  const int* free_atoms;
 };
-__device__ __forceinline__ void list_check_atom(const ListCheck& L, int g, const double* x, bool& mb, bool& mp) {
-  const double x_ = x[3 * g], y_ = x[3 * g + 1], z_ = x[3 * g + 2];
+__device__ __forceinline__ void list_check_at(const ListCheck& L, int g, const double p[3], bool& mb, bool& mp) {
+  const double x_ = p[0], y_ = p[1], z_ = p[2];
   const double bx = x_ - L.xb[3 * g], by = y_ - L.xb[3 * g + 1], bz = z_ - L.xb[3 * g + 2];
   const double px = x_ - L.xp[3 * g], py = y_ - L.xp[3 * g + 1], pz = z_ - L.xp[3 * g + 2];
   mb |= !(bx * bx + by * by + bz * bz <= L.lim_b2);   // NaN counts as moved
   mp |= !(px * px + py * py + pz * pz <= L.lim_p2);
+}
+__device__ __forceinline__ void list_check_atom(const ListCheck& L, int g, const double* x, bool& mb, bool& mp) {
+  const double p[3] = {x[3 * g], x[3 * g + 1], x[3 * g + 2]};
+  list_check_at(L, g, p, mb, mp);
 }
 // Raises the flags a warp's atoms call for (every lane of the warp calls it).
 __device__ __forceinline__ void list_check_flags(const ListCheck& L, bool mb, bool mp) {

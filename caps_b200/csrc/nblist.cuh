@@ -78,46 +78,30 @@ __device__ void scan_columns(const ListGeom& g, const ListBufs& b) {
     for (int s = b.col_sc[c]; s < b.col_sc[c + 1] && s < nsc; ++s) b.sc_col[s] = c;
 }
 
-// K-BIN: wrapped fractional coordinates, lattice offsets and the column of every atom; column counts. The last block
-// to finish (a ticket taken after a fence) runs the column scan, so the build has no launch of its own for it.
-constexpr int kBinThreads = 256;
-static __global__ void __launch_bounds__(kBinThreads) k_bin(int n, const double* __restrict__ x, DevCell cell, ListGeom g, ListBufs b) {
-  if (build_off(b.counters)) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    const double xi[3] = {x[3 * i], x[3 * i + 1], x[3 * i + 2]};
-    double f[3];
-    frac_of(cell, xi, f);
-    for (int k = 0; k < 3; ++k) {
-      const double fl = floor(f[k]);
-      double w = f[k] - fl;
-      w = fmin(fmax(w, 0.0), 1.0 - 1e-12);
-      b.frac[3 * i + k] = w;
-      b.ioff[3 * i + k] = -int(fl);
-    }
-    const int cu = min(g.nu - 1, int(b.frac[3 * i] * g.nu)), cv = min(g.nv - 1, int(b.frac[3 * i + 1] * g.nv));
-    const int c = cu * g.nv + cv;
-    b.col[i] = c;
-    // one atomic per distinct column in the warp (a column holds hundreds of atoms: the adds would contend)
-    const unsigned act = __activemask();
-    const unsigned same = __match_any_sync(act, c);
-    if ((threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(b.col_count + c, __popc(same));
+// Bin stage: wrapped fractional coordinates, lattice offsets and the column of atom i; column counts.
+constexpr int kListThreads = 256;   // block size of k_list (list.cuh), whose stages these are
+__device__ __forceinline__ void bin_atom(int n, int i, const double* __restrict__ x, const DevCell& cell, const ListGeom& g, const ListBufs& b) {
+  if (i >= n) return;
+  const double xi[3] = {x[3 * i], x[3 * i + 1], x[3 * i + 2]};
+  double f[3];
+  frac_of(cell, xi, f);
+  for (int k = 0; k < 3; ++k) {
+    const double fl = floor(f[k]);
+    f[k] = fmin(fmax(f[k] - fl, 0.0), 1.0 - 1e-12);
+    b.frac[3 * i + k] = f[k];
+    b.ioff[3 * i + k] = -int(fl);
   }
-  __shared__ bool s_last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(b.counters + kCntBinDone, 1) == int(gridDim.x) - 1;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  scan_columns<kBinThreads>(g, b);
-  if (threadIdx.x == 0) b.counters[kCntBinDone] = 0;
+  const int cu = min(g.nu - 1, int(f[0] * g.nu)), cv = min(g.nv - 1, int(f[1] * g.nv));
+  const int c = cu * g.nv + cv;
+  b.col[i] = c;
+  // one atomic per distinct column in the warp (a column holds hundreds of atoms: the adds would contend)
+  const unsigned act = __activemask();
+  const unsigned same = __match_any_sync(act, c);
+  if ((threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(b.col_count + c, __popc(same));
 }
 
-// K-SCATTER: atoms into their column's range (unordered; the sort that follows fixes the order).
-static __global__ void k_scatter(int n, ListBufs b) {
-  if (build_off(b.counters)) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Scatter stage: atom i into its column's range (unordered; the sort that follows fixes the order).
+__device__ __forceinline__ void scatter_atom(int n, int i, const ListBufs& b) {
   if (i >= n) return;
   const int c = b.col[i];
   // warp-aggregated: the lowest lane of each column group reserves the group's places
@@ -234,62 +218,54 @@ __device__ void form_supercluster(const DevCell& cell, const ListBufs& b, int sc
   }
 }
 
-// K-SORT (block per column): atoms by fractional c, ties by index, then the column's super-clusters (K-SUPER). A
+// Sort stage (a block per column): atoms by fractional c, ties by index, then the column's super-clusters (K-SUPER). A
 // bitonic sorting network in shared memory over the column padded to a power of two (pad keys sort last):
-// log2(n)(log2(n)+1)/2 compare-exchange rounds, one barrier each.
-constexpr int kSortThreads = 1024;
-constexpr int kScWarps = 16;   // warps of the sort block that form the column's super-clusters
-static_assert(sizeof(double) * 3 * 64 * kScWarps + sizeof(int) * 64 * kScWarps <= size_t(kSortMax) * (sizeof(double) + sizeof(int)),
-              "the super-cluster stage fits the sort's shared memory");
-static __global__ void __launch_bounds__(kSortThreads) k_sort_columns(DevCell cell, ListGeom g, ListBufs b) {
-  if (build_off(b.counters)) return;
-  extern __shared__ unsigned char smem_raw[];
+// log2(n)(log2(n)+1)/2 compare-exchange rounds, one barrier each. smem_raw: kSortMax keys and ids.
+constexpr int kScWarps = kListThreads / 32;   // the block's warps form the column's super-clusters
+constexpr size_t kSortSmem = size_t(kSortMax) * (sizeof(double) + sizeof(int));
+static_assert(sizeof(double) * 3 * 64 * kScWarps + sizeof(int) * 64 * kScWarps <= kSortSmem, "the super-cluster stage fits the sort's shared memory");
+__device__ void sort_column(int c, const DevCell& cell, const ListBufs& b, unsigned char* smem_raw) {
   const int nsc = min(b.counters[kCntNsc], b.nsc_cap);
   double* key = reinterpret_cast<double*>(smem_raw);
   int* id = reinterpret_cast<int*>(key + kSortMax);
-  for (int c = blockIdx.x; c < g.ncol; c += gridDim.x) {
-    const int s0 = b.col_start[c], n = min(b.col_start[c + 1] - s0, kSortMax);
-    int np = 1;
-    while (np < n) np <<= 1;
-    for (int k = threadIdx.x; k < np; k += blockDim.x) {
-      if (k < n) {
-        const int a = b.order[s0 + k];
-        id[k] = a;
-        key[k] = b.frac[3 * a + 2];
-      } else {
-        id[k] = 0x7fffffff;
-        key[k] = 2.0;   // fractional coordinates are below 1
-      }
+  const int s0 = b.col_start[c], n = min(b.col_start[c + 1] - s0, kSortMax);
+  int np = 1;
+  while (np < n) np <<= 1;
+  for (int k = threadIdx.x; k < np; k += blockDim.x) {
+    if (k < n) {
+      const int a = b.order[s0 + k];
+      id[k] = a;
+      key[k] = b.frac[3 * a + 2];
+    } else {
+      id[k] = 0x7fffffff;
+      key[k] = 2.0;   // fractional coordinates are below 1
     }
-    __syncthreads();
-    for (int kk = 2; kk <= np; kk <<= 1)
-      for (int j = kk >> 1; j > 0; j >>= 1) {
-        for (int t = threadIdx.x; t < (np >> 1); t += blockDim.x) {
-          const int lo = 2 * j * (t / j) + (t & (j - 1)), hi = lo + j;
-          const double ka = key[lo], kb = key[hi];
-          const int ia = id[lo], ib = id[hi];
-          const bool gt = ka > kb || (ka == kb && ia > ib);
-          if (gt == ((lo & kk) == 0)) {
-            key[lo] = kb, key[hi] = ka;
-            id[lo] = ib, id[hi] = ia;
-          }
-        }
-        __syncthreads();
-      }
-    for (int k = threadIdx.x; k < n; k += blockDim.x) b.order[s0 + k] = id[k];
-    __syncthreads();
-    // the column's super-clusters, a warp each, in the shared memory the sort is done with
-    const int w = threadIdx.x >> 5;
-    if (w < kScWarps) {
-      double(*s_w)[3] = reinterpret_cast<double(*)[3]>(smem_raw) + 64 * w;
-      int* s_a = reinterpret_cast<int*>(smem_raw + sizeof(double) * 3 * 64 * kScWarps) + 64 * w;
-      const int sc1 = min(b.col_sc[c + 1], nsc);
-      for (int sc = b.col_sc[c] + w; sc < sc1; sc += kScWarps) form_supercluster(cell, b, sc, c, threadIdx.x & 31, s_w, s_a);
-    }
-    __syncthreads();
   }
+  __syncthreads();
+  for (int kk = 2; kk <= np; kk <<= 1)
+    for (int j = kk >> 1; j > 0; j >>= 1) {
+      for (int t = threadIdx.x; t < (np >> 1); t += blockDim.x) {
+        const int lo = 2 * (t & ~(j - 1)) + (t & (j - 1)), hi = lo + j;
+        const double ka = key[lo], kb = key[hi];
+        const int ia = id[lo], ib = id[hi];
+        const bool gt = ka > kb || (ka == kb && ia > ib);
+        if (gt == ((lo & kk) == 0)) {
+          key[lo] = kb, key[hi] = ka;
+          id[lo] = ib, id[hi] = ia;
+        }
+      }
+      __syncthreads();
+    }
+  for (int k = threadIdx.x; k < n; k += blockDim.x) b.order[s0 + k] = id[k];
+  __syncthreads();
+  // the column's super-clusters, a warp each, in the shared memory the sort is done with
+  const int w = threadIdx.x >> 5;
+  double(*s_w)[3] = reinterpret_cast<double(*)[3]>(smem_raw) + 64 * w;
+  int* s_a = reinterpret_cast<int*>(smem_raw + sizeof(double) * 3 * 64 * kScWarps) + 64 * w;
+  const int sc1 = min(b.col_sc[c + 1], nsc);
+  for (int sc = b.col_sc[c] + w; sc < sc1; sc += kScWarps) form_supercluster(cell, b, sc, c, threadIdx.x & 31, s_w, s_a);
+  __syncthreads();
 }
-
 
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kSearchWarps = 8;       // warps per super-cluster in the search
@@ -362,22 +338,20 @@ static __device__ void flush_batch(SearchBatch& B, int sc, int cnt, int lane, co
   if (lane == 0) b.work[wi] = make_int4(sc, base, cnt, 0);
 }
 
-// K-SEARCH: one block of kSearchWarps warps per super-cluster. The block records the super-cluster's excluded pairs and
+// Search stage: one block of kSearchWarps warps per super-cluster. The block records the super-cluster's excluded pairs and
 // builds the atom masks of every (j cluster, image) they touch; then each warp takes a contiguous share of the
 // neighbouring columns (with their images) and batches its own entries. Exclusions (ForceField::excluded) hold at their
 // nearest image only (core/src/nbnxm.cpp:229-252): each of the super-cluster's excluded atom pairs is recorded with the
 // image that is nearest at the build, and the entry for that j cluster under that image carries masks with those pairs
 // cleared. The super-cluster's own clusters under the zero image always carry masks (each pair of a cluster with
 // itself once).
-static __global__ void __launch_bounds__(32 * kSearchWarps, 4) k_search(DevCell cell, ListGeom g, const uint32_t* __restrict__ excl_off,
-                                                                     const uint32_t* __restrict__ excl_list, ListBufs b) {
-  if (build_off(b.counters)) return;
-  extern __shared__ unsigned char smem_raw[];
-  SearchShared& S = *reinterpret_cast<SearchShared*>(smem_raw);
+static_assert(kListThreads == 32 * kSearchWarps, "the search runs in k_list's blocks");
+__device__ void search_supercluster(int sc, const DevCell& cell, const ListGeom& g, const uint32_t* __restrict__ excl_off,
+                                    const uint32_t* __restrict__ excl_list, const ListBufs& b, SearchShared& S) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   SearchBatch& B = S.batch[warp];
   const int nsc = min(b.counters[kCntNsc], b.nsc_cap);
-  for (int sc = blockIdx.x; sc < nsc; sc += gridDim.x) {
+  {
     // --- the super-cluster's boxes and exclusion records (the whole block)
     for (int t = threadIdx.x; t < kExclHash; t += blockDim.x) S.key[t] = ~0ull;
     if (threadIdx.x < 8)

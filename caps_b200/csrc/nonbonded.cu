@@ -7,15 +7,11 @@
 #include <vector>
 
 #include "engine.h"
-#include "pair.cuh"
+#include "list.cuh"
 
 namespace capsb {
 
 namespace {
-
-__global__ void k_set_flag(int* counters, int slot, int v) {
-  counters[slot] = v;
-}
 
 // Forces to the caller's AoS doubles: atom-order sums plus the pair kernel's slot-order sums.
 __global__ void k_reduce_f32(int n, const long long* __restrict__ F, const long long* __restrict__ Fs, int nslots, const int* __restrict__ iperm,
@@ -60,42 +56,12 @@ void Engine::fork(int k, const std::function<void()>& launch) {
 
 void Engine::join(int k) { CK(cudaStreamWaitEvent(stream_, ev_join_[k], 0)); }
 
-// Autotuner for the j-tile depth: the list is built with 32, 24 and 16 entries per work item and the pair kernel timed
-// on each (fewer entries per item balance small systems better, more amortise the per-item work); the fastest is kept
-// for this engine. Runs once, at the first non-bonded evaluation (never inside a stream capture).
-void Engine::tune_batch(const double* d_x) {
-  batch_tuned_ = true;
+// Chooses the launch shapes by timing, once per engine, at its first non-bonded evaluation (never inside a capture).
+void Engine::tune_shapes(const double* d_x) {
+  shapes_tuned_ = true;
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
-  float best = 1e30f;
-  int pick = batch_;
-  const size_t ns = size_t(nsc_cap_) * kScAtoms;
-  for (int bsz : {32, 24, 16}) {
-    geom_.batch = bsz;
-    launch_k(k_set_flag, 1, 1, 0, stream_, d_counters_.p, kCntRebuild, 1);
-    launch_build(d_x);
-    if (mixed_)
-      launch_k(k_pack_f32, blocks_for(ns, 256), 256, 0, stream_, int(ns), d_perm_.p, d_x, d_ioff_.p, dcell_, d_sc_org_.p, d_q_.p, d_type_.p, nt_,
-                                                           d_xq_.p, d_tslot_.p, d_counters_.p, d_x0_.p, d_Fs_.p);
-    else
-      launch_k(k_pack_f64, blocks_for(ns, 256), 256, 0, stream_, int(ns), d_perm_.p, d_x, d_ioff_.p, dcell_, d_q_.p, d_type_.p, nt_, d_xqd_.p, d_tslot_.p,
-                                                           d_counters_.p, d_x0_.p, d_Fsd_.p);
-    prune(d_x);
-    float ms = 0;
-    for (int rep = 0; rep < 4; ++rep) {
-      CK(cudaMemsetAsync(d_counters_.p + kCntPairNext, 0, sizeof(int), stream_));
-      if (rep == 1) CK(cudaEventRecord(e0, stream_));
-      pair_forces(false, false);
-    }
-    CK(cudaEventRecord(e1, stream_));
-    CK(cudaEventSynchronize(e1));
-    CK(cudaEventElapsedTime(&ms, e0, e1));
-    if (ms < best) best = ms, pick = bsz;
-  }
-  batch_ = pick;
-  geom_.batch = pick;
-  list_valid_ = false;   // the evaluation that follows builds the list with the chosen depth
   // The pair kernel's persistent grid holds every SM slot while it runs, so the bonded and PME branches of the same
   // evaluation wait for it to end unless it leaves room; PME's line transforms, on the other hand, run in fewer waves
   // on the slots left when their grid is capped. Time whole force-only evaluations for each pair (pair grid full or one
@@ -151,18 +117,38 @@ int Engine::counter(int slot) {
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-void Engine::launch_build(const double* d_x) {
-  const ListGeom& g = geom_;
-  // binning (its last block scans the columns), the scatter into columns, and the sort of each column (its block then
-  // forms the column's super-clusters): three launches before the search
-  launch_k(k_bin, blocks_for(size_t(n_), kBinThreads), kBinThreads, 0, stream_, n_, d_x, dcell_, g, lb_);
-  launch_k(k_scatter, blocks_for(size_t(n_), 256), 256, 0, stream_, n_, lb_);
-  const size_t sort_smem = size_t(kSortMax) * (sizeof(double) + sizeof(int));
-  launch_k(k_sort_columns, std::min(g.ncol, dev_sms_ * 8), kSortThreads, sort_smem, stream_, dcell_, g, lb_);
-  if (sizeof(SearchShared) > 48 * 1024) CK(cudaFuncSetAttribute(k_search, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(SearchShared))));
-  launch_k(k_search, std::max(1, std::min(nsc_cap_, dev_sms_ * 8)), 32 * kSearchWarps, sizeof(SearchShared), stream_, dcell_, g, d_excl_off_.p,
-                                                                                                          d_excl_list_.p, lb_);
-  CK(cudaGetLastError());
+// The list kernel (list.cuh): build and prune where flagged (build: forced), and the packed positions. The grid is what
+// fits at its four blocks per SM, and no more than the stages have units for.
+void Engine::launch_list(const double* d_x, bool build) {
+  const double b = std::min(0.8, skin_);   // the prune margin (field.cpp:1306-1312)
+  const double rp = rc_ + b;
+  const int nslots = nsc_cap_ * kScAtoms;
+  ListArgs L{};
+  L.n = n_;
+  L.nslots = nslots;
+  L.x = d_x;
+  L.cell = dcell_;
+  L.g = geom_;
+  L.b = lb_;
+  L.excl_off = d_excl_off_.p;
+  L.excl_list = d_excl_list_.p;
+  L.force = build ? 1 : 0;
+  L.pack_only = frozen_ ? 1 : 0;
+  L.q = d_q_.p;
+  L.type = d_type_.p;
+  L.pad_type = nt_;
+  L.xq = d_xq_.p;
+  L.xqd = d_xqd_.p;
+  L.tslot = d_tslot_.p;
+  L.x0 = d_x0_.p;
+  L.xp = d_xp_.p;
+  L.fs = d_Fs_.p;
+  L.fsd = d_Fsd_.p;
+  L.rprune2 = rp * rp;
+  auto* kernel = mixed_ ? k_list<false> : k_list<true>;
+  const size_t smem = sizeof(ListShared);
+  CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));   // above 48 KB with the static part
+  launch_k(kernel, std::min(4 * dev_sms_, std::max(dev_sms_, nsc_cap_)), kListThreads, smem, stream_, L);
 }
 
 PairArgs Engine::pair_args() {
@@ -213,22 +199,12 @@ PairArgs Engine::pair_args() {
   return A;
 }
 
-ListCheck Engine::list_check(int nfree, const int* free_atoms) const {
-  const double b = std::min(0.8, skin_);   // the prune margin (see prune())
-  return ListCheck{d_x0_.p, d_xp_.p, 0.25 * skin_ * skin_, 0.25 * b * b, d_counters_.p, nfree, free_atoms};
+ListCheck Engine::list_check() const {
+  const double b = std::min(0.8, skin_);   // the prune margin (launch_list)
+  return ListCheck{d_x0_.p, d_xp_.p, 0.25 * skin_ * skin_, 0.25 * b * b, d_counters_.p};
 }
 
 bool Engine::list_check_fusable() const { return (opt_.parts & 2) != 0 && list_valid_ && !frozen_; }
-
-// Dynamic pruning: when an atom has moved b/2 since the last prune (b = min(0.8 Å, skin), as field.cpp:1306-1312; the
-// step's displacement check tests it), or a build set the flag, every entry's masks are rewritten for r_c + b.
-void Engine::prune(const double* d_x) {
-  const double b = std::min(0.8, skin_);
-  const PairArgs A = pair_args();
-  const double rp = rc_ + b;
-  if (mixed_) launch_k(k_prune<false>, dev_sms_ * 8, 128, 0, stream_, A, rp * rp, d_ent_.p, n_, d_x, d_xp_.p);
-  else launch_k(k_prune<true>, dev_sms_ * 8, 128, 0, stream_, A, rp * rp, d_ent_.p, n_, d_x, d_xp_.p);
-}
 
 void Engine::pair_forces(bool ener, bool vir) {
   PairArgs A = pair_args();
@@ -368,8 +344,8 @@ void Engine::forces(const double* d_x, bool ener, bool vir, bool check_rebuild, 
   const int pm = parts >= 0 ? parts : ((opt_.parts & 1) | ((opt_.parts & 2) ? 6 : 0));
   const bool nonb = (pm & 2) != 0;
   double* out = d_out ? d_out : d_f_.p;
-  if (nonb && !batch_tuned_) tune_batch(d_x);
-  // the atom-order sums start at zero (the integrator's kick may have cleared them already); the pack kernel clears the
+  if (nonb && !shapes_tuned_) tune_shapes(d_x);
+  // the atom-order sums start at zero (the integrator's kick may have cleared them already); the list kernel clears the
   // pair kernel's slot-order sums
   if (!sums_cleared_) {
     if (mixed_) CK(cudaMemsetAsync(d_F_.p, 0, d_F_.n * sizeof(long long), stream_));
@@ -382,27 +358,14 @@ void Engine::forces(const double* d_x, bool ener, bool vir, bool check_rebuild, 
   }
   // Three branches: bonded terms and PME beside the list and pair kernels. All add into order-free fixed-point (or
   // atomic FP64) sums, so how the branches interleave does not change the mixed path's result.
-  fork(0, [&] { bonded_forces(d_x, ener, vir, pm); });
   const bool pme = (pm & 4) != 0 && pme_;
   if (pme) fork(1, [&] { pme_forces(d_x, ener, vir); });
+  fork(0, [&] { bonded_forces(d_x, ener, vir, pm); });
   if (nonb) {
-    if (frozen_) {
-      // a frozen pair set: no displacement check, build or prune; the pack and the pair kernel run on the frozen list
-    } else if (!list_valid_) {
-      launch_k(k_set_flag, 1, 1, 0, stream_, d_counters_.p, kCntRebuild, 1);
-      list_valid_ = true;
-    } else if (check_rebuild) {
-      launch_k(k_check_step, blocks_for(size_t(n_), 256), 256, 0, stream_, n_, d_x, list_check(0, nullptr));
-    }
-    if (!frozen_) launch_build(d_x);
-    const size_t ns = size_t(nsc_cap_) * kScAtoms;
-    if (mixed_)
-      launch_k(k_pack_f32, blocks_for(ns, 256), 256, 0, stream_, int(ns), d_perm_.p, d_x, d_ioff_.p, dcell_, d_sc_org_.p, d_q_.p, d_type_.p, nt_,
-                                                           d_xq_.p, d_tslot_.p, d_counters_.p, d_x0_.p, d_Fs_.p);
-    else
-      launch_k(k_pack_f64, blocks_for(ns, 256), 256, 0, stream_, int(ns), d_perm_.p, d_x, d_ioff_.p, dcell_, d_q_.p, d_type_.p, nt_, d_xqd_.p, d_tslot_.p,
-                                                           d_counters_.p, d_x0_.p, d_Fsd_.p);
-    if (!frozen_) prune(d_x);
+    const bool build = !frozen_ && !list_valid_;
+    if (build) list_valid_ = true;
+    else if (!frozen_ && check_rebuild) launch_k(k_check_step, blocks_for(size_t(n_), 256), 256, 0, stream_, n_, d_x, list_check());
+    launch_list(d_x, build);
     pair_forces(ener, vir);
   }
   join(0);

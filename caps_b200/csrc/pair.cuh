@@ -1,4 +1,4 @@
-// K-PACK and K-PAIR: the LJ 12-6 plus real-space Coulomb pair kernels over the cluster pair list.
+// K-PAIR: the LJ 12-6 plus real-space Coulomb pair kernels over the cluster pair list.
 //
 // Reference: the FP64 atom-pair loop (core/src/field.cpp:1604-1686: 12-6 LJ with the cut-off shift, Ewald real space
 // from the cubic-Hermite table of erf(kappa sqrt s)/sqrt s, field.cpp:1126-1157 and 1593-1602, DSF) and the FP32
@@ -19,73 +19,6 @@
 namespace capsb {
 
 constexpr float kPadFar = 1.0e5f;   // padding slots sit this far from their super-cluster's origin (never within reach)
-
-// K-PACK (FP32): per slot, float4 (position relative to the super-cluster origin, charge) and the type index.
-static __global__ void k_pack_f32(int nslots, const int* __restrict__ perm, const double* __restrict__ x, const int* __restrict__ ioff, DevCell cell,
-                           const double* __restrict__ sc_org, const double* __restrict__ q, const int* __restrict__ type, int pad_type,
-                           float4* __restrict__ xq, int* __restrict__ tslot, int* counters, double* __restrict__ x0,
-                           long long* __restrict__ fs) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < nslots)   // the pair kernel's slot-order sums (3 x nslots) start at zero
-    for (int r = 0; r < 3; ++r) fs[size_t(r) * nslots + s] = 0;
-  const bool built = counters[kCntRebuild] != 0;   // a build ran this step: the list was built at these positions
-  if (s == 0) {
-    counters[kCntPairNext] = 0;   // the pair kernel's work-item counter
-    if (built) {
-      counters[kCntPrune] = 1;    // a fresh list is pruned at once
-      counters[kCntBuilds] += 1;
-    }
-  }
-  const int nsc = counters[kCntNsc];
-  if (s >= nslots || s >= 64 * nsc) return;
-  const int a = perm[s];
-  if (a < 0) {
-    xq[s] = make_float4(0.f, 0.f, kPadFar, 0.f);
-    tslot[s] = pad_type;
-    return;
-  }
-  if (built)
-    for (int r = 0; r < 3; ++r) x0[3 * a + r] = x[3 * a + r];
-  const int sc = s >> 6;
-  const int o0 = ioff[3 * a], o1 = ioff[3 * a + 1], o2 = ioff[3 * a + 2];
-  float p[3];
-  for (int r = 0; r < 3; ++r)
-    p[r] = float(x[3 * a + r] + (cell.h[r][0] * o0 + cell.h[r][1] * o1 + cell.h[r][2] * o2) - sc_org[3 * sc + r]);
-  xq[s] = make_float4(p[0], p[1], p[2], float(q[a]));
-  tslot[s] = type[a];
-}
-
-// K-PACK (FP64): per slot, double4 (wrapped absolute position, charge) and the type index.
-static __global__ void k_pack_f64(int nslots, const int* __restrict__ perm, const double* __restrict__ x, const int* __restrict__ ioff, DevCell cell,
-                           const double* __restrict__ q, const int* __restrict__ type, int pad_type, double4* __restrict__ xq, int* __restrict__ tslot,
-                           int* counters, double* __restrict__ x0, double* __restrict__ fs) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < nslots)   // the pair kernel's slot-order sums (3 x nslots) start at zero
-    for (int r = 0; r < 3; ++r) fs[size_t(r) * nslots + s] = 0;
-  const bool built = counters[kCntRebuild] != 0;
-  if (s == 0) {
-    counters[kCntPairNext] = 0;
-    if (built) {
-      counters[kCntPrune] = 1;
-      counters[kCntBuilds] += 1;
-    }
-  }
-  const int nsc = counters[kCntNsc];
-  if (s >= nslots || s >= 64 * nsc) return;
-  const int a = perm[s];
-  if (a < 0) {
-    xq[s] = make_double4(1e7, 1e7, 1e7 + 16.0 * (s & 63), 0.0);
-    tslot[s] = pad_type;
-    return;
-  }
-  if (built)
-    for (int r = 0; r < 3; ++r) x0[3 * a + r] = x[3 * a + r];
-  const int o0 = ioff[3 * a], o1 = ioff[3 * a + 1], o2 = ioff[3 * a + 2];
-  double p[3];
-  for (int r = 0; r < 3; ++r) p[r] = x[3 * a + r] + (cell.h[r][0] * o0 + cell.h[r][1] * o1 + cell.h[r][2] * o2);
-  xq[s] = make_double4(p[0], p[1], p[2], q[a]);
-  tslot[s] = type[a];
-}
 
 struct PairArgs {
   const int4* work;
@@ -124,8 +57,8 @@ struct PairArgs {
   int* err;              // the error word (range errors of the fixed-point sums)
 };
 
-// Work items are taken dynamically: each warp fetches the next unclaimed item from a device counter (reset by the pack
-// kernel before every force evaluation). Items differ in size, so a static split leaves SMs idle at the end of the launch.
+// Work items are taken dynamically: each warp fetches the next unclaimed item from a device counter (reset by k_list
+// before every force evaluation). Items differ in size, so a static split leaves SMs idle at the end of the launch.
 __device__ __forceinline__ int next_work_item(const int* counters, int lane) {
   int w = 0;
   if (lane == 0) w = atomicAdd(const_cast<int*>(counters) + kCntPairNext, 1);
@@ -238,7 +171,7 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
     c[kCntPrune] = 0;
   }
   // a list build that ran out of room leaves stale work items: skip the pass, the host reports the error
-  if (A.counters[kCntErr] & (kErrListOverflow | kErrMaskOverflow | kErrScOverflow | kErrColumnTooBig | kErrExclOverflow)) return;
+  if (A.counters[kCntErr] & kErrListBad) return;
   const int nwork = min(A.counters[kCntWork], A.work_cap);
   const int pad = A.ntab - 1;
   const float rc2 = float(A.rc2), beta = float(A.beta), kc = float(A.kc), kcoul = float(A.kcoul);
@@ -519,7 +452,7 @@ static __global__ void __launch_bounds__(128, 2) k_pair_f64(PairArgs A) {
     c[kCntRebuild] = 0;
     c[kCntPrune] = 0;
   }
-  if (A.counters[kCntErr] & (kErrListOverflow | kErrMaskOverflow | kErrScOverflow | kErrColumnTooBig | kErrExclOverflow)) return;
+  if (A.counters[kCntErr] & kErrListBad) return;
   const int nwork = min(A.counters[kCntWork], A.work_cap);
   const int pad = A.ntab - 1;
   double acc_v = 0, acc_c = 0, acc_w[6] = {0, 0, 0, 0, 0, 0};
@@ -687,7 +620,7 @@ static __global__ void __launch_bounds__(128, 2) k_pair_f64(PairArgs A) {
 // cluster the 64 atom pairs that are listed, real, not excluded and inside r_c at the packed positions; the entry's
 // half mask becomes their union, so that the pair kernel visits exactly those halves. One thread per entry.
 static __global__ void __launch_bounds__(128) k_freeze(PairArgs A, uint4* __restrict__ ent, unsigned long long* __restrict__ frozen) {
-  if (A.counters[kCntErr] & (kErrListOverflow | kErrMaskOverflow | kErrScOverflow | kErrColumnTooBig | kErrExclOverflow)) return;
+  if (A.counters[kCntErr] & kErrListBad) return;
   const int nwork = min(A.counters[kCntWork], A.work_cap);
   const int pad = A.ntab - 1;
   const int lane = threadIdx.x & 31;
@@ -737,7 +670,7 @@ static __global__ void __launch_bounds__(128) k_freeze(PairArgs A, uint4* __rest
 static __global__ void __launch_bounds__(128) k_count_pairs(PairArgs A, const uint4* __restrict__ ent, const int* __restrict__ perm,
                                                            const double* __restrict__ x0, const int* __restrict__ ioff, double rl2,
                                                            unsigned long long* __restrict__ out) {
-  if (A.counters[kCntErr] & (kErrListOverflow | kErrMaskOverflow | kErrScOverflow | kErrColumnTooBig | kErrExclOverflow)) return;
+  if (A.counters[kCntErr] & kErrListBad) return;
   const int nwork = min(A.counters[kCntWork], A.work_cap);
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -777,111 +710,5 @@ static __global__ void __launch_bounds__(128) k_count_pairs(PairArgs A, const ui
   }
   if (cnt) atomicAdd(out, cnt);
 }
-
-// K-PRUNE (dynamic pruning, as core/src/nbnxm.cpp:328-363 does on the CPU): each entry's mask is rewritten to the
-// (i cluster, j half) pairs with at least one atom pair inside r_prune = r_c + b at the present positions; the pair
-// kernels read that mask. The j halves are the cluster's lower-x and upper-x four atoms (the cluster split orders its
-// atoms along x), so a half mask drops the far half of a j cluster that reaches an i cluster with its near half only. Pruned again once an atom has moved b/2 since the last prune, so no pair inside r_c is lost. Gated by
-// the prune flag, set by the displacement check and by every list build. FP32 path: packed float positions; FP64 path:
-// packed double positions.
-template <bool DBL>
-static __global__ void __launch_bounds__(128) k_prune(PairArgs A, double rprune2, uint4* __restrict__ ent, int n, const double* __restrict__ x,
-                                                     double* __restrict__ xp) {
-  if (*(volatile const int*)(A.counters + kCntPrune) == 0) return;
-  // the positions of this prune, for the next displacement check; and the prune count
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * n; i += gridDim.x * blockDim.x) xp[i] = x[i];
-  if (blockIdx.x == 0 && threadIdx.x == 0) const_cast<int*>(A.counters)[kCntPrunes] += 1;
-  if (A.counters[kCntErr] & (kErrListOverflow | kErrMaskOverflow | kErrScOverflow | kErrColumnTooBig | kErrExclOverflow)) return;
-  // per warp: the work item's i atoms, its entries' j atoms (w: 1 real, 0 padding) and the new half masks
-  __shared__ float4 s_xi[4][64];
-  __shared__ float4 s_xj[4][kBatch * 8];
-  __shared__ unsigned s_keep[4][kBatch];
-  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int i8 = lane & 7, jq = lane >> 3;
-  const int nwork = min(A.counters[kCntWork], A.work_cap);
-  const int pad = A.ntab - 1;
-  const float rp2 = float(rprune2);
-  for (int w = blockIdx.x * 4 + wib; w < nwork; w += gridDim.x * 4) {
-    const int4 wk = A.work[w];
-    const int sc = wk.x;
-    const int ne = min(wk.z, kBatch);
-    // one batch of independent loads: i atoms, the entries, then every entry's 8 j atoms with the entry's image shift
-    uint4 en = make_uint4(0u, 0u, 0u, 0u);
-    float sx = 0.f, sy = 0.f, sz = 0.f;
-    if (lane < ne) {
-      en = ent[wk.y + lane];
-      if (DBL) {
-        int qa, qb, qc;
-        unpack_image(en.y >> 8, qa, qb, qc);
-        sx = float(A.cell.h[0][0] * qa + A.cell.h[0][1] * qb + A.cell.h[0][2] * qc);
-        sy = float(A.cell.h[1][0] * qa + A.cell.h[1][1] * qb + A.cell.h[1][2] * qc);
-        sz = float(A.cell.h[2][0] * qa + A.cell.h[2][1] * qb + A.cell.h[2][2] * qc);
-      } else {
-        const float4 sh = A.ent_shift[wk.y + lane];
-        sx = sh.x, sy = sh.y, sz = sh.z;
-      }
-    }
-    for (int t = lane; t < 64; t += 32) {
-      float4 v;
-      if (DBL) {
-        const double4 d = A.xqd[64 * sc + t];
-        v = make_float4(float(d.x), float(d.y), float(d.z), 0.f);
-      } else {
-        v = A.xq[64 * sc + t];
-      }
-      v.w = A.tslot[64 * sc + t] != pad ? 1.f : 0.f;
-      s_xi[wib][t] = v;
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int t = lane + 32 * k;   // entry t / 8, j atom t % 8
-      const int e = t >> 3;
-      const unsigned cj = __shfl_sync(0xffffffffu, en.x, e & 31);
-      const float ex = __shfl_sync(0xffffffffu, sx, e & 31), ey = __shfl_sync(0xffffffffu, sy, e & 31),
-                  ez = __shfl_sync(0xffffffffu, sz, e & 31);
-      if (e < ne) {
-        const int ja = 8 * int(cj) + (t & 7);
-        float4 v;
-        // FP64 path: absolute positions rounded to float (1e-5 Å at 100 Å), far inside the 0.8 Å prune margin
-        if (DBL) {
-          const double4 d = A.xqd[ja];
-          v = make_float4(float(d.x), float(d.y), float(d.z), 0.f);
-        } else {
-          v = A.xq[ja];
-        }
-        v.x += ex, v.y += ey, v.z += ez;
-        v.w = A.tslot[ja] != pad ? 1.f : 0.f;
-        s_xj[wib][t] = v;
-      }
-    }
-    __syncwarp();
-    for (int el = 0; el < ne; ++el) {
-      const unsigned built = __shfl_sync(0xffffffffu, en.y, el) & 255u;
-      const float4 a0 = s_xj[wib][8 * el + jq], a1 = s_xj[wib][8 * el + jq + 4];
-      unsigned keep = 0;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        if (!((built >> c) & 1u)) continue;
-        const float4 xi = s_xi[wib][8 * c + i8];
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-          const float4 xj = jj ? a1 : a0;
-          const float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-          const float r2 = dx * dx + dy * dy + dz * dz;
-          const bool in = xi.w != 0.f && xj.w != 0.f && r2 < rp2;
-          if (__any_sync(0xffffffffu, in)) keep |= 1u << (c + 8 * jj);
-        }
-      }
-      if (lane == 0) s_keep[wib][el] = keep;
-    }
-    __syncwarp();
-    if (lane < ne) {
-      en.w = s_keep[wib][lane];
-      ent[wk.y + lane] = en;
-    }
-    __syncwarp();
-  }
-}
-
 
 }  // namespace capsb

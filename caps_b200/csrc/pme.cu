@@ -26,6 +26,18 @@ void factor_radices(int n, int* rad, int& nst) {
 
 }  // namespace
 
+// The active path's spread grid, zero when it is made: every transform of it leaves it zero (k_fft_x_fwd).
+void Engine::ensure_grid() {
+  const size_t want = size_t(pk_[0]) * pk_[1] * pk_[2];
+  if (mixed_ && (!d_gridq_.p || d_gridq_.n < want)) {
+    d_gridq_.alloc(want);
+    d_gridq_.zero(stream_);
+  } else if (!mixed_ && (!d_grid_.p || d_grid_.n < want)) {
+    d_grid_.alloc(want);
+    d_grid_.zero(stream_);
+  }
+}
+
 template <class R>
 void Engine::pme_setup(PmePath<R>& P) {
   using T = typename Cpx<R>::T;
@@ -34,8 +46,7 @@ void Engine::pme_setup(PmePath<R>& P) {
   P.gr.alloc(size_t(pk_[0]) * pk_[1] * pk_[2]);
   P.gt.alloc(half);
   P.wt.alloc(6 * half);
-  if (mixed_) d_gridq_.alloc(size_t(pk_[0]) * pk_[1] * pk_[2]);
-  d_grid_.alloc(size_t(pk_[0]) * pk_[1] * pk_[2]);
+  ensure_grid();
   for (int d = 0; d < 3; ++d)
     for (int dir = 0; dir < 2; ++dir) {
       const int nn = pk_[d];
@@ -86,7 +97,7 @@ void Engine::pin_tuning(const int32_t v[7]) {
   auto& lines = mixed_ ? pf_.lines : pd_.lines;
   for (int d = 0; d < 3; ++d) lines[d] = v[4 + d];
   tuning_pinned_ = true;
-  batch_tuned_ = true;
+  shapes_tuned_ = true;
   list_valid_ = false;
   drop_run_state();
 }
@@ -98,9 +109,11 @@ void Engine::ensure_pme() {
   auto same = [&](const int* k) { return k[0] == pk_[0] && k[1] == pk_[1] && k[2] == pk_[2]; };
   if (mixed_) {
     if (!same(pf_.k)) pme_setup(pf_);
-    d_gridq_.alloc(size_t(pk_[0]) * pk_[1] * pk_[2]);
+    ensure_grid();
   } else if (!same(pd_.k)) {
     pme_setup(pd_);
+  } else {
+    ensure_grid();
   }
 }
 
@@ -149,8 +162,6 @@ void Engine::pme_tune(PmePath<R>& P) {
   CK(cudaMemsetAsync(P.gt.p, 0, half * sizeof(R), stream_));
   CK(cudaMemsetAsync(P.wt.p, 0, 6 * half * sizeof(R), stream_));
   CK(cudaMemsetAsync(P.h.p, 0, half * sizeof(T), stream_));
-  if (mixed_) CK(cudaMemsetAsync(d_gridq_.p, 0, d_gridq_.n * sizeof(long long), stream_));
-  else CK(cudaMemsetAsync(d_grid_.p, 0, d_grid_.n * sizeof(double), stream_));
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -190,8 +201,6 @@ void Engine::pme_run(PmePath<R>& P, const double* d_x, bool ener, bool vir) {
     green_valid_ = true;
   }
   const int nb = blocks_for(size_t(n_), 128);
-  if (mixed_) CK(cudaMemsetAsync(d_gridq_.p, 0, d_gridq_.n * sizeof(long long), stream_));
-  else CK(cudaMemsetAsync(d_grid_.p, 0, d_grid_.n * sizeof(double), stream_));
 #define SPREAD(P_)                                                                            \
   do {                                                                                        \
     if (mixed_) launch_k(k_spread<float, P_>, nb, 128, 0, stream_, A, d_grid_.p, d_gridq_.p);      \

@@ -181,9 +181,11 @@ static __global__ void k_spread(PmeArgs A, double* __restrict__ g, long long* __
 }
 
 // Shared memory of the line-transform kernels: the twiddle table(s), then two buffers of `lines` lines of length n.
-// K-FFT-X forward: real lines (b, c) of length K1 to half spectra h(a, b, c), a <= K1/2. Input: g (double) or gq (fixed).
+// K-FFT-X forward: real lines (b, c) of length K1 to half spectra h(a, b, c), a <= K1/2. Input: g (double) or gq (fixed),
+// cleared as it is read: the grid is zero for the next spread, with no launch of its own for it (as a memset node of the
+// step's graph it started up to 10 us after the step's drift, and the spread behind it).
 template <class R>
-static __global__ void __launch_bounds__(128) k_fft_x_fwd(PmeArgs A, const double* __restrict__ g, const long long* __restrict__ gq,
+static __global__ void __launch_bounds__(128) k_fft_x_fwd(PmeArgs A, double* __restrict__ g, long long* __restrict__ gq,
                                                           typename Cpx<R>::T* __restrict__ h, FftPlan<R> P, int lines_per_block) {
   using T = typename Cpx<R>::T;
   extern __shared__ unsigned char smem_raw[];
@@ -197,7 +199,14 @@ static __global__ void __launch_bounds__(128) k_fft_x_fwd(PmeArgs A, const doubl
     const int nl = min(lines_per_block, nlines - l0);
     for (int t = threadIdx.x; t < nl * A.k1; t += blockDim.x) {
       const size_t gidx = size_t(l0) * A.k1 + t;   // lines are contiguous in the real grid
-      const R v = gq ? R(double(gq[gidx]) * kInvFixQ) : R(g[gidx]);
+      R v;
+      if (gq) {
+        v = R(double(gq[gidx]) * kInvFixQ);
+        gq[gidx] = 0;
+      } else {
+        v = R(g[gidx]);
+        g[gidx] = 0;
+      }
       s0[t] = {v, R(0)};
     }
     __syncthreads();
