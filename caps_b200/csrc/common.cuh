@@ -195,7 +195,7 @@ template <> struct ForceSink<float> {
     one(fy + i, y);
     one(fz + i, z);
   }
-  __device__ __forceinline__ void add1(int comp, int i, double v) const { one(comp == 0 ? fx : comp == 1 ? fy : fz, v); }
+  __device__ __forceinline__ void add1(int comp, int i, double v) const { one((comp == 0 ? fx : comp == 1 ? fy : fz) + i, v); }
 };
 template <> struct ForceSink<double> {
   double* fx;

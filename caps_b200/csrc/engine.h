@@ -119,10 +119,10 @@ struct PmePath {
   DevBuf<T> h;          // half spectrum
   DevBuf<R> gr;         // real grid after the inverse transform
   DevBuf<R> gt, wt;     // influence function, virial weights
-  DevBuf<T> tw[3][2];   // twiddles per axis: forward, inverse
-  FftPlan<R> plan[3][2];
+  DevBuf<T> tw[3];      // twiddles per axis
+  FftPlan<R> plan[3];
   int k[3] = {0, 0, 0};      // the grid these were set up for
-  int lines[3] = {1, 1, 1};  // line-transform block shapes (x lines per block; y, z consecutive a per block), tuned
+  int lines[3] = {1, 1, 1};  // line-transform block shapes (x pairs of lines per block; y, z consecutive a per block), tuned
 };
 
 class Engine {

@@ -16,12 +16,25 @@ namespace capsb {
 
 namespace {
 
-void factor_radices(int n, int* rad, int& nst) {
+// The passes of a length: as few radices as can be (at most 16 each), and among those with odd ones first, whose first
+// pass writes shared memory at an odd stride. Grid lengths are 2^a 3^b 5^c 7^d.
+void plan_radices(int n, int* rad, int& nst) {
+  static const int radices[] = {16, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+  std::vector<int> best(size_t(n) + 1, kMaxRadices + 1), from(size_t(n) + 1, 0);
+  best[1] = 0;
+  for (int m = 2; m <= n; ++m)
+    for (int r : radices)
+      if (m % r == 0 && best[size_t(m / r)] + 1 < best[size_t(m)]) best[size_t(m)] = best[size_t(m / r)] + 1, from[size_t(m)] = r;
+  if (best[size_t(n)] > kMaxRadices) throw ModelError(CAPS_GPU_EINVAL, "PME grid length " + std::to_string(n) + " cannot be factored for the line FFT");
   nst = 0;
-  int r = n;
-  while (r % 4 == 0 && nst < kMaxRadices) rad[nst++] = 4, r /= 4;
-  for (int p : {2, 3, 5, 7}) while (r % p == 0 && nst < kMaxRadices) rad[nst++] = p, r /= p;
-  if (r != 1) throw ModelError(CAPS_GPU_EINVAL, "PME grid length " + std::to_string(n) + " cannot be factored for the line FFT");
+  for (int m = n; m > 1; m /= from[size_t(m)]) rad[nst++] = from[size_t(m)];
+  std::sort(rad, rad + nst, [](int a, int b) { return (a & 1) != (b & 1) ? (a & 1) > (b & 1) : a < b; });
+}
+
+int log2_floor(int v) {
+  int s = 0;
+  while ((2 << s) <= v) ++s;
+  return s;
 }
 
 }  // namespace
@@ -47,26 +60,31 @@ void Engine::pme_setup(PmePath<R>& P) {
   P.gt.alloc(half);
   P.wt.alloc(6 * half);
   ensure_grid();
-  for (int d = 0; d < 3; ++d)
-    for (int dir = 0; dir < 2; ++dir) {
-      const int nn = pk_[d];
-      const int sign = dir == 0 ? -1 : +1;   // forward e^{-i}, inverse e^{+i}: the convolution is the same either way
-      std::vector<T> tw(static_cast<size_t>(nn));
-      for (int k = 0; k < nn; ++k) {
-        const double ang = 2 * kPi * k / nn;
-        tw[size_t(k)] = T{R(std::cos(ang)), R(sign * std::sin(ang))};
-      }
-      P.tw[d][dir].upload(tw, stream_);
-      FftPlan<R>& pl = P.plan[d][dir];
-      pl.n = nn;
-      factor_radices(nn, pl.rad, pl.nst);
-      pl.tw = P.tw[d][dir].p;
-      pl.sign = sign;
+  for (int d = 0; d < 3; ++d) {
+    const int nn = pk_[d];
+    std::vector<T> tw(static_cast<size_t>(nn));
+    for (int k = 0; k < nn; ++k) {
+      const double ang = 2 * kPi * k / nn;
+      tw[size_t(k)] = T{R(std::cos(ang)), R(-std::sin(ang))};
     }
-  // Lines per block. x: contiguous lines, enough blocks for four per SM, two buffers within 40 KB of shared memory.
-  // y, z: `la` consecutive a per block so that each row read is 128 bytes.
+    P.tw[d].upload(tw, stream_);
+    FftPlan<R>& pl = P.plan[d];
+    pl.n = nn;
+    plan_radices(nn, pl.rad, pl.nst);
+    int ns = 1;
+    for (int p = 0; p < pl.nst; ++p) {
+      pl.nb[p] = nn / pl.rad[p];
+      pl.ns[p] = ns;
+      pl.m_nb[p] = div_magic(unsigned(pl.nb[p]));
+      pl.m_ns[p] = div_magic(unsigned(ns));
+      ns *= pl.rad[p];
+    }
+    pl.tw = P.tw[d].p;
+  }
+  // Lines per block. x: pairs of contiguous lines, enough blocks for four per SM, two buffers within 40 KB of shared
+  // memory. y, z: consecutive a per block (a power of two of them) so that each row read is 128 bytes.
   const int cap = int(40 * 1024 / (2 * sizeof(T)));
-  const int nlx = pk_[1] * pk_[2];
+  const int nlx = (pk_[1] * pk_[2] + 1) / 2;
   P.lines[0] = std::max(1, std::min({cap / pk_[0], 16, (nlx + 4 * dev_sms_ - 1) / (4 * dev_sms_)}));
   const int la = int(128 / sizeof(T));
   P.lines[1] = std::max(1, std::min({la, cap / pk_[1], ph1_}));
@@ -122,27 +140,32 @@ template <class R>
 void Engine::fft_passes(PmePath<R>& P, bool ener, bool vir) {
   using T = typename Cpx<R>::T;
   PmeArgs A{pk_[0], pk_[1], pk_[2], ph1_, dcell_, nullptr, d_q_.p, n_};
-  // shared memory: twiddle table(s) + two line buffers
-  const size_t sx = (size_t(P.lines[0]) * 2 + 1) * pk_[0] * sizeof(T), sy = (size_t(P.lines[1]) * 2 + 1) * pk_[1] * sizeof(T),
-               sz = (size_t(P.lines[2]) + 1) * 2 * pk_[2] * sizeof(T);
-  const int nlx = pk_[1] * pk_[2];
+  // shared memory: twiddle table + two line buffers (y, z: 1 << ly, lz lines, the powers of two in P.lines)
+  const int ly = log2_floor(P.lines[1]), lz = log2_floor(P.lines[2]);
+  const size_t sx = (size_t(P.lines[0]) * 2 * (pk_[0] | 1) + pk_[0]) * sizeof(T), sy = ((size_t(2) << ly) + 1) * pk_[1] * sizeof(T),
+               sz = ((size_t(2) << lz) + 1) * pk_[2] * sizeof(T);
+  const int nlx = (pk_[1] * pk_[2] + 1) / 2;
   // the kernels stride over their line groups: a grid cap (the tuner's pme_cap_, 0 for none) leaves SM slots to the
   // pair kernel that runs beside them
   auto capped = [&](int g) { return pme_cap_ > 0 ? std::min(g, pme_cap_) : g; };
-  launch_k(k_fft_x_fwd<R>, capped(blocks_for(size_t(nlx), P.lines[0])), 128, sx, stream_, A, mixed_ ? nullptr : d_grid_.p, mixed_ ? d_gridq_.p : nullptr, P.h.p,
-                                                                        P.plan[0][0], P.lines[0]);
-  const int gy = capped(((ph1_ + P.lines[1] - 1) / P.lines[1]) * pk_[2]);
-  launch_k(k_fft_y<R>, gy, 128, sy, stream_, A, P.h.p, P.plan[1][0], P.lines[1]);
-  const int gz = capped(((ph1_ + P.lines[2] - 1) / P.lines[2]) * pk_[1]);
+  auto allow = [&](auto* kernel, size_t smem) {   // long lines need more than the default 48 KB
+    if (smem > 48 * 1024) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    return kernel;
+  };
+  const int gx = capped(blocks_for(size_t(nlx), P.lines[0]));
+  launch_k(allow(k_fft_x_fwd<R>, sx), gx, 128, sx, stream_, A, mixed_ ? nullptr : d_grid_.p, mixed_ ? d_gridq_.p : nullptr, P.h.p, P.plan[0], P.lines[0]);
+  const int gy = capped(blocks_for(size_t(ph1_), 1 << ly) * pk_[2]);
+  launch_k(allow(k_fft_y<R, false>, sy), gy, 128, sy, stream_, A, P.h.p, P.plan[1], ly);
+  const int gz = capped(blocks_for(size_t(ph1_), 1 << lz) * pk_[1]);
   EnergySink en{d_efix_.p, d_edbl_.p};
-  if (ener) { if (vir) launch_k(k_fft_z_solve<R, true, true>, gz, 128, sz, stream_, A, P.h.p, P.gt.p, P.wt.p, P.plan[2][0], P.plan[2][1], P.lines[2], en, mixed_); else launch_k(k_fft_z_solve<R, true, false>, gz, 128, sz, stream_, A, P.h.p, P.gt.p, P.wt.p, P.plan[2][0], P.plan[2][1], P.lines[2], en, mixed_); }
-  else { if (vir) launch_k(k_fft_z_solve<R, false, true>, gz, 128, sz, stream_, A, P.h.p, P.gt.p, P.wt.p, P.plan[2][0], P.plan[2][1], P.lines[2], en, mixed_); else launch_k(k_fft_z_solve<R, false, false>, gz, 128, sz, stream_, A, P.h.p, P.gt.p, P.wt.p, P.plan[2][0], P.plan[2][1], P.lines[2], en, mixed_); }
-  launch_k(k_fft_y<R>, gy, 128, sy, stream_, A, P.h.p, P.plan[1][1], P.lines[1]);
-  launch_k(k_fft_x_inv<R>, capped(blocks_for(size_t(nlx), P.lines[0])), 128, sx, stream_, A, P.h.p, P.gr.p, P.plan[0][1], P.lines[0]);
+  auto* solve = ener ? (vir ? k_fft_z_solve<R, true, true> : k_fft_z_solve<R, true, false>) : (vir ? k_fft_z_solve<R, false, true> : k_fft_z_solve<R, false, false>);
+  launch_k(allow(solve, sz), gz, 128, sz, stream_, A, P.h.p, P.gt.p, P.wt.p, P.plan[2], lz, en, mixed_);
+  launch_k(allow(k_fft_y<R, true>, sy), gy, 128, sy, stream_, A, P.h.p, P.plan[1], ly);
+  launch_k(allow(k_fft_x_inv<R>, sx), gx, 128, sx, stream_, A, P.h.p, P.gr.p, P.plan[0], P.lines[0]);
 }
 
-// Autotuner for the line transforms: every block shape that fits (x: 1-16 lines per block; y, z: 1-8 consecutive a per
-// block) is timed on this grid (the transforms' time does not depend on the values), and the fastest kept. Results are
+// Autotuner for the line transforms: every block shape that fits (x: 1-8 pairs of lines per block; y, z: 1-16 consecutive
+// a per block) is timed on this grid (the transforms' time does not depend on the values), and the fastest kept. Results are
 // cached per grid, precision and SM count for the process.
 template <class R>
 void Engine::pme_tune(PmePath<R>& P) {
@@ -168,12 +191,11 @@ void Engine::pme_tune(PmePath<R>& P) {
   const size_t smax = 48 * 1024;
   float best = 1e30f;
   std::array<int, 3> pick{P.lines[0], P.lines[1], P.lines[2]};
-  for (int lx : {1, 2, 4, 8, 16})
-    for (int la : {1, 2, 4, 8}) {
-      if ((size_t(lx) * 2 + 1) * pk_[0] * sizeof(T) > smax) continue;
-      const int ly = std::min(la, ph1_), lz = std::min(la, ph1_);
-      if ((size_t(ly) * 2 + 1) * pk_[1] * sizeof(T) > smax || (size_t(lz) + 1) * 2 * pk_[2] * sizeof(T) > smax) continue;
-      P.lines[0] = lx, P.lines[1] = ly, P.lines[2] = lz;
+  for (int lx : {1, 2, 4, 8})
+    for (int la : {1, 2, 4, 8, 16}) {
+      if (((size_t(lx) * 2) * (pk_[0] | 1) + pk_[0]) * sizeof(T) > smax) continue;
+      if ((size_t(la) * 2 + 1) * std::max(pk_[1], pk_[2]) * sizeof(T) > smax) continue;
+      P.lines[0] = lx, P.lines[1] = la, P.lines[2] = la;
       fft_passes(P, false, false);   // warm
       CK(cudaEventRecord(e0, stream_));
       for (int rep = 0; rep < 3; ++rep) fft_passes(P, false, false);
@@ -181,7 +203,7 @@ void Engine::pme_tune(PmePath<R>& P) {
       CK(cudaEventSynchronize(e1));
       float ms = 0;
       CK(cudaEventElapsedTime(&ms, e0, e1));
-      if (ms < best) best = ms, pick = {lx, ly, lz};
+      if (ms < best) best = ms, pick = {lx, la, la};
     }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -200,11 +222,11 @@ void Engine::pme_run(PmePath<R>& P, const double* d_x, bool ener, bool vir) {
     std::memcpy(green_cell_, cell_h_, sizeof cell_h_);
     green_valid_ = true;
   }
-  const int nb = blocks_for(size_t(n_), 128);
+  const int nb = blocks_for(size_t(n_), kPmeAtoms);
 #define SPREAD(P_)                                                                            \
   do {                                                                                        \
-    if (mixed_) launch_k(k_spread<float, P_>, nb, 128, 0, stream_, A, d_grid_.p, d_gridq_.p);      \
-    else launch_k(k_spread<double, P_>, nb, 128, 0, stream_, A, d_grid_.p, d_gridq_.p);            \
+    if (mixed_) launch_k(k_spread<float, P_>, nb, kPmeThreads, 0, stream_, A, d_grid_.p, d_gridq_.p);      \
+    else launch_k(k_spread<double, P_>, nb, kPmeThreads, 0, stream_, A, d_grid_.p, d_gridq_.p);            \
   } while (0)
   switch (order_) {
     case 3: SPREAD(3); break;
@@ -220,8 +242,8 @@ void Engine::pme_run(PmePath<R>& P, const double* d_x, bool ener, bool vir) {
   const ForceSink<double> Fd{d_Fd_.p, d_Fd_.p + n_, d_Fd_.p + 2 * size_t(n_)};
 #define GATHER(P_)                                                                            \
   do {                                                                                        \
-    if (mixed_) launch_k(k_gather<float, R, P_>, nb, 128, 0, stream_, A, P.gr.p, Ff);              \
-    else launch_k(k_gather<double, R, P_>, nb, 128, 0, stream_, A, P.gr.p, Fd);                     \
+    if (mixed_) launch_k(k_gather<float, R, P_>, blocks_for(size_t(n_), 128), 128, 0, stream_, A, P.gr.p, Ff);              \
+    else launch_k(k_gather<double, R, P_>, blocks_for(size_t(n_), 128), 128, 0, stream_, A, P.gr.p, Fd);                     \
   } while (0)
   switch (order_) {
     case 3: GATHER(3); break;

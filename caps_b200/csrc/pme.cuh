@@ -6,91 +6,217 @@
 // convention are the reference's: g(a, b, c) at a + K1 (b + K2 c), and theta(a) weighs grid point floor(u) - p + a.
 //
 // Precision: the FP64 path is double throughout. The mixed path spreads in FP32 arithmetic into an exact fixed-point
-// grid, runs the transforms and the influence function in FP64 (a 70^3 grid is a few MB: the FFT is a small share of the
-// step, and FP32 transforms measured 1.3e-5 RMS relative force error on a relaxed cell against the 5e-6 target), and
-// gathers in FP32 arithmetic.
+// grid, transforms, solves and gathers in FP32 arithmetic (twiddles and butterfly constants computed in double and rounded
+// once).
 //
-// Kernels: K-SPREAD (thread per atom, fixed-point atomics on the FP32 path: deterministic), K-FFT-X (real lines to half
-// spectra), K-FFT-Y, K-FFT-Z+SOLVE (forward z transform, G multiply with energy/virial, inverse z transform, fused in one
-// pass over the grid), K-FFT-Y inverse, K-FFT-X inverse (half spectra to real lines), K-GATHER. Each line transform is a
-// Stockham autosort FFT in shared memory (radix 2, 3, 4, 5, 7 butterflies unrolled in registers), twiddles staged from
-// host-computed tables into shared memory.
+// Kernels: K-SPREAD (an atom's splines by one thread, its grid points by a group of lanes along x), K-GATHER, K-FFT-X
+// (pairs of real lines as one complex line, to half spectra), K-FFT-Y, K-FFT-Z+SOLVE (forward z transform, G multiply with
+// energy/virial, inverse z transform, fused in one pass over the grid), K-FFT-Y inverse, K-FFT-X inverse (half spectra to
+// pairs of real lines). Each line transform is a Stockham autosort FFT of two or three passes: butterflies of radix up to
+// 16 in registers, the first pass straight from global memory, one exchange through shared memory per pass. These kernels
+// are bound by latency (a 70^3 grid is 1.4 MB of half spectrum), so fewer passes and exchanges per line, not fewer bytes,
+// are what counts.
 #pragma once
 #include "pme_types.cuh"
 
 namespace capsb {
 
-// One radix-RAD Stockham pass over `nl` lines of length n, line-major, from `in` to `out`; Ns = product of the radices
-// before this pass. tw is the plan's twiddle table staged in shared memory. Every index stays below n: r k stride <=
-// (RAD-1)(Ns-1) n / (Ns RAD) < n. Butterflies are unrolled in registers; the small-radix DFT constants W_RAD^e = tw[e n/RAD].
-template <class T, int RAD>
-__device__ __forceinline__ void stockham_pass(const T* __restrict__ in, T* __restrict__ out, const T* __restrict__ tw, int n, int Ns, int nl,
-                                              int sign) {
-  using R = decltype(T::x);
-  const int nb = n / RAD, stride = n / (Ns * RAD);
-  T w[RAD];
-#pragma unroll
-  for (int e = 0; e < RAD; ++e) w[e] = tw[e * nb];
-  for (int t = threadIdx.x; t < nl * nb; t += blockDim.x) {
-    const int l = t / nb, j = t - l * nb;
-    const int k = j % Ns;
-    const T* src = in + l * n;
-    T v[RAD];
-    v[0] = src[j];
-#pragma unroll
-    for (int r = 1; r < RAD; ++r) v[r] = cmul(src[j + r * nb], tw[r * k * stride]);
-    T o[RAD];
-    if constexpr (RAD == 2) {
-      o[0] = cadd(v[0], v[1]);
-      o[1] = csub(v[0], v[1]);
-    } else if constexpr (RAD == 4) {
-      const T s0 = cadd(v[0], v[2]), s1 = csub(v[0], v[2]), s2 = cadd(v[1], v[3]), s3 = csub(v[1], v[3]);
-      const T is3 = {R(-sign) * s3.y, R(sign) * s3.x};   // sign * i * s3
-      o[0] = cadd(s0, s2);
-      o[2] = csub(s0, s2);
-      o[1] = cadd(s1, is3);
-      o[3] = csub(s1, is3);
-    } else {
-#pragma unroll
-      for (int m = 0; m < RAD; ++m) {
-        T acc = v[0];
-#pragma unroll
-        for (int r = 1; r < RAD; ++r) acc = cadd(acc, cmul(v[r], w[(m * r) % RAD]));
-        o[m] = acc;
-      }
-    }
-    T* dst = out + l * n + (j - k) * RAD + k;   // (j / Ns) Ns RAD + k
-#pragma unroll
-    for (int r = 0; r < RAD; ++r) dst[r * Ns] = o[r];
+// cos and sin of 2 pi e / n in double, at compile time (Taylor series after reduction to [-pi, pi]).
+constexpr double tw_series(double x, bool sine) {
+  double term = sine ? x : 1.0, sum = term;
+  for (int k = 1; k < 24; ++k) {
+    term *= -x * x / (sine ? (2.0 * k) * (2.0 * k + 1.0) : (2.0 * k - 1.0) * (2.0 * k));
+    sum += term;
   }
+  return sum;
 }
+constexpr double tw_angle(int e, int n) {
+  const int r = ((e % n) + n) % n;
+  return 2.0 * kPi * double(2 * r > n ? r - n : r) / double(n);
+}
+template <class R, int N, int E>
+struct TwConst {   // exp(-2 pi i E / N)
+  static constexpr double c = tw_series(tw_angle(E, N), false), s = -tw_series(tw_angle(E, N), true);
+};
 
-// All passes of a plan over `nl` lines held line-major in a (scratch b; tw in shared memory). Returns the buffer holding
-// the result (a or b). The plans hold radices 2, 3, 4, 5 and 7 only (grid lengths are 2^a 3^b 5^c 7^d).
-template <class R>
-__device__ typename Cpx<R>::T* fft_lines_smem(typename Cpx<R>::T* a, typename Cpx<R>::T* b, const typename Cpx<R>::T* tw, int nl,
-                                              const FftPlan<R>& P) {
-  using T = typename Cpx<R>::T;
-  int Ns = 1;
-  T* in = a;
-  T* out = b;
-  for (int s = 0; s < P.nst; ++s) {
-    const int Rr = P.rad[s];
-    switch (Rr) {
-      case 2: stockham_pass<T, 2>(in, out, tw, P.n, Ns, nl, P.sign); break;
-      case 3: stockham_pass<T, 3>(in, out, tw, P.n, Ns, nl, P.sign); break;
-      case 4: stockham_pass<T, 4>(in, out, tw, P.n, Ns, nl, P.sign); break;
-      case 5: stockham_pass<T, 5>(in, out, tw, P.n, Ns, nl, P.sign); break;
-      default: stockham_pass<T, 7>(in, out, tw, P.n, Ns, nl, P.sign); break;
-    }
-    __syncthreads();
-    T* tmp = in;
-    in = out;
-    out = tmp;
-    Ns *= Rr;
+// The forward DFT of N values in registers: o_m = sum_k v_k exp(-2 pi i m k / N).
+template <class T, int N>
+struct Dft;
+template <class T>
+struct Dft<T, 1> {
+  static __device__ __forceinline__ void run(T*) {}
+};
+template <class T>
+struct Dft<T, 2> {
+  static __device__ __forceinline__ void run(T* v) {
+    const T a = v[0], b = v[1];
+    v[0] = cadd(a, b), v[1] = csub(a, b);
   }
-  return in;
+};
+template <class T>
+struct Dft<T, 4> {
+  static __device__ __forceinline__ void run(T* v) {
+    const T s0 = cadd(v[0], v[2]), s1 = csub(v[0], v[2]), s2 = cadd(v[1], v[3]), s3 = csub(v[1], v[3]);
+    const T is3 = {s3.y, -s3.x};   // -i s3
+    v[0] = cadd(s0, s2), v[2] = csub(s0, s2);
+    v[1] = cadd(s1, is3), v[3] = csub(s1, is3);
+  }
+};
+// odd prime lengths: the sums and differences of v_k and v_(N-k) against real constants
+template <class T, int N, int M, int K>
+struct OddTerm {
+  static __device__ __forceinline__ void run(const T* s, const T* d, T& re, T& im) {
+    using R = decltype(T::x);
+    constexpr R c = R(TwConst<R, N, M * K>::c), q = R(TwConst<R, N, M * K>::s);
+    re.x += c * s[K].x, re.y += c * s[K].y;
+    im.x -= q * d[K].y, im.y += q * d[K].x;   // i q d
+    if constexpr (K < (N - 1) / 2) OddTerm<T, N, M, K + 1>::run(s, d, re, im);
+  }
+};
+template <class T, int N, int M>
+struct OddOut {
+  static __device__ __forceinline__ void run(const T* s, const T* d, T v0, T* o) {
+    T re = v0, im = {0, 0};
+    OddTerm<T, N, M, 1>::run(s, d, re, im);
+    o[M] = cadd(re, im);
+    o[N - M] = csub(re, im);
+    if constexpr (M < (N - 1) / 2) OddOut<T, N, M + 1>::run(s, d, v0, o);
+  }
+};
+template <class T, int N>
+struct DftOdd {
+  static __device__ __forceinline__ void run(T* v) {
+    constexpr int H = (N - 1) / 2;
+    T s[H + 1], d[H + 1], o[N], sum = v[0];
+#pragma unroll
+    for (int k = 1; k <= H; ++k) {
+      s[k] = cadd(v[k], v[N - k]), d[k] = csub(v[k], v[N - k]);
+      sum = cadd(sum, s[k]);
+    }
+    o[0] = sum;
+    OddOut<T, N, 1>::run(s, d, v[0], o);
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = o[k];
+  }
+};
+template <class T> struct Dft<T, 3> : DftOdd<T, 3> {};
+template <class T> struct Dft<T, 5> : DftOdd<T, 5> {};
+template <class T> struct Dft<T, 7> : DftOdd<T, 7> {};
+// N = A B: B transforms of length A over the stride B, twiddles, A transforms of length B
+template <class T, int N, int A, int B, int I, int J>
+struct SplitTw {
+  static __device__ __forceinline__ void run(T (&u)[B][A]) {
+    using R = decltype(T::x);
+    if constexpr (I * J != 0) {
+      constexpr R c = R(TwConst<R, N, I * J>::c), q = R(TwConst<R, N, I * J>::s);
+      u[J][I] = cmul(u[J][I], T{c, q});
+    }
+    if constexpr (I + 1 < A) SplitTw<T, N, A, B, I + 1, J>::run(u);
+    else if constexpr (J + 1 < B) SplitTw<T, N, A, B, 0, J + 1>::run(u);
+  }
+};
+template <class T, int A, int B>
+struct DftSplit {
+  static __device__ __forceinline__ void run(T* v) {
+    T u[B][A];
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+#pragma unroll
+      for (int a = 0; a < A; ++a) u[b][a] = v[B * a + b];
+      Dft<T, A>::run(u[b]);
+    }
+    SplitTw<T, A * B, A, B, 0, 0>::run(u);
+#pragma unroll
+    for (int a = 0; a < A; ++a) {
+      T w[B];
+#pragma unroll
+      for (int b = 0; b < B; ++b) w[b] = u[b][a];
+      Dft<T, B>::run(w);
+#pragma unroll
+      for (int b = 0; b < B; ++b) v[a + A * b] = w[b];
+    }
+  }
+};
+template <class T> struct Dft<T, 6> : DftSplit<T, 3, 2> {};
+template <class T> struct Dft<T, 8> : DftSplit<T, 4, 2> {};
+template <class T> struct Dft<T, 9> : DftSplit<T, 3, 3> {};
+template <class T> struct Dft<T, 10> : DftSplit<T, 5, 2> {};
+template <class T> struct Dft<T, 12> : DftSplit<T, 4, 3> {};
+template <class T> struct Dft<T, 16> : DftSplit<T, 4, 4> {};
+
+// A block's lines in shared memory: element i of line l at l ls + i is. LFAST: consecutive threads take consecutive lines
+// (y and z, whose rows in global memory run across the lines), 1 << lsh lines to the block; else consecutive elements (x).
+struct LineBuf {
+  int nl, ls, is, lsh;
+};
+
+// One radix-RAD Stockham pass (pass p of plan P): butterfly j of line l takes elements j + r nb, from `load(l, i)`, and
+// leaves element (j - k) RAD + k + r ns, k = j mod ns, in `out`.
+template <class T, int RAD, bool LFAST, class R, class LOAD>
+__device__ __forceinline__ void fft_pass(const LOAD& load, T* __restrict__ out, const T* __restrict__ tw, const FftPlan<R>& P, int p, const LineBuf& B) {
+  const int nb = P.nb[p], ns = P.ns[p], stride = nb / ns;   // n / (ns RAD)
+  const int total = LFAST ? nb << B.lsh : nb * B.nl;
+  for (int t = threadIdx.x; t < total; t += blockDim.x) {
+    int l, j;
+    if (LFAST) {
+      l = t & ((1 << B.lsh) - 1), j = t >> B.lsh;
+      if (l >= B.nl) continue;
+    } else {
+      l = div_by(t, P.m_nb[p]);
+      j = t - l * nb;
+    }
+    const int k = j - div_by(j, P.m_ns[p]) * ns;
+    T v[RAD];
+#pragma unroll
+    for (int r = 0; r < RAD; ++r) v[r] = load(l, j + r * nb);
+    if (ns > 1) {
+#pragma unroll
+      for (int r = 1; r < RAD; ++r) v[r] = cmul(v[r], tw[r * k * stride]);
+    }
+    Dft<T, RAD>::run(v);
+    T* dst = out + l * B.ls + ((j - k) * RAD + k) * B.is;
+#pragma unroll
+    for (int r = 0; r < RAD; ++r) dst[r * ns * B.is] = v[r];
+  }
 }
+template <class T, bool LFAST, class R, class LOAD>
+__device__ __forceinline__ void fft_pass_any(const LOAD& load, T* out, const T* tw, const FftPlan<R>& P, int p, const LineBuf& B) {
+  switch (P.rad[p]) {
+    case 2: fft_pass<T, 2, LFAST>(load, out, tw, P, p, B); break;
+    case 3: fft_pass<T, 3, LFAST>(load, out, tw, P, p, B); break;
+    case 4: fft_pass<T, 4, LFAST>(load, out, tw, P, p, B); break;
+    case 5: fft_pass<T, 5, LFAST>(load, out, tw, P, p, B); break;
+    case 6: fft_pass<T, 6, LFAST>(load, out, tw, P, p, B); break;
+    case 7: fft_pass<T, 7, LFAST>(load, out, tw, P, p, B); break;
+    case 8: fft_pass<T, 8, LFAST>(load, out, tw, P, p, B); break;
+    case 9: fft_pass<T, 9, LFAST>(load, out, tw, P, p, B); break;
+    case 10: fft_pass<T, 10, LFAST>(load, out, tw, P, p, B); break;
+    case 12: fft_pass<T, 12, LFAST>(load, out, tw, P, p, B); break;
+    default: fft_pass<T, 16, LFAST>(load, out, tw, P, p, B); break;
+  }
+}
+// The forward transform of a block's lines from `load` (first pass) into shared memory; a and b are the buffers, and the
+// one that holds the result is returned (every thread may read it). tw in shared memory; the caller has synchronised after
+// staging it and after the last use of the buffers.
+template <bool LFAST, class R, class LOAD>
+__device__ __forceinline__ typename Cpx<R>::T* fft_lines(const LOAD& load, typename Cpx<R>::T* a, typename Cpx<R>::T* b, const typename Cpx<R>::T* tw,
+                                                         const FftPlan<R>& P, const LineBuf& B) {
+  using T = typename Cpx<R>::T;
+  fft_pass_any<T, LFAST>(load, a, tw, P, 0, B);
+  __syncthreads();
+  for (int p = 1; p < P.nst; ++p) {
+    const T* in = a;
+    fft_pass_any<T, LFAST>([&](int l, int i) { return in[l * B.ls + i * B.is]; }, b, tw, P, p, B);
+    __syncthreads();
+    T* t = a;
+    a = b;
+    b = t;
+  }
+  return a;
+}
+// The inverse transform is the forward one of the values with real and imaginary parts exchanged, exchanged back.
+template <class T>
+__device__ __forceinline__ T swap_ri(T v) { return {v.y, v.x}; }
 
 template <class T>
 __device__ __forceinline__ void stage_twiddles(T* dst, const T* __restrict__ src, int n) {
@@ -151,129 +277,153 @@ __device__ __forceinline__ int wrapk(int v, int K) {
   return v < 0 ? v + K : v;
 }
 
-// K-SPREAD. FP64: double atomics into g. FP32: fixed point (2^40 per e) into gq, exact and order-free.
+// An atom's grid points are worked on by a group of lanes: P^2 lanes of P = 3 and 4 (two atoms and more to a warp), a warp
+// for the higher orders; a lane's points follow one another G lanes apart, x fastest.
+template <int P>
+constexpr int pme_group() { return P == 3 ? 9 : P == 4 ? 16 : 32; }
+constexpr int kPmeThreads = 128;
+constexpr int kPmeAtoms = 64;   // atoms per block
 template <class R, int P>
-static __global__ void k_spread(PmeArgs A, double* __restrict__ g, long long* __restrict__ gq) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.n) return;
-  const double qi = A.q[i];
-  if (qi == 0) return;
+struct PmeAtom {
   R th[3][P], dth[3][P];
   int base[3];
-  atom_splines<R, P>(A, i, th, dth, base);
-  int ia[P], ib[P];
+  R q;
+};
+
+// K-SPREAD. FP64: double atomics into g. FP32: fixed point (2^40 per e) into gq, exact and order-free. A row of P points
+// along x is P neighbouring lanes', so that it reaches L2 as one or two sectors of adds instead of P: the kernel is bound
+// by its atomics there (64 per atom at order 4).
+template <class R, int P>
+static __global__ void __launch_bounds__(kPmeThreads) k_spread(PmeArgs A, double* __restrict__ g, long long* __restrict__ gq) {
+  __shared__ PmeAtom<R, P> S[kPmeAtoms];
+  const int i0 = blockIdx.x * kPmeAtoms, n = min(kPmeAtoms, A.n - i0);
+  for (int t = threadIdx.x; t < n; t += kPmeThreads) {
+    atom_splines<R, P>(A, i0 + t, S[t].th, S[t].dth, S[t].base);
+    S[t].q = R(A.q[i0 + t]);
+  }
+  __syncthreads();
+  constexpr int G = pme_group<P>(), NG = kPmeThreads / G;
+  const int grp = threadIdx.x / G, lane = threadIdx.x % G;
+  if (grp >= NG) return;
+  for (int t = grp; t < n; t += NG) {
+    const PmeAtom<R, P>& a = S[t];
+    if (a.q == 0) continue;
 #pragma unroll
-  for (int a = 0; a < P; ++a) ia[a] = wrapk(base[0] + a, A.k1), ib[a] = wrapk(base[1] + a, A.k2);
-  for (int c = 0; c < P; ++c) {
-    const int ic = wrapk(base[2] + c, A.k3);
-#pragma unroll
-    for (int b = 0; b < P; ++b) {
-      const R st = R(qi) * th[1][b] * th[2][c];
-      const size_t row = size_t(A.k1) * (size_t(ib[b]) + size_t(A.k2) * size_t(ic));
-#pragma unroll
-      for (int a = 0; a < P; ++a) {
-        const R v = st * th[0][a];
-        if (sizeof(R) == 8) atomicAdd(g + row + ia[a], double(v));
-        else atomic_add_fix(gq + row + ia[a], to_fix(double(v), kFixQ));
-      }
+    for (int k = 0; k < (P * P * P + G - 1) / G; ++k) {
+      const int pt = lane + k * G;
+      if (P * P * P % G != 0 && pt >= P * P * P) break;
+      const int ia = pt % P, ib = pt / P % P, ic = pt / (P * P);
+      const R st = a.q * a.th[1][ib] * a.th[2][ic];
+      const size_t at = size_t(wrapk(a.base[0] + ia, A.k1)) + size_t(A.k1) * (size_t(wrapk(a.base[1] + ib, A.k2)) + size_t(A.k2) * size_t(wrapk(a.base[2] + ic, A.k3)));
+      const R v = st * a.th[0][ia];
+      if (sizeof(R) == 8) atomicAdd(g + at, double(v));
+      else atomic_add_fix(gq + at, __float2ll_rn(float(v) * float(kFixQ)));   // the scale is a power of two: no rounding
     }
   }
 }
 
-// Shared memory of the line-transform kernels: the twiddle table(s), then two buffers of `lines` lines of length n.
-// K-FFT-X forward: real lines (b, c) of length K1 to half spectra h(a, b, c), a <= K1/2. Input: g (double) or gq (fixed),
+// Shared memory of the line-transform kernels: the twiddle table, then two buffers of the block's lines.
+// K-FFT-X forward: real lines (b, c) of length K1 to half spectra h(a, b, c), a <= K1/2; lines 2 m and 2 m + 1 are the real
+// and imaginary parts of one complex line, parted again in the spectrum by its symmetry. Input: g (double) or gq (fixed),
 // cleared as it is read: the grid is zero for the next spread, with no launch of its own for it (as a memset node of the
-// step's graph it started up to 10 us after the step's drift, and the spread behind it).
+// step's graph it started up to 10 us after the step's drift, and the spread behind it). lpb: pairs of lines per block.
 template <class R>
 static __global__ void __launch_bounds__(128) k_fft_x_fwd(PmeArgs A, double* __restrict__ g, long long* __restrict__ gq,
-                                                          typename Cpx<R>::T* __restrict__ h, FftPlan<R> P, int lines_per_block) {
+                                                          typename Cpx<R>::T* __restrict__ h, FftPlan<R> P, int lpb) {
   using T = typename Cpx<R>::T;
-  extern __shared__ unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int ls = A.k1 | 1;
   T* tw = reinterpret_cast<T*>(smem_raw);
   T* s0 = tw + A.k1;
-  T* s1 = s0 + lines_per_block * A.k1;
-  const int nlines = A.k2 * A.k3;
+  T* s1 = s0 + lpb * ls;
+  const int nlines = A.k2 * A.k3, npairs = (nlines + 1) / 2;
   stage_twiddles(tw, P.tw, A.k1);
-  // groups of lines_per_block lines, strided over the grid (the grid may be smaller than the group count)
-  for (int l0 = blockIdx.x * lines_per_block; l0 < nlines; l0 += gridDim.x * lines_per_block) {
-    const int nl = min(lines_per_block, nlines - l0);
-    for (int t = threadIdx.x; t < nl * A.k1; t += blockDim.x) {
-      const size_t gidx = size_t(l0) * A.k1 + t;   // lines are contiguous in the real grid
-      R v;
-      if (gq) {
-        v = R(double(gq[gidx]) * kInvFixQ);
-        gq[gidx] = 0;
-      } else {
-        v = R(g[gidx]);
-        g[gidx] = 0;
-      }
-      s0[t] = {v, R(0)};
-    }
+  auto take = [&](int line, int i) {
+    if (line >= nlines) return R(0);
+    const size_t at = size_t(line) * A.k1 + i;   // lines are contiguous in the real grid
+    return gq ? R(double(gq[at]) * kInvFixQ) : R(g[at]);
+  };
+  const unsigned m_h1 = div_magic(unsigned(A.h1));
+  // groups of lpb pairs, strided over the grid (the grid may be smaller than the group count)
+  for (int l0 = blockIdx.x * lpb; l0 < npairs; l0 += gridDim.x * lpb) {
+    const LineBuf B{min(lpb, npairs - l0), ls, 1, 0};
     __syncthreads();
-    const T* res = fft_lines_smem<R>(s0, s1, tw, nl, P);
-    for (int t = threadIdx.x; t < nl * A.h1; t += blockDim.x) {
-      const int l = t / A.h1, a = t - l * A.h1;
-      h[size_t(l0 + l) * A.h1 + a] = res[l * A.k1 + a];
+    const T* z = fft_lines<false, R>([&](int l, int i) { return T{take(2 * (l0 + l), i), take(2 * (l0 + l) + 1, i)}; }, s0, s1, tw, P, B);
+    // every value is read: cleared together, so that no store stands between two loads
+    const size_t first = size_t(2 * l0) * A.k1, cells = size_t(min(2 * B.nl, nlines - 2 * l0)) * A.k1;
+    for (size_t t = threadIdx.x; t < cells; t += blockDim.x) {
+      if (gq) gq[first + t] = 0;
+      else g[first + t] = 0;
     }
-    __syncthreads();
+    for (int t = threadIdx.x; t < 2 * B.nl * A.h1; t += blockDim.x) {
+      const int l = div_by(t, m_h1), a = t - l * A.h1;
+      if (2 * l0 + l >= nlines) continue;
+      const T u = z[(l >> 1) * ls + a], w = z[(l >> 1) * ls + (a ? A.k1 - a : 0)];   // Z(a), Z(-a)
+      h[size_t(2 * l0 + l) * A.h1 + a] = (l & 1) ? T{R(0.5) * (u.y + w.y), R(0.5) * (w.x - u.x)} : T{R(0.5) * (u.x + w.x), R(0.5) * (u.y - w.y)};
+    }
   }
 }
 
-// K-FFT-X inverse: half spectra back to real lines (the missing half by Hermitian symmetry), real part kept.
+// K-FFT-X inverse: half spectra back to real lines, two at a time (the missing halves by Hermitian symmetry).
 template <class R>
-static __global__ void __launch_bounds__(128) k_fft_x_inv(PmeArgs A, const typename Cpx<R>::T* __restrict__ h, R* __restrict__ gr, FftPlan<R> P,
-                                                          int lines_per_block) {
+static __global__ void __launch_bounds__(128) k_fft_x_inv(PmeArgs A, const typename Cpx<R>::T* __restrict__ h, R* __restrict__ gr, FftPlan<R> P, int lpb) {
   using T = typename Cpx<R>::T;
-  extern __shared__ unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int ls = A.k1 | 1;
   T* tw = reinterpret_cast<T*>(smem_raw);
   T* s0 = tw + A.k1;
-  T* s1 = s0 + lines_per_block * A.k1;
-  const int nlines = A.k2 * A.k3;
+  T* s1 = s0 + lpb * ls;
+  const int nlines = A.k2 * A.k3, npairs = (nlines + 1) / 2;
   stage_twiddles(tw, P.tw, A.k1);
-  for (int l0 = blockIdx.x * lines_per_block; l0 < nlines; l0 += gridDim.x * lines_per_block) {
-    const int nl = min(lines_per_block, nlines - l0);
-    for (int t = threadIdx.x; t < nl * A.k1; t += blockDim.x) {
-      const int l = t / A.k1, m = t - l * A.k1;
-      const size_t lb = size_t(l0 + l) * A.h1;
-      T v;
-      if (m <= A.k1 / 2) v = h[lb + m];
-      else {
-        const T c = h[lb + (A.k1 - m)];
-        v = {c.x, -c.y};
-      }
-      s0[t] = v;
+  const unsigned m_k1 = div_magic(unsigned(A.k1));
+  for (int l0 = blockIdx.x * lpb; l0 < npairs; l0 += gridDim.x * lpb) {
+    const LineBuf B{min(lpb, npairs - l0), ls, 1, 0};
+    __syncthreads();
+    const T* z = fft_lines<false, R>(
+        [&](int l, int m) {
+          const int line = 2 * (l0 + l), a = 2 * m <= A.k1 ? m : A.k1 - m;
+          const R sg = 2 * m <= A.k1 ? R(1) : R(-1);
+          const T u = h[size_t(line) * A.h1 + a];
+          const T w = line + 1 < nlines ? h[size_t(line + 1) * A.h1 + a] : T{R(0), R(0)};
+          // Z = U + i W with conjugates past the middle, real and imaginary parts exchanged
+          return T{sg * u.y + w.x, u.x - sg * w.y};
+        },
+        s0, s1, tw, P, B);
+    for (int t = threadIdx.x; t < 2 * B.nl * A.k1; t += blockDim.x) {
+      const int l = div_by(t, m_k1), i = t - l * A.k1;
+      if (2 * l0 + l >= nlines) continue;
+      const T v = z[(l >> 1) * ls + i];
+      gr[size_t(2 * l0 + l) * A.k1 + i] = (l & 1) ? v.x : v.y;
     }
-    __syncthreads();
-    const T* res = fft_lines_smem<R>(s0, s1, tw, nl, P);
-    for (int t = threadIdx.x; t < nl * A.k1; t += blockDim.x) gr[size_t(l0) * A.k1 + t] = res[t].x;
-    __syncthreads();
   }
 }
 
-// K-FFT-Y: lines along b for fixed (a, c); a block takes `la` consecutive a (coalesced rows) of one c.
-template <class R>
-static __global__ void __launch_bounds__(128) k_fft_y(PmeArgs A, typename Cpx<R>::T* __restrict__ h, FftPlan<R> P, int la) {
+// K-FFT-Y: lines along b for fixed (a, c); a block takes 1 << lsh consecutive a (coalesced rows) of one c.
+template <class R, bool INV>
+static __global__ void __launch_bounds__(128) k_fft_y(PmeArgs A, typename Cpx<R>::T* __restrict__ h, FftPlan<R> P, int lsh) {
   using T = typename Cpx<R>::T;
-  extern __shared__ unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int la = 1 << lsh;
   T* tw = reinterpret_cast<T*>(smem_raw);
   T* s0 = tw + A.k2;
   T* s1 = s0 + la * A.k2;
-  const int ngrp = (A.h1 + la - 1) / la;
+  const int ngrp = (A.h1 + la - 1) >> lsh;
   stage_twiddles(tw, P.tw, A.k2);
   for (int grp = blockIdx.x; grp < ngrp * A.k3; grp += gridDim.x) {
-    const int c = grp / ngrp, a0 = (grp % ngrp) * la;
-    const int nl = min(la, A.h1 - a0);
-    for (int t = threadIdx.x; t < nl * A.k2; t += blockDim.x) {
-      const int b = t / nl, al = t - b * nl;
-      s0[al * A.k2 + b] = h[size_t(a0 + al) + size_t(A.h1) * (size_t(b) + size_t(A.k2) * c)];
-    }
+    const int c = grp / ngrp, a0 = (grp - c * ngrp) << lsh;
+    const LineBuf B{min(la, A.h1 - a0), 1, la, lsh};
+    T* row = h + size_t(a0) + size_t(A.h1) * size_t(A.k2) * c;
     __syncthreads();
-    const T* res = fft_lines_smem<R>(s0, s1, tw, nl, P);
-    for (int t = threadIdx.x; t < nl * A.k2; t += blockDim.x) {
-      const int b = t / nl, al = t - b * nl;
-      h[size_t(a0 + al) + size_t(A.h1) * (size_t(b) + size_t(A.k2) * c)] = res[al * A.k2 + b];
+    const T* res = fft_lines<true, R>(
+        [&](int l, int i) {
+          const T v = row[l + size_t(A.h1) * i];
+          return INV ? swap_ri(v) : v;
+        },
+        s0, s1, tw, P, B);
+    for (int t = threadIdx.x; t < A.k2 << lsh; t += blockDim.x) {
+      const int l = t & (la - 1), i = t >> lsh;
+      if (l < B.nl) row[l + size_t(A.h1) * i] = INV ? swap_ri(res[t]) : res[t];
     }
-    __syncthreads();
   }
 }
 
@@ -281,62 +431,54 @@ static __global__ void __launch_bounds__(128) k_fft_y(PmeArgs A, typename Cpx<R>
 // for 0 < a < K1/2), multiply by G, inverse transform, in one pass.
 template <class R, bool ENER, bool VIR>
 static __global__ void __launch_bounds__(128) k_fft_z_solve(PmeArgs A, typename Cpx<R>::T* __restrict__ h, const R* __restrict__ gt,
-                                                            const R* __restrict__ wt, FftPlan<R> Pf, FftPlan<R> Pi, int la, EnergySink en,
-                                                            int fixed) {
+                                                            const R* __restrict__ wt, FftPlan<R> P, int lsh, EnergySink en, int fixed) {
   using T = typename Cpx<R>::T;
-  extern __shared__ unsigned char smem_raw[];
-  T* twf = reinterpret_cast<T*>(smem_raw);
-  T* twi = twf + A.k3;
-  T* s0 = twi + A.k3;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int la = 1 << lsh;
+  T* tw = reinterpret_cast<T*>(smem_raw);
+  T* s0 = tw + A.k3;
   T* s1 = s0 + la * A.k3;
-  const int ngrp = (A.h1 + la - 1) / la;
+  const int ngrp = (A.h1 + la - 1) >> lsh;
   const size_t plane = size_t(A.h1) * A.k2;
-  stage_twiddles(twf, Pf.tw, A.k3);
-  stage_twiddles(twi, Pi.tw, A.k3);
+  stage_twiddles(tw, P.tw, A.k3);
   double e = 0, w[6] = {0, 0, 0, 0, 0, 0};
   long long ef = 0, wf[6] = {0, 0, 0, 0, 0, 0};
   for (int grp = blockIdx.x; grp < ngrp * A.k2; grp += gridDim.x) {
-    const int b = grp / ngrp, a0 = (grp % ngrp) * la;
-    const int nl = min(la, A.h1 - a0);
-    for (int t = threadIdx.x; t < nl * A.k3; t += blockDim.x) {
-      const int c = t / nl, al = t - c * nl;
-      s0[al * A.k3 + c] = h[size_t(a0 + al) + size_t(A.h1) * b + plane * c];
-    }
+    const int b = grp / ngrp, a0 = (grp - b * ngrp) << lsh;
+    const LineBuf B{min(la, A.h1 - a0), 1, la, lsh};
+    const size_t first = size_t(a0) + size_t(A.h1) * b;
+    T* row = h + first;
     __syncthreads();
-    T* res = fft_lines_smem<R>(s0, s1, twf, nl, Pf);
-    T* other = res == s0 ? s1 : s0;
-    for (int t = threadIdx.x; t < nl * A.k3; t += blockDim.x) {
-      const int al = t / A.k3, c = t - al * A.k3;
-      const int a = a0 + al;
-      const size_t gi = size_t(a) + size_t(A.h1) * b + plane * c;
-      T v = res[t];
-      const R G = gt[gi];
-      if (ENER || VIR) {
-        double em = 0.5 * (double(v.x) * v.x + double(v.y) * v.y);
-        if (a > 0 && 2 * a != A.k1) em *= 2;
-        // mixed path: every term rounded to fixed point on its own, so the sum does not depend on which block took
-        // which line group
-        if (ENER) {
-          if (fixed) ef += to_fix(em * double(G), kFixE);
-          else e += em * double(G);
-        }
-        if (VIR)
-          for (int k = 0; k < 6; ++k) {
-            if (fixed) wf[k] += to_fix(em * double(wt[6 * gi + k]), kFixE);
-            else w[k] += em * double(wt[6 * gi + k]);
+    T* res = fft_lines<true, R>([&](int l, int i) { return row[l + plane * i]; }, s0, s1, tw, P, B);
+    // the inverse transform's first pass reads the spectrum times G (parts exchanged); every point is read once
+    const T* back = fft_lines<true, R>(
+        [&](int l, int i) {
+          const T v = res[l + (i << lsh)];
+          const size_t gi = first + l + plane * i;
+          const R G = gt[gi];
+          if (ENER || VIR) {
+            const int a = a0 + l;
+            double em = 0.5 * (double(v.x) * v.x + double(v.y) * v.y);
+            if (a > 0 && 2 * a != A.k1) em *= 2;
+            // mixed path: every term rounded to fixed point on its own, so the sum does not depend on which block took
+            // which line group
+            if (ENER) {
+              if (fixed) ef += to_fix(em * double(G), kFixE);
+              else e += em * double(G);
+            }
+            if (VIR)
+              for (int k = 0; k < 6; ++k) {
+                if (fixed) wf[k] += to_fix(em * double(wt[6 * gi + k]), kFixE);
+                else w[k] += em * double(wt[6 * gi + k]);
+              }
           }
-      }
-      v.x *= G;
-      v.y *= G;
-      res[t] = v;
+          return T{v.y * G, v.x * G};
+        },
+        res == s0 ? s1 : s0, res, tw, P, B);
+    for (int t = threadIdx.x; t < A.k3 << lsh; t += blockDim.x) {
+      const int l = t & (la - 1), i = t >> lsh;
+      if (l < B.nl) row[l + plane * i] = swap_ri(back[t]);
     }
-    __syncthreads();
-    const T* back = fft_lines_smem<R>(res, other, twi, nl, Pi);
-    for (int t = threadIdx.x; t < nl * A.k3; t += blockDim.x) {
-      const int c = t / nl, al = t - c * nl;
-      h[size_t(a0 + al) + size_t(A.h1) * b + plane * c] = back[al * A.k3 + c];
-    }
-    __syncthreads();
   }
   if ((ENER || VIR) && fixed) {
     __shared__ long long scratch_q[32];
@@ -419,7 +561,9 @@ static __global__ void k_pme_green(PmeArgs A, const double* __restrict__ b1, con
   }
 }
 
-// K-GATHER: F_i -= q_i sum_d K_d (row d of h^-1) dE/du_d (caps_kspace.f90:965-992).
+// K-GATHER: F_i -= q_i sum_d K_d (row d of h^-1) dE/du_d (caps_kspace.f90:965-992). A thread per atom: its rows of P values
+// along x are a sector each, which the loads of one thread share in L1; a group of 16 lanes per atom, as in the spread,
+// measured 11 us against 6 at 32,000 atoms (its sums go through twelve shuffles).
 template <class R, class G, int P>
 static __global__ void k_gather(PmeArgs A, const G* __restrict__ gr, ForceSink<R> F) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

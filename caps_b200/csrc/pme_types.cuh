@@ -4,7 +4,7 @@
 
 namespace capsb {
 
-constexpr int kMaxRadices = 16;
+constexpr int kMaxRadices = 8;
 constexpr int kMaxOrder = 8;
 
 template <class R> struct Cpx;
@@ -15,12 +15,18 @@ template <class T> __device__ __forceinline__ T cmul(T a, T b) { return {a.x * b
 template <class T> __device__ __forceinline__ T cadd(T a, T b) { return {a.x + b.x, a.y + b.y}; }
 template <class T> __device__ __forceinline__ T csub(T a, T b) { return {a.x - b.x, a.y - b.y}; }
 
+// A line transform of length n = rad[0] rad[1] ... as Stockham passes. For pass p: nb = n / rad[p] butterflies per line,
+// ns = the product of the radices before it; m_nb and m_ns divide by them (div_by).
 template <class R>
 struct FftPlan {
   int n, nst;
-  int rad[kMaxRadices];
-  const typename Cpx<R>::T* tw;   // exp(sign 2 pi i k / n), k < n
-  int sign;                        // +1 / -1 (the sign of tw)
+  int rad[kMaxRadices], nb[kMaxRadices], ns[kMaxRadices];
+  unsigned m_nb[kMaxRadices], m_ns[kMaxRadices];
+  const typename Cpx<R>::T* tw;   // exp(-2 pi i k / n), k < n
 };
+
+// t / d by the multiplier m = floor(2^32 / d) + 1 (0 for d = 1), exact for t d < 2^32.
+__host__ __device__ inline unsigned div_magic(unsigned d) { return d == 1 ? 0u : unsigned(0xffffffffu / d) + 1u; }
+__device__ __forceinline__ int div_by(int t, unsigned m) { return m ? int(__umulhi(unsigned(t), m)) : t; }
 
 }  // namespace capsb
