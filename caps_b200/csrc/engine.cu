@@ -390,7 +390,14 @@ void Engine::setup_options() {
       gt[2 * k + 1] = h * dG;
     }
     d_gtab_.upload(gt, stream_);
-    gnodes_ = int(m + 2);
+    // the pair kernel's form of the same interpolant: per interval its polynomial (pair.cuh, EwaldTab)
+    std::vector<double4> gc(m + 1);
+    for (size_t k = 0; k <= m; ++k) {
+      const double g0 = gt[2 * k], g1 = gt[2 * k + 1], d = gt[2 * k + 2] - g0, g3 = gt[2 * k + 3];
+      gc[k] = make_double4(2 * g1 / h, 4 * (3 * d - 2 * g1 - g3) / h, 6 * (g1 + g3 - 2 * d) / h, g0);
+    }
+    d_gcoef_.upload(gc, stream_);
+    gnodes_ = int(m + 1);
     ghi_ = 1 / h;
   }
   // pair coefficient tables, the padding type last (all zero)

@@ -253,6 +253,7 @@ class Engine {
   std::vector<double> h_tr0dr_, h_te_, h_tf_;
   PairTables pair_tables() const { return PairTables{d_toff_.p, d_tr0dr_.p, d_te_.p, d_tf_.p}; }
   DevBuf<double> d_gtab_;
+  DevBuf<double4> d_gcoef_;
   int gnodes_ = 0;
   double ghi_ = 0;
   DevBuf<uint32_t> d_bond_ij_, d_angle_ijk_, d_dih_ijkl_, d_imp_ijkl_, d_p14_ij_, d_excl_ij_, d_fene_ij_;

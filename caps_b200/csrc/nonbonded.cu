@@ -172,7 +172,7 @@ PairArgs Engine::pair_args() {
   A.lj_inner = lj_inner_;
   A.lj_fsw = lj_fsw_ && !lj96_ ? 1 : 0;
   A.tables = pair_tables();
-  A.gtab = d_gtab_.p;
+  A.gcoef = d_gcoef_.p;
   A.ntab = nt_ + 1;
   A.gnodes = coul_ ? gnodes_ : 0;   // a table only with Coulomb: the FP64 kernel's shared memory holds it then
   A.ghi = ghi_;
@@ -244,13 +244,24 @@ void Engine::pair_forces(bool ener, bool vir) {
 #undef PAIR32
 #undef PAIR32L
   } else {
-    const size_t smem = sizeof(double4) * (size_t(ntab) * ntab + 4 * 64) + sizeof(double) * 2 * size_t(coul ? gnodes_ : 0) + sizeof(int) * 4 * 64;
+    // LJ table, Ewald table, the 4 warps' i atoms and types, and their staged entries with j atoms, types and masks
+    const size_t staged = sizeof(double4) * (size_t(ntab) * ntab + 4 * 64) + sizeof(int) * 4 * 64 +
+                          4 * size_t(A.batch) * (sizeof(uint4) + 8 * (sizeof(double4) + sizeof(unsigned long long) + sizeof(int)));
+    const size_t table = coul ? sizeof(double4) * size_t(gnodes_) : 0;
+    // a table past about 100 KB leaves room for one block per SM: then through L1 (the rare variants always do)
+    const bool gsm = table <= 100 * 1024;
+#define PAIR64LG(C, E, V, CAP, L, F, G)                                                                              \
+  do {                                                                                                               \
+    const size_t smem = staged + ((G) ? table : 0);                                                                  \
+    if (smem > 48 * 1024) CK(cudaFuncSetAttribute(k_pair_f64<C, E, V, CAP, L, F, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))); \
+    int per_sm = 0;                                                                                                  \
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_f64<C, E, V, CAP, L, F, G>, 128, smem));        \
+    launch_k(k_pair_f64<C, E, V, CAP, L, F, G>, dev_sms_ * std::max(1, per_sm - pair_cut_), 128, smem, stream_, A);  \
+  } while (0)
 #define PAIR64LF(C, E, V, CAP, L, F)                                                                                 \
   do {                                                                                                               \
-    if (smem > 48 * 1024) CK(cudaFuncSetAttribute(k_pair_f64<C, E, V, CAP, L, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))); \
-    int per_sm = 0;                                                                                                  \
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_f64<C, E, V, CAP, L, F>, 128, smem));           \
-    launch_k(k_pair_f64<C, E, V, CAP, L, F>, dev_sms_ * std::max(1, per_sm - pair_cut_), 128, smem, stream_, A);                       \
+    if ((CAP) || (F) || !gsm) PAIR64LG(C, E, V, CAP, L, F, false);                                                   \
+    else PAIR64LG(C, E, V, CAP, L, F, !(CAP) && !(F));                                                               \
   } while (0)
 #define PAIR64L(C, E, V, CAP, L) PAIR64LF(C, E, V, CAP, L, false)
 #define PAIR64(C, E, V, CAP)                                                                                         \
@@ -281,6 +292,7 @@ void Engine::pair_forces(bool ener, bool vir) {
 #undef PAIR64
 #undef PAIR64L
 #undef PAIR64LF
+#undef PAIR64LG
   }
   CK(cudaGetLastError());
 }

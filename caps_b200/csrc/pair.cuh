@@ -40,7 +40,7 @@ struct PairArgs {
   double lj_inner;
   int lj_fsw;            // FP64: CHARMM's force switch on the 12-6 pairs
   PairTables tables;
-  const double* gtab;    // FP64 Ewald table: 2 per node (G, h dG/ds)
+  const double4* gcoef;  // FP64 Ewald table: per node the polynomial of its interval (EwaldTab)
   int ntab;              // types incl. the padding type
   int gnodes;            // table nodes
   double ghi;            // 1 / node spacing
@@ -407,16 +407,41 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
 
 // --- FP64 path ---------------------------------------------------------------------------------------------------
 
-// The reference's ewald_ef (field.cpp:1593-1602): E = 1/r - G(s), F = 1/r^3 + 2 dG/ds by cubic Hermite interpolation.
-__device__ __forceinline__ void ewald_ef(const double* __restrict__ gt, double ghi, double s, double rinv, double& E, double& F) {
-  const double u = s * ghi;
-  const int k = int(u);
-  const double t = u - double(k), t2 = t * t;
-  const double g0 = gt[2 * k], g1 = gt[2 * k + 1], g2 = gt[2 * k + 2], g3 = gt[2 * k + 3];
-  const double G = g0 + t2 * (3 - 2 * t) * (g2 - g0) + t * (1 - t) * ((1 - t) * g1 - t * g3);
-  const double dG = (6 * t * (1 - t) * (g2 - g0) * ghi) + (1 - t) * (1 - 3 * t) * g1 * ghi + t * (3 * t - 2) * g3 * ghi;
-  E = rinv - G;
-  F = rinv * rinv * rinv + 2 * dG;
+// The reference's ewald_ef (field.cpp:1593-1602): E = 1/r - G(s), F = 1/r^3 + 2 dG/ds by cubic Hermite interpolation of G
+// over nodes of spacing h. The interpolant is held as its polynomial in t = s/h - k, c[k] = (a1, a2, a3, G_k) with
+// 2 dG/ds = a1 + t (a2 + t a3): a force takes three loads and two multiply-adds.
+struct EwaldTab {
+  const double4* c;
+  double ghi, hh;   // 1 / h, h / 2
+};
+__device__ __forceinline__ int ewald_node(double u, double& t) {   // node and offset of u = s / h in [0, 2^31)
+  const double m = (u - 0.5) + 6755399441055744.0;   // 1.5 2^52: the sum's low word is u - 1/2 rounded to an integer
+  t = u - (m - 6755399441055744.0);                  // in [0, 1] (a tie may take either end)
+  return __double2loint(m);
+}
+template <bool ENER>
+__device__ __forceinline__ double ewald_f(const EwaldTab& T, double s, double& G) {
+  double t;
+  const double4* c = T.c + ewald_node(s * T.ghi, t);
+  const double2 a = *reinterpret_cast<const double2*>(c);
+  if (ENER) {
+    const double2 g = *(reinterpret_cast<const double2*>(c) + 1);
+    G = g.y + t * T.hh * (a.x + t * (0.5 * a.y + t * (g.x * (1.0 / 3.0))));
+    return a.x + t * (a.y + t * g.x);
+  }
+  return a.x + t * (a.y + t * c->z);
+}
+
+// 1/sqrt(x) and 1/x in double from the hardware's 20-bit estimate y: with e = 1 - x y^2, y (1 + e/2 + 3 e^2/8) is off by
+// 5 e^3 / 16 < 2^-58, and its square is corrected once. x is a squared distance, neither 0 nor denormal.
+__device__ __forceinline__ double rsqrt_sq(double x, double& inv) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x * y, y, 1.0);
+  y = fma(y * e, fma(e, 0.375, 0.5), y);
+  inv = y * y;
+  inv = fma(inv, fma(-x, inv, 1.0), inv);
+  return y;
 }
 
 // erfc(x) and exp(-x^2) by Abramowitz & Stegun 7.1.26, the reference's erfc_exp (field.cpp:585-590): the closed form a
@@ -428,25 +453,95 @@ __device__ __forceinline__ double erfc_exp_as(double x, double& ex2) {
   return t * (A1 + t * (A2 + t * (A3 + t * (A4 + t * A5)))) * ex2;
 }
 
-// FROZEN: the pairs are those of the frozen set (A.frozen), whatever their distance now (field.cpp:1700); one beyond
-// the cut-off takes the closed-form Coulomb term (field.cpp:1759-1768).
+// One pair at squared distance r2 of types (ti, tj): |F| / r, energies added to ev and ec.
+// FROZEN: a pair of the frozen set beyond the cut-off takes the closed-form Coulomb term (field.cpp:1759-1768).
 // CAP: the rare forms' variant (the push-off force cap, the generic pair forms, CHARMM's force switch), taken with energies
 // and virial on; the plain variants carry none of their branches.
-template <int COUL, bool ENER, bool VIR, bool CAP = false, bool LJ96 = false, bool FROZEN = false>
-static __global__ void __launch_bounds__(128, 2) k_pair_f64(PairArgs A) {
+template <int COUL, bool ENER, bool CAP, bool LJ96, bool FROZEN>
+__device__ __forceinline__ double pair_f64(const PairArgs& A, const EwaldTab& T, const double4* tab, int tt, double r2, double qq, double& ev, double& ec) {
+  double r2i;
+  const double rinv = rsqrt_sq(r2, r2i);
+  const double r6i = r2i * r2i * r2i;
+  const double2 c = *reinterpret_cast<const double2*>(tab + tt);
+  double fr;
+  const double4 cc = (ENER || CAP || FROZEN) ? tab[tt] : make_double4(c.x, c.y, 0, 0);
+  const double4 cp = CAP ? A.tabcap[tt] : make_double4(0, 0, 0, 0);
+  if (CAP && r2 < cp.x) {
+    // the push-off cap (field.cpp:1534-1538): LJ continued linearly inside the radius where |F| reaches the cap
+    fr = cp.z * rinv;   // F / r with |F| = the cap
+    if (ENER) ev += cp.y + cp.z * (sqrt(cp.x) - r2 * rinv) - cc.z;
+  } else if ((CAP || FROZEN) && cc.w != 0) {
+    // a generic form (field.cpp:1381-1396), nothing beyond the pair's own cut-off (and no shift there)
+    const double4 g = A.tabg[tt];
+    double e = 0;
+    fr = (g.w > 0 && r2 > g.w) ? 0.0 : generic_pair(int(cc.w), g, A.tabg2[tt], A.lj_inner, A.tables, r2, e);
+    if (ENER && !(g.w > 0 && r2 > g.w)) ev += e - cc.z;
+  } else if (LJ96) {   // field.cpp:1658-1661
+    const double r9i = r6i * r2i * rinv;
+    fr = (9 * cc.y * r9i - 6 * cc.x * r6i) * r2i;
+    if (ENER) ev += cc.y * r9i - cc.x * r6i - cc.z;
+  } else if ((CAP || FROZEN) && A.lj_fsw) {
+    fr = charmm_fsw(cc.y, cc.x, A.lj_inner, A.rc, r2, ev, ENER);
+  } else {
+    fr = r6i * (12 * cc.y * r6i - 6 * cc.x) * r2i;
+    if (ENER) ev += r6i * (cc.y * r6i - cc.x) - cc.z;
+  }
+  if (COUL != 0 && FROZEN && !(r2 < A.rc2)) {
+    const double r = sqrt(r2);
+    double ex2;
+    const double er = erfc_exp_as(A.beta * r, ex2);   // beta: the Ewald or DSF coefficient; kc = 2 beta / sqrt(pi)
+    if (COUL == 1) {
+      if (ENER) ec += qq * er / r;
+      fr += qq * (er / r2 + A.kc * ex2 / r) / r;
+    } else {
+      if (ENER) ec += qq * (er / r - A.dsf_e0 + A.dsf_f0 * (r - A.rc));
+      fr += qq * (er / r2 + A.kc * ex2 / r - A.dsf_f0) / r;
+    }
+  } else if (COUL != 0) {
+    double G = 0;
+    const double Fc = fma(rinv, r2i, ewald_f<ENER>(T, r2, G));
+    if (COUL == 1) {
+      if (ENER) ec += qq * (rinv - G);
+      fr += qq * Fc;
+    } else {
+      if (ENER) ec += qq * (rinv - G - A.dsf_e0 + A.dsf_f0 * (r2 * rinv - A.rc));
+      fr += qq * (Fc - A.dsf_f0 * rinv);
+    }
+  }
+  return fr;
+}
+
+// The FP64 pair kernel, staged as the FP32 one: a work item's i atoms, entries, shifted j atoms and exclusion masks by one
+// batch of loads into shared memory, a lane's pairs of an entry in one 16-bit word, and both of the lane's j atoms of an
+// entry evaluated side by side, so that two independent chains of FP64 operations fill the pipe's latency. FROZEN: the
+// pairs are those of the frozen set (A.frozen), whatever their distance now (field.cpp:1700).
+// Bound by FP64 issue: 46 double operations per pair (a division and a square root made it 75) on half-rate units, 3 warps
+// per scheduler. GSM: the Ewald table in shared memory (else read through L1, for tables too large for it).
+template <int COUL, bool ENER, bool VIR, bool CAP = false, bool LJ96 = false, bool FROZEN = false, bool GSM = true>
+static __global__ void __launch_bounds__(128, 3) k_pair_f64(PairArgs A) {
   extern __shared__ double4 smem_d4[];
-  double4* tab = smem_d4;                                   // ntab * ntab
-  double* gt = reinterpret_cast<double*>(tab + A.ntab * A.ntab);   // 2 * gnodes with Coulomb, none without (as the launch sizes it)
-  double4* s_xi = reinterpret_cast<double4*>(gt + (COUL != 0 ? 2 * A.gnodes : 0));   // 4 x 64
-  int* s_ti = reinterpret_cast<int*>(s_xi + 4 * 64);
+  const int nb = A.batch;
+  double4* tab = smem_d4;                                            // ntab * ntab
+  double4* gt = tab + A.ntab * A.ntab;                               // gnodes with Coulomb, none without (as the launch sizes it)
+  double4* s_xi_all = gt + (COUL != 0 && GSM ? A.gnodes : 0);        // 4 warps x 64
+  double4* s_xj_all = s_xi_all + 4 * 64;                             // 4 warps x nb entries x 8, shifted by the entry's image
+  unsigned long long* s_mk_all = reinterpret_cast<unsigned long long*>(s_xj_all + 4 * nb * 8);   // 4 warps x nb x 8
+  uint4* s_en_all = reinterpret_cast<uint4*>(s_mk_all + 4 * nb * 8); // 4 warps x nb entries
+  int* s_ti_all = reinterpret_cast<int*>(s_en_all + 4 * nb);         // 4 warps x 64, a type's row in tab
+  int* s_tj_all = s_ti_all + 4 * 64;                                 // 4 warps x nb x 8
   for (int t = threadIdx.x; t < A.ntab * A.ntab; t += blockDim.x) tab[t] = A.tabd[t];
-  if (COUL != 0)
-    for (int t = threadIdx.x; t < 2 * A.gnodes; t += blockDim.x) gt[t] = A.gtab[t];
+  if (COUL != 0 && GSM)
+    for (int t = threadIdx.x; t < A.gnodes; t += blockDim.x) gt[t] = A.gcoef[t];
   __syncthreads();
+  const EwaldTab T{COUL != 0 && GSM ? gt : A.gcoef, A.ghi, 0.5 / A.ghi};
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i8 = lane & 7, jq = lane >> 3;
-  double4* xi_s = s_xi + 64 * wib;
-  int* ti_s = s_ti + 64 * wib;
+  double4* xi_s = s_xi_all + 64 * wib;
+  double4* xj_s = s_xj_all + 8 * nb * wib;
+  unsigned long long* mk_s = s_mk_all + 8 * nb * wib;
+  uint4* en_s = s_en_all + nb * wib;
+  int* ti_s = s_ti_all + 64 * wib;
+  int* tj_s = s_tj_all + 8 * nb * wib;
   if (blockIdx.x == 0 && threadIdx.x == 0) {   // the step's list work is done: lower the rebuild and prune flags
     int* c = const_cast<int*>(A.counters);
     c[kCntRebuild] = 0;
@@ -459,119 +554,95 @@ static __global__ void __launch_bounds__(128, 2) k_pair_f64(PairArgs A) {
   for (int w = next_work_item(A.counters, lane); w < nwork; w = next_work_item(A.counters, lane)) {
     const int4 wk = A.work[w];
     const int sc = wk.x;
+    const int ne = min(wk.z, nb);
+    if (lane < ne) en_s[lane] = A.ent[wk.y + lane];
     for (int t = lane; t < 64; t += 32) {
       double4 v = A.xqd[64 * sc + t];
       v.w *= A.kcoul;
       xi_s[t] = v;
-      ti_s[t] = A.tslot[64 * sc + t];
+      ti_s[t] = A.tslot[64 * sc + t] * A.ntab;
     }
     __syncwarp();
+    for (int t = lane; t < 8 * ne; t += 32) {   // entry t / 8, j atom (and i cluster of the mask) t % 8
+      const uint4 en = en_s[t >> 3];
+      int qa, qb, qc;
+      unpack_image(en.y >> 8, qa, qb, qc);
+      const int ja = 8 * int(en.x) + (t & 7);
+      double4 v = A.xqd[ja];
+      v.x += A.cell.h[0][0] * qa + A.cell.h[0][1] * qb + A.cell.h[0][2] * qc;
+      v.y += A.cell.h[1][0] * qa + A.cell.h[1][1] * qb + A.cell.h[1][2] * qc;
+      v.z += A.cell.h[2][0] * qa + A.cell.h[2][1] * qb + A.cell.h[2][2] * qc;
+      xj_s[t] = v;
+      tj_s[t] = A.tslot[ja];
+      mk_s[t] = FROZEN ? A.frozen[8 * size_t(wk.y) + t] : en.z ? A.masks[8 * size_t(en.z - 1) + (t & 7)] : ~0ull;
+    }
     unsigned ireal = 0;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) ireal |= unsigned(ti_s[8 * c + i8] != pad) << c;
+    for (int c = 0; c < 8; ++c) ireal |= unsigned(ti_s[8 * c + i8] != pad * A.ntab) << c;
+    ireal |= ireal << 8;
     double fix[8], fiy[8], fiz[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) fix[c] = fiy[c] = fiz[c] = 0.0;
     double ev = 0, ec = 0, vw[6] = {0, 0, 0, 0, 0, 0};
-    for (int e = wk.y; e < wk.y + wk.z; ++e) {
-      const uint4 en = A.ent[e];
-      const int cj = int(en.x);
+    __syncwarp();
+    for (int el = 0; el < ne; ++el) {
+      const uint4 en = en_s[el];
       const unsigned hmask = en.w & 0xffffu;
       if (!hmask) continue;
       const unsigned imask = (hmask | (hmask >> 8)) & 255u;
-      int qa, qb, qc;
-      unpack_image(en.y >> 8, qa, qb, qc);
-      const double Sx = A.cell.h[0][0] * qa + A.cell.h[0][1] * qb + A.cell.h[0][2] * qc;
-      const double Sy = A.cell.h[1][0] * qa + A.cell.h[1][1] * qb + A.cell.h[1][2] * qc;
-      const double Sz = A.cell.h[2][0] * qa + A.cell.h[2][1] * qb + A.cell.h[2][2] * qc;
-      const int j0 = 8 * cj + jq, j1 = j0 + 4;
-      const double4 a0 = A.xqd[j0], a1 = A.xqd[j1];
-      const int t0 = A.tslot[j0], t1 = A.tslot[j1];
+      // the lane's listed pairs of the entry (as the FP32 kernel)
+      unsigned lv = hmask & ireal;
+      if (FROZEN || en.z) {
+        unsigned xm = 0;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const unsigned b = unsigned(mk_s[8 * el + c] >> (8 * i8 + jq));
+          xm |= ((b & 1u) << c) | (((b >> 4) & 1u) << (c + 8));
+        }
+        lv &= xm;
+      }
+      const double4 a0 = xj_s[8 * el + jq], a1 = xj_s[8 * el + jq + 4];
+      const int t0 = tj_s[8 * el + jq], t1 = tj_s[8 * el + jq + 4];
       double f0x = 0, f0y = 0, f0z = 0, f1x = 0, f1y = 0, f1z = 0;
-#pragma unroll 2
+#pragma unroll
       for (int c = 0; c < 8; ++c) {
         if (!((imask >> c) & 1u)) continue;
-        const unsigned long long mm = FROZEN ? A.frozen[8 * size_t(e) + c] : en.z ? A.masks[8 * size_t(en.z - 1) + c] : ~0ull;
         const double4 xi = xi_s[8 * c + i8];
         const int ti = ti_s[8 * c + i8];
-        const bool oki = (ireal >> c) & 1u;
-        // d = xs_j - (xs_i - S), as field.cpp:1628-1636
-        const double xs = xi.x - Sx, ys = xi.y - Sy, zs = xi.z - Sz;
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-          if (!((hmask >> (c + 8 * jj)) & 1u)) continue;
-          const double4 aj = jj ? a1 : a0;
-          const int tj = jj ? t1 : t0;
-          const int bit = 8 * i8 + jq + 4 * jj;
-          const double dx = aj.x - xs, dy = aj.y - ys, dz = aj.z - zs;
-          const double r2 = dx * dx + dy * dy + dz * dz;
-          const bool ok = oki && ((mm >> bit) & 1ull) && (FROZEN || r2 < A.rc2);
-          if (!ok) continue;
-          const double r2i = 1 / r2, r6i = r2i * r2i * r2i, rinv = sqrt(r2i);
-          const double4 cc = tab[ti * A.ntab + tj];
-          double fr;
-          const double4 cp = CAP ? A.tabcap[ti * A.ntab + tj] : make_double4(0, 0, 0, 0);
-          if (CAP && r2 < cp.x) {
-            // the push-off cap (field.cpp:1534-1538): LJ continued linearly inside the radius where |F| reaches the cap
-            const double r = r2 * rinv, rcp = sqrt(cp.x);
-            fr = cp.z * rinv;   // F / r with |F| = the cap
-            if (ENER) ev += cp.y + cp.z * (rcp - r) - cc.z;
-          } else if ((CAP || FROZEN) && cc.w != 0) {
-            // a generic form (field.cpp:1381-1396), nothing beyond the pair's own cut-off (and no shift there)
-            const double4 g = A.tabg[ti * A.ntab + tj];
-            double e = 0;
-            fr = (g.w > 0 && r2 > g.w) ? 0.0 : generic_pair(int(cc.w), g, A.tabg2[ti * A.ntab + tj], A.lj_inner, A.tables, r2, e);
-            if (ENER && !(g.w > 0 && r2 > g.w)) ev += e - cc.z;
-          } else {
-            if (LJ96) {   // field.cpp:1658-1661
-              const double r9i = r6i * r2i * rinv;
-              fr = (9 * cc.y * r9i - 6 * cc.x * r6i) * r2i;
-              if (ENER) ev += cc.y * r9i - cc.x * r6i - cc.z;
-            } else if ((CAP || FROZEN) && A.lj_fsw) {
-              fr = charmm_fsw(cc.y, cc.x, A.lj_inner, A.rc, r2, ev, ENER);
-            } else {
-              fr = r6i * (12 * cc.y * r6i - 6 * cc.x) * r2i;
-              if (ENER) ev += r6i * (cc.y * r6i - cc.x) - cc.z;
-            }
-          }
-          if (COUL != 0 && FROZEN && !(r2 < A.rc2)) {
-            const double qq = xi.w * aj.w;
-            const double r = sqrt(r2);
-            double ex2;
-            const double er = erfc_exp_as(A.beta * r, ex2);   // beta: the Ewald or DSF coefficient; kc = 2 beta / sqrt(pi)
-            if (COUL == 1) {
-              if (ENER) ec += qq * er / r;
-              fr += qq * (er / r2 + A.kc * ex2 / r) / r;
-            } else {
-              if (ENER) ec += qq * (er / r - A.dsf_e0 + A.dsf_f0 * (r - A.rc));
-              fr += qq * (er / r2 + A.kc * ex2 / r - A.dsf_f0) / r;
-            }
-          } else if (COUL != 0) {
-            const double qq = xi.w * aj.w;
-            double E, Fc;
-            ewald_ef(gt, A.ghi, r2, rinv, E, Fc);
-            if (COUL == 1) {
-              if (ENER) ec += qq * E;
-              fr += qq * Fc;
-            } else {
-              if (ENER) ec += qq * (E - A.dsf_e0 + A.dsf_f0 * (r2 * rinv - A.rc));
-              fr += qq * (Fc - A.dsf_f0 * rinv);
-            }
-          }
-          const double fx = fr * dx, fy = fr * dy, fz = fr * dz;
-          if (jj) f1x += fx, f1y += fy, f1z += fz;
-          else f0x += fx, f0y += fy, f0z += fz;
-          fix[c] -= fx;
-          fiy[c] -= fy;
-          fiz[c] -= fz;
-          if (VIR) {
-            vw[0] += fx * dx;
-            vw[1] += fy * dy;
-            vw[2] += fz * dz;
-            vw[3] += fx * dy;
-            vw[4] += fx * dz;
-            vw[5] += fy * dz;
-          }
+        const double dx0 = a0.x - xi.x, dy0 = a0.y - xi.y, dz0 = a0.z - xi.z;
+        const double dx1 = a1.x - xi.x, dy1 = a1.y - xi.y, dz1 = a1.z - xi.z;
+        const double r20 = dx0 * dx0 + dy0 * dy0 + dz0 * dz0, r21 = dx1 * dx1 + dy1 * dy1 + dz1 * dz1;
+        const bool ok0 = ((lv >> c) & 1u) && (FROZEN || r20 < A.rc2), ok1 = ((lv >> (c + 8)) & 1u) && (FROZEN || r21 < A.rc2);
+        if (!__any_sync(0xffffffffu, ok0 || ok1)) continue;
+        double e0 = 0, e1 = 0, q0 = 0, q1 = 0;
+        double fr0 = 0, fr1 = 0;
+        if (CAP || FROZEN) {   // the rare variants branch within a pair: a pair at a time
+          if (ok0) fr0 = pair_f64<COUL, ENER, CAP, LJ96, FROZEN>(A, T, tab, ti + t0, r20, xi.w * a0.w, e0, q0);
+          if (ok1) fr1 = pair_f64<COUL, ENER, CAP, LJ96, FROZEN>(A, T, tab, ti + t1, r21, xi.w * a1.w, e1, q1);
+        } else {               // a pair left out is evaluated at a distance inside the table and dropped
+          fr0 = pair_f64<COUL, ENER, CAP, LJ96, FROZEN>(A, T, tab, ti + t0, ok0 ? r20 : 0.5 * A.rc2, xi.w * a0.w, e0, q0);
+          fr1 = pair_f64<COUL, ENER, CAP, LJ96, FROZEN>(A, T, tab, ti + t1, ok1 ? r21 : 0.5 * A.rc2, xi.w * a1.w, e1, q1);
+          fr0 = ok0 ? fr0 : 0.0, fr1 = ok1 ? fr1 : 0.0;
+        }
+        if (ENER) {
+          ev += (ok0 ? e0 : 0.0) + (ok1 ? e1 : 0.0);
+          ec += (ok0 ? q0 : 0.0) + (ok1 ? q1 : 0.0);
+        }
+        // a padding slot's separation may overflow a product, never reach a sum
+        const double fx0 = ok0 ? fr0 * dx0 : 0.0, fy0 = ok0 ? fr0 * dy0 : 0.0, fz0 = ok0 ? fr0 * dz0 : 0.0;
+        const double fx1 = ok1 ? fr1 * dx1 : 0.0, fy1 = ok1 ? fr1 * dy1 : 0.0, fz1 = ok1 ? fr1 * dz1 : 0.0;
+        f0x += fx0, f0y += fy0, f0z += fz0;
+        f1x += fx1, f1y += fy1, f1z += fz1;
+        fix[c] -= fx0 + fx1;
+        fiy[c] -= fy0 + fy1;
+        fiz[c] -= fz0 + fz1;
+        if (VIR) {
+          vw[0] += fx0 * dx0 + fx1 * dx1;
+          vw[1] += fy0 * dy0 + fy1 * dy1;
+          vw[2] += fz0 * dz0 + fz1 * dz1;
+          vw[3] += fx0 * dy0 + fx1 * dy1;
+          vw[4] += fx0 * dz0 + fx1 * dz1;
+          vw[5] += fy0 * dz0 + fy1 * dz1;
         }
       }
       {
@@ -581,7 +652,7 @@ static __global__ void __launch_bounds__(128, 2) k_pair_f64(PairArgs A) {
         if (comp < 3) {
           const double v = comp == 0 ? kx : comp == 1 ? ky : kz;
           double* dst = comp == 0 ? A.fdx : comp == 1 ? A.fdy : A.fdz;
-          if (v != 0.0) atomicAdd(dst + ((i8 & 4) ? j1 : j0), v);
+          if (v != 0.0) atomicAdd(dst + 8 * int(en.x) + jq + (i8 & 4), v);
         }
       }
     }
