@@ -129,6 +129,9 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
   return y;
 }
 
+// A position times a force in fixed point (2^24 per kcal/mol); the product of two floats is exact in double.
+__device__ __forceinline__ long long vir_fix(float x, float f) { return to_fix(double(x) * double(f), kFixE); }
+
 // COUL: 0 none; 1 Ewald real space (PME) and 2 damped shifted force through the rational fits of ewald_fit.cuh
 // (kappa r_c <= 4); 3 and 4 the same through erfcf and expf (any kappa). COMB: the LJ coefficients of a type pair are
 // products of per-type factors (geometric mixing: c6_ab = sqrt(c6_aa c6_bb), the same for c12), taken from a
@@ -177,9 +180,12 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
   const float rc2 = float(A.rc2), beta = float(A.beta), kc = float(A.kc), kcoul = float(A.kcoul);
   const float2 ku = p_dup(float(A.beta * A.beta / kEwUMax)), nkap3 = p_dup(-float(A.beta * A.beta * A.beta));
   const float e0 = float(A.dsf_e0), f0 = float(A.dsf_f0), rcf = float(A.rc);
-  // energy and virial: every pair's terms rounded to fixed point on their own (2^24 per kcal/mol), so that the totals do
-  // not depend on the list's grouping of pairs into entries and work items
-  long long acc_v = 0, acc_c = 0, acc_w[6] = {0, 0, 0, 0, 0, 0};
+  // energies: every pair's terms rounded to fixed point on their own (2^24 per kcal/mol), so that the totals do not depend
+  // on the list's grouping of pairs. Virial: sum of d F over a work item's pairs, d = x_j - x_i, as sum x_j F_j + sum x_i F_i
+  // over its atoms with the force sums the kernel has anyway (positions from the super-cluster's origin, products exact in
+  // double, each rounded to fixed point): per pair it took six products and twelve conversions to 64-bit integers, which
+  // made this variant twice as long as the force-only one
+  long long acc_v = 0, acc_c = 0, acc_w[6] = {0, 0, 0, 0, 0, 0}, acc_wj[2] = {0, 0};
   double acc_np = 0, acc_nl = 0;
   constexpr float kq = 16777216.f;
   for (int w = next_work_item(A.counters, lane); w < nwork; w = next_work_item(A.counters, lane)) {
@@ -349,11 +355,6 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
         fix[c] -= fx.x + fx.y;
         fiy[c] -= fy.x + fy.y;
         fiz[c] -= fz.x + fz.y;
-        if (VIR) {   // fr is 0 for the pairs left out
-          const float2 w6[6] = {p_mul(fx, dx), p_mul(fy, dy), p_mul(fz, dz), p_mul(fx, dy), p_mul(fx, dz), p_mul(fy, dz)};
-#pragma unroll
-          for (int k = 0; k < 6; ++k) acc_w[k] += __float2ll_rn(w6[k].x * kq) + __float2ll_rn(w6[k].y * kq);
-        }
       }
       // j forces: summed over the 8 lanes holding the same j atoms, then one fixed-point add per component
       {
@@ -364,6 +365,12 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
           const float v = comp == 0 ? kx : comp == 1 ? ky : kz;
           long long* dst = comp == 0 ? A.fsx : comp == 1 ? A.fsy : A.fsz;
           if (v != 0.f) fix_add_f(dst + ((i8 & 4) ? j1 : j0), v, A.err);
+          if (VIR) {   // the j atoms' share of the virial: lane comp 0 takes xx and xy, 1 yy and yz, 2 zz and xz
+            const bool h = (i8 & 4) != 0;
+            const float px = h ? xj.y : xj.x, py = h ? yj.y : yj.x, pz = h ? zj.y : zj.x;
+            acc_wj[0] += vir_fix(comp == 0 ? px : comp == 1 ? py : pz, v);
+            acc_wj[1] += vir_fix(comp == 1 ? py : px, comp == 0 ? ky : kz);
+          }
         }
       }
     }
@@ -379,6 +386,16 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
         if (fo[3 * m] != 0.f) fix_add_f(A.fsx + s, fo[3 * m], A.err);
         if (fo[3 * m + 1] != 0.f) fix_add_f(A.fsy + s, fo[3 * m + 1], A.err);
         if (fo[3 * m + 2] != 0.f) fix_add_f(A.fsz + s, fo[3 * m + 2], A.err);
+        if (VIR) {   // the i atoms' share (staged negated)
+          const float4 pa = xi_s[3 * (8 * c + i8)];
+          const float px = -pa.x, py = -pa.z, pz = -xi_s[3 * (8 * c + i8) + 1].x;
+          acc_w[0] += vir_fix(px, fo[3 * m]);
+          acc_w[1] += vir_fix(py, fo[3 * m + 1]);
+          acc_w[2] += vir_fix(pz, fo[3 * m + 2]);
+          acc_w[3] += vir_fix(px, fo[3 * m + 1]);
+          acc_w[4] += vir_fix(px, fo[3 * m + 2]);
+          acc_w[5] += vir_fix(py, fo[3 * m + 2]);
+        }
       }
     }
     if (ENER) {
@@ -391,8 +408,14 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
     acc_v = warp_sum(acc_v);
     acc_c = warp_sum(acc_c);
   }
-  if (VIR)
+  if (VIR) {
+    const int comp = i8 & 3;
+    if (comp < 3) {
+      acc_w[0] += comp == 0 ? acc_wj[0] : 0, acc_w[1] += comp == 1 ? acc_wj[0] : 0, acc_w[2] += comp == 2 ? acc_wj[0] : 0;
+      acc_w[3] += comp == 0 ? acc_wj[1] : 0, acc_w[5] += comp == 1 ? acc_wj[1] : 0, acc_w[4] += comp == 2 ? acc_wj[1] : 0;
+    }
     for (int k = 0; k < 6; ++k) acc_w[k] = warp_sum(acc_w[k]);
+  }
   if (lane == 0) {
     if (ENER) {
       atomic_add_fix(A.en.fix + kEVdw, acc_v);
@@ -550,7 +573,8 @@ static __global__ void __launch_bounds__(128, 3) k_pair_f64(PairArgs A) {
   if (A.counters[kCntErr] & kErrListBad) return;
   const int nwork = min(A.counters[kCntWork], A.work_cap);
   const int pad = A.ntab - 1;
-  double acc_v = 0, acc_c = 0, acc_w[6] = {0, 0, 0, 0, 0, 0};
+  // energies, and the virial from the atoms' force sums as in the FP32 kernel (positions from the first i atom)
+  double acc_v = 0, acc_c = 0, acc_w[6] = {0, 0, 0, 0, 0, 0}, acc_wj[2] = {0, 0};
   for (int w = next_work_item(A.counters, lane); w < nwork; w = next_work_item(A.counters, lane)) {
     const int4 wk = A.work[w];
     const int sc = wk.x;
@@ -583,7 +607,7 @@ static __global__ void __launch_bounds__(128, 3) k_pair_f64(PairArgs A) {
     double fix[8], fiy[8], fiz[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) fix[c] = fiy[c] = fiz[c] = 0.0;
-    double ev = 0, ec = 0, vw[6] = {0, 0, 0, 0, 0, 0};
+    double ev = 0, ec = 0;
     __syncwarp();
     for (int el = 0; el < ne; ++el) {
       const uint4 en = en_s[el];
@@ -636,14 +660,6 @@ static __global__ void __launch_bounds__(128, 3) k_pair_f64(PairArgs A) {
         fix[c] -= fx0 + fx1;
         fiy[c] -= fy0 + fy1;
         fiz[c] -= fz0 + fz1;
-        if (VIR) {
-          vw[0] += fx0 * dx0 + fx1 * dx1;
-          vw[1] += fy0 * dy0 + fy1 * dy1;
-          vw[2] += fz0 * dz0 + fz1 * dz1;
-          vw[3] += fx0 * dy0 + fx1 * dy1;
-          vw[4] += fx0 * dz0 + fx1 * dz1;
-          vw[5] += fy0 * dz0 + fy1 * dz1;
-        }
       }
       {
         double kx, ky, kz;
@@ -653,6 +669,11 @@ static __global__ void __launch_bounds__(128, 3) k_pair_f64(PairArgs A) {
           const double v = comp == 0 ? kx : comp == 1 ? ky : kz;
           double* dst = comp == 0 ? A.fdx : comp == 1 ? A.fdy : A.fdz;
           if (v != 0.0) atomicAdd(dst + 8 * int(en.x) + jq + (i8 & 4), v);
+          if (VIR && v != 0.0) {
+            const double4 a = xj_s[8 * el + jq + (i8 & 4)], r = xi_s[0];
+            acc_wj[0] += (comp == 0 ? a.x - r.x : comp == 1 ? a.y - r.y : a.z - r.z) * v;
+            acc_wj[1] += (comp == 1 ? a.y - r.y : a.x - r.x) * (comp == 0 ? ky : kz);
+          }
         }
       }
     }
@@ -667,15 +688,33 @@ static __global__ void __launch_bounds__(128, 3) k_pair_f64(PairArgs A) {
         if (fo[3 * m] != 0.0) atomicAdd(A.fdx + s, fo[3 * m]);
         if (fo[3 * m + 1] != 0.0) atomicAdd(A.fdy + s, fo[3 * m + 1]);
         if (fo[3 * m + 2] != 0.0) atomicAdd(A.fdz + s, fo[3 * m + 2]);
+        if (VIR) {
+          const double4 x = xi_s[8 * c + i8], r = xi_s[0];
+          const double px = x.x - r.x, py = x.y - r.y, pz = x.z - r.z;
+          acc_w[0] += px * fo[3 * m];
+          acc_w[1] += py * fo[3 * m + 1];
+          acc_w[2] += pz * fo[3 * m + 2];
+          acc_w[3] += px * fo[3 * m + 1];
+          acc_w[4] += px * fo[3 * m + 2];
+          acc_w[5] += py * fo[3 * m + 2];
+        }
       }
     }
-    if (ENER) {
-      acc_v += warp_sum(ev);
-      acc_c += warp_sum(ec);
-    }
-    if (VIR)
-      for (int k = 0; k < 6; ++k) acc_w[k] += warp_sum(vw[k]);
+    acc_v += ev;
+    acc_c += ec;
     __syncwarp();
+  }
+  if (ENER) {
+    acc_v = warp_sum(acc_v);
+    acc_c = warp_sum(acc_c);
+  }
+  if (VIR) {
+    const int comp = i8 & 3;
+    if (comp < 3) {
+      acc_w[0] += comp == 0 ? acc_wj[0] : 0, acc_w[1] += comp == 1 ? acc_wj[0] : 0, acc_w[2] += comp == 2 ? acc_wj[0] : 0;
+      acc_w[3] += comp == 0 ? acc_wj[1] : 0, acc_w[5] += comp == 1 ? acc_wj[1] : 0, acc_w[4] += comp == 2 ? acc_wj[1] : 0;
+    }
+    for (int k = 0; k < 6; ++k) acc_w[k] = warp_sum(acc_w[k]);
   }
   if (lane == 0) {
     if (ENER) {
