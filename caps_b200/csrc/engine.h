@@ -94,6 +94,8 @@ void DevBuf<T>::zero(cudaStream_t s) {
   const cudaError_t e = cudaMemsetAsync(p, 0, n * sizeof(T), s);
   if (e != cudaSuccess) throw CudaError(std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
 }
+// Kernel launches of this thread (the runs' launch counts).
+inline thread_local long long g_launches = 0;
 // Launches a kernel on a stream and turns a launch error into an exception. Arguments convert to the kernel's parameter
 // types.
 template <class... KP, class... A>
@@ -103,6 +105,7 @@ void launch_k(void (*kernel)(KP...), dim3 grid, dim3 block, size_t smem, cudaStr
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
+  ++g_launches;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
   if (e != cudaSuccess) throw CudaError(std::string("kernel launch: ") + cudaGetErrorString(e));
 }

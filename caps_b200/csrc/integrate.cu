@@ -722,6 +722,24 @@ __global__ void k_scale_by(int n, double* __restrict__ v, double f) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < 3 * n) v[i] *= f;
 }
+// The barostat's rescaling (dynamics.cpp:684-723): x = o + mu (x - o) by component; with vel, v /= mu (one mu for the three
+// components). The step's constraint virial, each component r_a F_b, is scaled with the cell (dynamics.cpp:448-456), and the
+// kinetic energy before the rescaling kept for the bath.
+__global__ void k_rescale(int n, double* __restrict__ x, double* __restrict__ v, double* __restrict__ sc, double3 org, double3 mu, int vel) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const double m[3] = {mu.x, mu.y, mu.z}, o[3] = {org.x, org.y, org.z};
+  if (i < 3 * n) {
+    const int c = i % 3;
+    x[i] = o[c] + m[c] * (x[i] - o[c]);
+    if (vel) v[i] /= m[0];
+  }
+  if (i < 6) {
+    const int ia = i < 3 ? i : i < 5 ? 0 : 1, ib = i < 3 ? i : i == 3 ? 1 : 2;
+    sc[kScCW0 + i] *= sqrt(m[ia] * m[ib]);
+  } else if (i == 6) {
+    sc[kScKE0] = sc[kScKE];
+  }
+}
 // The MTK remap (dynamics.cpp:560-570): x = c0 + mu (x - c0) about the cell's centre c0.
 __global__ void k_remap(int n, double* __restrict__ x, double c0x, double c0y, double c0z, double mu) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -778,15 +796,17 @@ __device__ double nhc_half(Chain& c, double& ke, double tt, double ndof, double 
 }
 
 // Bussi velocity rescaling (Bussi, Donadio & Parrinello 2007, appendix; dynamics.cpp:466-477) from this step's draws
-// (r1, sum of ndof - 1 squared normals) read from the host-made table.
-__device__ void bussi_body(double* sc, const double2* __restrict__ draws, long long first_step, double h, double tau, double ndof) {
+// (r1, sum of ndof - 1 squared normals) read from the host-made table, a ring over the steps: its captured kernel has no
+// parameter that a refill would change.
+constexpr long long kDrawRing = 8192;
+__device__ void bussi_body(double* sc, const double2* __restrict__ draws, double h, double tau, double ndof) {
   const double k = sc[kScKE];
   const long long step = (long long)sc[kScStep];
   if (k <= 0) {
     sc[kScFactor] = 1;
     return;
   }
-  const double2 d = draws[step - first_step];
+  const double2 d = draws[step & (kDrawRing - 1)];
   const double c = exp(-h / tau), kt = sc[kScKtarget];
   const double r1 = d.x, sum = d.y;
   const double knew = k + (1 - c) * (kt * (r1 * r1 + sum) / ndof - k) + 2 * r1 * sqrt(c * (1 - c) * kt * k / ndof);
@@ -813,7 +833,6 @@ struct KeArgs {
   const Chain* chain_half;   // the chain after the step's first half (kThenNhc)
   double t_freq, dt;
   const double2* draws;
-  long long draws_first;
   double tau;
 };
 
@@ -869,7 +888,7 @@ __device__ void ke_blocks(const KeArgs& A, double e, double t[6]) {
     *A.chain = c;
   }
   sc[A.slot] = ke;
-  if (A.then == kThenBussi) bussi_body(sc, A.draws, A.draws_first, A.dt, A.tau, A.ndof);
+  if (A.then == kThenBussi) bussi_body(sc, A.draws, A.dt, A.tau, A.ndof);
   else if (A.then == kThenLang) sc[kScKE0] = 0.5 * tt[0] / kAcc;
   if (A.then == kThenBath || A.then == kThenLang) sc[kScBath] -= sc[kScKE] - sc[kScKE0];
 }
@@ -1474,7 +1493,7 @@ struct Stepper {
     auto put = [&k](const void* p, size_t bytes) { k.append(static_cast<const char*>(p), bytes); };
     const double dv[] = {o.dt, o.temperature, o.temperature_end, o.tau_t, ndof, t_freq};
     put(dv, sizeof dv);
-    const long long iv[] = {(long long)o.steps, (long long)o.seed, o.thermostat, o.respa, o.respa_split, o.constraints, draws_first,
+    const long long iv[] = {(long long)o.steps, (long long)o.seed, o.thermostat, o.respa, o.respa_split, o.constraints,
                             ncons, nfree, nparts, respa, slow_parts, fast_parts, thermo ? 1 : 0};
     put(iv, sizeof iv);
     put(&C, sizeof C);
@@ -1483,11 +1502,23 @@ struct Stepper {
     return k;
   }
 
+  // A capture costs as much as some twenty plain launches of the step, and the barostats change the cell, a parameter of the
+  // captured kernels: runs with fewer steps than that between rescalings launch their steps directly (6,192 atoms with a
+  // rescaling every 10 steps: 157 us per step with a capture after each, 105 without).
+  bool direct() const { return (o.barostat == 1 || o.barostat == 2) && o.barostat_every < 32; }
+
   // Replays the step graph. It is captured when the run's key differs from the one it was made with; an instantiated
   // graph is then updated in place (cudaGraphExecUpdate), and instantiated anew only if the update is refused.
   // Returns its kernel count.
   int launch_step(bool thermo) {
     const int k = thermo ? 1 : 0;
+    if (direct()) {
+      const long long before = g_launches;
+      step(thermo, thermo);
+      graph_kernels[k] = int(g_launches - before);
+      if (k == 0) E.graph_kernels_ = graph_kernels[k];
+      return graph_kernels[k];
+    }
     ensure_graph(thermo);
     if (k == 0) E.graph_kernels_ = graph_kernels[k];
     CK(cudaGraphLaunch(graph[k], E.stream_));
@@ -1563,7 +1594,6 @@ struct Stepper {
     A.t_freq = t_freq;
     A.dt = o.dt;
     A.draws = draws.p;
-    A.draws_first = draws_first;
     A.tau = o.tau_t;
     return A;
   }
@@ -1713,7 +1743,7 @@ struct Stepper {
   }
 
   // Bussi draws for steps [first, first + count): r1 = gauss, then the chi-squared of ndof - 1 by a fresh Gamma
-  static constexpr long long kDrawChunk = 4096;   // draws made ahead at most (the buffer holds one chunk and one more)
+  static constexpr long long kDrawChunk = kDrawRing / 2;   // draws made ahead at most
   void make_draws(long long first, long long count) {
     std::vector<double2> d(static_cast<size_t>(count));
     for (long long s = 0; s < count; ++s) {
@@ -1721,7 +1751,12 @@ struct Stepper {
       const double sum = ndof > 1 ? rng->gamma((ndof - 1) / 2, 2.0) : 0.0;
       d[size_t(s)] = make_double2(r1, sum);
     }
-    draws.upload(d, E.stream_);
+    // into the ring, after the steps queued so far, which read earlier slots (a chunk is half a ring at most)
+    for (long long s = 0; s < count;) {
+      const long long slot = (first + s) & (kDrawRing - 1), run = std::min(count - s, kDrawRing - slot);
+      CK(cudaMemcpyAsync(draws.p + slot, d.data() + s, size_t(run) * sizeof(double2), cudaMemcpyHostToDevice, E.stream_));
+      s += run;
+    }
     draws_first = first;
     draws_count = count;
   }
@@ -2011,7 +2046,7 @@ struct MdRun {
   void advance(long long s, bool stop = false);
   // steps s .. s + kBlockSteps - 1 are plain steps (no row, frame, checkpoint, cell rescaling or thermostat refill)
   bool block_due(long long s) const {
-    if (mtk() || s + Stepper::kBlockSteps - 1 >= o.steps) return false;
+    if (mtk() || S.direct() || s + Stepper::kBlockSteps - 1 >= o.steps) return false;
     for (long long t = s; t < s + Stepper::kBlockSteps; ++t)
       if (special(t)) return false;
     return true;
@@ -2079,7 +2114,7 @@ void MdRun::start() {
   S.part.alloc(size_t(7) * std::max(S.nparts, blocks(size_t(n_), 128)));   // k_ke's blocks, or k_vel_rattle's
   S.done.alloc(1);
   S.done.zero(stream_);
-  S.draws.alloc(size_t(Stepper::kDrawChunk) + 1);
+  S.draws.alloc(size_t(kDrawRing));
   S.respa = std::max(1, o.respa);
   S.slow_parts = 6, S.fast_parts = 1;
   if (o.respa_split == 1) {
@@ -2181,10 +2216,7 @@ void MdRun::start() {
 // One step s: the captured plain step, or a special one (thermo row, frame, cell rescaling, new thermostat draws).
 void MdRun::advance(long long s, bool stop) {
   if (refill_due(s)) {
-    CK(cudaStreamSynchronize(E.stream_));
     S.make_draws(s, draw_chunk(s));
-    S.drop_graphs();   // the draw table's first step is a parameter of the captured thermostat kernel
-    ++generation;
   }
   if (mtk()) {
     mtk_step(s);
@@ -2338,8 +2370,8 @@ void MdRun::baro_step(long long s) {
   E.read_terms(&t, true, true);
   for (int c = 0; c < 6; ++c) t.w[c] += S.h_sc[kScCW0 + c];
   t.virial = t.w[0] + t.w[1] + t.w[2];
-  const double k = S.h_sc[kScKE], vol = E.dcell_.vol;
-  const double p = (2 * k + t.virial) / (3 * vol) * kAtm;
+  const double vol = E.dcell_.vol;
+  const double p = (2 * S.h_sc[kScKE] + t.virial) / (3 * vol) * kAtm;
   const double hp = o.dt * baro_every;
   const double tnow = S.h_sc[kScTnow];
   // per-axis factors (the isotropic update scales all three by the same mu)
@@ -2364,30 +2396,18 @@ void MdRun::baro_step(long long s) {
     deps = std::max(-0.01, std::min(0.01, deps));   // at most 1 % in volume per update
     mu[0] = mu[1] = mu[2] = std::exp(deps / 3);
   }
-  std::vector<double> hx(n3);
-  CK(cudaMemcpyAsync(hx.data(), S.x.p, n3 * sizeof(double), cudaMemcpyDeviceToHost, stream_));
-  CK(cudaMemcpyAsync(hv.data(), S.v.p, n3 * sizeof(double), cudaMemcpyDeviceToHost, stream_));
-  CK(cudaStreamSynchronize(stream_));
+  // positions about the cell origin, and every cell vector's component c, by mu[c]; with cell rescaling the velocities
+  // follow the cell and the bath takes the kinetic energy's change
   double cell[12];
   std::memcpy(cell, E.cell_h_, sizeof cell);
-  // positions about the cell origin, and every cell vector's component c, by mu[c]
-  for (int i = 0; i < E.n_; ++i)
-    for (int c = 0; c < 3; ++c) hx[3 * size_t(i) + c] = cell[c] + mu[c] * (hx[3 * size_t(i) + c] - cell[c]);
+  launch_k(k_rescale, blocks(n3, 256), 256, 0, stream_, E.n_, S.x.p, S.v.p, S.sc.p, make_double3(cell[0], cell[1], cell[2]),
+           make_double3(mu[0], mu[1], mu[2]), o.barostat == 1 ? 1 : 0);
   for (int q = 3; q < 12; ++q) cell[q] *= mu[q % 3];
-  if (o.barostat == 1) {   // the velocities follow the cell, and the bath takes the kinetic energy's change
-    for (auto& q : hv) q /= mu[0];
-    const double k2 = host_ke(hv);
-    S.h_sc[kScBath] -= k2 - k;
-    CK(cudaMemcpyAsync(S.sc.p + kScBath, S.h_sc + kScBath, sizeof(double), cudaMemcpyHostToDevice, stream_));
+  if (o.barostat == 1) {
+    KeArgs A = S.ke_args(kScKE, false);
+    A.then = kThenBath;
+    S.ke_launch(A);
   }
-  // the step's constraint virial, each component r_a F_b scaled with the cell (dynamics.cpp:448-456)
-  {
-    static const int ia[6] = {0, 1, 2, 0, 0, 1}, ib[6] = {0, 1, 2, 1, 2, 2};
-    for (int c = 0; c < 6; ++c) S.h_sc[kScCW0 + c] *= std::sqrt(mu[ia[c]] * mu[ib[c]]);
-    CK(cudaMemcpyAsync(S.sc.p + kScCW0, S.h_sc + kScCW0, 6 * sizeof(double), cudaMemcpyHostToDevice, stream_));
-  }
-  S.x.upload(hx, stream_);
-  S.v.upload(hv, stream_);
   E.set_cell(cell);
   S.C.cell = E.dcell_;
   if (S.ncons) {
@@ -2397,7 +2417,7 @@ void MdRun::baro_step(long long s) {
   }
   S.forces(true, true);
   S.ke(kScKE, false);   // the rescaled velocities' kinetic energy, which the next Nose-Hoover step starts from
-  S.drop_graphs();   // the cell is a parameter of the captured kernels
+  S.drop_graphs();   // the cell is a parameter of the captured kernels (a run with few steps per cell captures none)
   ++generation;
 }
 
@@ -2422,7 +2442,7 @@ void Engine::run(caps_gpu_state* st, const caps_gpu_md_opts* md, caps_gpu_progre
   }
   // the step graphs are captured before the step loop, as set-up (like the first force evaluation), so that no step's
   // time holds a capture
-  if (o.steps > 0 && !R.mtk() && !R.baro_due(1) && !R.refill_due(1)) {
+  if (o.steps > 0 && !R.mtk() && !S.direct() && !R.baro_due(1) && !R.refill_due(1)) {
     S.ensure_graph(false);
     S.ensure_graph(true);
     if (!timed && o.steps > Stepper::kBlockSteps) S.ensure_graph(false, true);
@@ -2545,6 +2565,8 @@ void run_batch(const std::vector<Engine*>& es, caps_gpu_state* const* states, co
   for (auto& e : res.ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   std::vector<int> seen(R, -1);
   long long batch_kernels = 0, graph_nodes = 0;
+  bool direct = true;
+  for (size_t r = 0; r < R; ++r) direct = direct && runs[r]->S.direct();
   bool on_replicas = true;   // the replicas' own streams hold the latest work
   // orders the batch stream after every replica stream, or every replica stream after the batch stream
   auto join_to_batch = [&] {
@@ -2578,6 +2600,11 @@ void run_batch(const std::vector<Engine*>& es, caps_gpu_state* const* states, co
         stopped_at = s;
         break;
       }
+      continue;
+    }
+    if (direct) {   // no graph worth capturing: every replica's step on its own stream
+      if (!on_replicas) fork_to_replicas(), on_replicas = true;
+      for (size_t r = 0; r < R; ++r) runs[r]->kernels += runs[r]->S.launch_step(false);
       continue;
     }
     if (on_replicas) join_to_batch(), on_replicas = false;

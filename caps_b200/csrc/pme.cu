@@ -240,10 +240,14 @@ void Engine::pme_run(PmePath<R>& P, const double* d_x, bool ener, bool vir) {
   fft_passes(P, ener, vir);
   const ForceSink<float> Ff{d_F_.p, d_F_.p + n_, d_F_.p + 2 * size_t(n_), d_counters_.p + kCntErr};
   const ForceSink<double> Fd{d_Fd_.p, d_Fd_.p + n_, d_Fd_.p + 2 * size_t(n_)};
+  // four lanes per atom up to four waves of threads, 75,000 atoms: there the gather waits for its loads, beyond it the
+  // splines' repetition costs more
+  const bool split = n_ <= 512 * dev_sms_;
+  const int gb = blocks_for(size_t(n_) * (split ? 4 : 1), 128);
 #define GATHER(P_)                                                                            \
   do {                                                                                        \
-    if (mixed_) launch_k(k_gather<float, R, P_>, blocks_for(size_t(n_), 128), 128, 0, stream_, A, P.gr.p, Ff);              \
-    else launch_k(k_gather<double, R, P_>, blocks_for(size_t(n_), 128), 128, 0, stream_, A, P.gr.p, Fd);                     \
+    if (mixed_) launch_k(split ? k_gather<float, R, P_, 4> : k_gather<float, R, P_, 1>, gb, 128, 0, stream_, A, P.gr.p, Ff);   \
+    else launch_k(split ? k_gather<double, R, P_, 4> : k_gather<double, R, P_, 1>, gb, 128, 0, stream_, A, P.gr.p, Fd);       \
   } while (0)
   switch (order_) {
     case 3: GATHER(3); break;

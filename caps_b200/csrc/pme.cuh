@@ -324,7 +324,7 @@ static __global__ void __launch_bounds__(kPmeThreads) k_spread(PmeArgs A, double
 
 // Shared memory of the line-transform kernels: the twiddle table, then two buffers of the block's lines.
 // K-FFT-X forward: real lines (b, c) of length K1 to half spectra h(a, b, c), a <= K1/2; lines 2 m and 2 m + 1 are the real
-// and imaginary parts of one complex line, parted again in the spectrum by its symmetry. Input: g (double) or gq (fixed),
+// and imaginary parts of one complex line, parted again in the spectrum by its symmetry. Input: g (FP64 path) or gq (mixed path, fixed),
 // cleared as it is read: the grid is zero for the next spread, with no launch of its own for it (as a memset node of the
 // step's graph it started up to 10 us after the step's drift, and the spread behind it). lpb: pairs of lines per block.
 template <class R>
@@ -338,10 +338,13 @@ static __global__ void __launch_bounds__(128) k_fft_x_fwd(PmeArgs A, double* __r
   T* s1 = s0 + lpb * ls;
   const int nlines = A.k2 * A.k3, npairs = (nlines + 1) / 2;
   stage_twiddles(tw, P.tw, A.k1);
+  // no branch around a load, so that a butterfly's loads go out together (a line past the last reads the last, times 0)
   auto take = [&](int line, int i) {
-    if (line >= nlines) return R(0);
-    const size_t at = size_t(line) * A.k1 + i;   // lines are contiguous in the real grid
-    return gq ? R(double(gq[at]) * kInvFixQ) : R(g[at]);
+    const size_t at = size_t(min(line, nlines - 1)) * A.k1 + i;   // lines are contiguous in the real grid
+    R v;
+    if constexpr (sizeof(R) == 4) v = R(double(gq[at]) * kInvFixQ);
+    else v = g[at];
+    return line < nlines ? v : R(0);
   };
   const unsigned m_h1 = div_magic(unsigned(A.h1));
   // groups of lpb pairs, strided over the grid (the grid may be smaller than the group count)
@@ -352,7 +355,7 @@ static __global__ void __launch_bounds__(128) k_fft_x_fwd(PmeArgs A, double* __r
     // every value is read: cleared together, so that no store stands between two loads
     const size_t first = size_t(2 * l0) * A.k1, cells = size_t(min(2 * B.nl, nlines - 2 * l0)) * A.k1;
     for (size_t t = threadIdx.x; t < cells; t += blockDim.x) {
-      if (gq) gq[first + t] = 0;
+      if constexpr (sizeof(R) == 4) gq[first + t] = 0;
       else g[first + t] = 0;
     }
     for (int t = threadIdx.x; t < 2 * B.nl * A.h1; t += blockDim.x) {
@@ -384,7 +387,8 @@ static __global__ void __launch_bounds__(128) k_fft_x_inv(PmeArgs A, const typen
           const int line = 2 * (l0 + l), a = 2 * m <= A.k1 ? m : A.k1 - m;
           const R sg = 2 * m <= A.k1 ? R(1) : R(-1);
           const T u = h[size_t(line) * A.h1 + a];
-          const T w = line + 1 < nlines ? h[size_t(line + 1) * A.h1 + a] : T{R(0), R(0)};
+          T w = h[size_t(min(line + 1, nlines - 1)) * A.h1 + a];
+          if (line + 1 >= nlines) w = {R(0), R(0)};
           // Z = U + i W with conjugates past the middle, real and imaginary parts exchanged
           return T{sg * u.y + w.x, u.x - sg * w.y};
         },
@@ -561,15 +565,16 @@ static __global__ void k_pme_green(PmeArgs A, const double* __restrict__ b1, con
   }
 }
 
-// K-GATHER: F_i -= q_i sum_d K_d (row d of h^-1) dE/du_d (caps_kspace.f90:965-992). A thread per atom: its rows of P values
-// along x are a sector each, which the loads of one thread share in L1; a group of 16 lanes per atom, as in the spread,
-// measured 11 us against 6 at 32,000 atoms (its sums go through twelve shuffles).
-template <class R, class G, int P>
-static __global__ void k_gather(PmeArgs A, const G* __restrict__ gr, ForceSink<R> F) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// K-GATHER: F_i -= q_i sum_d K_d (row d of h^-1) dE/du_d (caps_kspace.f90:965-992), L lanes per atom, each taking every
+// L-th plane c of its P^3 points (the splines by each lane for itself: cheaper than a stage in shared memory). One lane per
+// atom reads fewest instructions, four fill the GPU and shorten the chain of loads where atoms are few (gather_lanes).
+template <class R, class G, int P, int L>
+static __global__ void __launch_bounds__(128) k_gather(PmeArgs A, const G* __restrict__ gr, ForceSink<R> F) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = t / L, lane = t % L;
   if (i >= A.n) return;
   const double qi = A.q[i];
-  if (qi == 0) return;
+  if (qi == 0) return;   // the same for an atom's lanes
   R th[3][P], dth[3][P];
   int base[3];
   atom_splines<R, P>(A, i, th, dth, base);
@@ -577,9 +582,15 @@ static __global__ void k_gather(PmeArgs A, const G* __restrict__ gr, ForceSink<R
 #pragma unroll
   for (int a = 0; a < P; ++a) ia[a] = wrapk(base[0] + a, A.k1), ib[a] = wrapk(base[1] + a, A.k2);
   R gs0 = 0, gs1 = 0, gs2 = 0;
-  for (int c = 0; c < P; ++c) {
+#pragma unroll
+  for (int c0 = 0; c0 < P; c0 += L) {
+    const int c = c0 + lane;
+    if (P % L != 0 && c >= P) break;
+    R tc = th[2][c0], dc = dth[2][c0];   // of plane c, by selects (an index would put the arrays in memory)
+#pragma unroll
+    for (int m = 1; m < L; ++m)
+      if (c0 + m < P && lane == m) tc = th[2][c0 + m], dc = dth[2][c0 + m];
     const int ic = wrapk(base[2] + c, A.k3);
-    const R tc = th[2][c], dc = dth[2][c];
 #pragma unroll
     for (int b = 0; b < P; ++b) {
       const R tb = th[1][b], db = dth[1][b];
@@ -592,6 +603,16 @@ static __global__ void k_gather(PmeArgs A, const G* __restrict__ gr, ForceSink<R
         gs2 += th[0][a] * tb * dc * st;
       }
     }
+  }
+  if (L > 1) {
+    const unsigned m = (L == 32 ? 0xffffffffu : (1u << L) - 1) << (threadIdx.x & 31 & ~(L - 1));
+#pragma unroll
+    for (int o = 1; o < L; o <<= 1) {
+      gs0 += __shfl_xor_sync(m, gs0, o);
+      gs1 += __shfl_xor_sync(m, gs1, o);
+      gs2 += __shfl_xor_sync(m, gs2, o);
+    }
+    if (lane) return;
   }
   R f[3];
   for (int r = 0; r < 3; ++r)
