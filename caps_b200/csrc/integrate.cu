@@ -181,6 +181,7 @@ struct ConsArgs {
   const double* d2;        // squared lengths
   const double* invm;      // per atom
   DevCell cell;
+  int direct;              // the mixed path: RATTLE's multipliers of stars and waters from their linear system at once
   // LINCS (every cluster in the general layout): the constraints' lengths, and per cluster its couplings, pairs of its
   // constraints (local indices) that share an atom with the coefficient -S_k S_l s_ka s_la / m_a, in the reference's
   // order (atoms ascending, then the constraints on each)
@@ -595,6 +596,33 @@ __device__ __forceinline__ void vel_op(const VelOp& op, int g, double* vv, const
   }
 }
 
+// The multipliers of N coupled velocity constraints, M lam = -rv (M symmetric), by elimination. RATTLE's Gauss-Seidel sweep
+// reaches them to 1e-8 in ten to twenty rounds of dependent operations, which took 22 us a step for 1,000 rigid waters; the
+// sweep that follows finds nothing left to do. The FP64 path keeps the sweep alone, whose stopping point its velocities
+// (and the reference's) carry.
+template <int N>
+__device__ __forceinline__ void rattle_solve(double M[N][N], const double rv[N], double lam[N]) {
+  double b[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) b[k] = -rv[k];
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+#pragma unroll
+    for (int l = k + 1; l < N; ++l) {
+      const double q = M[l][k] / M[k][k];
+#pragma unroll
+      for (int c = k; c < N; ++c) M[l][c] -= q * M[k][c];
+      b[l] -= q * b[k];
+    }
+#pragma unroll
+  for (int k = N - 1; k >= 0; --k) {
+    double v = b[k];
+#pragma unroll
+    for (int c = k + 1; c < N; ++c) v -= M[k][c] * lam[c];
+    lam[k] = v / M[k][k];
+  }
+}
+
 // RATTLE on a star cluster with NK constraints, in registers (the general kernel's sweep, constraints as (centre, partner)).
 template <int NK>
 __device__ void rattle_star(const ConsArgs& C, int s, const double* __restrict__ x, double* __restrict__ v, const VelOp& op, const double* sc,
@@ -619,6 +647,22 @@ __device__ void rattle_star(const ConsArgs& C, int s, const double* __restrict__
     min_image(C.cell, d0, d1, d2v);
     rr[k][0] = d0, rr[k][1] = d1, rr[k][2] = d2v;
     lam[k] = 0;
+  }
+  if (C.direct) {
+    double M[NK][NK], rv[NK];
+#pragma unroll
+    for (int k = 0; k < NK; ++k) {
+      rv[k] = rr[k][0] * (pv[0][0] - pv[k + 1][0]) + rr[k][1] * (pv[0][1] - pv[k + 1][1]) + rr[k][2] * (pv[0][2] - pv[k + 1][2]);
+#pragma unroll
+      for (int l = 0; l < NK; ++l) M[k][l] = (im[0] + (k == l ? im[k + 1] : 0.0)) * dot3d(rr[k], rr[l]);
+    }
+    rattle_solve<NK>(M, rv, lam);
+#pragma unroll
+    for (int k = 0; k < NK; ++k)
+      for (int r = 0; r < 3; ++r) {
+        pv[0][r] += lam[k] * im[0] * rr[k][r];
+        pv[k + 1][r] -= lam[k] * im[k + 1] * rr[k][r];
+      }
   }
   bool done = false;
   for (int it = 0; it < kShakeIter && !done; ++it) {
@@ -677,6 +721,26 @@ __device__ void rattle_water(const ConsArgs& C, int wi, const double* __restrict
     min_image(C.cell, d0, d1, d2v);
     rr[k][0] = d0, rr[k][1] = d1, rr[k][2] = d2v;
     lam[k] = 0;
+  }
+  if (C.direct) {
+    double M[3][3], rv[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int i = pi[k], j = pj[k];
+      rv[k] = rr[k][0] * (pv[i][0] - pv[j][0]) + rr[k][1] * (pv[i][1] - pv[j][1]) + rr[k][2] * (pv[i][2] - pv[j][2]);
+#pragma unroll
+      for (int l = 0; l < 3; ++l) {   // atoms i and j of constraint k move by +im rr_l and -im rr_l where l holds them
+        const double wi = (pi[l] == i ? im[i] : 0.0) - (pj[l] == i ? im[i] : 0.0), wj = (pi[l] == j ? im[j] : 0.0) - (pj[l] == j ? im[j] : 0.0);
+        M[k][l] = (wi - wj) * dot3d(rr[k], rr[l]);
+      }
+    }
+    rattle_solve<3>(M, rv, lam);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      for (int r = 0; r < 3; ++r) {
+        pv[pi[k]][r] += lam[k] * im[pi[k]] * rr[k][r];
+        pv[pj[k]][r] -= lam[k] * im[pj[k]] * rr[k][r];
+      }
   }
   bool done = false;
   for (int it = 0; it < kShakeIter && !done; ++it) {
@@ -1505,7 +1569,8 @@ struct Stepper {
   // A capture costs as much as some twenty plain launches of the step, and the barostats change the cell, a parameter of the
   // captured kernels: runs with fewer steps than that between rescalings launch their steps directly (6,192 atoms with a
   // rescaling every 10 steps: 157 us per step with a capture after each, 105 without).
-  bool direct() const { return (o.barostat == 1 || o.barostat == 2) && o.barostat_every < 32; }
+  bool direct() const { return (o.barostat == 1 || o.barostat == 2) && o.barostat_every < 6; }
+  bool blocks_worth() const { return !(o.barostat == 1 || o.barostat == 2) || o.barostat_every >= 32; }
 
   // Replays the step graph. It is captured when the run's key differs from the one it was made with; an instantiated
   // graph is then updated in place (cudaGraphExecUpdate), and instantiated anew only if the update is refused.
@@ -2046,7 +2111,7 @@ struct MdRun {
   void advance(long long s, bool stop = false);
   // steps s .. s + kBlockSteps - 1 are plain steps (no row, frame, checkpoint, cell rescaling or thermostat refill)
   bool block_due(long long s) const {
-    if (mtk() || S.direct() || s + Stepper::kBlockSteps - 1 >= o.steps) return false;
+    if (mtk() || !S.blocks_worth() || s + Stepper::kBlockSteps - 1 >= o.steps) return false;
     for (long long t = s; t < s + Stepper::kBlockSteps; ++t)
       if (special(t)) return false;
     return true;
@@ -2134,6 +2199,7 @@ void MdRun::start() {
   S.C.cell = E.dcell_;
   S.build_constraints(st->x);
   S.C.cell = E.dcell_;
+  S.C.direct = E.mixed_ ? 1 : 0;
   S.ndof = 3.0 * double(n_) - 3.0 - double(S.ncons);
   if (S.ndof < 1) throw ModelError(CAPS_GPU_EINVAL, "the constraints leave no degree of freedom");
   S.rng = std::make_unique<HostRng>(o.seed);
@@ -2444,8 +2510,8 @@ void Engine::run(caps_gpu_state* st, const caps_gpu_md_opts* md, caps_gpu_progre
   // time holds a capture
   if (o.steps > 0 && !R.mtk() && !S.direct() && !R.baro_due(1) && !R.refill_due(1)) {
     S.ensure_graph(false);
-    S.ensure_graph(true);
-    if (!timed && o.steps > Stepper::kBlockSteps) S.ensure_graph(false, true);
+    if (S.blocks_worth()) S.ensure_graph(true);
+    if (!timed && S.blocks_worth() && o.steps > Stepper::kBlockSteps) S.ensure_graph(false, true);
   }
   const auto w0 = std::chrono::steady_clock::now();
   CK(cudaEventRecord(ev0, stream_));

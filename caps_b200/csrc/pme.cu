@@ -222,11 +222,12 @@ void Engine::pme_run(PmePath<R>& P, const double* d_x, bool ener, bool vir) {
     std::memcpy(green_cell_, cell_h_, sizeof cell_h_);
     green_valid_ = true;
   }
-  const int nb = blocks_for(size_t(n_), kPmeAtoms);
+  // enough blocks of the spread for two per SM where atoms are few
+  const int pb = std::clamp(n_ / (2 * dev_sms_), 8, kPmeAtoms), nb = blocks_for(size_t(n_), pb);
 #define SPREAD(P_)                                                                            \
   do {                                                                                        \
-    if (mixed_) launch_k(k_spread<float, P_>, nb, kPmeThreads, 0, stream_, A, d_grid_.p, d_gridq_.p);      \
-    else launch_k(k_spread<double, P_>, nb, kPmeThreads, 0, stream_, A, d_grid_.p, d_gridq_.p);            \
+    if (mixed_) launch_k(k_spread<float, P_>, nb, kPmeThreads, 0, stream_, A, pb, d_grid_.p, d_gridq_.p);      \
+    else launch_k(k_spread<double, P_>, nb, kPmeThreads, 0, stream_, A, pb, d_grid_.p, d_gridq_.p);            \
   } while (0)
   switch (order_) {
     case 3: SPREAD(3); break;

@@ -282,11 +282,11 @@ __device__ __forceinline__ int wrapk(int v, int K) {
 template <int P>
 constexpr int pme_group() { return P == 3 ? 9 : P == 4 ? 16 : 32; }
 constexpr int kPmeThreads = 128;
-constexpr int kPmeAtoms = 64;   // atoms per block
+constexpr int kPmeAtoms = 64;   // atoms per block at most
 template <class R, int P>
 struct PmeAtom {
-  R th[3][P], dth[3][P];
-  int base[3];
+  R th[3][P];
+  int at[3][P];   // grid offsets of the P points along each axis
   R q;
 };
 
@@ -294,11 +294,18 @@ struct PmeAtom {
 // along x is P neighbouring lanes', so that it reaches L2 as one or two sectors of adds instead of P: the kernel is bound
 // by its atomics there (64 per atom at order 4).
 template <class R, int P>
-static __global__ void __launch_bounds__(kPmeThreads) k_spread(PmeArgs A, double* __restrict__ g, long long* __restrict__ gq) {
+static __global__ void __launch_bounds__(kPmeThreads) k_spread(PmeArgs A, int per_block, double* __restrict__ g, long long* __restrict__ gq) {
   __shared__ PmeAtom<R, P> S[kPmeAtoms];
-  const int i0 = blockIdx.x * kPmeAtoms, n = min(kPmeAtoms, A.n - i0);
+  const int i0 = blockIdx.x * per_block, n = min(per_block, A.n - i0);
   for (int t = threadIdx.x; t < n; t += kPmeThreads) {
-    atom_splines<R, P>(A, i0 + t, S[t].th, S[t].dth, S[t].base);
+    R th[3][P], dth[3][P];
+    int base[3];
+    atom_splines<R, P>(A, i0 + t, th, dth, base);
+    const int K[3] = {A.k1, A.k2, A.k3}, step[3] = {1, A.k1, A.k1 * A.k2};
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+      for (int k = 0; k < P; ++k) S[t].th[d][k] = th[d][k], S[t].at[d][k] = wrapk(base[d] + k, K[d]) * step[d];
     S[t].q = R(A.q[i0 + t]);
   }
   __syncthreads();
@@ -314,7 +321,7 @@ static __global__ void __launch_bounds__(kPmeThreads) k_spread(PmeArgs A, double
       if (P * P * P % G != 0 && pt >= P * P * P) break;
       const int ia = pt % P, ib = pt / P % P, ic = pt / (P * P);
       const R st = a.q * a.th[1][ib] * a.th[2][ic];
-      const size_t at = size_t(wrapk(a.base[0] + ia, A.k1)) + size_t(A.k1) * (size_t(wrapk(a.base[1] + ib, A.k2)) + size_t(A.k2) * size_t(wrapk(a.base[2] + ic, A.k3)));
+      const int at = a.at[0][ia] + a.at[1][ib] + a.at[2][ic];
       const R v = st * a.th[0][ia];
       if (sizeof(R) == 8) atomicAdd(g + at, double(v));
       else atomic_add_fix(gq + at, __float2ll_rn(float(v) * float(kFixQ)));   // the scale is a power of two: no rounding
