@@ -170,6 +170,7 @@ __device__ __forceinline__ void kick_drift_atom(const KickArgs& K, int i, double
 struct ConsArgs {
   int ncl;                 // all clusters: e3 star clusters, then e4 - e3 rigid waters, then ncl - e4 general ones
   int e1, e2, e3, e4;
+  int w1, w2, w3, w4, w5;  // first thread of the second kind of cluster ... of the free atoms: kinds start at whole warps
   const int4* star;        // e3: centre, then up to three partners (-1 unused)
   const double4* star_d2;  // e3: squared lengths of (centre, partner k)
   const int4* water;       // e4 - e3: O, H1, H2
@@ -191,6 +192,19 @@ struct ConsArgs {
   const int2* cp;
   const double* cpc;
 };
+// The cluster of thread t (or ncl + its free atom); past them all for a thread between two kinds. A warp with several kinds
+// would run their paths one after another, and the kernel last as long as that warp (6,192 atoms: 21 us against 14).
+__device__ __forceinline__ int cluster_of(const ConsArgs& C, int t) {
+  const int none = 0x3fffffff;
+  int c, end;
+  if (t < C.w1) c = t, end = C.e1;
+  else if (t < C.w2) c = C.e1 + t - C.w1, end = C.e2;
+  else if (t < C.w3) c = C.e2 + t - C.w2, end = C.e3;
+  else if (t < C.w4) c = C.e3 + t - C.w3, end = C.e4;
+  else if (t < C.w5) c = C.e4 + t - C.w4, end = C.ncl;
+  else return C.ncl + t - C.w5;
+  return c < end ? c : none;
+}
 constexpr int kMaxCouple = 56;   // couplings of a cluster of 8 constraints
 
 // SHAKE on a star cluster with NK constraints, in registers: p the positions (solved in place), o the old ones. The same
@@ -1035,13 +1049,13 @@ __device__ __forceinline__ void move_water(const KickArgs& K, const ConsArgs& C,
 }
 __global__ void __launch_bounds__(128) k_move(KickArgs K, ConsArgs C, ListCheck L, int nfree, const int* __restrict__ free_atoms, KeArgs A) {
   __shared__ double s_half;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, c = cluster_of(C, tid);
   const int stride = gridDim.x * blockDim.x;
-  for (int i = c; i < 3 * K.n; i += stride) {
+  for (int i = tid; i < 3 * K.n; i += stride) {
     if (K.fq) K.fq[i] = 0;
     if (K.fd) K.fd[i] = 0;
   }
-  if (K.zero_cw && c < 6) K.sc[kScCW0 + c] = 0;
+  if (K.zero_cw && tid < 6) K.sc[kScCW0 + tid] = 0;
   if (K.chain) {
     if (threadIdx.x == 0) {
       Chain ch = *K.chain;
@@ -1097,7 +1111,7 @@ __global__ void __launch_bounds__(128) k_move(KickArgs K, ConsArgs C, ListCheck 
 // velocities and runs K's thermostat update in its last block (what k_ke does in a launch of its own).
 __global__ void k_vel_rattle(ConsArgs C, int nfree, const int* __restrict__ free_atoms, const double* __restrict__ x, double* __restrict__ v, VelOp op,
                              double h, double* sc, int* counters, KeArgs K) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = cluster_of(C, blockIdx.x * blockDim.x + threadIdx.x);
   double w[6] = {0, 0, 0, 0, 0, 0};
   if (c >= C.ncl && c < C.ncl + nfree) {
     const int g = free_atoms ? free_atoms[c - C.ncl] : c - C.ncl;
@@ -1526,6 +1540,12 @@ struct Stepper {
       C.cpc = cpc.p;
     }
     C.ncl = C.e4 + int(st.size()) - 1;
+    auto warps = [](int k) { return (k + 31) / 32 * 32; };
+    C.w1 = warps(C.e1);
+    C.w2 = C.w1 + warps(C.e2 - C.e1);
+    C.w3 = C.w2 + warps(C.e3 - C.e2);
+    C.w4 = C.w3 + warps(C.e4 - C.e3);
+    C.w5 = C.w4 + warps(C.ncl - C.e4);
     C.cl_start = cl_start.p;
     C.cl_atom0 = cl_atom0.p;
     C.cl_atoms = cl_atoms.p;
@@ -1665,7 +1685,7 @@ struct Stepper {
   void ke_launch(const KeArgs& A) { launch_k(k_ke, nparts, 256, 0, E.stream_, A); }
   void ke(int slot, bool tensor) { ke_launch(ke_args(slot, tensor)); }
   // threads of the per-atom kernels: one per constraint cluster and one per atom in none
-  int movers() const { return ncons ? C.ncl + nfree : n; }
+  int movers() const { return ncons ? C.w5 + nfree : n; }
   // a step's first kernel (k_move): half kick, drift, constraints. pending: the step before left its velocity factor to
   // apply. The kick also clears the force evaluation's atom-order sums for the evaluation that follows (Engine::forces then
   // skips its own clearing). check: the list's displacement check runs here too, and the evaluation skips its own.
@@ -2176,7 +2196,7 @@ void MdRun::start() {
   S.chain_half.alloc(1);
   CK(cudaMemsetAsync(S.chain.p, 0, sizeof(Chain), stream_));
   S.nparts = blocks(size_t(n_), 256);
-  S.part.alloc(size_t(7) * std::max(S.nparts, blocks(size_t(n_), 128)));   // k_ke's blocks, or k_vel_rattle's
+  S.part.alloc(size_t(7) * (blocks(size_t(n_), 128) + 2));   // k_ke's blocks, or k_move's and k_vel_rattle's
   S.done.alloc(1);
   S.done.zero(stream_);
   S.draws.alloc(size_t(kDrawRing));
