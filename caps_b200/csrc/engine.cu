@@ -148,6 +148,7 @@ Engine::~Engine() {
   if (h_counters_) cudaFreeHost(h_counters_);
   if (h_efix_) cudaFreeHost(h_efix_);
   if (h_edbl_) cudaFreeHost(h_edbl_);
+  if (h_xf_) cudaFreeHost(h_xf_);
   if (stream_) cudaStreamDestroy(stream_);
   for (auto st : side_)
     if (st) cudaStreamDestroy(st);
@@ -166,6 +167,9 @@ void Engine::setup_ff(const caps_gpu_ff* ff) {
     if (t < 0 || t >= nt_) throw ModelError(CAPS_GPU_EINVAL, "type index out of range");
   h_q_.assign(ff->charge, ff->charge + n_);
   h_mass_.assign(ff->mass, ff->mass + n_);
+  charge_ = charge2_ = mass_ = 0;
+  for (double c : h_q_) charge2_ += c * c, charge_ += c;
+  for (double m : h_mass_) mass_ += m;
   h_eps_.assign(ff->pair_eps, ff->pair_eps + size_t(nt_) * nt_);
   h_sig_.assign(ff->pair_sigma, ff->pair_sigma + size_t(nt_) * nt_);
   // generic pair forms (field.cpp:478-487): both orders of each type pair; the pair is evaluated whatever its LJ eps
@@ -749,8 +753,7 @@ void Engine::host_constants(caps_gpu_terms* t, bool ener, bool vir) const {
   (void)vir;
   const bool nonb = (opt_.parts & 2) != 0;
   if (!nonb) return;
-  double q2 = 0, qt = 0;
-  for (double c : h_q_) q2 += c * c, qt += c;
+  const double q2 = charge2_, qt = charge_;
   if (coul_) {
     if (pme_) {
       if (ener) t->coulomb -= kCoulomb * beta_ / std::sqrt(kPi) * q2;
@@ -858,13 +861,24 @@ bool Engine::grow_list_for_run() {
   return true;
 }
 
-void Engine::compute_dev(const double* d_x, const double* cell, double* d_f, caps_gpu_terms* out) {
-  set_cell(cell);
+// What the host reads of an evaluation (counters, energies), written by the device into pinned memory: one small launch
+// in place of three copies of a few hundred bytes, each of which waits for the one before.
+__global__ void k_publish(const int* counters, const long long* efix, const double* edbl, int* h_counters, long long* h_efix, double* h_edbl) {
+  const int t = threadIdx.x;
+  if (t < kCntNum) h_counters[t] = counters[t];
+  if (t < kENumSlots) h_efix[t] = efix[t], h_edbl[t] = edbl[t];
+}
+
+void Engine::publish() {
+  launch_k(k_publish, 1, 32, 0, stream_, d_counters_.p, d_efix_.p, d_edbl_.p, h_counters_, h_efix_, h_edbl_);
+}
+
+// Evaluates and reads the results; h_f (pinned): the forces too, by the same synchronisation.
+void Engine::evaluate(const double* d_x, double* h_f, caps_gpu_terms* out) {
   for (int attempt = 0;; ++attempt) {
     forces(d_x, true, true, true);
-    CK(cudaMemcpyAsync(h_counters_, d_counters_.p, sizeof(int) * kCntNum, cudaMemcpyDeviceToHost, stream_));
-    CK(cudaMemcpyAsync(h_efix_, d_efix_.p, sizeof(long long) * kENumSlots, cudaMemcpyDeviceToHost, stream_));
-    CK(cudaMemcpyAsync(h_edbl_, d_edbl_.p, sizeof(double) * kENumSlots, cudaMemcpyDeviceToHost, stream_));
+    publish();
+    if (h_f) CK(cudaMemcpyAsync(h_f, d_f_.p, sizeof(double) * 3 * size_t(n_), cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
     try {
       check_errors();
@@ -875,21 +889,41 @@ void Engine::compute_dev(const double* d_x, const double* cell, double* d_f, cap
     }
     break;
   }
-  const bool ener_pairs = energies_ || !mixed_;
-  (void)ener_pairs;
   read_terms(out, true, true);
+}
+
+void Engine::compute_dev(const double* d_x, const double* cell, double* d_f, caps_gpu_terms* out) {
+  set_cell(cell);
+  evaluate(d_x, nullptr, out);
   if (d_f != d_f_.p) CK(cudaMemcpyAsync(d_f, d_f_.p, sizeof(double) * 3 * size_t(n_), cudaMemcpyDeviceToDevice, stream_));
   CK(cudaStreamSynchronize(stream_));
 }
 
+// Host arrays in and out through pinned staging (kept with the engine): the coordinates are checked and staged a piece at a
+// time, each piece's copy running while the next is staged.
 void Engine::compute_host(const double* x, const double* cell, double* f, caps_gpu_terms* out) {
-  for (size_t k = 0; k < size_t(3) * n_; ++k)
-    if (!std::isfinite(x[k])) throw ModelError(CAPS_GPU_EFIELD, "non-finite coordinates: atom " + std::to_string(k / 3 + 1));
+  const size_t n3 = size_t(3) * n_;
+  if (!h_xf_) CK(cudaMallocHost(&h_xf_, 2 * n3 * sizeof(double)));
+  d_x_.alloc(n3);
+  constexpr size_t piece = 32768;
+  constexpr uint64_t exponent = 0x7ff0000000000000ull;
+  for (size_t k0 = 0; k0 < n3; k0 += piece) {
+    const size_t m = std::min(piece, n3 - k0);
+    uint64_t bad = 0;   // the sign bit: an exponent of all ones (infinity or NaN) carries into it
+    for (size_t k = 0; k < m; ++k) {
+      uint64_t u;
+      std::memcpy(&u, x + k0 + k, sizeof u);
+      bad |= (u & exponent) + 0x0010000000000000ull;
+      h_xf_[k0 + k] = x[k0 + k];
+    }
+    if (bad >> 63)
+      for (size_t k = k0; k < n3; ++k)
+        if (!std::isfinite(x[k])) throw ModelError(CAPS_GPU_EFIELD, "non-finite coordinates: atom " + std::to_string(k / 3 + 1));
+    CK(cudaMemcpyAsync(d_x_.p + k0, h_xf_ + k0, m * sizeof(double), cudaMemcpyHostToDevice, stream_));
+  }
   set_cell(cell);
-  CK(cudaMemcpyAsync(d_x_.p, x, sizeof(double) * 3 * size_t(n_), cudaMemcpyHostToDevice, stream_));
-  compute_dev(d_x_.p, cell, d_f_.p, out);
-  CK(cudaMemcpyAsync(f, d_f_.p, sizeof(double) * 3 * size_t(n_), cudaMemcpyDeviceToHost, stream_));
-  CK(cudaStreamSynchronize(stream_));
+  evaluate(d_x_.p, h_xf_ + n3, out);
+  std::memcpy(f, h_xf_ + n3, n3 * sizeof(double));
 }
 
 

@@ -137,6 +137,8 @@ class Engine {
   // compute on host arrays (copies in and out) or on device arrays
   void compute_host(const double* x, const double* cell, double* f, caps_gpu_terms* out);
   void compute_dev(const double* d_x, const double* cell, double* d_f, caps_gpu_terms* out);
+  void publish();
+  void evaluate(const double* d_x, double* h_f, caps_gpu_terms* out);
   int list_builds();   // list builds so far (counted on the device)
   void list_counts(int64_t* v);   // v[0] list builds, v[1] dynamic prunes so far
   // Evaluator::freeze_pairs / unfreeze (field.hpp:341-347): later evaluations take exactly the pairs inside the cut-off
@@ -234,6 +236,7 @@ class Engine {
   std::vector<int> h_type_;
   std::vector<double> h_q_, h_mass_, h_eps_, h_sig_;   // per type pair
   std::vector<double> type_count_;
+  double charge_ = 0, charge2_ = 0, mass_ = 0;   // sums over the atoms: q, q^2, m
   std::vector<std::array<uint32_t, 2>> hb_;   // bonds (harmonic, then FENE) and their r0 (0: none), for constraints
   std::vector<double> hr0_;
   std::vector<std::array<uint32_t, 3>> ha_;   // angles and theta0, for rigid waters
@@ -313,6 +316,7 @@ class Engine {
   int* h_counters_ = nullptr;       // pinned
   long long* h_efix_ = nullptr;     // pinned
   double* h_edbl_ = nullptr;        // pinned
+  double* h_xf_ = nullptr;          // pinned: a host call's positions in and forces out (2 x 3 n)
 
   // PME
   int pk_[3] = {0, 0, 0}, ph1_ = 0;

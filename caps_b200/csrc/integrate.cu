@@ -2001,9 +2001,7 @@ struct MdRun {
     r.potential = t.bond + t.angle + t.dihedral + t.improper + t.vdw + t.coulomb;
     r.total = r.potential + r.kinetic;
     r.volume = E.dcell_.vol;
-    double mtot = 0;
-    for (double mm : E.h_mass_) mtot += mm;
-    r.density = mtot / kNA / (r.volume * 1e-24);
+    r.density = E.mass_ / kNA / (r.volume * 1e-24);
     r.pressure = (2 * r.kinetic + t.virial) / (3 * r.volume) * kAtm;
     for (int c = 0; c < 6; ++c) r.p[c] = (sc[kScKin0 + c] + t.w[c]) / r.volume * kAtm;
     if (S.nhc || mtk()) {
@@ -2029,10 +2027,8 @@ struct MdRun {
   void sync_scalars() {
     cudaStream_t stream_ = E.stream_;
     CK(cudaMemcpyAsync(S.h_sc, S.sc.p, sizeof(double) * kScNum, cudaMemcpyDeviceToHost, stream_));
-    CK(cudaMemcpyAsync(S.h_chain, S.chain.p, sizeof(Chain), cudaMemcpyDeviceToHost, stream_));
-    CK(cudaMemcpyAsync(E.h_counters_, E.d_counters_.p, sizeof(int) * kCntNum, cudaMemcpyDeviceToHost, stream_));
-    CK(cudaMemcpyAsync(E.h_efix_, E.d_efix_.p, sizeof(long long) * kENumSlots, cudaMemcpyDeviceToHost, stream_));
-    CK(cudaMemcpyAsync(E.h_edbl_, E.d_edbl_.p, sizeof(double) * kENumSlots, cudaMemcpyDeviceToHost, stream_));
+    if (S.nhc) CK(cudaMemcpyAsync(S.h_chain, S.chain.p, sizeof(Chain), cudaMemcpyDeviceToHost, stream_));
+    E.publish();
     CK(cudaStreamSynchronize(stream_));
     E.check_errors();
   }
@@ -2126,7 +2122,11 @@ struct MdRun {
     return mtk() || s % thermo_every == 0 || s == o.steps || frame_due(s) || checkpoint_due(s) || baro_due(s) || refill_due(s);
   }
 
-  void start();
+  // set-up to step 0: queued on the run's stream up to the first force, then finished (start() does both; a batch queues
+  // every replica before it waits for the first)
+  void start_queue();
+  void start_finish();
+  void start() { start_queue(), start_finish(); }
   // step s; stop: a stop was asked for before it (and s < steps), so the run ends after it
   void advance(long long s, bool stop = false);
   // steps s .. s + kBlockSteps - 1 are plain steps (no row, frame, checkpoint, cell rescaling or thermostat refill)
@@ -2139,7 +2139,7 @@ struct MdRun {
   void baro_step(long long s);
 };
 
-void MdRun::start() {
+void MdRun::start_queue() {
   cudaStream_t stream_ = E.stream_;
   Engine& e = E;
   const int n_ = E.n_;
@@ -2266,11 +2266,13 @@ void MdRun::start() {
   if (S.ncons) S.rattle(0);
   if (S.bussi) S.make_draws(1, draw_chunk(1));
 
-  // the first force, energies and virial; a list without room enough for the run is grown and built again
-  for (int attempt = 0;; ++attempt) {
-    S.forces(true, true);
-    if (attempt >= 3 || !E.grow_list_for_run()) break;
-  }
+  S.forces(true, true);   // the first force, energies and virial
+}
+
+void MdRun::start_finish() {
+  cudaStream_t stream_ = E.stream_;
+  // a list without room enough for the run is grown and built again
+  for (int attempt = 0; attempt < 3 && E.grow_list_for_run(); ++attempt) S.forces(true, true);
   if (S.ncons) {
     // step 0's constraint virial from one trial step on copies (dynamics.cpp:582-600)
     DevBuf<double>& xs = S.xs;
@@ -2626,8 +2628,9 @@ void run_batch(const std::vector<Engine*>& es, caps_gpu_state* const* states, co
   std::vector<std::unique_ptr<MdRun>> runs;
   for (size_t r = 0; r < R; ++r) {
     runs.emplace_back(new MdRun(*es[r], states[r], mds[r], progress, frame, users ? users[r] : nullptr));
-    runs.back()->start();
+    runs.back()->start_queue();
   }
+  for (auto& run : runs) run->start_finish();
   struct Res {
     cudaStream_t bs = nullptr;
     cudaEvent_t fork = nullptr, t0 = nullptr, t1 = nullptr;
@@ -2650,6 +2653,8 @@ void run_batch(const std::vector<Engine*>& es, caps_gpu_state* const* states, co
   res.ev.assign(R, nullptr);
   for (auto& e : res.ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   std::vector<int> seen(R, -1);
+  // one step to a graph: blocks of 2, 4 and 8 steps measured 232-235 us a step against 236 (six replicas of 2,064 to 16,512
+  // atoms), for 1 to 8 ms more to capture
   long long batch_kernels = 0, graph_nodes = 0;
   bool direct = true;
   for (size_t r = 0; r < R; ++r) direct = direct && runs[r]->S.direct();
@@ -2743,14 +2748,20 @@ void run_batch(const std::vector<Engine*>& es, caps_gpu_state* const* states, co
   const long long done = stopped_at >= 0 ? stopped_at : steps;
   for (size_t r = 0; r < R; ++r) {
     MdRun& M = *runs[r];
+    double* px = M.S.pinned_xv(M.n3);
+    CK(cudaMemcpyAsync(px, M.S.x.p, M.n3 * sizeof(double), cudaMemcpyDeviceToHost, M.E.stream_));
+    if (M.st->v) CK(cudaMemcpyAsync(px + M.n3, M.S.v.p, M.n3 * sizeof(double), cudaMemcpyDeviceToHost, M.E.stream_));
+  }
+  for (size_t r = 0; r < R; ++r) {
+    MdRun& M = *runs[r];
     Engine& E = M.E;
     M.sync_scalars();
     E.last_step_ms_ = done > 0 ? double(ms) / double(done) : 0.0;
     E.last_sps_ = done > 0 && ms > 0 ? double(done) / (ms * 1e-3) : 0.0;
     E.kernels_run_ = M.kernels + M.emits + (r == 0 ? batch_kernels : 0);
-    CK(cudaMemcpyAsync(M.st->x, M.S.x.p, M.n3 * sizeof(double), cudaMemcpyDeviceToHost, E.stream_));
-    if (M.st->v) CK(cudaMemcpyAsync(M.st->v, M.S.v.p, M.n3 * sizeof(double), cudaMemcpyDeviceToHost, E.stream_));
-    CK(cudaStreamSynchronize(E.stream_));
+    const double* px = M.S.pinned_xv(M.n3);   // copied above, before the scalars
+    std::memcpy(M.st->x, px, M.n3 * sizeof(double));
+    if (M.st->v) std::memcpy(M.st->v, px + M.n3, M.n3 * sizeof(double));
     std::memcpy(M.st->cell, E.cell_h_, sizeof E.cell_h_);
     M.completed = true;
   }

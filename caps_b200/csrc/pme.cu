@@ -153,15 +153,15 @@ void Engine::fft_passes(PmePath<R>& P, bool ener, bool vir) {
     return kernel;
   };
   const int gx = capped(blocks_for(size_t(nlx), P.lines[0]));
-  launch_k(allow(k_fft_x_fwd<R>, sx), gx, 128, sx, stream_, A, mixed_ ? nullptr : d_grid_.p, mixed_ ? d_gridq_.p : nullptr, P.h.p, P.plan[0], P.lines[0]);
+  launch_k(allow(k_fft_x_fwd<R>, sx), gx, kFftThreads, sx, stream_, A, mixed_ ? nullptr : d_grid_.p, mixed_ ? d_gridq_.p : nullptr, P.h.p, P.plan[0], P.lines[0]);
   const int gy = capped(blocks_for(size_t(ph1_), 1 << ly) * pk_[2]);
-  launch_k(allow(k_fft_y<R, false>, sy), gy, 128, sy, stream_, A, P.h.p, P.plan[1], ly);
+  launch_k(allow(k_fft_y<R, false>, sy), gy, kFftThreads, sy, stream_, A, P.h.p, P.plan[1], ly);
   const int gz = capped(blocks_for(size_t(ph1_), 1 << lz) * pk_[1]);
   EnergySink en{d_efix_.p, d_edbl_.p};
   auto* solve = ener ? (vir ? k_fft_z_solve<R, true, true> : k_fft_z_solve<R, true, false>) : (vir ? k_fft_z_solve<R, false, true> : k_fft_z_solve<R, false, false>);
-  launch_k(allow(solve, sz), gz, 128, sz, stream_, A, P.h.p, P.gt.p, P.wt.p, P.plan[2], lz, en, mixed_);
-  launch_k(allow(k_fft_y<R, true>, sy), gy, 128, sy, stream_, A, P.h.p, P.plan[1], ly);
-  launch_k(allow(k_fft_x_inv<R>, sx), gx, 128, sx, stream_, A, P.h.p, P.gr.p, P.plan[0], P.lines[0]);
+  launch_k(allow(solve, sz), gz, kFftThreads, sz, stream_, A, P.h.p, P.gt.p, P.wt.p, P.plan[2], lz, en, mixed_);
+  launch_k(allow(k_fft_y<R, true>, sy), gy, kFftThreads, sy, stream_, A, P.h.p, P.plan[1], ly);
+  launch_k(allow(k_fft_x_inv<R>, sx), gx, kFftThreads, sx, stream_, A, P.h.p, P.gr.p, P.plan[0], P.lines[0]);
 }
 
 // Autotuner for the line transforms: every block shape that fits (x: 1-8 pairs of lines per block; y, z: 1-16 consecutive

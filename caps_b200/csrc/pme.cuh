@@ -329,13 +329,15 @@ static __global__ void __launch_bounds__(kPmeThreads) k_spread(PmeArgs A, int pe
   }
 }
 
+// Block size of the line transforms. At 64 registers (FP32) two blocks fit an SM beside a pair grid one block short of full.
+constexpr int kFftThreads = 128;
 // Shared memory of the line-transform kernels: the twiddle table, then two buffers of the block's lines.
 // K-FFT-X forward: real lines (b, c) of length K1 to half spectra h(a, b, c), a <= K1/2; lines 2 m and 2 m + 1 are the real
 // and imaginary parts of one complex line, parted again in the spectrum by its symmetry. Input: g (FP64 path) or gq (mixed path, fixed),
 // cleared as it is read: the grid is zero for the next spread, with no launch of its own for it (as a memset node of the
 // step's graph it started up to 10 us after the step's drift, and the spread behind it). lpb: pairs of lines per block.
 template <class R>
-static __global__ void __launch_bounds__(128) k_fft_x_fwd(PmeArgs A, double* __restrict__ g, long long* __restrict__ gq,
+static __global__ void __launch_bounds__(kFftThreads) k_fft_x_fwd(PmeArgs A, double* __restrict__ g, long long* __restrict__ gq,
                                                           typename Cpx<R>::T* __restrict__ h, FftPlan<R> P, int lpb) {
   using T = typename Cpx<R>::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -376,7 +378,7 @@ static __global__ void __launch_bounds__(128) k_fft_x_fwd(PmeArgs A, double* __r
 
 // K-FFT-X inverse: half spectra back to real lines, two at a time (the missing halves by Hermitian symmetry).
 template <class R>
-static __global__ void __launch_bounds__(128) k_fft_x_inv(PmeArgs A, const typename Cpx<R>::T* __restrict__ h, R* __restrict__ gr, FftPlan<R> P, int lpb) {
+static __global__ void __launch_bounds__(kFftThreads) k_fft_x_inv(PmeArgs A, const typename Cpx<R>::T* __restrict__ h, R* __restrict__ gr, FftPlan<R> P, int lpb) {
   using T = typename Cpx<R>::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ls = A.k1 | 1;
@@ -411,7 +413,7 @@ static __global__ void __launch_bounds__(128) k_fft_x_inv(PmeArgs A, const typen
 
 // K-FFT-Y: lines along b for fixed (a, c); a block takes 1 << lsh consecutive a (coalesced rows) of one c.
 template <class R, bool INV>
-static __global__ void __launch_bounds__(128) k_fft_y(PmeArgs A, typename Cpx<R>::T* __restrict__ h, FftPlan<R> P, int lsh) {
+static __global__ void __launch_bounds__(kFftThreads) k_fft_y(PmeArgs A, typename Cpx<R>::T* __restrict__ h, FftPlan<R> P, int lsh) {
   using T = typename Cpx<R>::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int la = 1 << lsh;
@@ -441,7 +443,7 @@ static __global__ void __launch_bounds__(128) k_fft_y(PmeArgs A, typename Cpx<R>
 // K-FFT-Z+SOLVE: lines along c for fixed (a, b): forward transform, energy and virial of the half spectrum (e_m doubled
 // for 0 < a < K1/2), multiply by G, inverse transform, in one pass.
 template <class R, bool ENER, bool VIR>
-static __global__ void __launch_bounds__(128) k_fft_z_solve(PmeArgs A, typename Cpx<R>::T* __restrict__ h, const R* __restrict__ gt,
+static __global__ void __launch_bounds__(kFftThreads) k_fft_z_solve(PmeArgs A, typename Cpx<R>::T* __restrict__ h, const R* __restrict__ gt,
                                                             const R* __restrict__ wt, FftPlan<R> P, int lsh, EnergySink en, int fixed) {
   using T = typename Cpx<R>::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];

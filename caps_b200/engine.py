@@ -271,7 +271,7 @@ class Evaluator:
     def compute(self, x, cell) -> tuple[dict, np.ndarray]:
         x = np.ascontiguousarray(np.asarray(x, dtype=np.float64).reshape(-1))
         c = cell_array(cell)
-        f = np.zeros_like(x)
+        f = np.empty_like(x)   # the call writes all of it, or raises
         t = _abi.Terms()
         self._check(self.lib.caps_gpu_compute(self.h, x.ctypes.data_as(C.c_void_p), c.ctypes.data_as(C.c_void_p),
                                               f.ctypes.data_as(C.c_void_p), C.byref(t)))
