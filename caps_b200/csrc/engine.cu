@@ -570,11 +570,15 @@ void Engine::set_cell(const double* cell) {
   g.nv = std::clamp(int(g.w[1] / side), 1, 1024);
   g.ncol = g.nu * g.nv;
   g.rlist = rc_ + skin_;
-  g.rlist2 = g.rlist * g.rlist;
+  // wrapped coordinates lie within the cell: rounded to float, and shifted by an image, they are off by a few ulps of its size
+  double span = 0;
+  for (int k = 0; k < 12; ++k) span += std::fabs(cell[k]);
+  const double reach = g.rlist + 1e-3 + 1e-6 * span;
+  g.reach2 = float(reach * reach);
   g.ru = int(std::floor(g.rlist * g.nu / g.w[0])) + 1;
   g.rv = int(std::floor(g.rlist * g.nv / g.w[1])) + 1;
   g.rq = int(std::ceil(g.rlist / g.w[2])) + 1;
-  g.dw = g.rlist / g.w[2];
+  g.dw = (g.rlist + 1e-3) / g.w[2];   // the columns are sorted by c in units of 2^-32 of the cell
   if (!tuning_pinned_ && !frozen_) batch_ = list_depth(g);
   g.batch = batch_;
   // periodic images in range along each axis: 2 ceil(r_list / w) + 1 for the perpendicular width w (the reference counts
@@ -646,7 +650,7 @@ void Engine::ensure_list_capacity() {
     d_sc_col_.alloc(size_t(nsc_cap_));
     d_sc_z_.alloc(size_t(2) * nsc_cap_);
     d_sc_org_.alloc(size_t(3) * nsc_cap_);
-    d_cl_box_.alloc(size_t(6) * 8 * nsc_cap_);
+    d_cl_box_.alloc(size_t(2) * 8 * nsc_cap_);
     d_cl_real_.alloc(size_t(8) * nsc_cap_);
     d_perm_.alloc(ns);
     d_xq_.alloc(ns);

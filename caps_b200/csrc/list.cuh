@@ -1,5 +1,5 @@
 // K-LIST: everything between a step's drift and its pair kernel in one launch: the gated list build (bin, scan, scatter,
-// column sort with the super-clusters, search), the packed positions and the gated dynamic prune.
+// column sort, super-clusters, search), the packed positions and the gated dynamic prune.
 //
 // A step without a build or a prune (about three in four at 500 K) only packs: the blocks stride over the slots and
 // leave. On the others the work is cut into units, numbered in the order of the stages, and every block takes the next
@@ -16,7 +16,7 @@
 
 namespace capsb {
 
-enum ListStage { kStBin = 0, kStScan, kStScatter, kStSort, kStSearch, kStPack, kStNum };
+enum ListStage { kStBin = 0, kStScan, kStScatter, kStSort, kStSuper, kStSearch, kStPack, kStNum };
 static_assert(kStNum == kCntNum - kCntStage, "a counter per stage");
 constexpr int kListSpin = 1 << 21;   // polls (with a pause of about 0.1 us each) before a wait gives up
 
@@ -77,90 +77,92 @@ __device__ __forceinline__ void pack_slot(const ListArgs& L, int s, int nsc, boo
   L.tslot[s] = L.type[a];
 }
 
-struct PruneShared {   // per warp: a work item's i atoms, its entries' j atoms (w: 1 real, 0 padding), the new half masks
-  float4 xi[kListThreads / 32][64];
+struct PruneShared {   // per warp: its entries' j atoms (x, y, z, (|x|^2 - r_prune^2) / 2) from the work item's origin
   float4 xj[kListThreads / 32][kBatch * 8];
-  unsigned keep[kListThreads / 32][kBatch];
+  float4 sh[kListThreads / 32][kBatch];   // the entries' shifts, and their j clusters
 };
 
 // Dynamic pruning (as core/src/nbnxm.cpp:328-363 does on the CPU), a warp per work item w: each entry's mask is rewritten
 // to the (i cluster, j half) pairs with at least one atom pair inside r_prune = r_c + b at the present positions; the pair
 // kernels read that mask. The j halves are the cluster's lower-x and upper-x four atoms (the cluster split orders its
 // atoms along x), so a half mask drops the far half of a j cluster that reaches an i cluster with its near half only.
-// Pruned again once an atom has moved b/2 since the last prune, so no pair inside r_c is lost. FP32 path: packed float
-// positions; FP64 path: packed double positions.
+// Pruned again once an atom has moved b/2 since the last prune, so no pair inside r_c is lost.
+//
+// Bound by issue. A lane keeps its eight i atoms in registers and tests them against its two j atoms of an entry without a
+// branch, as x_i x_j - |x_i|^2 / 2 > (|x_j|^2 - r^2) / 2, positions from the work item's origin (three multiply-adds and a
+// compare per pair; the squares a millionth low and r^2 0.02 Å^2 high, so that rounding only ever keeps a pair); one
+// reduction over the warp per entry. Branches and two votes per
+// i cluster took 54 us for 45 million listed pairs, a box test before them 57.
 template <bool DBL>
 __device__ void prune_item(const ListArgs& L, int w, PruneShared& S) {
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i8 = lane & 7, jq = lane >> 3;
-  const float rp2 = float(L.rprune2);
+  const float rp2 = float(L.rprune2) + 0.02f;
   const int4 wk = L.b.work[w];
   const int sc = wk.x;
   const int ne = min(wk.z, kBatch);
-  // one batch of independent loads: i atoms, the entries, then every entry's 8 j atoms with the entry's image shift
   uint4 en = make_uint4(0u, 0u, 0u, 0u);
-  float sx = 0.f, sy = 0.f, sz = 0.f;
-  if (lane < ne) {
-    en = L.b.ent[wk.y + lane];
-    if (DBL) {
-      int qa, qb, qc;
-      unpack_image(en.y >> 8, qa, qb, qc);
-      sx = float(L.cell.h[0][0] * qa + L.cell.h[0][1] * qb + L.cell.h[0][2] * qc);
-      sy = float(L.cell.h[1][0] * qa + L.cell.h[1][1] * qb + L.cell.h[1][2] * qc);
-      sz = float(L.cell.h[2][0] * qa + L.cell.h[2][1] * qb + L.cell.h[2][2] * qc);
-    } else {
-      const float4 sh = L.b.ent_shift[wk.y + lane];
-      sx = sh.x, sy = sh.y, sz = sh.z;
-    }
-  }
-  // FP64 path: absolute positions rounded to float (1e-5 Å at 100 Å), far inside the 0.8 Å prune margin
+  if (lane < ne) en = L.b.ent[wk.y + lane];
+  // positions from the super-cluster's origin (FP32 path: packed so) or first atom (FP64 path: slot 0 is always real)
+  double4 o = make_double4(0, 0, 0, 0);
+  if (DBL) o = L.xqd[64 * sc];
   auto at = [&](int s) {
     float4 v;
     if (DBL) {
       const double4 d = L.xqd[s];
-      v = make_float4(float(d.x), float(d.y), float(d.z), 0.f);
+      v = make_float4(float(d.x - o.x), float(d.y - o.y), float(d.z - o.z), 0.f);
     } else {
       v = L.xq[s];
     }
-    v.w = L.tslot[s] != L.pad_type ? 1.f : 0.f;
     return v;
   };
-  for (int t = lane; t < 64; t += 32) S.xi[wib][t] = at(64 * sc + t);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const int t = lane + 32 * k;   // entry t / 8, j atom t % 8
-    const int e = t >> 3;
-    const unsigned cj = __shfl_sync(0xffffffffu, en.x, e & 31);
-    const float ex = __shfl_sync(0xffffffffu, sx, e & 31), ey = __shfl_sync(0xffffffffu, sy, e & 31), ez = __shfl_sync(0xffffffffu, sz, e & 31);
-    if (e < ne) {
-      float4 v = at(8 * int(cj) + (t & 7));
-      v.x += ex, v.y += ey, v.z += ez;
-      S.xj[wib][t] = v;
+  if (lane < ne) {
+    float4 sh;
+    if (DBL) {
+      int qa, qb, qc;
+      unpack_image(en.y >> 8, qa, qb, qc);
+      sh = make_float4(float(L.cell.h[0][0] * qa + L.cell.h[0][1] * qb + L.cell.h[0][2] * qc), float(L.cell.h[1][0] * qa + L.cell.h[1][1] * qb + L.cell.h[1][2] * qc),
+                       float(L.cell.h[2][0] * qa + L.cell.h[2][1] * qb + L.cell.h[2][2] * qc), 0.f);
+    } else {
+      sh = L.b.ent_shift[wk.y + lane];
     }
+    sh.w = __int_as_float(int(en.x));
+    S.sh[wib][lane] = sh;
+  }
+  float xi[8], yi[8], zi[8], hi[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const int s = 64 * sc + 8 * c + i8;
+    const float4 v = at(s);
+    xi[c] = v.x, yi[c] = v.y, zi[c] = v.z;
+    hi[c] = L.tslot[s] != L.pad_type ? -0.4999995f * (v.x * v.x + v.y * v.y + v.z * v.z) : -1e30f;   // padding is never near
   }
   __syncwarp();
+  for (int t = lane; t < 8 * ne; t += 32) {   // entry t / 8, j atom t % 8
+    const float4 sh = S.sh[wib][t >> 3];
+    const int s = 8 * __float_as_int(sh.w) + (t & 7);
+    float4 v = at(s);
+    v.x += sh.x, v.y += sh.y, v.z += sh.z;
+    v.w = L.tslot[s] != L.pad_type ? 0.4999995f * (v.x * v.x + v.y * v.y + v.z * v.z) - 0.5f * rp2 : 1e30f;
+    S.xj[wib][t] = v;
+  }
+  __syncwarp();
+  unsigned mine = 0;   // lane e: entry e's new mask
   for (int el = 0; el < ne; ++el) {
-    const unsigned built = __shfl_sync(0xffffffffu, en.y, el) & 255u;
     const float4 a0 = S.xj[wib][8 * el + jq], a1 = S.xj[wib][8 * el + jq + 4];
     unsigned keep = 0;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      if (!((built >> c) & 1u)) continue;
-      const float4 xi = S.xi[wib][8 * c + i8];
-#pragma unroll
-      for (int jj = 0; jj < 2; ++jj) {
-        const float4 xj = jj ? a1 : a0;
-        const float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        const bool in = xi.w != 0.f && xj.w != 0.f && r2 < rp2;
-        if (__any_sync(0xffffffffu, in)) keep |= 1u << (c + 8 * jj);
-      }
+      const float d0 = fmaf(xi[c], a0.x, fmaf(yi[c], a0.y, fmaf(zi[c], a0.z, hi[c])));
+      const float d1 = fmaf(xi[c], a1.x, fmaf(yi[c], a1.y, fmaf(zi[c], a1.z, hi[c])));
+      if (d0 > a0.w) keep |= 1u << c;
+      if (d1 > a1.w) keep |= 256u << c;
     }
-    if (lane == 0) S.keep[wib][el] = keep;
+    keep = __reduce_or_sync(0xffffffffu, keep);
+    if (lane == el) mine = keep;
   }
-  __syncwarp();
   if (lane < ne) {
-    en.w = S.keep[wib][lane];
+    en.w = mine & ((en.y & 255u) * 0x101u);
     L.b.ent[wk.y + lane] = en;
   }
   __syncwarp();
@@ -217,8 +219,8 @@ static __global__ void __launch_bounds__(kListThreads, 4) k_list(ListArgs L) {
   }
   // units of each stage; the prune's are the grid's blocks, striding over the work items
   const int nbin = built ? (L.n + kListThreads - 1) / kListThreads : 0;
-  const int nsort = built ? L.g.ncol : 0, nsearch = built ? L.b.nsc_cap : 0;
-  const int e_bin = nbin, e_scat = e_bin + nbin, e_sort = e_scat + nsort, e_search = e_sort + nsearch, e_pack = e_search + npack;
+  const int nsort = built ? L.g.ncol : 0, nsuper = built ? (L.b.nsc_cap + kScWarps - 1) / kScWarps : 0, nsearch = built ? L.b.nsc_cap : 0;
+  const int e_bin = nbin, e_scat = e_bin + nbin, e_sort = e_scat + nsort, e_super = e_sort + nsuper, e_search = e_super + nsearch, e_pack = e_search + npack;
   const int total = e_pack + int(gridDim.x);
   for (;;) {
     __syncthreads();
@@ -242,16 +244,20 @@ static __global__ void __launch_bounds__(kListThreads, 4) k_list(ListArgs L) {
       list_done(cnt, kStScatter);
     } else if (t < e_sort) {
       if (!list_wait(cnt, kStScatter, nbin, &s_ok)) break;
-      sort_column(t - e_scat, L.cell, L.b, S.sort);
+      sort_column(t - e_scat, L.b, S.sort);
       list_done(cnt, kStSort);
-    } else if (t < e_search) {
+    } else if (t < e_super) {
       if (!list_wait(cnt, kStSort, nsort, &s_ok)) break;
-      const int sc = t - e_sort;
+      super_unit(t - e_sort, L.cell, L.b);
+      list_done(cnt, kStSuper);
+    } else if (t < e_search) {
+      if (!list_wait(cnt, kStSuper, nsuper, &s_ok)) break;
+      const int sc = t - e_super;
       if (sc < min(L.b.counters[kCntNsc], L.b.nsc_cap)) search_supercluster(sc, L.cell, L.g, L.excl_off, L.excl_list, L.b, S.search);
       list_done(cnt, kStSearch);
     } else if (t < e_pack) {
-      // the pack reads the order the sort made; it runs beside the last of the search
-      if (built && !list_wait(cnt, kStSort, nsort, &s_ok)) break;
+      // the pack reads the slots that the super-clusters' stage made; it runs beside the last of the search
+      if (built && !list_wait(cnt, kStSuper, nsuper, &s_ok)) break;
       const int u = t - e_search;
       if (u == 0 && threadIdx.x == 0) {
         cnt[kCntPairNext] = 0;

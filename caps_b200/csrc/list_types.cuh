@@ -15,7 +15,8 @@ struct ListGeom {
   int nu, nv, ncol;
   int ru, rv, rq;
   double w[3];        // perpendicular widths of the cell
-  double rlist, rlist2;
+  double rlist;
+  float reach2;       // the search's squared radius: rlist and what the float boxes may be off by
   double dw;          // rlist / w[2]
   int batch;          // entries per work item (the pair kernels' j-tile depth), at most kBatch (Engine::list_depth)
 };
@@ -37,7 +38,7 @@ struct ListBufs {
   double* sc_z;       // 2 per sc: fractional c range
   double* sc_org;     // 3 per sc: origin (centre of its bounding box)
   // per cluster
-  double* cl_box;     // 6 per cluster: lo xyz, hi xyz (wrapped Cartesian)
+  float4* cl_box;     // 2 per cluster: lo xyz, hi xyz at the build (wrapped Cartesian)
   unsigned char* cl_real;   // 8-bit mask of real atoms
   // per slot
   int* perm;
@@ -58,7 +59,7 @@ struct ListBufs {
 enum Counter { kCntEnt = 0, kCntWork, kCntMask, kCntErr, kCntRebuild, kCntNsc, kCntMaxCol, kCntPrune, kCntBuilds, kCntPrunes, kCntPairNext,
                kCntFeneClaim, kCntNanClaim,   // *Claim: 1 once the first failure of that kind left its details
                // k_list: the next unit of work, the blocks that left, and the finished units of each stage
-               kCntTicket, kCntLeft, kCntStage, kCntNum = kCntStage + 6 };
+               kCntTicket, kCntLeft, kCntStage, kCntNum = kCntStage + 7 };
 
 __device__ __forceinline__ void raise_error(int* counters, unsigned bit) { atomicOr(reinterpret_cast<unsigned*>(counters + kCntErr), bit); }
 

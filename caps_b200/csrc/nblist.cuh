@@ -24,41 +24,42 @@ static __global__ void k_check_step(int n, const double* __restrict__ x, ListChe
   list_check_flags(L, mb, mp);
 }
 
-// K-SCAN (one block, NT threads): column starts, super-cluster starts (64 atoms each, the last one of a column
+// Scan stage (one block, NT threads): column starts, super-cluster starts (64 atoms each, the last one of a column
 // partial), and the column of every super-cluster. Also resets the list counters for the search. The column counts are
 // read through L2 (the other blocks of the binning made them with atomics).
 template <int NT>
 __device__ void scan_columns(const ListGeom& g, const ListBufs& b) {
-  __shared__ int s_a[NT], s_s[NT];
-  __shared__ int carry_a, carry_s, s_max;
-  if (threadIdx.x == 0) carry_a = carry_s = s_max = 0;
+  __shared__ int s_a[NT / 32], s_s[NT / 32];
+  __shared__ int s_max;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int carry_a = 0, carry_s = 0;
+  if (threadIdx.x == 0) s_max = 0;
   __syncthreads();
   for (int base = 0; base < g.ncol; base += NT) {
     const int c = base + threadIdx.x;
     const int cnt = c < g.ncol ? __ldcg(b.col_count + c) : 0;
     if (c < g.ncol) b.col_count[c] = 0;   // cleared for the next build's binning
-    if (c < g.ncol) atomicMax(&s_max, cnt);
-    s_a[threadIdx.x] = cnt;
-    s_s[threadIdx.x] = (cnt + kScAtoms - 1) / kScAtoms;
+    if (cnt) atomicMax(&s_max, cnt);
+    int a = cnt, sc = (cnt + kScAtoms - 1) / kScAtoms;   // inclusive scans of both, by warp and then over the warps
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int ta = __shfl_up_sync(0xffffffffu, a, o), ts = __shfl_up_sync(0xffffffffu, sc, o);
+      if (lane >= o) a += ta, sc += ts;
+    }
+    if (lane == 31) s_a[warp] = a, s_s[warp] = sc;
     __syncthreads();
-    for (int off = 1; off < NT; off <<= 1) {   // inclusive Hillis-Steele scan
-      const int ta = threadIdx.x >= unsigned(off) ? s_a[threadIdx.x - off] : 0;
-      const int ts = threadIdx.x >= unsigned(off) ? s_s[threadIdx.x - off] : 0;
-      __syncthreads();
-      s_a[threadIdx.x] += ta;
-      s_s[threadIdx.x] += ts;
-      __syncthreads();
+    int tot_a = 0, tot_s = 0;
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) {
+      if (w < warp) a += s_a[w], sc += s_s[w];
+      tot_a += s_a[w], tot_s += s_s[w];
     }
     if (c < g.ncol) {
-      b.col_start[c + 1] = carry_a + s_a[threadIdx.x];
-      b.col_sc[c + 1] = carry_s + s_s[threadIdx.x];
+      b.col_start[c + 1] = carry_a + a;
+      b.col_sc[c + 1] = carry_s + sc;
       b.col_fill[c] = 0;
     }
-    __syncthreads();
-    if (threadIdx.x == NT - 1) {
-      carry_a += s_a[threadIdx.x];
-      carry_s += s_s[threadIdx.x];
-    }
+    carry_a += tot_a, carry_s += tot_s;
     __syncthreads();
   }
   if (threadIdx.x == 0) {
@@ -114,157 +115,165 @@ __device__ __forceinline__ void scatter_atom(int n, int i, const ListBufs& b) {
   b.order[b.col_start[c] + base + __popc(same & ((1u << lane) - 1))] = i;
 }
 
-// K-SUPER (a warp per super-cluster, inside the sort of its column): the 2 x 2 x 2 split into clusters, perm / iperm,
-// cluster boxes and real-atom masks, the super-cluster's origin and its c range. Lane l holds atoms l (lower c half) and
-// l + 32 (upper c half): the ranks along y and x come from shuffles, the boxes from butterfly reductions over the 8 lanes
-// of a cluster. s_w and s_a: the warp's world positions and atoms by local slot (-1 padding).
-__device__ void form_supercluster(const DevCell& cell, const ListBufs& b, int sc, int c, int lane, double (*s_w)[3], int* s_a) {
-  const unsigned full = 0xffffffffu;
-  {
-    const int k = sc - b.col_sc[c];
-    const int s0 = b.col_start[c] + kScAtoms * k;
-    const int m = min(kScAtoms, b.col_start[c + 1] - s0);
-    if (m <= 0) {   // not made by the scan (every super-cluster holds at least one atom); kept empty
-      b.perm[64 * sc + lane] = b.perm[64 * sc + lane + 32] = -1;
-      return;
-    }
-    int id[2];
-    double fx[2], fy[2], w[2][3];
+// One compare-exchange of a bitonic network over the lanes: the pair (lane, lane ^ j) ascending where up.
+__device__ __forceinline__ void lane_exchange(float& key, int& id, int j, bool up) {
+  const float k = __shfl_xor_sync(0xffffffffu, key, j);
+  const int i = __shfl_xor_sync(0xffffffffu, id, j);
+  const bool low = (threadIdx.x & j) == 0;   // the pair's lower lane keeps the smaller key
+  if (low == up ? k < key : k > key) key = k, id = i;
+}
+// Sorts key (and id) over groups of N lanes, ascending. Deterministic: the network's exchanges depend on the keys alone.
+template <int N>
+__device__ __forceinline__ void lane_sort(float& key, int& id) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int t = lane + 32 * h;
-      id[h] = -1;
-      fx[h] = fy[h] = 0;
-      w[h][0] = w[h][1] = w[h][2] = 0;
-      if (t < m) {
-        const int a = b.order[s0 + t];
-        id[h] = a;
-        const double f0 = b.frac[3 * a], f1 = b.frac[3 * a + 1], f2 = b.frac[3 * a + 2];
-        fx[h] = f0, fy[h] = f1;
-        for (int r = 0; r < 3; ++r) w[h][r] = cell.o[r] + cell.h[r][0] * f0 + cell.h[r][1] * f1 + cell.h[r][2] * f2;
-      }
-      s_a[t] = -1;
-    }
-    // rank along y within the c half, then along x within the y half of the c half (ties by atom index)
-    int ry[2] = {0, 0}, rx[2] = {0, 0};
-    for (int u = 0; u < 32; ++u) {
+  for (int kk = 2; kk <= N; kk <<= 1)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const double yu = __shfl_sync(full, fy[h], u);
-        const int iu = __shfl_sync(full, id[h], u);
-        ry[h] += (u + 32 * h < m) && (yu < fy[h] || (yu == fy[h] && iu < id[h]));
-      }
-    }
-    for (int u = 0; u < 32; ++u) {
+    for (int j = kk >> 1; j > 0; j >>= 1) lane_exchange(key, id, j, kk == N || (lane & kk) == 0);
+}
+
+// K-SUPER (a warp per super-cluster): the 2 x 2 x 2 split into clusters, perm / iperm, cluster boxes and real-atom masks,
+// the super-cluster's origin and its c range. Lane l holds atoms l (lower c half) and l + 32 (upper c half), sorted along b
+// over the warp and then along a over each half of it, which leaves slot 32 h + l in lane l; padding sorts last. (Ranks by
+// comparing with every other atom took some 2,600 instructions of one warp: 17 us a build at any size.)
+__device__ void form_supercluster(const DevCell& cell, const ListBufs& b, int sc, int c, int lane) {
+  const int k = sc - b.col_sc[c];
+  const int s0 = b.col_start[c] + kScAtoms * k;
+  const int m = min(kScAtoms, b.col_start[c + 1] - s0);
+  if (m <= 0) {   // not made by the scan (every super-cluster holds at least one atom); kept empty
+    b.perm[64 * sc + lane] = b.perm[64 * sc + lane + 32] = -1;
+    return;
+  }
+  const int first = b.order[s0], last = b.order[s0 + m - 1];
+  int id[2];
+  float key[2];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const double xu = __shfl_sync(full, fx[h], u);
-        const int iu = __shfl_sync(full, id[h], u);
-        const int qu = __shfl_sync(full, ry[h] >> 4, u);
-        rx[h] += (u + 32 * h < m) && qu == (ry[h] >> 4) && (xu < fx[h] || (xu == fx[h] && iu < id[h]));
-      }
-    }
-    __syncwarp();
+  for (int h = 0; h < 2; ++h) {
+    const int t = lane + 32 * h;
+    id[h] = t < m ? b.order[s0 + t] : -1;
+    key[h] = id[h] >= 0 ? float(b.frac[3 * id[h] + 1]) : 3.f;   // fractional coordinates are below 1
+  }
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (lane + 32 * h >= m) continue;
-      const int slot = 8 * (4 * h + 2 * (ry[h] >> 4) + (rx[h] >> 3)) + (rx[h] & 7);
-      s_a[slot] = id[h];
-      for (int r = 0; r < 3; ++r) s_w[slot][r] = w[h][r];
-      b.iperm[id[h]] = 64 * sc + slot;
-    }
-    __syncwarp();
-    // cluster boxes and real masks: slot lane + 32 h belongs to cluster (lane >> 3) + 4 h
-    double slo[3] = {1e300, 1e300, 1e300}, shi[3] = {-1e300, -1e300, -1e300};
+  for (int h = 0; h < 2; ++h) lane_sort<32>(key[h], id[h]);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int t = lane + 32 * h;
-      const int a = s_a[t];
-      b.perm[64 * sc + t] = a;
-      double lo[3], hi[3];
+  for (int h = 0; h < 2; ++h) {
+    key[h] = id[h] >= 0 ? float(b.frac[3 * id[h]]) : 3.f;
+    lane_sort<16>(key[h], id[h]);
+  }
+  // cluster boxes and real masks: slot lane + 32 h belongs to cluster (lane >> 3) + 4 h. The origin, which the packed
+  // positions are rounded from, is the middle of the atoms' own extent, in double.
+  double slo[3] = {1e300, 1e300, 1e300}, shi[3] = {-1e300, -1e300, -1e300};
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int a = id[h];
+    b.perm[64 * sc + lane + 32 * h] = a;
+    float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
+    if (a >= 0) {
+      b.iperm[a] = 64 * sc + lane + 32 * h;
+      const double f0 = b.frac[3 * a], f1 = b.frac[3 * a + 1], f2 = b.frac[3 * a + 2];
       for (int r = 0; r < 3; ++r) {
-        lo[r] = a >= 0 ? s_w[t][r] : 1e300;
-        hi[r] = a >= 0 ? s_w[t][r] : -1e300;
+        const double p = cell.o[r] + cell.h[r][0] * f0 + cell.h[r][1] * f1 + cell.h[r][2] * f2;
+        lo[r] = hi[r] = float(p);
+        slo[r] = fmin(slo[r], p), shi[r] = fmax(shi[r], p);
       }
-#pragma unroll
-      for (int o = 1; o < 8; o <<= 1)
-        for (int r = 0; r < 3; ++r) {
-          lo[r] = fmin(lo[r], __shfl_xor_sync(full, lo[r], o));
-          hi[r] = fmax(hi[r], __shfl_xor_sync(full, hi[r], o));
-        }
-      const unsigned real = __ballot_sync(full, a >= 0);
-      if ((lane & 7) == 0) {
-        const int cg = 8 * sc + (lane >> 3) + 4 * h;
-        for (int r = 0; r < 3; ++r) b.cl_box[6 * cg + r] = lo[r], b.cl_box[6 * cg + 3 + r] = hi[r];
-        b.cl_real[cg] = (unsigned char)((real >> (lane & 24)) & 255u);
-      }
-      for (int r = 0; r < 3; ++r) slo[r] = fmin(slo[r], lo[r]), shi[r] = fmax(shi[r], hi[r]);
     }
 #pragma unroll
-    for (int o = 8; o < 32; o <<= 1)
+    for (int o = 1; o < 8; o <<= 1)
       for (int r = 0; r < 3; ++r) {
-        slo[r] = fmin(slo[r], __shfl_xor_sync(full, slo[r], o));
-        shi[r] = fmax(shi[r], __shfl_xor_sync(full, shi[r], o));
+        lo[r] = fminf(lo[r], __shfl_xor_sync(0xffffffffu, lo[r], o));
+        hi[r] = fmaxf(hi[r], __shfl_xor_sync(0xffffffffu, hi[r], o));
       }
-    const int last = m - 1;
-    const int id_first = __shfl_sync(full, id[0], 0);
-    const int id_last = __shfl_sync(full, (last >> 5) ? id[1] : id[0], last & 31);
-    if (lane == 0) {
-      for (int r = 0; r < 3; ++r) b.sc_org[3 * sc + r] = 0.5 * (slo[r] + shi[r]);
-      b.sc_z[2 * sc] = b.frac[3 * id_first + 2];
-      b.sc_z[2 * sc + 1] = b.frac[3 * id_last + 2];
+    const unsigned real = __ballot_sync(0xffffffffu, a >= 0);
+    if ((lane & 7) == 0) {
+      const int cg = 8 * sc + (lane >> 3) + 4 * h;
+      b.cl_box[2 * cg] = make_float4(lo[0], lo[1], lo[2], 0.f);   // an empty cluster: lo above every hi
+      b.cl_box[2 * cg + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
+      b.cl_real[cg] = (unsigned char)((real >> (lane & 24)) & 255u);
     }
-    __syncwarp();
+  }
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1)
+    for (int r = 0; r < 3; ++r) {
+      slo[r] = fmin(slo[r], __shfl_xor_sync(0xffffffffu, slo[r], o));
+      shi[r] = fmax(shi[r], __shfl_xor_sync(0xffffffffu, shi[r], o));
+    }
+  if (lane == 0) {
+    for (int r = 0; r < 3; ++r) b.sc_org[3 * sc + r] = 0.5 * (slo[r] + shi[r]);
+    b.sc_z[2 * sc] = b.frac[3 * first + 2];
+    b.sc_z[2 * sc + 1] = b.frac[3 * last + 2];
   }
 }
 
-// Sort stage (a block per column): atoms by fractional c, ties by index, then the column's super-clusters (K-SUPER). A
-// bitonic sorting network in shared memory over the column padded to a power of two (pad keys sort last):
-// log2(n)(log2(n)+1)/2 compare-exchange rounds, one barrier each. smem_raw: kSortMax keys and ids.
-constexpr int kScWarps = kListThreads / 32;   // the block's warps form the column's super-clusters
-constexpr size_t kSortSmem = size_t(kSortMax) * (sizeof(double) + sizeof(int));
-static_assert(sizeof(double) * 3 * 64 * kScWarps + sizeof(int) * 64 * kScWarps <= kSortSmem, "the super-cluster stage fits the sort's shared memory");
-__device__ void sort_column(int c, const DevCell& cell, const ListBufs& b, unsigned char* smem_raw) {
-  const int nsc = min(b.counters[kCntNsc], b.nsc_cap);
-  double* key = reinterpret_cast<double*>(smem_raw);
-  int* id = reinterpret_cast<int*>(key + kSortMax);
+// Sort stage (a block per column): atoms by fractional c, ties by index, as one 64-bit key each (c in units of 2^-32 of the
+// cell, the index). Runs of 32 are sorted by the lanes of a warp, then runs are merged in pairs: every key finds its place
+// among the sibling run's by binary search. Columns past kSortMax / 2, whose second buffer has no room, take a bitonic
+// network in place (55 rounds with a barrier each took 40 us for columns of 650 atoms).
+constexpr size_t kSortSmem = size_t(kSortMax) * sizeof(unsigned long long);
+__device__ void sort_column(int c, const ListBufs& b, unsigned char* smem_raw) {
+  using Key = unsigned long long;
+  Key* A = reinterpret_cast<Key*>(smem_raw);
   const int s0 = b.col_start[c], n = min(b.col_start[c + 1] - s0, kSortMax);
-  int np = 1;
-  while (np < n) np <<= 1;
-  for (int k = threadIdx.x; k < np; k += blockDim.x) {
-    if (k < n) {
-      const int a = b.order[s0 + k];
-      id[k] = a;
-      key[k] = b.frac[3 * a + 2];
-    } else {
-      id[k] = 0x7fffffff;
-      key[k] = 2.0;   // fractional coordinates are below 1
-    }
-  }
-  __syncthreads();
-  for (int kk = 2; kk <= np; kk <<= 1)
-    for (int j = kk >> 1; j > 0; j >>= 1) {
-      for (int t = threadIdx.x; t < (np >> 1); t += blockDim.x) {
-        const int lo = 2 * (t & ~(j - 1)) + (t & (j - 1)), hi = lo + j;
-        const double ka = key[lo], kb = key[hi];
-        const int ia = id[lo], ib = id[hi];
-        const bool gt = ka > kb || (ka == kb && ia > ib);
-        if (gt == ((lo & kk) == 0)) {
-          key[lo] = kb, key[hi] = ka;
-          id[lo] = ib, id[hi] = ia;
+  auto key_of = [&](int k) {
+    const int a = b.order[s0 + k];
+    return (Key(unsigned(b.frac[3 * a + 2] * 4294967296.0)) << 32) | unsigned(a);   // fractional coordinates are below 1 - 1e-12
+  };
+  if (n <= kSortMax / 2) {
+    Key* B = A + kSortMax / 2;
+    const int lane = threadIdx.x & 31;
+    for (int k0 = (threadIdx.x >> 5) * 32; k0 < n; k0 += kListThreads) {
+      Key key = k0 + lane < n ? key_of(k0 + lane) : ~0ull;
+#pragma unroll
+      for (int kk = 2; kk <= 32; kk <<= 1)
+#pragma unroll
+        for (int j = kk >> 1; j > 0; j >>= 1) {
+          const Key o = __shfl_xor_sync(0xffffffffu, key, j);
+          const bool low = (lane & j) == 0, up = kk == 32 || (lane & kk) == 0;
+          if (low == up ? o < key : o > key) key = o;
         }
+      if (k0 + lane < n) A[k0 + lane] = key;
+    }
+    __syncthreads();
+    for (int ws = 5; (1 << ws) < n; ++ws) {
+      const int width = 1 << ws;
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const Key key = A[i];
+        const int run = i >> ws, sib = (run ^ 1) << ws;
+        int lo = sib, hi = min(sib + width, n);   // the sibling's first key above this one (keys are distinct)
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (A[mid] < key) lo = mid + 1;
+          else hi = mid;
+        }
+        B[((run & ~1) << ws) + (i & (width - 1)) + max(0, lo - sib)] = key;
       }
       __syncthreads();
+      Key* t = A;
+      A = B;
+      B = t;
     }
-  for (int k = threadIdx.x; k < n; k += blockDim.x) b.order[s0 + k] = id[k];
-  __syncthreads();
-  // the column's super-clusters, a warp each, in the shared memory the sort is done with
-  const int w = threadIdx.x >> 5;
-  double(*s_w)[3] = reinterpret_cast<double(*)[3]>(smem_raw) + 64 * w;
-  int* s_a = reinterpret_cast<int*>(smem_raw + sizeof(double) * 3 * 64 * kScWarps) + 64 * w;
-  const int sc1 = min(b.col_sc[c + 1], nsc);
-  for (int sc = b.col_sc[c] + w; sc < sc1; sc += kScWarps) form_supercluster(cell, b, sc, c, threadIdx.x & 31, s_w, s_a);
-  __syncthreads();
+  } else {
+    int np = 1;
+    while (np < n) np <<= 1;
+    for (int k = threadIdx.x; k < np; k += blockDim.x) A[k] = k < n ? key_of(k) : ~0ull;
+    __syncthreads();
+    for (int kk = 2; kk <= np; kk <<= 1)
+      for (int j = kk >> 1; j > 0; j >>= 1) {
+        for (int t = threadIdx.x; t < (np >> 1); t += blockDim.x) {
+          const int lo = 2 * (t & ~(j - 1)) + (t & (j - 1)), hi = lo + j;
+          const Key ka = A[lo], kb = A[hi];
+          if ((ka > kb) == ((lo & kk) == 0)) A[lo] = kb, A[hi] = ka;
+        }
+        __syncthreads();
+      }
+  }
+  for (int k = threadIdx.x; k < n; k += blockDim.x) b.order[s0 + k] = int(unsigned(A[k]));
+}
+
+// Super-cluster stage: kScWarps of them to a unit, a warp each.
+constexpr int kScWarps = kListThreads / 32;
+__device__ __forceinline__ void super_unit(int unit, const DevCell& cell, const ListBufs& b) {
+  const int sc = unit * kScWarps + int(threadIdx.x >> 5);
+  if (sc < min(b.counters[kCntNsc], b.nsc_cap)) form_supercluster(cell, b, sc, b.sc_col[sc], threadIdx.x & 31);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -278,11 +287,14 @@ struct SearchBatch {
 };
 
 struct SearchShared {
+  int xfirst[65];                         // exclusions of the super-cluster's atoms: where each atom's begin
+  int xatom[64];                          // the atoms
+  unsigned xoff[64];                      // and their places in the exclusion list
   uint2 rec[kExclRecMax];                 // x: j cluster, y: i local (6 bits) | j in cluster (3) << 6 | image << 9
   unsigned long long key[kExclHash];      // distinct (j cluster, image) of the records; ~0 empty
   unsigned short krank[kExclHash];        // rank of each occupied key slot: its masks are number mbase + rank
   int mbase;
-  double ibox[8][6];
+  float ilo[8][3], ihi[8][3];   // the i clusters' boxes, from the super-cluster's origin
   double org_i[3];
   int nrec;
   SearchBatch batch[kSearchWarps];
@@ -312,20 +324,22 @@ static __device__ int key_insert(SearchShared& S, unsigned long long key, int* c
   raise_error(counters, kErrExclOverflow);
   return -1;
 }
-// Writes the batch [0, cnt) of B as one work item. One atomic reserves the entries and the work item: the entry and work
+// Writes the entries [0, cnt) of B as work items of up to `depth` entries. One atomic reserves them all: the entry and work
 // counters are the two halves of one 64-bit word (entries low, work items high), shared by every warp of the build.
-static __device__ void flush_batch(SearchBatch& B, int sc, int cnt, int lane, const ListBufs& b) {
+static __device__ void flush_entries(SearchBatch& B, int sc, int cnt, int depth, int lane, const ListBufs& b) {
   if (cnt <= 0) return;
   static_assert(kCntEnt == 0 && kCntWork == 1, "entry and work counters form one 64-bit word");
+  const int items = (cnt + depth - 1) / depth;
   int base = 0, wi = 0;
   if (lane == 0) {
-    const unsigned long long old = atomicAdd(reinterpret_cast<unsigned long long*>(b.counters + kCntEnt), (1ull << 32) | unsigned(cnt));
+    const unsigned long long old =
+        atomicAdd(reinterpret_cast<unsigned long long*>(b.counters + kCntEnt), ((unsigned long long)(unsigned)items << 32) | unsigned(cnt));
     base = int(unsigned(old & 0xffffffffull));
     wi = int(unsigned(old >> 32));
   }
   base = __shfl_sync(0xffffffffu, base, 0);
   wi = __shfl_sync(0xffffffffu, wi, 0);
-  if (base + cnt > b.ent_cap || wi >= b.work_cap) {
+  if (base + cnt > b.ent_cap || wi + items > b.work_cap) {
     if (lane == 0) raise_error(b.counters, kErrListOverflow);
     return;
   }
@@ -335,7 +349,7 @@ static __device__ void flush_batch(SearchBatch& B, int sc, int cnt, int lane, co
     b.ent[base + e] = en;
     b.ent_shift[base + e] = B.sh[e];
   }
-  if (lane == 0) b.work[wi] = make_int4(sc, base, cnt, 0);
+  for (int k = lane; k < items; k += 32) b.work[wi + k] = make_int4(sc, base + k * depth, min(depth, cnt - k * depth), 0);
 }
 
 // Search stage: one block of kSearchWarps warps per super-cluster. The block records the super-cluster's excluded pairs and
@@ -354,32 +368,56 @@ __device__ void search_supercluster(int sc, const DevCell& cell, const ListGeom&
   {
     // --- the super-cluster's boxes and exclusion records (the whole block)
     for (int t = threadIdx.x; t < kExclHash; t += blockDim.x) S.key[t] = ~0ull;
-    if (threadIdx.x < 8)
-      for (int r = 0; r < 6; ++r) S.ibox[threadIdx.x][r] = b.cl_box[6 * (8 * sc + threadIdx.x) + r];
-    if (threadIdx.x < 3) S.org_i[threadIdx.x] = b.sc_org[3 * sc + threadIdx.x];
+    if (threadIdx.x < 24) {
+      const int c = threadIdx.x / 3, r = threadIdx.x % 3;
+      const float* box = reinterpret_cast<const float*>(b.cl_box + 2 * (8 * sc + c));
+      const double o = b.sc_org[3 * sc + r];
+      S.ilo[c][r] = float(double(box[r]) - o), S.ihi[c][r] = float(double(box[4 + r]) - o);
+      if (c == 0) S.org_i[r] = o;
+    }
     if (threadIdx.x == 0) S.nrec = 0;
     if (lane == 0) B.nent = 0;
     __syncthreads();
     if (threadIdx.x < 8) key_insert(S, excl_key(unsigned(8 * sc + threadIdx.x), pack_image(0, 0, 0)), b.counters);
-    // kSearchWarps / 2 threads per atom, each taking every (kSearchWarps / 2)-th of the atom's excluded partners
-    for (int u = threadIdx.x; u < 64 * (kSearchWarps / 2); u += blockDim.x) {
-      const int t = u & 63;
-      const int a = b.perm[64 * sc + t];
-      if (a < 0) continue;
-      const double* fa = b.frac + 3 * a;
-      for (uint32_t p = excl_off[a] + uint32_t(u >> 6); p < excl_off[a + 1]; p += kSearchWarps / 2) {
-        const int bb = int(excl_list[p]);
-        const int sb = b.iperm[bb];
-        const double* fb = b.frac + 3 * bb;
-        // nearest image of bb seen from a: bb + q, q = -round(fb - fa)
-        const int qa = -int(rint(fb[0] - fa[0])), qb = -int(rint(fb[1] - fa[1])), qc = -int(rint(fb[2] - fa[2]));
-        if (qa < -63 || qa > 63 || qb < -63 || qb > 63 || qc < -63 || qc > 63) { raise_error(b.counters, kErrImageRange); continue; }
-        const unsigned img = pack_image(qa, qb, qc);
-        const int r = atomicAdd(&S.nrec, 1);
-        if (r >= kExclRecMax) { raise_error(b.counters, kErrExclOverflow); continue; }
-        S.rec[r] = make_uint2(unsigned(sb >> 3), unsigned(t) | (unsigned(sb & 7) << 6) | (img << 9));
-        key_insert(S, excl_key(unsigned(sb >> 3), img), b.counters);
+    // the super-cluster's exclusions, one to a thread: their counts per atom, the running sums, then each (atom, partner)
+    if (threadIdx.x < 64) {
+      const int a = b.perm[64 * sc + threadIdx.x];
+      const unsigned o = a >= 0 ? excl_off[a] : 0u;
+      S.xatom[threadIdx.x] = a;
+      S.xoff[threadIdx.x] = o;
+      int sum = a >= 0 ? int(excl_off[a + 1] - o) : 0;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, sum, d);
+        if (lane >= d) sum += y;
       }
+      S.xfirst[threadIdx.x + 1] = sum;   // within each half; the upper half's offset is added below
+    }
+    if (threadIdx.x == 0) S.xfirst[0] = 0;
+    __syncthreads();
+    const int xhalf = S.xfirst[32], nexcl = xhalf + S.xfirst[64];
+    for (int q = threadIdx.x; q < nexcl; q += blockDim.x) {
+      // the atom of exclusion q: the last whose first is at most q
+      const int up = q >= xhalf ? 32 : 0, qq = q - (up ? xhalf : 0);
+      int t = 0;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1)
+        if ((t + d ? S.xfirst[up + t + d] : 0) <= qq) t += d;
+      const int firstq = t ? S.xfirst[up + t] : 0;
+      t += up;
+      const int a = S.xatom[t];
+      const int bb = int(excl_list[S.xoff[t] + unsigned(qq - firstq)]);
+      const int sb = b.iperm[bb];
+      const double* fa = b.frac + 3 * a;
+      const double* fb = b.frac + 3 * bb;
+      // nearest image of bb seen from a: bb + q, q = -round(fb - fa)
+      const int qa = -int(rint(fb[0] - fa[0])), qb = -int(rint(fb[1] - fa[1])), qc = -int(rint(fb[2] - fa[2]));
+      if (qa < -63 || qa > 63 || qb < -63 || qb > 63 || qc < -63 || qc > 63) { raise_error(b.counters, kErrImageRange); continue; }
+      const unsigned img = pack_image(qa, qb, qc);
+      const int r = atomicAdd(&S.nrec, 1);
+      if (r >= kExclRecMax) { raise_error(b.counters, kErrExclOverflow); continue; }
+      S.rec[r] = make_uint2(unsigned(sb >> 3), unsigned(t) | (unsigned(sb & 7) << 6) | (img << 9));
+      key_insert(S, excl_key(unsigned(sb >> 3), img), b.counters);
     }
     __syncthreads();
     if (threadIdx.x == 0 && S.nrec > kExclRecMax) S.nrec = kExclRecMax;
@@ -444,7 +482,6 @@ __device__ void search_supercluster(int sc, const DevCell& cell, const ListGeom&
     const int col = b.sc_col[sc];
     const int cu = col / g.nv, cv = col % g.nv;
     const double zlo = b.sc_z[2 * sc], zhi = b.sc_z[2 * sc + 1];
-    const int ci0 = 8 * sc;
     const int nvw = 2 * g.rv + 1, ncols = (2 * g.ru + 1) * nvw;
     const int kper = (ncols + kSearchWarps - 1) / kSearchWarps;
     for (int k = warp * kper; k < min(ncols, (warp + 1) * kper); ++k) {
@@ -465,84 +502,76 @@ __device__ void search_supercluster(int sc, const DevCell& cell, const ListGeom&
         const bool positive = qa > 0 || (qa == 0 && (qb > 0 || (qb == 0 && qc > 0)));
         const unsigned img = pack_image(qa, qb, qc);
         const double lo = zlo - g.dw - qc, hi = zhi + g.dw - qc;
-        // super-clusters of column cc whose c range meets [lo, hi]: their ranges rise along the column
-        int sj = b.col_sc[cc];
-        const int sje = min(b.col_sc[cc + 1], nsc);
-        {
-          int lo_i = sj, hi_i = sje;   // first with z_hi >= lo
-          while (lo_i < hi_i) {
-            const int mid = (lo_i + hi_i) >> 1;
-            if (b.sc_z[2 * mid + 1] < lo) lo_i = mid + 1;
-            else hi_i = mid;
+        // the image's shift as seen from the super-cluster's origin
+        const float F0 = float(S0 - S.org_i[0]), F1 = float(S1 - S.org_i[1]), F2 = float(S2 - S.org_i[2]);
+        // super-clusters of column cc whose c range meets [lo, hi]: their ranges rise along the column, 32 looked at at once
+        const int sj0 = b.col_sc[cc], sje = min(b.col_sc[cc + 1], nsc);
+        for (int sjb = sj0; sjb < sje; sjb += 32) {
+          unsigned in = 0;
+          {
+            const int t = sjb + lane;
+            const double2 z = t < sje ? *reinterpret_cast<const double2*>(b.sc_z + 2 * t) : make_double2(3e300, -3e300);
+            in = __ballot_sync(0xffffffffu, z.y >= lo && z.x <= hi);
           }
-          sj = lo_i;
-        }
-        for (; sj < sje && b.sc_z[2 * sj] <= hi; sj += 4) {
-          // four candidate super-clusters per pass: lane = 8 * which + j cluster
-          const int sjl = sj + (lane >> 3);
-          bool have = false;
-          unsigned imask = 0;
-          int cj = -1;
-          if (sjl < sje && b.sc_z[2 * sjl] <= hi) {
-            cj = 8 * sjl + (lane & 7);
-            const double* bj = b.cl_box + 6 * cj;
-            const double jlo[3] = {bj[0] + S0, bj[1] + S1, bj[2] + S2}, jhi[3] = {bj[3] + S0, bj[4] + S1, bj[5] + S2};
-            for (int c = 0; c < 8; ++c) {
-              const int ci = ci0 + c;
-              // half list: one side of each cluster pair by parity; a cluster with itself under zero or + images
-              bool keep;
-              if (cj != ci) keep = (cj > ci) == (((ci + cj) & 1) == 0);
-              else keep = zero || positive;
-              if (!keep) continue;
-              double d2 = 0;
-              for (int r = 0; r < 3; ++r) {
-                const double g1 = jlo[r] - S.ibox[c][3 + r], g2 = S.ibox[c][r] - jhi[r];
-                const double gg = g1 > 0 ? g1 : (g2 > 0 ? g2 : 0.0);
-                d2 += gg * gg;
+          if (!in) continue;
+          const int sj1 = sjb + __ffs(in) - 1, sj2 = sjb + 32 - __clz(in);
+          for (int sj = sj1; sj < sj2; sj += 4) {
+            // four candidate super-clusters per pass: lane = 8 * which + j cluster
+            const int sjl = sj + (lane >> 3);
+            bool have = false;
+            unsigned imask = 0;
+            int cj = -1;
+            if (sjl < sj2) {
+              cj = 8 * sjl + (lane & 7);
+              const float4 bl = b.cl_box[2 * cj], bh = b.cl_box[2 * cj + 1];
+              const float l0 = bl.x + F0, l1 = bl.y + F1, l2 = bl.z + F2, h0 = bh.x + F0, h1 = bh.y + F1, h2 = bh.z + F2;
+  #pragma unroll
+              for (int c = 0; c < 8; ++c) {
+                const float g0 = fmaxf(fmaxf(l0 - S.ihi[c][0], S.ilo[c][0] - h0), 0.f), g1 = fmaxf(fmaxf(l1 - S.ihi[c][1], S.ilo[c][1] - h1), 0.f),
+                            g2 = fmaxf(fmaxf(l2 - S.ihi[c][2], S.ilo[c][2] - h2), 0.f);
+                imask |= unsigned(g0 * g0 + g1 * g1 + g2 * g2 < g.reach2) << c;
               }
-              if (d2 < g.rlist2) imask |= 1u << c;
+              // half list: one side of each cluster pair by parity; a cluster with itself under zero or + images
+              const unsigned even = 0x55u << (cj & 1);   // the i clusters ci with ci + cj even (8 sc is)
+              if (sjl != sc) imask &= sjl > sc ? even : ~even;
+              else {
+                const int k = lane & 7;
+                const unsigned below = (1u << k) - 1;
+                imask &= (even & below) | (~even & ~below & ~(1u << k)) | (zero || positive ? 1u << k : 0u);
+              }
+              have = imask != 0;
             }
-            have = imask != 0;
-          }
-          const unsigned ball = __ballot_sync(0xffffffffu, have);
-          if (have) {
-            const int pos = B.nent + __popc(ball & ((1u << lane) - 1));   // < batch + 32 <= 2 kBatch (flushed below)
-            const int sjc = cj >> 3;
-            const int h = key_slot(S, excl_key(unsigned(cj), img));
-            const int mi = h >= 0 ? S.mbase + S.krank[h] : -1;
-            B.ent[pos] = make_uint4(unsigned(cj), imask | (img << 8), mi >= 0 && mi < b.mask_cap ? unsigned(mi + 1) : 0u, 0u);
-            B.sh[pos] = make_float4(float(b.sc_org[3 * sjc] + S0 - S.org_i[0]), float(b.sc_org[3 * sjc + 1] + S1 - S.org_i[1]),
-                                    float(b.sc_org[3 * sjc + 2] + S2 - S.org_i[2]), 0.f);
-          }
-          __syncwarp();
-          if (lane == 0) B.nent += __popc(ball);
-          __syncwarp();
-          while (B.nent >= g.batch) {   // a pass adds up to 32 entries: with a depth below 32 more than one batch fills
-            flush_batch(B, sc, g.batch, lane, b);
-            __syncwarp();
-            // the rest (< 2 kBatch - batch entries) moves down: read all, then write (the ranges can overlap)
-            const int rest = B.nent - g.batch;
-            uint4 te[2];
-            float4 ts[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              const int e = lane + 32 * k;
-              if (e < rest) te[k] = B.ent[g.batch + e], ts[k] = B.sh[g.batch + e];
+            const unsigned ball = __ballot_sync(0xffffffffu, have);
+            if (have) {
+              const int pos = B.nent + __popc(ball & ((1u << lane) - 1));   // < batch + 32 <= 2 kBatch (flushed below)
+              const int sjc = cj >> 3;
+              const int h = key_slot(S, excl_key(unsigned(cj), img));
+              const int mi = h >= 0 ? S.mbase + S.krank[h] : -1;
+              B.ent[pos] = make_uint4(unsigned(cj), imask | (img << 8), mi >= 0 && mi < b.mask_cap ? unsigned(mi + 1) : 0u, 0u);
+              B.sh[pos] = make_float4(float(b.sc_org[3 * sjc] + S0 - S.org_i[0]), float(b.sc_org[3 * sjc + 1] + S1 - S.org_i[1]),
+                                      float(b.sc_org[3 * sjc + 2] + S2 - S.org_i[2]), 0.f);
             }
             __syncwarp();
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              const int e = lane + 32 * k;
-              if (e < rest) B.ent[e] = te[k], B.sh[e] = ts[k];
+            if (lane == 0) B.nent += __popc(ball);
+            __syncwarp();
+            if (B.nent >= g.batch) {   // a pass adds up to 32 entries: all full work items go together
+              const int full = B.nent / g.batch * g.batch, rest = B.nent - full;
+              flush_entries(B, sc, full, g.batch, lane, b);
+              __syncwarp();
+              // the rest (fewer than a work item's, at most 31) moves down: read, then write (the ranges can overlap)
+              uint4 te;
+              float4 ts;
+              if (lane < rest) te = B.ent[full + lane], ts = B.sh[full + lane];
+              __syncwarp();
+              if (lane < rest) B.ent[lane] = te, B.sh[lane] = ts;
+              if (lane == 0) B.nent = rest;
+              __syncwarp();
             }
-            __syncwarp();
-            if (lane == 0) B.nent = rest;
-            __syncwarp();
           }
         }
       }
     }
-    flush_batch(B, sc, B.nent, lane, b);
+    flush_entries(B, sc, B.nent, g.batch, lane, b);
     __syncthreads();   // S is rewritten for the next super-cluster
   }
 }

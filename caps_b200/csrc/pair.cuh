@@ -129,9 +129,6 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
   return y;
 }
 
-// A position times a force in fixed point (2^24 per kcal/mol); the product of two floats is exact in double.
-__device__ __forceinline__ long long vir_fix(float x, float f) { return to_fix(double(x) * double(f), kFixE); }
-
 // COUL: 0 none; 1 Ewald real space (PME) and 2 damped shifted force through the rational fits of ewald_fit.cuh
 // (kappa r_c <= 4); 3 and 4 the same through erfcf and expf (any kappa). COMB: the LJ coefficients of a type pair are
 // products of per-type factors (geometric mixing: c6_ab = sqrt(c6_aa c6_bb), the same for c12), taken from a
@@ -181,11 +178,11 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
   const float2 ku = p_dup(float(A.beta * A.beta / kEwUMax)), nkap3 = p_dup(-float(A.beta * A.beta * A.beta));
   const float e0 = float(A.dsf_e0), f0 = float(A.dsf_f0), rcf = float(A.rc);
   // energies: every pair's terms rounded to fixed point on their own (2^24 per kcal/mol), so that the totals do not depend
-  // on the list's grouping of pairs. Virial: sum of d F over a work item's pairs, d = x_j - x_i, as sum x_j F_j + sum x_i F_i
-  // over its atoms with the force sums the kernel has anyway (positions from the super-cluster's origin, products exact in
-  // double, each rounded to fixed point): per pair it took six products and twelve conversions to 64-bit integers, which
-  // made this variant twice as long as the force-only one
-  long long acc_v = 0, acc_c = 0, acc_w[6] = {0, 0, 0, 0, 0, 0}, acc_wj[2] = {0, 0};
+  // on the list's grouping of pairs. Virial: a lane's at most eight pairs of an entry and half summed by multiply-adds, one
+  // rounding each, then to fixed point (an entry's pairs are the same whatever work item holds it); with six products and
+  // twelve conversions to 64-bit integers per pair this variant took 226 us at 32,000 atoms. From the atoms' force sums
+  // instead (sum x F, as the FP64 kernel) it is off twice as far: those sums' rounding times positions of 20 Å.
+  long long acc_v = 0, acc_c = 0, acc_w[6] = {0, 0, 0, 0, 0, 0};
   double acc_np = 0, acc_nl = 0;
   constexpr float kq = 16777216.f;
   for (int w = next_work_item(A.counters, lane); w < nwork; w = next_work_item(A.counters, lane)) {
@@ -285,6 +282,9 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
         t1 = s_tj[8 * el + jq + 4];
       }
       float2 fjx = p_dup(0.f), fjy = p_dup(0.f), fjz = p_dup(0.f);
+      float2 w6[6];   // the entry's virial in the lane
+      if (VIR)
+        for (int k = 0; k < 6; ++k) w6[k] = p_dup(0.f);
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         if (!((imask >> c) & 1u)) continue;
@@ -355,7 +355,14 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
         fix[c] -= fx.x + fx.y;
         fiy[c] -= fy.x + fy.y;
         fiz[c] -= fz.x + fz.y;
+        if (VIR) {
+          w6[0] = p_fma(fx, dx, w6[0]), w6[1] = p_fma(fy, dy, w6[1]), w6[2] = p_fma(fz, dz, w6[2]);
+          w6[3] = p_fma(fx, dy, w6[3]), w6[4] = p_fma(fx, dz, w6[4]), w6[5] = p_fma(fy, dz, w6[5]);
+        }
       }
+      if (VIR)
+#pragma unroll
+        for (int k = 0; k < 6; ++k) acc_w[k] += __float2ll_rn(w6[k].x * kq) + __float2ll_rn(w6[k].y * kq);
       // j forces: summed over the 8 lanes holding the same j atoms, then one fixed-point add per component
       {
         float kx, ky, kz;
@@ -365,12 +372,6 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
           const float v = comp == 0 ? kx : comp == 1 ? ky : kz;
           long long* dst = comp == 0 ? A.fsx : comp == 1 ? A.fsy : A.fsz;
           if (v != 0.f) fix_add_f(dst + ((i8 & 4) ? j1 : j0), v, A.err);
-          if (VIR) {   // the j atoms' share of the virial: lane comp 0 takes xx and xy, 1 yy and yz, 2 zz and xz
-            const bool h = (i8 & 4) != 0;
-            const float px = h ? xj.y : xj.x, py = h ? yj.y : yj.x, pz = h ? zj.y : zj.x;
-            acc_wj[0] += vir_fix(comp == 0 ? px : comp == 1 ? py : pz, v);
-            acc_wj[1] += vir_fix(comp == 1 ? py : px, comp == 0 ? ky : kz);
-          }
         }
       }
     }
@@ -386,16 +387,6 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
         if (fo[3 * m] != 0.f) fix_add_f(A.fsx + s, fo[3 * m], A.err);
         if (fo[3 * m + 1] != 0.f) fix_add_f(A.fsy + s, fo[3 * m + 1], A.err);
         if (fo[3 * m + 2] != 0.f) fix_add_f(A.fsz + s, fo[3 * m + 2], A.err);
-        if (VIR) {   // the i atoms' share (staged negated)
-          const float4 pa = xi_s[3 * (8 * c + i8)];
-          const float px = -pa.x, py = -pa.z, pz = -xi_s[3 * (8 * c + i8) + 1].x;
-          acc_w[0] += vir_fix(px, fo[3 * m]);
-          acc_w[1] += vir_fix(py, fo[3 * m + 1]);
-          acc_w[2] += vir_fix(pz, fo[3 * m + 2]);
-          acc_w[3] += vir_fix(px, fo[3 * m + 1]);
-          acc_w[4] += vir_fix(px, fo[3 * m + 2]);
-          acc_w[5] += vir_fix(py, fo[3 * m + 2]);
-        }
       }
     }
     if (ENER) {
@@ -408,14 +399,8 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
     acc_v = warp_sum(acc_v);
     acc_c = warp_sum(acc_c);
   }
-  if (VIR) {
-    const int comp = i8 & 3;
-    if (comp < 3) {
-      acc_w[0] += comp == 0 ? acc_wj[0] : 0, acc_w[1] += comp == 1 ? acc_wj[0] : 0, acc_w[2] += comp == 2 ? acc_wj[0] : 0;
-      acc_w[3] += comp == 0 ? acc_wj[1] : 0, acc_w[5] += comp == 1 ? acc_wj[1] : 0, acc_w[4] += comp == 2 ? acc_wj[1] : 0;
-    }
+  if (VIR)
     for (int k = 0; k < 6; ++k) acc_w[k] = warp_sum(acc_w[k]);
-  }
   if (lane == 0) {
     if (ENER) {
       atomic_add_fix(A.en.fix + kEVdw, acc_v);
@@ -573,7 +558,8 @@ static __global__ void __launch_bounds__(128, 3) k_pair_f64(PairArgs A) {
   if (A.counters[kCntErr] & kErrListBad) return;
   const int nwork = min(A.counters[kCntWork], A.work_cap);
   const int pad = A.ntab - 1;
-  // energies, and the virial from the atoms' force sums as in the FP32 kernel (positions from the first i atom)
+  // energies; virial: sum of d F over a work item's pairs, d = x_j - x_i, as sum x_j F_j + sum x_i F_i over its atoms with
+  // the force sums the kernel has anyway (positions from the first i atom)
   double acc_v = 0, acc_c = 0, acc_w[6] = {0, 0, 0, 0, 0, 0}, acc_wj[2] = {0, 0};
   for (int w = next_work_item(A.counters, lane); w < nwork; w = next_work_item(A.counters, lane)) {
     const int4 wk = A.work[w];
