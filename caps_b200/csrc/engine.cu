@@ -573,8 +573,10 @@ void Engine::set_cell(const double* cell) {
   // wrapped coordinates lie within the cell: rounded to float, and shifted by an image, they are off by a few ulps of its size
   double span = 0;
   for (int k = 0; k < 12; ++k) span += std::fabs(cell[k]);
-  const double reach = g.rlist + 1e-3 + 1e-6 * span;
-  g.reach2 = float(reach * reach);
+  const double off = 1e-3 + 1e-6 * span;
+  g.rlist2 = g.rlist * g.rlist;
+  g.far2 = float((g.rlist + off) * (g.rlist + off));
+  g.near2 = g.rlist > off ? float((g.rlist - off) * (g.rlist - off)) : 0.f;
   g.ru = int(std::floor(g.rlist * g.nu / g.w[0])) + 1;
   g.rv = int(std::floor(g.rlist * g.nv / g.w[1])) + 1;
   g.rq = int(std::ceil(g.rlist / g.w[2])) + 1;
@@ -632,6 +634,9 @@ int Engine::list_depth(const ListGeom& g) const {
   const double reach = s * s * s + 6 * s * s * R + 3 * kPi * s * R * R + 4.0 / 3.0 * kPi * R * R * R;
   const double entries = 1.5 * (n_ / 64.0 + 0.5 * g.ncol) * 0.5 * reach * rho / 8.0;
   const double per_warp = entries / (20.0 * dev_sms_);
+  // The mixed path sums a work item's i forces in float, so the depth shows in their last bits. In melts of hard beads (no
+  // Coulomb) that grows past 1e-4 of the velocities within two hundred steps: their depth stays what it has been.
+  if (mixed_ && !coul_) return 16;
   return per_warp < 3 ? 2 : per_warp < 5 ? 4 : per_warp < 20 ? 8 : per_warp < 200 ? 16 : 24;
 }
 
@@ -650,7 +655,8 @@ void Engine::ensure_list_capacity() {
     d_sc_col_.alloc(size_t(nsc_cap_));
     d_sc_z_.alloc(size_t(2) * nsc_cap_);
     d_sc_org_.alloc(size_t(3) * nsc_cap_);
-    d_cl_box_.alloc(size_t(2) * 8 * nsc_cap_);
+    d_cl_box_.alloc(size_t(6) * 8 * nsc_cap_);
+    d_cl_boxf_.alloc(size_t(2) * 8 * nsc_cap_);
     d_cl_real_.alloc(size_t(8) * nsc_cap_);
     d_perm_.alloc(ns);
     d_xq_.alloc(ns);
@@ -701,6 +707,7 @@ void Engine::ensure_list_capacity() {
   b.sc_z = d_sc_z_.p;
   b.sc_org = d_sc_org_.p;
   b.cl_box = d_cl_box_.p;
+  b.cl_boxf = d_cl_boxf_.p;
   b.cl_real = d_cl_real_.p;
   b.perm = d_perm_.p;
   b.ent = d_ent_.p;

@@ -291,7 +291,8 @@ class Engine {
   DevBuf<int> d_col_, d_ioff_, d_order_, d_iperm_, d_col_count_, d_col_fill_, d_col_start_, d_col_sc_, d_sc_col_, d_perm_, d_counters_;
   DevBuf<double> d_frac_, d_sc_z_, d_sc_org_, d_x0_, d_xp_;
   DevBuf<unsigned char> d_cl_real_;
-  DevBuf<float4> d_cl_box_;
+  DevBuf<double> d_cl_box_;
+  DevBuf<float4> d_cl_boxf_;
   DevBuf<uint4> d_ent_;
   DevBuf<float4> d_ent_shift_;
   DevBuf<unsigned long long> d_masks_;

@@ -16,7 +16,8 @@ struct ListGeom {
   int ru, rv, rq;
   double w[3];        // perpendicular widths of the cell
   double rlist;
-  float reach2;       // the search's squared radius: rlist and what the float boxes may be off by
+  double rlist2;
+  float near2, far2;  // squared box distances in float below and above which they decide; between them, in double
   double dw;          // rlist / w[2]
   int batch;          // entries per work item (the pair kernels' j-tile depth), at most kBatch (Engine::list_depth)
 };
@@ -38,7 +39,8 @@ struct ListBufs {
   double* sc_z;       // 2 per sc: fractional c range
   double* sc_org;     // 3 per sc: origin (centre of its bounding box)
   // per cluster
-  float4* cl_box;     // 2 per cluster: lo xyz, hi xyz at the build (wrapped Cartesian)
+  double* cl_box;     // 6 per cluster: lo xyz, hi xyz at the build (wrapped Cartesian)
+  float4* cl_boxf;    // 2 per cluster: the same in float
   unsigned char* cl_real;   // 8-bit mask of real atoms
   // per slot
   int* perm;

@@ -116,15 +116,15 @@ __device__ __forceinline__ void scatter_atom(int n, int i, const ListBufs& b) {
 }
 
 // One compare-exchange of a bitonic network over the lanes: the pair (lane, lane ^ j) ascending where up.
-__device__ __forceinline__ void lane_exchange(float& key, int& id, int j, bool up) {
-  const float k = __shfl_xor_sync(0xffffffffu, key, j);
+__device__ __forceinline__ void lane_exchange(unsigned& key, int& id, int j, bool up) {
+  const unsigned k = __shfl_xor_sync(0xffffffffu, key, j);
   const int i = __shfl_xor_sync(0xffffffffu, id, j);
   const bool low = (threadIdx.x & j) == 0;   // the pair's lower lane keeps the smaller key
   if (low == up ? k < key : k > key) key = k, id = i;
 }
 // Sorts key (and id) over groups of N lanes, ascending. Deterministic: the network's exchanges depend on the keys alone.
 template <int N>
-__device__ __forceinline__ void lane_sort(float& key, int& id) {
+__device__ __forceinline__ void lane_sort(unsigned& key, int& id) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int kk = 2; kk <= N; kk <<= 1)
@@ -134,7 +134,8 @@ __device__ __forceinline__ void lane_sort(float& key, int& id) {
 
 // K-SUPER (a warp per super-cluster): the 2 x 2 x 2 split into clusters, perm / iperm, cluster boxes and real-atom masks,
 // the super-cluster's origin and its c range. Lane l holds atoms l (lower c half) and l + 32 (upper c half), sorted along b
-// over the warp and then along a over each half of it, which leaves slot 32 h + l in lane l; padding sorts last. (Ranks by
+// over the warp and then along a over each half of it (keys in units of 2^-32 of the cell), which leaves slot 32 h + l in
+// lane l; padding sorts last. (Ranks by
 // comparing with every other atom took some 2,600 instructions of one warp: 17 us a build at any size.)
 __device__ void form_supercluster(const DevCell& cell, const ListBufs& b, int sc, int c, int lane) {
   const int k = sc - b.col_sc[c];
@@ -146,18 +147,19 @@ __device__ void form_supercluster(const DevCell& cell, const ListBufs& b, int sc
   }
   const int first = b.order[s0], last = b.order[s0 + m - 1];
   int id[2];
-  float key[2];
+  unsigned key[2];
+  auto key_of = [&](int a, int axis) { return a >= 0 ? unsigned(b.frac[3 * a + axis] * 4294967295.0) : ~0u; };
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int t = lane + 32 * h;
     id[h] = t < m ? b.order[s0 + t] : -1;
-    key[h] = id[h] >= 0 ? float(b.frac[3 * id[h] + 1]) : 3.f;   // fractional coordinates are below 1
+    key[h] = key_of(id[h], 1);
   }
 #pragma unroll
   for (int h = 0; h < 2; ++h) lane_sort<32>(key[h], id[h]);
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    key[h] = id[h] >= 0 ? float(b.frac[3 * id[h]]) : 3.f;
+    key[h] = key_of(id[h], 0);
     lane_sort<16>(key[h], id[h]);
   }
   // cluster boxes and real masks: slot lane + 32 h belongs to cluster (lane >> 3) + 4 h. The origin, which the packed
@@ -167,32 +169,30 @@ __device__ void form_supercluster(const DevCell& cell, const ListBufs& b, int sc
   for (int h = 0; h < 2; ++h) {
     const int a = id[h];
     b.perm[64 * sc + lane + 32 * h] = a;
-    float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
+    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
     if (a >= 0) {
       b.iperm[a] = 64 * sc + lane + 32 * h;
       const double f0 = b.frac[3 * a], f1 = b.frac[3 * a + 1], f2 = b.frac[3 * a + 2];
-      for (int r = 0; r < 3; ++r) {
-        const double p = cell.o[r] + cell.h[r][0] * f0 + cell.h[r][1] * f1 + cell.h[r][2] * f2;
-        lo[r] = hi[r] = float(p);
-        slo[r] = fmin(slo[r], p), shi[r] = fmax(shi[r], p);
-      }
+      for (int r = 0; r < 3; ++r) lo[r] = hi[r] = cell.o[r] + cell.h[r][0] * f0 + cell.h[r][1] * f1 + cell.h[r][2] * f2;
     }
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1)
       for (int r = 0; r < 3; ++r) {
-        lo[r] = fminf(lo[r], __shfl_xor_sync(0xffffffffu, lo[r], o));
-        hi[r] = fmaxf(hi[r], __shfl_xor_sync(0xffffffffu, hi[r], o));
+        lo[r] = fmin(lo[r], __shfl_xor_sync(0xffffffffu, lo[r], o));
+        hi[r] = fmax(hi[r], __shfl_xor_sync(0xffffffffu, hi[r], o));
       }
     const unsigned real = __ballot_sync(0xffffffffu, a >= 0);
     if ((lane & 7) == 0) {
       const int cg = 8 * sc + (lane >> 3) + 4 * h;
-      b.cl_box[2 * cg] = make_float4(lo[0], lo[1], lo[2], 0.f);   // an empty cluster: lo above every hi
-      b.cl_box[2 * cg + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
+      for (int r = 0; r < 3; ++r) b.cl_box[6 * cg + r] = lo[r], b.cl_box[6 * cg + 3 + r] = hi[r];
+      b.cl_boxf[2 * cg] = make_float4(float(lo[0]), float(lo[1]), float(lo[2]), 0.f);   // an empty cluster: +inf and -inf
+      b.cl_boxf[2 * cg + 1] = make_float4(float(hi[0]), float(hi[1]), float(hi[2]), 0.f);
       b.cl_real[cg] = (unsigned char)((real >> (lane & 24)) & 255u);
     }
+    for (int r = 0; r < 3; ++r) slo[r] = fmin(slo[r], lo[r]), shi[r] = fmax(shi[r], hi[r]);
   }
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1)
+  for (int o = 8; o < 32; o <<= 1)
     for (int r = 0; r < 3; ++r) {
       slo[r] = fmin(slo[r], __shfl_xor_sync(0xffffffffu, slo[r], o));
       shi[r] = fmax(shi[r], __shfl_xor_sync(0xffffffffu, shi[r], o));
@@ -294,7 +294,8 @@ struct SearchShared {
   unsigned long long key[kExclHash];      // distinct (j cluster, image) of the records; ~0 empty
   unsigned short krank[kExclHash];        // rank of each occupied key slot: its masks are number mbase + rank
   int mbase;
-  float ilo[8][3], ihi[8][3];   // the i clusters' boxes, from the super-cluster's origin
+  double ibox[8][6];            // the i clusters' boxes
+  float ilo[8][3], ihi[8][3];   // the same in float, from the super-cluster's origin
   double org_i[3];
   int nrec;
   SearchBatch batch[kSearchWarps];
@@ -370,9 +371,10 @@ __device__ void search_supercluster(int sc, const DevCell& cell, const ListGeom&
     for (int t = threadIdx.x; t < kExclHash; t += blockDim.x) S.key[t] = ~0ull;
     if (threadIdx.x < 24) {
       const int c = threadIdx.x / 3, r = threadIdx.x % 3;
-      const float* box = reinterpret_cast<const float*>(b.cl_box + 2 * (8 * sc + c));
+      const double* box = b.cl_box + 6 * (8 * sc + c);
       const double o = b.sc_org[3 * sc + r];
-      S.ilo[c][r] = float(double(box[r]) - o), S.ihi[c][r] = float(double(box[4 + r]) - o);
+      S.ibox[c][r] = box[r], S.ibox[c][3 + r] = box[3 + r];
+      S.ilo[c][r] = float(box[r] - o), S.ihi[c][r] = float(box[3 + r] - o);
       if (c == 0) S.org_i[r] = o;
     }
     if (threadIdx.x == 0) S.nrec = 0;
@@ -519,17 +521,19 @@ __device__ void search_supercluster(int sc, const DevCell& cell, const ListGeom&
             // four candidate super-clusters per pass: lane = 8 * which + j cluster
             const int sjl = sj + (lane >> 3);
             bool have = false;
-            unsigned imask = 0;
+            unsigned imask = 0, sure = 0;
             int cj = -1;
             if (sjl < sj2) {
               cj = 8 * sjl + (lane & 7);
-              const float4 bl = b.cl_box[2 * cj], bh = b.cl_box[2 * cj + 1];
+              const float4 bl = b.cl_boxf[2 * cj], bh = b.cl_boxf[2 * cj + 1];
               const float l0 = bl.x + F0, l1 = bl.y + F1, l2 = bl.z + F2, h0 = bh.x + F0, h1 = bh.y + F1, h2 = bh.z + F2;
   #pragma unroll
               for (int c = 0; c < 8; ++c) {
                 const float g0 = fmaxf(fmaxf(l0 - S.ihi[c][0], S.ilo[c][0] - h0), 0.f), g1 = fmaxf(fmaxf(l1 - S.ihi[c][1], S.ilo[c][1] - h1), 0.f),
                             g2 = fmaxf(fmaxf(l2 - S.ihi[c][2], S.ilo[c][2] - h2), 0.f);
-                imask |= unsigned(g0 * g0 + g1 * g1 + g2 * g2 < g.reach2) << c;
+                const float d2 = g0 * g0 + g1 * g1 + g2 * g2;
+                imask |= unsigned(d2 < g.far2) << c;
+                sure |= unsigned(d2 < g.near2) << c;
               }
               // half list: one side of each cluster pair by parity; a cluster with itself under zero or + images
               const unsigned even = 0x55u << (cj & 1);   // the i clusters ci with ci + cj even (8 sc is)
@@ -538,6 +542,19 @@ __device__ void search_supercluster(int sc, const DevCell& cell, const ListGeom&
                 const int k = lane & 7;
                 const unsigned below = (1u << k) - 1;
                 imask &= (even & below) | (~even & ~below & ~(1u << k)) | (zero || positive ? 1u << k : 0u);
+              }
+              // the few that float cannot decide
+              for (unsigned open = imask & ~sure; open; open &= open - 1) {
+                const int c = __ffs(open) - 1;
+                const double* bj = b.cl_box + 6 * cj;
+                const double jlo[3] = {bj[0] + S0, bj[1] + S1, bj[2] + S2}, jhi[3] = {bj[3] + S0, bj[4] + S1, bj[5] + S2};
+                double d2 = 0;
+                for (int r = 0; r < 3; ++r) {
+                  const double g1 = jlo[r] - S.ibox[c][3 + r], g2 = S.ibox[c][r] - jhi[r];
+                  const double gg = g1 > 0 ? g1 : (g2 > 0 ? g2 : 0.0);
+                  d2 += gg * gg;
+                }
+                if (!(d2 < g.rlist2)) imask &= ~(1u << c);
               }
               have = imask != 0;
             }
