@@ -196,8 +196,10 @@ class Engine {
   void forces(const double* d_x, bool ener, bool vir, bool check_rebuild, int parts = -1, double* d_out = nullptr, bool clear_energies = true,
               bool reduce = true);
   // Concurrent branches of a force evaluation: `launch` runs with stream_ pointing at side stream k, after everything
-  // queued on the main stream so far; join(k) makes the main stream wait for it. Captured, these are graph branches.
-  void fork(int k, const std::function<void()>& launch);
+  // queued on the main stream up to mark_fork(); join(k) makes the main stream wait for it. Captured, these are graph
+  // branches.
+  void mark_fork();
+  void branch(int k, const std::function<void()>& launch);
   void join(int k);
   cudaStream_t side_[2] = {nullptr, nullptr};
   int counter(int slot);   // a device counter (synchronises the stream)

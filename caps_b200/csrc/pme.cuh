@@ -576,7 +576,7 @@ static __global__ void k_pme_green(PmeArgs A, const double* __restrict__ b1, con
 
 // K-GATHER: F_i -= q_i sum_d K_d (row d of h^-1) dE/du_d (caps_kspace.f90:965-992), L lanes per atom, each taking every
 // L-th plane c of its P^3 points (the splines by each lane for itself: cheaper than a stage in shared memory). One lane per
-// atom reads fewest instructions, four fill the GPU and shorten the chain of loads where atoms are few (gather_lanes).
+// atom reads fewest instructions, four fill the GPU and shorten the chain of loads where atoms are few.
 template <class R, class G, int P, int L>
 static __global__ void __launch_bounds__(128) k_gather(PmeArgs A, const G* __restrict__ gr, ForceSink<R> F) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
