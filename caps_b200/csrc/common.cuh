@@ -249,6 +249,22 @@ __device__ T block_sum(T v, T* scratch /* >= 32 */) {
   return s;
 }
 
+// N block-wide sums at once, each the bits of block_sum's: two barriers in all. Results valid in thread 0.
+template <int N>
+__device__ __forceinline__ void block_sums(double (&v)[N], double* scratch /* >= 32 N */) {
+#pragma unroll
+  for (int q = 0; q < N; ++q) v[q] = warp_sum(v[q]);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  __syncthreads();
+  if (lane == 0)
+#pragma unroll
+    for (int q = 0; q < N; ++q) scratch[32 * q + w] = v[q];
+  __syncthreads();
+  if (w == 0)
+#pragma unroll
+    for (int q = 0; q < N; ++q) v[q] = warp_sum(lane < int(blockDim.x >> 5) ? scratch[32 * q + lane] : 0.0);
+}
+
 // Philox4x32-10 (Salmon, Moraes, Dror & Shaw, SC'11): counter-based random numbers, so every atom's noise at every
 // step is a pure function of (seed, step, atom) whatever the launch shape.
 struct Philox {

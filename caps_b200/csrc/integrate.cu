@@ -571,7 +571,8 @@ struct VelOp {
   int nat, nslots;
   double* fout;
 };
-// The force on atom g for a kick: f, or the evaluation's sums (stored to fout).
+// The force on atom g for a kick: f, or the evaluation's sums. Loads alone: a store to fout among them would make each
+// load that follows it wait (the two may overlap for all the compiler knows), a trip to L2 per component and atom.
 __device__ __forceinline__ void kick_force(const VelOp& op, int g, double f[3]) {
   if (!op.fq && !op.fd) {
     for (int r = 0; r < 3; ++r) f[r] = op.f[3 * g + r];
@@ -589,13 +590,12 @@ __device__ __forceinline__ void kick_force(const VelOp& op, int g, double f[3]) 
       if (ok) q += op.fsd[size_t(r) * op.nslots + s];
       f[r] = q;
     }
-    op.fout[3 * g + r] = f[r];
   }
 }
-__device__ __forceinline__ void vel_op(const VelOp& op, int g, double* vv, const double* __restrict__ invm, const double* sc) {
+// Atom g's updated velocity from vv; f: the force it was kicked with, for vel_store.
+__device__ __forceinline__ void vel_op(const VelOp& op, int g, double* vv, double f[3], const double* __restrict__ invm, const double* sc) {
   if (op.kind == 1) {
     const double a = op.hk * kAcc * invm[g];
-    double f[3];
     kick_force(op, g, f);
     for (int r = 0; r < 3; ++r) vv[r] += a * f[r];
     if (op.f2) {
@@ -608,6 +608,45 @@ __device__ __forceinline__ void vel_op(const VelOp& op, int g, double* vv, const
     const double sd = sqrt(kB * sc[kScTnow] * kAcc * invm[g]);
     for (int r = 0; r < 3; ++r) vv[r] = op.c1 * vv[r] + op.c2 * sd * z[r];
   }
+}
+__device__ __forceinline__ void vel_store(const VelOp& op, int g, const double* vv, const double f[3], double* v) {
+  for (int r = 0; r < 3; ++r) v[3 * g + r] = vv[r];
+  if (op.kind == 1 && (op.fq || op.fd))
+    for (int r = 0; r < 3; ++r) op.fout[3 * g + r] = f[r];
+}
+
+// What the last block of k_ke does with the fresh kinetic energy.
+enum KeThen { kThenNone = 0, kThenNhc, kThenBussi, kThenBath, kThenLang };
+struct KeArgs {
+  int n;
+  const double* v;
+  const double* m;
+  double* part;          // 7 per block
+  unsigned* done;        // blocks finished; the last block resets it
+  double* sc;
+  int slot;              // sc slot receiving 0.5 sum m v^2 / kAcc
+  int extra;             // further sums: 6 the kinetic tensor into kScKin0.., 1 the energy before the O step into kScKE0
+  int begin;             // run the step-begin update first
+  int then;              // KeThen
+  double t0, t1, ndof;
+  long long steps;
+  Chain* chain;
+  const Chain* chain_half;   // the chain after the step's first half (kThenNhc)
+  double t_freq, dt;
+  const double2* draws;
+  double tau;
+};
+
+// The share of one atom with velocity v: m v^2, and the tensor terms on request.
+__device__ __forceinline__ void ke_share(const KeArgs& A, double mi, const double v[3], double& e, double t[6]) {
+  e += mi * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+  if (A.extra == 6)
+    t[0] += mi * v[0] * v[0], t[1] += mi * v[1] * v[1], t[2] += mi * v[2] * v[2], t[3] += mi * v[0] * v[1], t[4] += mi * v[0] * v[2],
+        t[5] += mi * v[1] * v[2];
+}
+__device__ __forceinline__ void ke_atom(const KeArgs& A, int i, double& e, double t[6]) {
+  const double v[3] = {A.v[3 * i], A.v[3 * i + 1], A.v[3 * i + 2]};
+  ke_share(A, A.m[i], v, e, t);
 }
 
 // The multipliers of N coupled velocity constraints, M lam = -rv (M symmetric), by elimination. RATTLE's Gauss-Seidel sweep
@@ -640,18 +679,19 @@ __device__ __forceinline__ void rattle_solve(double M[N][N], const double rv[N],
 // RATTLE on a star cluster with NK constraints, in registers (the general kernel's sweep, constraints as (centre, partner)).
 template <int NK>
 __device__ void rattle_star(const ConsArgs& C, int s, const double* __restrict__ x, double* __restrict__ v, const VelOp& op, const double* sc,
-                            double h, double w[6], int* counters) {
+                            double h, double w[6], int* counters, const KeArgs& K, double& e, double t[6]) {
   const int4 at = C.star[s];
   const double4 d4 = C.star_d2[s];
   const int ids[4] = {at.x, at.y, at.z, at.w};
   const double dd[3] = {d4.x, d4.y, d4.z};
-  double pv[NK + 1][3], im[NK + 1];
+  double pv[NK + 1][3], im[NK + 1], ff[NK + 1][3], ma[NK + 1];
 #pragma unroll
   for (int a = 0; a <= NK; ++a) {
     const int g = ids[a];
     for (int r = 0; r < 3; ++r) pv[a][r] = v[3 * g + r];
-    vel_op(op, g, pv[a], C.invm, sc);
+    vel_op(op, g, pv[a], ff[a], C.invm, sc);
     im[a] = C.invm[g];
+    ma[a] = K.n > 0 ? K.m[g] : 0.0;
   }
   double rr[NK][3], lam[NK];
 #pragma unroll
@@ -696,8 +736,10 @@ __device__ void rattle_star(const ConsArgs& C, int s, const double* __restrict__
   }
   if (!done) atomicOr(reinterpret_cast<unsigned*>(counters + kCntErr), kErrRattle);
 #pragma unroll
-  for (int a = 0; a <= NK; ++a)
-    for (int r = 0; r < 3; ++r) v[3 * ids[a] + r] = pv[a][r];
+  for (int a = 0; a <= NK; ++a) {
+    vel_store(op, ids[a], pv[a], ff[a], v);
+    if (K.n > 0) ke_share(K, ma[a], pv[a], e, t);
+  }
   if (h > 0)
 #pragma unroll
     for (int k = 0; k < NK; ++k) {
@@ -713,19 +755,20 @@ __device__ void rattle_star(const ConsArgs& C, int s, const double* __restrict__
 
 // RATTLE on a rigid water in registers: Gauss-Seidel over (O, H1), (O, H2), (H1, H2).
 __device__ void rattle_water(const ConsArgs& C, int wi, const double* __restrict__ x, double* __restrict__ v, const VelOp& op, const double* sc,
-                             double h, double w[6], int* counters) {
+                             double h, double w[6], int* counters, const KeArgs& K, double& e, double t[6]) {
   const int4 at = C.water[wi];
   const double2 geo = C.water_geo[wi];
   const int ids[3] = {at.x, at.y, at.z};
   const int pi[3] = {0, 0, 1}, pj[3] = {1, 2, 2};
   const double dd[3] = {geo.x * geo.x, geo.x * geo.x, geo.y * geo.y};
-  double pv[3][3], im[3];
+  double pv[3][3], im[3], ff[3][3], ma[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const int g = ids[a];
     for (int r = 0; r < 3; ++r) pv[a][r] = v[3 * g + r];
-    vel_op(op, g, pv[a], C.invm, sc);
+    vel_op(op, g, pv[a], ff[a], C.invm, sc);
     im[a] = C.invm[g];
+    ma[a] = K.n > 0 ? K.m[g] : 0.0;
   }
   double rr[3][3], lam[3];
 #pragma unroll
@@ -775,8 +818,10 @@ __device__ void rattle_water(const ConsArgs& C, int wi, const double* __restrict
   }
   if (!done) atomicOr(reinterpret_cast<unsigned*>(counters + kCntErr), kErrRattle);
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
-    for (int r = 0; r < 3; ++r) v[3 * ids[a] + r] = pv[a][r];
+  for (int a = 0; a < 3; ++a) {
+    vel_store(op, ids[a], pv[a], ff[a], v);
+    if (K.n > 0) ke_share(K, ma[a], pv[a], e, t);
+  }
   if (h > 0)
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -845,18 +890,22 @@ __global__ void k_step_begin(double* sc, double t0, double t1, long long steps, 
 
 // Nose-Hoover chain over half a step (LAMMPS FixNH::nhc_temp_integrate, as dynamics.cpp:479-508) on chain c at target
 // temperature tt: returns the velocity factor and scales the kinetic energy ke by its square; the caller scales v.
-__device__ double nhc_half(Chain& c, double& ke, double tt, double ndof, double t_freq, double dt) {
-  const double dthalf = 0.5 * dt, dt4 = 0.25 * dt, dt8 = 0.125 * dt;
-  const double kt = kB * tt, ke_target = ndof * kt;
+// It runs in two parts: what the chain alone gives (returned: the first link's friction factor), then the rest.
+__device__ __forceinline__ double nhc_before(Chain& c, double tt, double ndof, double t_freq, double dt) {
+  const double dt4 = 0.25 * dt, dt8 = 0.125 * dt, kt = kB * tt;
   c.eta_mass[0] = ndof * kt / (t_freq * t_freq);
   for (int q = 1; q < 3; ++q) c.eta_mass[q] = kt / (t_freq * t_freq);
-  double kecur = 2 * ke;
-  c.eta_dotdot[0] = (kecur - ke_target) / c.eta_mass[0];
   for (int q = 2; q > 0; --q) {
     const double ex = exp(-dt8 * c.eta_dot[q + 1]);
     c.eta_dot[q] = (c.eta_dot[q] * ex + c.eta_dotdot[q] * dt4) * ex;
   }
-  double ex = exp(-dt8 * c.eta_dot[1]);
+  return exp(-dt8 * c.eta_dot[1]);
+}
+__device__ __forceinline__ double nhc_after(Chain& c, double ex, double& ke, double tt, double ndof, double dt) {
+  const double dthalf = 0.5 * dt, dt4 = 0.25 * dt, dt8 = 0.125 * dt;
+  const double kt = kB * tt, ke_target = ndof * kt;
+  double kecur = 2 * ke;
+  c.eta_dotdot[0] = (kecur - ke_target) / c.eta_mass[0];
   c.eta_dot[0] = (c.eta_dot[0] * ex + c.eta_dotdot[0] * dt4) * ex;
   const double factor = exp(-dthalf * c.eta_dot[0]);
   kecur *= factor * factor;
@@ -872,103 +921,107 @@ __device__ double nhc_half(Chain& c, double& ke, double tt, double ndof, double 
   ke = 0.5 * kecur;
   return factor;
 }
+__device__ double nhc_half(Chain& c, double& ke, double tt, double ndof, double t_freq, double dt) {
+  const double ex = nhc_before(c, tt, ndof, t_freq, dt);
+  return nhc_after(c, ex, ke, tt, ndof, dt);
+}
 
-// Bussi velocity rescaling (Bussi, Donadio & Parrinello 2007, appendix; dynamics.cpp:466-477) from this step's draws
-// (r1, sum of ndof - 1 squared normals) read from the host-made table, a ring over the steps: its captured kernel has no
+// Bussi velocity rescaling (Bussi, Donadio & Parrinello 2007, appendix; dynamics.cpp:466-477) takes this step's draws
+// (r1, sum of ndof - 1 squared normals) from a host-made table, a ring over the steps: its captured kernel has no
 // parameter that a refill would change.
 constexpr long long kDrawRing = 8192;
-__device__ void bussi_body(double* sc, const double2* __restrict__ draws, double h, double tau, double ndof) {
-  const double k = sc[kScKE];
-  const long long step = (long long)sc[kScStep];
-  if (k <= 0) {
-    sc[kScFactor] = 1;
-    return;
-  }
-  const double2 d = draws[step & (kDrawRing - 1)];
-  const double c = exp(-h / tau), kt = sc[kScKtarget];
-  const double r1 = d.x, sum = d.y;
-  const double knew = k + (1 - c) * (kt * (r1 * r1 + sum) / ndof - k) + 2 * r1 * sqrt(c * (1 - c) * kt * k / ndof);
-  sc[kScFactor] = sqrt(fmax(knew, 0.0) / k);
-  sc[kScBath] -= knew - k;
-}
 
-// What the last block of k_ke does with the fresh kinetic energy.
-enum KeThen { kThenNone = 0, kThenNhc, kThenBussi, kThenBath, kThenLang };
-struct KeArgs {
-  int n;
-  const double* v;
-  const double* m;
-  double* part;          // 7 per block
-  unsigned* done;        // blocks finished; the last block resets it
-  double* sc;
-  int slot;              // sc slot receiving 0.5 sum m v^2 / kAcc
-  int extra;             // further sums: 6 the kinetic tensor into kScKin0.., 1 the energy before the O step into kScKE0
-  int begin;             // run the step-begin update first
-  int then;              // KeThen
-  double t0, t1, ndof;
-  long long steps;
-  Chain* chain;
-  const Chain* chain_half;   // the chain after the step's first half (kThenNhc)
-  double t_freq, dt;
-  const double2* draws;
-  double tau;
+// The scalars an update reads, asked for when its kernel starts (in thread 0 of every block: any may be the last).
+struct KePre {
+  double step, tnow, ktarget, bath, ke0;
 };
-
-// The share of one atom with velocity v: m v^2, and the tensor terms on request.
-__device__ __forceinline__ void ke_share(const KeArgs& A, double mi, const double v[3], double& e, double t[6]) {
-  e += mi * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-  if (A.extra == 6)
-    t[0] += mi * v[0] * v[0], t[1] += mi * v[1] * v[1], t[2] += mi * v[2] * v[2], t[3] += mi * v[0] * v[1], t[4] += mi * v[0] * v[2],
-        t[5] += mi * v[1] * v[2];
-}
-__device__ __forceinline__ void ke_atom(const KeArgs& A, int i, double& e, double t[6]) {
-  const double v[3] = {A.v[3 * i], A.v[3 * i + 1], A.v[3 * i + 2]};
-  ke_share(A, A.m[i], v, e, t);
+__device__ __forceinline__ KePre ke_pre(const KeArgs& A) {
+  KePre p{};
+  if (threadIdx.x == 0 && A.n > 0) {
+    p.step = A.sc[kScStep], p.tnow = A.sc[kScTnow], p.ktarget = A.sc[kScKtarget], p.bath = A.sc[kScBath], p.ke0 = A.sc[kScKE0];
+  }
+  return p;
 }
 
 // The block sums of every thread's share into A.part (7 per block), then in the last block to finish: the partials in
 // block order and the scalar update. Every thread of every block calls it.
-__device__ void ke_blocks(const KeArgs& A, double e, double t[6]) {
-  __shared__ double scratch[32];
+//
+// A chain of waits: the block's sum, its fence, the counter, the partials, then the update's own arithmetic. Thread 0 of
+// every block asks for what the update reads before that chain, and does the part of it that needs no kinetic energy while
+// the counter's answer is on its way; with loads and all of it at the chain's end the kernel of 594 atoms took 8.8 us.
+template <int NS>
+__device__ __forceinline__ void ke_blocks_n(const KeArgs& A, const KePre& pre, double e, const double* t) {
+  __shared__ double scratch[NS * 32];
   __shared__ bool last;
-  const double s = block_sum(e, scratch);
-  if (threadIdx.x == 0) A.part[blockIdx.x * 7] = s;
-  for (int q = 0; q < A.extra; ++q) {
-    const double st = block_sum(t[q], scratch);
-    if (threadIdx.x == 0) A.part[blockIdx.x * 7 + 1 + q] = st;
-  }
+  Chain ch;
+  double2 d = {0, 0};
+  double step = pre.step, tnow = pre.tnow, ktarget = pre.ktarget;
   if (threadIdx.x == 0) {
+    if (A.begin) {
+      step += 1;
+      tnow = target_at(step, A.t0, A.t1, A.steps);
+      ktarget = 0.5 * A.ndof * kB * tnow;
+    }
+    if (A.then == kThenNhc) ch = *A.chain_half;   // the chain after the first half that the step's first kernel left
+    else if (A.then == kThenBussi) d = A.draws[(long long)step & (kDrawRing - 1)];
+  }
+  double s[NS];
+  s[0] = e;
+#pragma unroll
+  for (int q = 1; q < NS; ++q) s[q] = t[q - 1];
+  block_sums(s, scratch);
+  double c = 0, kick = 0, root = 0;
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) A.part[blockIdx.x * 7 + q] = s[q];
     __threadfence();
-    last = atomicAdd(A.done, 1u) == gridDim.x - 1;
+    const unsigned before = atomicAdd(A.done, 1u);
+    if (A.then == kThenNhc) c = nhc_before(ch, tnow, A.ndof, A.t_freq, A.dt);
+    else if (A.then == kThenBussi) {
+      c = exp(-A.dt / A.tau);
+      kick = ktarget * (d.x * d.x + d.y) / A.ndof;
+      root = c * (1 - c) * ktarget;
+    }
+    last = before == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  e = 0;
-  for (int q = 0; q < 6; ++q) t[q] = 0;
-  for (int b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-    e += __ldcg(A.part + 7 * b);
-    for (int q = 0; q < A.extra; ++q) t[q] += __ldcg(A.part + 7 * b + 1 + q);
-  }
-  const double tot = block_sum(e, scratch);
-  double tt[6];
-  for (int q = 0; q < A.extra; ++q) tt[q] = block_sum(t[q], scratch);
+#pragma unroll
+  for (int q = 0; q < NS; ++q) s[q] = 0;
+  for (int b = threadIdx.x; b < gridDim.x; b += blockDim.x)
+#pragma unroll
+    for (int q = 0; q < NS; ++q) s[q] += __ldcg(A.part + 7 * b + q);
+  block_sums(s, scratch);
   if (threadIdx.x != 0) return;
   *A.done = 0;
   double* sc = A.sc;
-  double ke = 0.5 * tot / kAcc;
-  if (A.extra == 6)
-    for (int q = 0; q < 6; ++q) sc[kScKin0 + q] = tt[q] / kAcc;
-  if (A.begin) step_begin_body(sc, A.t0, A.t1, A.steps, A.ndof);
-  if (A.then == kThenNhc) {   // the second half of the chain, after the first that the step's first kernel left
-    Chain c = *A.chain_half;
-    sc[kScFactor] = nhc_half(c, ke, sc[kScTnow], A.ndof, A.t_freq, A.dt);
-    *A.chain = c;
+  double ke = 0.5 * s[0] / kAcc;
+  if (NS == 7)
+    for (int q = 1; q < NS; ++q) sc[kScKin0 + q - 1] = s[q] / kAcc;
+  if (A.begin) sc[kScStep] = step, sc[kScTnow] = tnow, sc[kScKtarget] = ktarget;
+  if (A.then == kThenNhc) {
+    sc[kScFactor] = nhc_after(ch, c, ke, tnow, A.ndof, A.dt);
+    *A.chain = ch;
   }
-  sc[A.slot] = ke;
-  if (A.then == kThenBussi) bussi_body(sc, A.draws, A.dt, A.tau, A.ndof);
-  else if (A.then == kThenLang) sc[kScKE0] = 0.5 * tt[0] / kAcc;
-  if (A.then == kThenBath || A.then == kThenLang) sc[kScBath] -= sc[kScKE] - sc[kScKE0];
+  sc[A.slot] = ke;   // kScKE where a thermostat follows
+  if (A.then == kThenBussi) {
+    double factor = 1;
+    if (ke > 0) {
+      const double knew = ke + (1 - c) * (kick - ke) + 2 * d.x * sqrt(root * ke / A.ndof);
+      factor = sqrt(fmax(knew, 0.0) / ke);
+      sc[kScBath] = pre.bath - (knew - ke);
+    }
+    sc[kScFactor] = factor;
+  }
+  double ke0 = pre.ke0;
+  if (NS == 2) sc[kScKE0] = ke0 = 0.5 * s[1] / kAcc;   // kThenLang
+  if (A.then == kThenBath || A.then == kThenLang) sc[kScBath] = pre.bath - (ke - ke0);
+}
+__device__ void ke_blocks(const KeArgs& A, const KePre& pre, double e, const double* t) {
+  if (A.extra == 6) ke_blocks_n<7>(A, pre, e, t);
+  else if (A.extra == 1) ke_blocks_n<2>(A, pre, e, t);
+  else ke_blocks_n<1>(A, pre, e, t);
 }
 
 // Thread c's share: the atoms of its constraint cluster, or its free atom.
@@ -1099,8 +1152,9 @@ __global__ void __launch_bounds__(128) k_move(KickArgs K, ConsArgs C, ListCheck 
   }
   if (L.xb) list_check_flags(L, mb, mp);
   if (A.n > 0) {
+    const KePre pre = ke_pre(A);
     if (!K.lang) cluster_ke(A, C, c, nfree, free_atoms, e, t);
-    ke_blocks(A, e, t);
+    ke_blocks(A, pre, e, t);
   }
 }
 
@@ -1112,17 +1166,20 @@ __global__ void __launch_bounds__(128) k_move(KickArgs K, ConsArgs C, ListCheck 
 __global__ void k_vel_rattle(ConsArgs C, int nfree, const int* __restrict__ free_atoms, const double* __restrict__ x, double* __restrict__ v, VelOp op,
                              double h, double* sc, int* counters, KeArgs K) {
   const int c = cluster_of(C, blockIdx.x * blockDim.x + threadIdx.x);
-  double w[6] = {0, 0, 0, 0, 0, 0};
+  double w[6] = {0, 0, 0, 0, 0, 0}, e = 0, t[6] = {0, 0, 0, 0, 0, 0};
+  const KePre pre = ke_pre(K);
   if (c >= C.ncl && c < C.ncl + nfree) {
     const int g = free_atoms ? free_atoms[c - C.ncl] : c - C.ncl;
-    double vv[3] = {v[3 * g], v[3 * g + 1], v[3 * g + 2]};
-    vel_op(op, g, vv, C.invm, sc);
-    for (int r = 0; r < 3; ++r) v[3 * g + r] = vv[r];
+    const double mi = K.n > 0 ? K.m[g] : 0.0;
+    double vv[3] = {v[3 * g], v[3 * g + 1], v[3 * g + 2]}, ff[3];
+    vel_op(op, g, vv, ff, C.invm, sc);
+    vel_store(op, g, vv, ff, v);
+    if (K.n > 0) ke_share(K, mi, vv, e, t);
   }
-  if (c < C.e1) rattle_star<1>(C, c, x, v, op, sc, h, w, counters);
-  else if (c < C.e2) rattle_star<2>(C, c, x, v, op, sc, h, w, counters);
-  else if (c < C.e3) rattle_star<3>(C, c, x, v, op, sc, h, w, counters);
-  else if (c < C.e4) rattle_water(C, c - C.e3, x, v, op, sc, h, w, counters);
+  if (c < C.e1) rattle_star<1>(C, c, x, v, op, sc, h, w, counters, K, e, t);
+  else if (c < C.e2) rattle_star<2>(C, c, x, v, op, sc, h, w, counters, K, e, t);
+  else if (c < C.e3) rattle_star<3>(C, c, x, v, op, sc, h, w, counters, K, e, t);
+  else if (c < C.e4) rattle_water(C, c - C.e3, x, v, op, sc, h, w, counters, K, e, t);
   else if (c < C.ncl) {
     const int cg = c - C.e4;
     const int k0 = C.cl_start[cg], k1 = C.cl_start[cg + 1], a0 = C.cl_atom0[cg], a1 = C.cl_atom0[cg + 1];
@@ -1131,7 +1188,9 @@ __global__ void k_vel_rattle(ConsArgs C, int nfree, const int* __restrict__ free
     for (int a = 0; a < na; ++a) {
       const int g = C.cl_atoms[a0 + a];
       for (int r = 0; r < 3; ++r) pv[a][r] = v[3 * g + r];
-      vel_op(op, g, pv[a], C.invm, sc);
+      double ff[3];
+      vel_op(op, g, pv[a], ff, C.invm, sc);
+      vel_store(op, g, pv[a], ff, v);
       im[a] = C.invm[g];
     }
     double rr[kMaxClCons][3], lam[kMaxClCons], dd[kMaxClCons];
@@ -1165,6 +1224,7 @@ __global__ void k_vel_rattle(ConsArgs C, int nfree, const int* __restrict__ free
     for (int a = 0; a < na; ++a) {
       const int g = C.cl_atoms[a0 + a];
       for (int r = 0; r < 3; ++r) v[3 * g + r] = pv[a][r];
+      if (K.n > 0) ke_share(K, K.m[g], pv[a], e, t);
     }
     if (h > 0)
       for (int k = 0; k < nk; ++k) {
@@ -1178,20 +1238,16 @@ __global__ void k_vel_rattle(ConsArgs C, int nfree, const int* __restrict__ free
       }
   }
   if (h > 0) {
-    __shared__ double scratch[32];
-    for (int q = 0; q < 6; ++q) {
-      const double s = block_sum(w[q], scratch);
-      if (threadIdx.x == 0 && s != 0) atomicAdd(sc + kScCW0 + q, s);
-    }
+    __shared__ double scratch[6 * 32];
+    block_sums(w, scratch);
+    if (threadIdx.x == 0)
+      for (int q = 0; q < 6; ++q)
+        if (w[q] != 0) atomicAdd(sc + kScCW0 + q, w[q]);
   }
-  // the kinetic energy of the updated velocities (this thread's atoms, read back) and the thermostat update, as k_ke
-  if (K.n > 0) {
-    double e = 0, t[6] = {0, 0, 0, 0, 0, 0};
-    cluster_ke(K, C, c, nfree, free_atoms, e, t);
-    ke_blocks(K, e, t);
-  } else if (K.begin && blockIdx.x == 0 && threadIdx.x == 0) {   // no thermostat: the step's scalars alone
+  // the kinetic energy of the updated velocities and the thermostat update, as k_ke
+  if (K.n > 0) ke_blocks(K, pre, e, t);
+  else if (K.begin && blockIdx.x == 0 && threadIdx.x == 0)   // no thermostat: the step's scalars alone
     step_begin_body(sc, K.t0, K.t1, K.steps, K.ndof);
-  }
 }
 
 
@@ -1200,9 +1256,10 @@ __global__ void k_vel_rattle(ConsArgs C, int nfree, const int* __restrict__ free
 // runs the scalar update. No block waits on another.
 __global__ void k_ke(KeArgs A) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const KePre pre = ke_pre(A);
   double e = 0, t[6] = {0, 0, 0, 0, 0, 0};
   if (i < A.n) ke_atom(A, i, e, t);
-  ke_blocks(A, e, t);
+  ke_blocks(A, pre, e, t);
 }
 
 }  // namespace
