@@ -1822,9 +1822,10 @@ struct Stepper {
   // kinetic energy, thermostat update in its last block). Langevin (BAOAB) takes kick, half drift, O step and half drift in
   // k_move, or with constraints k_move, O + RATTLE, k_move.
   // A thermostat's velocity factor is left pending for the next step's kick (pend_out) where that step follows in the same
-  // graph, or applied at once. pend_in: the step before left one.
+  // graph, or applied at once. pend_in: the step before left one (none without a thermostat that scales).
   void step(bool ener, bool vir, bool pend_in = false, bool pend_out = false) {
     const double dt = o.dt;
+    pend_in = pend_in && (nhc || bussi);
     const double hw = vir ? dt : 0.0;   // the constraint virial only on steps that report it
     if (respa > 1) {
       // r-RESPA (dynamics.cpp:643-657): outer half kick with the slow forces; `respa` velocity-Verlet steps of dt/respa
@@ -2249,6 +2250,8 @@ void MdRun::start_queue() {
   }
   S.sc.alloc(kScNum);
   S.sc.zero(stream_);
+  static const double unscaled = 1;   // the velocity factor until a thermostat writes one
+  CK(cudaMemcpyAsync(S.sc.p + kScFactor, &unscaled, sizeof unscaled, cudaMemcpyHostToDevice, stream_));
   S.chain.alloc(1);
   S.chain_half.alloc(1);
   CK(cudaMemsetAsync(S.chain.p, 0, sizeof(Chain), stream_));
