@@ -657,7 +657,7 @@ static __global__ void __launch_bounds__(128, 3) k_pair_f64(PairArgs A) {
           const double v = comp == 0 ? kx : comp == 1 ? ky : kz;
           double* dst = comp == 0 ? A.fdx : comp == 1 ? A.fdy : A.fdz;
           if (v != 0.0) atomicAdd(dst + 8 * int(en.x) + jq + (i8 & 4), v);
-          if (VIR && v != 0.0) {
+          if (VIR) {   // not for v alone: the lane's second product is another component's, and v may be exactly zero
             const double4 a = xj_s[8 * el + jq + (i8 & 4)], r = xi_s[0];
             acc_wj[0] += (comp == 0 ? a.x - r.x : comp == 1 ? a.y - r.y : a.z - r.z) * v;
             acc_wj[1] += (comp == 1 ? a.y - r.y : a.x - r.x) * (comp == 0 ? ky : kz);
