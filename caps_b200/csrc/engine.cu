@@ -122,6 +122,7 @@ Engine::Engine(const caps_gpu_ff* ff, const caps_gpu_opts* o) {
   int dev = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&dev_sms_, cudaDevAttrMultiProcessorCount, dev));
+  CK(cudaDeviceGetAttribute(&dev_smem_, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
   // the main stream (integrator, list, pair kernel) runs at the highest priority, PME's chain of dependent launches one
   // level below and the bonded terms at the lowest: the chain that leads to the pair kernel takes SM slots first, then

@@ -340,7 +340,7 @@ class Engine {
   int graph_kernels_ = 0;
   long long kernels_run_ = 0;
   DevBuf<unsigned char> d_flush_;
-  int dev_sms_ = 148;
+  int dev_sms_ = 148, dev_smem_ = 0;   // multiprocessors; shared memory a block may ask for
   // The MD state kept between runs (integrate.cu): state and work buffers, pinned scalars, the constraint clusters and
   // the instantiated step graphs, so that a run on the same engine pays none of their set-up again.
   std::unique_ptr<Stepper, StepperDeleter> stepper_;

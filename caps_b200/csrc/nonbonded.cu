@@ -249,8 +249,10 @@ void Engine::pair_forces(bool ener, bool vir) {
     const size_t staged = sizeof(double4) * (size_t(ntab) * ntab + 4 * 64) + sizeof(int) * 4 * 64 +
                           4 * size_t(A.batch) * (sizeof(uint4) + 8 * (sizeof(double4) + sizeof(unsigned long long) + sizeof(int)));
     const size_t table = coul ? sizeof(double4) * size_t(gnodes_) : 0;
-    // a table past about 100 KB leaves room for one block per SM: then through L1 (the rare variants always do)
-    const bool gsm = table <= 100 * 1024;
+    // an Ewald table past about 100 KB leaves room for one block per SM, and one that does not fit beside the LJ table of
+    // many types and the staged entries for none (63 types, 24 entries: 1,776 nodes): then through L1 (the rare variants
+    // always do)
+    const bool gsm = table <= 100 * 1024 && staged + table <= size_t(dev_smem_);
 #define PAIR64LG(C, E, V, CAP, L, F, G)                                                                              \
   do {                                                                                                               \
     const size_t smem = staged + ((G) ? table : 0);                                                                  \
