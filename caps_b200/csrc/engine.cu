@@ -529,6 +529,11 @@ void Engine::set_options(const caps_gpu_opts* o) {
   setup_options();
 }
 
+void Engine::set_list_wait(int polls) {
+  drop_run_state();   // a parameter of the captured list kernels
+  list_polls_ = polls;
+}
+
 std::string Engine::capture_state() const {
   std::string k;
   auto put = [&k](const void* p, size_t bytes) { k.append(static_cast<const char*>(p), bytes); };
@@ -732,6 +737,7 @@ void Engine::check_errors() {
   CK(cudaMemsetAsync(d_counters_.p + kCntFeneClaim, 0, 2 * sizeof(int), stream_));
   d_errinfo_.zero(stream_);
   CK(cudaStreamSynchronize(stream_));
+  if (e & (kErrListBad | kErrImageRange)) list_valid_ = false;   // what the build left is not the list of its positions
   if (e & kErrFene) {   // the reference's text (field.cpp:2157-2159), with the first stretched bond found
     const int b = int(info[kInfoFeneBond]);
     const double r0 = b >= 0 && b < int(h_fene_r0_.size()) ? h_fene_r0_[size_t(b)] : 0.0;
@@ -739,6 +745,7 @@ void Engine::check_errors() {
                                           " Å; lower --dt or relax the structure first");
   }
   if (e & (kErrListOverflow | kErrMaskOverflow | kErrScOverflow)) throw ModelError(-100, "pair list capacity exceeded");
+  if (e & kErrListWait) throw ModelError(CAPS_GPU_ECUDA, "the pair-list kernel gave up waiting for one of its stages");
   if (e & kErrColumnTooBig) throw ModelError(CAPS_GPU_EINVAL, "a grid column holds more atoms than the device sort takes (the cell is too dense or too thin)");
   if (e & kErrExclOverflow) throw ModelError(CAPS_GPU_EINVAL, "too many excluded partners in one super-cluster for the device list");
   if (e & kErrImageRange) throw ModelError(CAPS_GPU_EFIELD, "an excluded pair is more than 63 cells apart: unwrap the molecules first");
@@ -756,7 +763,6 @@ void Engine::check_errors() {
   if (e & kErrNonFinite)   // the reference's text (dynamics.cpp:757), with the step whose positions were not finite
     throw ModelError(CAPS_GPU_EFIELD, "the simulation became unstable at step " + std::to_string((long long)info[kInfoNonFiniteStep]) +
                                           "; lower the time step or relax first");
-  if (e & kErrListWait) throw ModelError(CAPS_GPU_ECUDA, "the pair-list kernel gave up waiting for one of its stages");
   throw ModelError(CAPS_GPU_EINVAL, "device error word " + std::to_string(e));
 }
 
@@ -1104,6 +1110,11 @@ int32_t caps_gpu_diag_set_timing(caps_gpu_engine* e, int64_t flush_bytes) {
   if (!e) return CAPS_GPU_EINVAL;
   e->e->set_timing(flush_bytes);
   return CAPS_GPU_OK;
+}
+
+int32_t caps_gpu_diag_set_list_wait(caps_gpu_engine* e, int32_t polls) {
+  if (!e || polls < 0) return CAPS_GPU_EINVAL;
+  return guard(e, [&] { e->e->set_list_wait(polls); });
 }
 
 int32_t caps_gpu_diag_get_tuning(const caps_gpu_engine* e, int32_t* v) {

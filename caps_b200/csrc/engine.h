@@ -156,6 +156,7 @@ class Engine {
   double last_steps_per_second() const { return last_sps_; }
   // measurement support (include/caps_gpu_diag.h)
   void set_timing(int64_t flush_bytes) { timing_flush_ = flush_bytes; }
+  void set_list_wait(int polls);
   void time_pair_kernel(const double* x, const double* cell, int launches, int64_t flush_bytes, double* avg_ms, double* pairs_in,
                         double* pairs_listed, double* entries);
   void time_phases(const double* x, const double* cell, int launches, int64_t flush_bytes, double* ms);
@@ -337,6 +338,7 @@ class Engine {
 
   double last_sps_ = 0, last_step_ms_ = 0;
   int64_t timing_flush_ = -1;
+  int list_polls_ = kListPolls;
   int graph_kernels_ = 0;
   long long kernels_run_ = 0;
   DevBuf<unsigned char> d_flush_;

@@ -18,7 +18,6 @@ namespace capsb {
 
 enum ListStage { kStBin = 0, kStScan, kStScatter, kStSort, kStSuper, kStSearch, kStPack, kStNum };
 static_assert(kStNum == kCntNum - kCntStage, "a counter per stage");
-constexpr int kListSpin = 1 << 21;   // polls (with a pause of about 0.1 us each) before a wait gives up
 
 struct ListArgs {
   int n, nslots;
@@ -30,6 +29,7 @@ struct ListArgs {
   const uint32_t* excl_list;
   int force;      // 1: build whatever the flag says
   int pack_only;  // 1: a frozen list (no build, no prune)
+  int polls;      // of a wait before it gives up (Engine::list_polls_)
   // pack
   const double* q;
   const int* type;
@@ -174,12 +174,13 @@ union ListShared {
   PruneShared prune;
 };
 
-// Waits (every thread of the block calls it) until `want` units of a stage are finished; false after kListSpin polls.
-__device__ __forceinline__ bool list_wait(int* counters, int stage, int want, int* s_ok) {
+// Waits (every thread of the block calls it) until `want` units of a stage are finished; false after L.polls looks.
+__device__ __forceinline__ bool list_wait(const ListArgs& L, int stage, int want, int* s_ok) {
+  int* counters = L.b.counters;
   if (threadIdx.x == 0) {
     volatile const int* done = counters + kCntStage + stage;
     int k = 0;
-    while (*done < want && k < kListSpin) {
+    while (*done < want && k < L.polls) {
       __nanosleep(64);
       ++k;
     }
@@ -239,25 +240,25 @@ static __global__ void __launch_bounds__(kListThreads, 4) k_list(ListArgs L) {
         list_done(cnt, kStScan);
       }
     } else if (t < e_scat) {
-      if (!list_wait(cnt, kStScan, 1, &s_ok)) break;
+      if (!list_wait(L, kStScan, 1, &s_ok)) break;
       scatter_atom(L.n, (t - e_bin) * kListThreads + threadIdx.x, L.b);
       list_done(cnt, kStScatter);
     } else if (t < e_sort) {
-      if (!list_wait(cnt, kStScatter, nbin, &s_ok)) break;
+      if (!list_wait(L, kStScatter, nbin, &s_ok)) break;
       sort_column(t - e_scat, L.b, S.sort);
       list_done(cnt, kStSort);
     } else if (t < e_super) {
-      if (!list_wait(cnt, kStSort, nsort, &s_ok)) break;
+      if (!list_wait(L, kStSort, nsort, &s_ok)) break;
       super_unit(t - e_sort, L.cell, L.b);
       list_done(cnt, kStSuper);
     } else if (t < e_search) {
-      if (!list_wait(cnt, kStSuper, nsuper, &s_ok)) break;
+      if (!list_wait(L, kStSuper, nsuper, &s_ok)) break;
       const int sc = t - e_super;
       if (sc < min(L.b.counters[kCntNsc], L.b.nsc_cap)) search_supercluster(sc, L.cell, L.g, L.excl_off, L.excl_list, L.b, S.search);
       list_done(cnt, kStSearch);
     } else if (t < e_pack) {
       // the pack reads the slots that the super-clusters' stage made; it runs beside the last of the search
-      if (built && !list_wait(cnt, kStSuper, nsuper, &s_ok)) break;
+      if (built && !list_wait(L, kStSuper, nsuper, &s_ok)) break;
       const int u = t - e_search;
       if (u == 0 && threadIdx.x == 0) {
         cnt[kCntPairNext] = 0;
@@ -267,7 +268,7 @@ static __global__ void __launch_bounds__(kListThreads, 4) k_list(ListArgs L) {
       pack_slot<DBL>(L, u * kListThreads + threadIdx.x, min(L.b.counters[kCntNsc], L.b.nsc_cap), built);
       list_done(cnt, kStPack);
     } else {
-      if (!list_wait(cnt, kStPack, npack, &s_ok) || (built && !list_wait(cnt, kStSearch, nsearch, &s_ok))) break;
+      if (!list_wait(L, kStPack, npack, &s_ok) || (built && !list_wait(L, kStSearch, nsearch, &s_ok))) break;
       const int u = t - e_pack;
       // the positions of this prune, for the next displacement check
       for (int i = u * kListThreads + threadIdx.x; i < 3 * L.n; i += gridDim.x * kListThreads) L.xp[i] = L.x[i];

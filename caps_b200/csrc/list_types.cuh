@@ -9,6 +9,7 @@ constexpr int kClAtoms = 8;
 constexpr int kSortMax = 4096;         // largest column the in-block sort takes
 constexpr int kExclRecMax = 2048;      // exclusion records per super-cluster (64 atoms x 32 partners)
 constexpr int kExclHash = 256;         // distinct (cluster, image) keys of one super-cluster's exclusions
+constexpr int kListPolls = 1 << 21;    // looks (about 0.1 us each) before a wait in the list kernel gives up
 constexpr int kBatch = 32;             // entries per work item
 
 struct ListGeom {

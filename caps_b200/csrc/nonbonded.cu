@@ -135,6 +135,7 @@ void Engine::launch_list(const double* d_x, bool build) {
   L.excl_list = d_excl_list_.p;
   L.force = build ? 1 : 0;
   L.pack_only = frozen_ ? 1 : 0;
+  L.polls = list_polls_;
   L.q = d_q_.p;
   L.type = d_type_.p;
   L.pad_type = nt_;

@@ -281,6 +281,10 @@ class Evaluator:
         """Measurement mode for run(): per-step CUDA events, an L2 flush of flush_bytes between steps (< 0: off)."""
         self._check(self.lib.caps_gpu_diag_set_timing(self.h, int(flush_bytes)))
 
+    def set_list_wait(self, polls: int):
+        """How often a stage of the list kernel looks for the one before it before it gives up (include/caps_gpu_diag.h)."""
+        self._check(self.lib.caps_gpu_diag_set_list_wait(self.h, int(polls)))
+
     def tuning(self) -> list[int]:
         """The tuned launch shapes (include/caps_gpu_diag.h): entries per work item, pair-grid cut, PME grid cap, bonded
         cap, PME line blocks x, y, z."""

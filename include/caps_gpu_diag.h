@@ -14,6 +14,10 @@ extern "C" {
  * stream and, when > 0, writes flush_bytes (larger than the 126 MB L2) between steps, outside the events; < 0 turns it
  * off. caps_gpu_last_steps_per_second then reports K / (sum of the per-step event times). */
 int32_t caps_gpu_diag_set_timing(caps_gpu_engine* e, int64_t flush_bytes);
+/* How many times a stage of the list kernel looks for the one before it before it gives up (about 0.1 us a look; 2^21 at
+ * the start, some hundred times the longest wait): the evaluation then ends with an error, and the next one builds the
+ * list again. Shortened, it shows that path without a kernel that hangs. */
+int32_t caps_gpu_diag_set_list_wait(caps_gpu_engine* e, int32_t polls);
 /* The launch shapes the engine's tuners chose (v[7]: entries per work item, pair-grid blocks per SM left free, PME
  * line-transform grid cap, bonded blocks per term kind, PME line blocks along x, y, z; a cap of 0 means none), and
  * the same shapes pinned on an engine, which then tunes nothing: a profiler, which slows the kernels it replays and
