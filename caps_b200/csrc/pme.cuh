@@ -283,10 +283,12 @@ template <int P>
 constexpr int pme_group() { return P == 3 ? 9 : P == 4 ? 16 : 32; }
 constexpr int kPmeThreads = 128;
 constexpr int kPmeAtoms = 64;   // atoms per block at most
+// The place of grid point (a, b, c) in the grid, row = b K1, plane = K1 K2: past 2^31 for grids of 1,291^3 points and more.
+__host__ __device__ __forceinline__ size_t grid_cell(int a, int row, int c, int plane) { return size_t(c) * size_t(plane) + size_t(row + a); }
 template <class R, int P>
 struct PmeAtom {
   R th[3][P];
-  int at[3][P];   // grid offsets of the P points along each axis
+  int at[3][P];   // the P points along each axis: a, b K1 and c of grid_cell
   R q;
 };
 
@@ -301,7 +303,7 @@ static __global__ void __launch_bounds__(kPmeThreads) k_spread(PmeArgs A, int pe
     R th[3][P], dth[3][P];
     int base[3];
     atom_splines<R, P>(A, i0 + t, th, dth, base);
-    const int K[3] = {A.k1, A.k2, A.k3}, step[3] = {1, A.k1, A.k1 * A.k2};
+    const int K[3] = {A.k1, A.k2, A.k3}, step[3] = {1, A.k1, 1};
 #pragma unroll
     for (int d = 0; d < 3; ++d)
 #pragma unroll
@@ -321,7 +323,7 @@ static __global__ void __launch_bounds__(kPmeThreads) k_spread(PmeArgs A, int pe
       if (P * P * P % G != 0 && pt >= P * P * P) break;
       const int ia = pt % P, ib = pt / P % P, ic = pt / (P * P);
       const R st = a.q * a.th[1][ib] * a.th[2][ic];
-      const int at = a.at[0][ia] + a.at[1][ib] + a.at[2][ic];
+      const size_t at = grid_cell(a.at[0][ia], a.at[1][ib], a.at[2][ic], A.k1 * A.k2);
       const R v = st * a.th[0][ia];
       if (sizeof(R) == 8) atomicAdd(g + at, double(v));
       else atomic_add_fix(gq + at, __float2ll_rn(float(v) * float(kFixQ)));   // the scale is a power of two: no rounding
