@@ -2016,7 +2016,7 @@ struct MdRun {
   size_t n3;
   std::vector<double>& hv;
   int thermo_every = 1, baro_every = 1;
-  long long kernels = 0, emits = 0, baro_steps = 0;
+  long long kernels = 0;   // launched by the steps and rows so far
   int generation = 0;   // bumped whenever this replica's captured step changes (its graphs are dropped)
   SnapRing snaps;
   long long stopped_at = -1;   // the step a stop ended the run at
@@ -2366,11 +2366,13 @@ void MdRun::advance(long long s, bool stop) {
   if (refill_due(s)) {
     S.make_draws(s, draw_chunk(s));
   }
+  const long long before = g_launches;   // outside the graphs every kernel goes through launch_k
   if (mtk()) {
     mtk_step(s);
-    ++baro_steps;
+    kernels += g_launches - before;
   } else if (baro_due(s)) {
     baro_step(s);
+    kernels += g_launches - before;
   } else {
     // energies and virial only for a thermo row: a step that only records, refills or stops runs the plain graph
     kernels += S.launch_step(s % thermo_every == 0 || s == o.steps);
@@ -2381,8 +2383,9 @@ void MdRun::advance(long long s, bool stop) {
   take(s, frame_due(s), (checkpoint_due(s) ? 1 : 0) + (stop && o.checkpoint ? 1 : 0));
   deliver(s);
   if (s % thermo_every == 0 || s == o.steps) {
+    const long long row = g_launches;
     emit(s);
-    ++emits;
+    kernels += g_launches - row;
   }
   if (stop) {
     deliver(s + 1);
@@ -2511,7 +2514,6 @@ void MdRun::baro_step(long long s) {
   (void)s;
   cudaStream_t stream_ = E.stream_;
   S.step(true, true);
-  ++baro_steps;
   S.ke(kScKE, true);
   sync_scalars();
   caps_gpu_terms t{};
@@ -2623,7 +2625,7 @@ void Engine::run(caps_gpu_state* st, const caps_gpu_md_opts* md, caps_gpu_progre
   CK(cudaEventRecord(ev1, stream_));
   CK(cudaEventSynchronize(ev1));
   R.deliver(o.steps + 1);
-  kernels_run_ = R.kernels + R.emits + R.baro_steps * S.graph_kernels[1];
+  kernels_run_ = R.kernels;
   float ms = 0;
   CK(cudaEventElapsedTime(&ms, ev0, ev1));
   const long long done = R.stopped_at >= 0 ? R.stopped_at : o.steps;   // steps run
@@ -2818,7 +2820,7 @@ void run_batch(const std::vector<Engine*>& es, caps_gpu_state* const* states, co
     M.sync_scalars();
     E.last_step_ms_ = done > 0 ? double(ms) / double(done) : 0.0;
     E.last_sps_ = done > 0 && ms > 0 ? double(done) / (ms * 1e-3) : 0.0;
-    E.kernels_run_ = M.kernels + M.emits + (r == 0 ? batch_kernels : 0);
+    E.kernels_run_ = M.kernels + (r == 0 ? batch_kernels : 0);
     const double* px = M.S.pinned_xv(M.n3);   // copied above, before the scalars
     std::memcpy(M.st->x, px, M.n3 * sizeof(double));
     if (M.st->v) std::memcpy(M.st->v, px + M.n3, M.n3 * sizeof(double));

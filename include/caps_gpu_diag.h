@@ -29,8 +29,8 @@ double caps_gpu_diag_last_step_ms(const caps_gpu_engine* e);
 /* Kernel launches in one plain MD step of the last run (the kernel nodes of its captured CUDA graph; the list-build and
  * prune kernels among them return at once on steps that do not need them). */
 int32_t caps_gpu_diag_step_kernels(const caps_gpu_engine* e);
-/* Kernels the last caps_gpu_run launched in its step loop: per step the kernel nodes of the step graph it replayed, plus
- * the kinetic-energy kernel of each thermo row; a barostat step (run outside a graph) counts as one thermo step. */
+/* Kernels the last caps_gpu_run launched in its step loop: per step the kernel nodes of the step graph it replayed, or
+ * the kernels of a step outside a graph (one that rescales the cell), plus those of each thermo row. */
 int64_t caps_gpu_diag_kernels_run(const caps_gpu_engine* e);
 /* List builds and dynamic prunes the engine has run so far (counted on the device; v[0] builds, v[1] prunes). */
 int32_t caps_gpu_diag_list_counts(caps_gpu_engine* e, int64_t* v);
