@@ -214,6 +214,7 @@ class Engine {
   bool sums_cleared_ = false;   // the atom-order force sums were cleared by the integrator's kick (the next forces() skips it)
   bool shapes_tuned_ = false;
   void tune_shapes(const double* d_x);
+  std::function<void()> before_timing_;   // called before shapes are timed: a batch waits for its other replicas
   int list_depth(const ListGeom& g) const;
   template <class R> void fft_passes(PmePath<R>& P, bool ener, bool vir);
   template <class R> void pme_tune(PmePath<R>& P);

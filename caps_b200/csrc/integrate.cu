@@ -2690,6 +2690,13 @@ void run_batch(const std::vector<Engine*>& es, caps_gpu_state* const* states, co
   std::vector<std::unique_ptr<MdRun>> runs;
   for (size_t r = 0; r < R; ++r) {
     runs.emplace_back(new MdRun(*es[r], states[r], mds[r], progress, frame, users ? users[r] : nullptr));
+    struct Alone {   // launch shapes are timed with no earlier replica's first evaluation beside them
+      Engine& e;
+      ~Alone() { e.before_timing_ = nullptr; }
+    } alone{*es[r]};
+    es[r]->before_timing_ = [&es, r] {
+      for (size_t q = 0; q < r; ++q) CK(cudaStreamSynchronize(es[q]->stream_));
+    };
     runs.back()->start_queue();
   }
   for (auto& run : runs) run->start_finish();

@@ -60,6 +60,7 @@ void Engine::join(int k) { CK(cudaStreamWaitEvent(stream_, ev_join_[k], 0)); }
 // Chooses the launch shapes by timing, once per engine, at its first non-bonded evaluation (never inside a capture).
 void Engine::tune_shapes(const double* d_x) {
   shapes_tuned_ = true;
+  if (before_timing_) before_timing_();
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));

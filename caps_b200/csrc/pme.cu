@@ -181,6 +181,7 @@ void Engine::pme_tune(PmePath<R>& P) {
       return;
     }
   }
+  if (before_timing_) before_timing_();
   const size_t half = size_t(ph1_) * pk_[1] * pk_[2];
   CK(cudaMemsetAsync(P.gt.p, 0, half * sizeof(R), stream_));
   CK(cudaMemsetAsync(P.wt.p, 0, 6 * half * sizeof(R), stream_));
