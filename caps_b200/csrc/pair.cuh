@@ -178,11 +178,12 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
   const float rc2 = float(A.rc2), beta = float(A.beta), kc = float(A.kc), kcoul = float(A.kcoul);
   const float2 ku = p_dup(float(A.beta * A.beta / kEwUMax)), nkap3 = p_dup(-float(A.beta * A.beta * A.beta));
   const float e0 = float(A.dsf_e0), f0 = float(A.dsf_f0), rcf = float(A.rc);
-  // energies: every pair's terms rounded to fixed point on their own (2^24 per kcal/mol), so that the totals do not depend
-  // on the list's grouping of pairs. Virial: a lane's at most eight pairs of an entry and half summed by multiply-adds, one
-  // rounding each, then to fixed point (an entry's pairs are the same whatever work item holds it); with six products and
-  // twelve conversions to 64-bit integers per pair this variant took 226 us at 32,000 atoms. From the atoms' force sums
-  // instead (sum x F, as the FP64 kernel) it is off twice as far: those sums' rounding times positions of 20 Å.
+  // energies and virial: every pair's terms rounded to fixed point on their own (2^24 per kcal/mol), so that the totals do
+  // not depend on the list's grouping of pairs. The virial's six products and twelve conversions to 64-bit integers per
+  // pair of pairs take a seventh of this variant's time (32,000 atoms: 223 us; 194 with a lane's pairs of an entry summed in
+  // float first, which drops bits; 214 summed in double, 239 in two floats: no closer to 64 bits, 4.9e-7 of the trace
+  // against 4.8e-7 at 33,000 atoms). From the atoms' force sums instead (sum x F, as the FP64 kernel) it is off twice as
+  // far: those sums' rounding times positions of 20 Å.
   long long acc_v = 0, acc_c = 0, acc_w[6] = {0, 0, 0, 0, 0, 0};
   double acc_np = 0, acc_nl = 0;
   constexpr float kq = 16777216.f;
@@ -284,9 +285,6 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
         t1 = s_tj[8 * el + jq + 4];
       }
       float2 fjx = p_dup(0.f), fjy = p_dup(0.f), fjz = p_dup(0.f);
-      float2 w6[6];   // the entry's virial in the lane
-      if (VIR)
-        for (int k = 0; k < 6; ++k) w6[k] = p_dup(0.f);
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         if (!((imask >> c) & 1u)) continue;
@@ -357,14 +355,12 @@ static __global__ void __launch_bounds__(128, (ENER || VIR) ? 4 : 5) k_pair_f32(
         fix[c] -= fx.x + fx.y;
         fiy[c] -= fy.x + fy.y;
         fiz[c] -= fz.x + fz.y;
-        if (VIR) {
-          w6[0] = p_fma(fx, dx, w6[0]), w6[1] = p_fma(fy, dy, w6[1]), w6[2] = p_fma(fz, dz, w6[2]);
-          w6[3] = p_fma(fx, dy, w6[3]), w6[4] = p_fma(fx, dz, w6[4]), w6[5] = p_fma(fy, dz, w6[5]);
+        if (VIR) {   // fr is 0 for the pairs left out
+          const float2 w6[6] = {p_mul(fx, dx), p_mul(fy, dy), p_mul(fz, dz), p_mul(fx, dy), p_mul(fx, dz), p_mul(fy, dz)};
+#pragma unroll
+          for (int k = 0; k < 6; ++k) acc_w[k] += __float2ll_rn(w6[k].x * kq) + __float2ll_rn(w6[k].y * kq);
         }
       }
-      if (VIR)
-#pragma unroll
-        for (int k = 0; k < 6; ++k) acc_w[k] += __float2ll_rn(w6[k].x * kq) + __float2ll_rn(w6[k].y * kq);
       // j forces: summed over the 8 lanes holding the same j atoms, then one fixed-point add per component
       {
         float kx, ky, kz;

@@ -69,3 +69,29 @@ def test_virial_of_ordered_structures(name, kind):
     tol = 1e-12 if kind != "mixed" else 3e-6
     assert np.abs(np.array(t["w"]) - ref).max() <= tol * size, (t["w"], ref)
     assert abs(t["vdw"] - energy) <= tol * size, (t["vdw"], energy)
+
+
+def test_mixed_sums_do_not_depend_on_how_pairs_are_grouped():
+    """Every pair's energy and virial are rounded to fixed point on their own: the sums over all pairs equal, to the last
+    unit, those of the same atoms with one pair of types interacting at a time, which parts the pairs of each work item."""
+    rng = np.random.default_rng(7)
+    x, edge = _lattice((7, 7, 7), 2.9)
+    x = x + rng.uniform(-0.2, 0.2, x.shape)
+    n, nt = len(x), 4
+    types = rng.integers(0, nt, n)
+
+    def sums(eps):
+        ff = ForceField(type_index=types, charge=np.zeros(n), mass=np.full(n, 12.0), pair_eps=eps, pair_sigma=np.full((nt, nt), SIG),
+                        element=np.full(n, 6))
+        ev = Evaluator(ff, EnergyOptions(cutoff=RC, skin=1.0, coulomb=False, tail=False, precision="mixed"))
+        t, _ = ev.compute(x, np.concatenate([np.zeros(3), np.diag(edge).reshape(-1)]))
+        ev.close()
+        return np.array(t["w"] + [t["vdw"]])
+
+    parts = np.zeros(7)
+    for a in range(nt):
+        for b in range(a, nt):
+            eps = np.zeros((nt, nt))
+            eps[a, b] = eps[b, a] = EPS
+            parts += sums(eps)
+    assert np.array_equal(sums(np.full((nt, nt), EPS)), parts)
