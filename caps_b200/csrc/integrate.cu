@@ -1643,10 +1643,14 @@ struct Stepper {
     return k;
   }
 
-  // A capture costs as much as some twenty plain launches of the step, and the barostats change the cell, a parameter of the
-  // captured kernels: runs with fewer steps than that between rescalings launch their steps directly (6,192 atoms with a
-  // rescaling every 10 steps: 157 us per step with a capture after each, 105 without).
-  bool direct() const { return (o.barostat == 1 || o.barostat == 2) && o.barostat_every < 6; }
+  // The barostats change the cell, a parameter of the captured kernels, so every rescaling is followed by a capture. A single
+  // run's updates its graph in place and pays even every other step: 6,192 atoms, us a step captured / launched directly,
+  // with a rescaling every 2 steps 195 / 203, 4 135 / 147, 10 101 / 114, 31 85 / 100. A batch's graph of every replica's
+  // step is made anew (1.5 ms for six replicas), so its steps go directly up to a rescaling every 31 steps, where that was
+  // faster for every batch measured: six replicas of 2,064 to 16,512 atoms, every 4 steps 1,020 / 590, 10 560 / 404,
+  // 31 332 / 294, 64 288 / 280, 100 266 / 273; two of 2,064 atoms, 31 94 / 90, 48 86 / 88, 200 68 / 84.
+  bool direct = false;   // this run's steps are launched directly (set by run_batch)
+  bool direct_worth() const { return (o.barostat == 1 || o.barostat == 2) && o.barostat_every < 32; }
   bool blocks_worth() const { return !(o.barostat == 1 || o.barostat == 2) || o.barostat_every >= 32; }
 
   // Replays the step graph. It is captured when the run's key differs from the one it was made with; an instantiated
@@ -1654,7 +1658,7 @@ struct Stepper {
   // Returns its kernel count.
   int launch_step(bool thermo) {
     const int k = thermo ? 1 : 0;
-    if (direct()) {
+    if (direct) {
       const long long before = g_launches;
       step(thermo, thermo);
       graph_kernels[k] = int(g_launches - before);
@@ -2030,6 +2034,7 @@ struct MdRun {
   MdRun(Engine& e, caps_gpu_state* state, const caps_gpu_md_opts* md, caps_gpu_progress_fn prog, caps_gpu_frame_fn fr, void* u)
       : E(e), o(*md), st(state), progress(prog), frame(fr), user(u), S(kept_state(e)), n3(size_t(3) * e.n_), hv(S.hv) {
     S.o = *md;
+    S.direct = false;
   }
   // a run that ended in an error may have left its captured steps half-way: the next run captures them again
   ~MdRun() {
@@ -2567,7 +2572,7 @@ void MdRun::baro_step(long long s) {
   }
   S.forces(true, true);
   S.ke(kScKE, false);   // the rescaled velocities' kinetic energy, which the next Nose-Hoover step starts from
-  S.drop_graphs();   // the cell is a parameter of the captured kernels (a run with few steps per cell captures none)
+  S.drop_graphs();   // the cell is a parameter of the captured kernels
   ++generation;
 }
 
@@ -2592,7 +2597,7 @@ void Engine::run(caps_gpu_state* st, const caps_gpu_md_opts* md, caps_gpu_progre
   }
   // the step graphs are captured before the step loop, as set-up (like the first force evaluation), so that no step's
   // time holds a capture
-  if (o.steps > 0 && !R.mtk() && !S.direct() && !R.baro_due(1) && !R.refill_due(1)) {
+  if (o.steps > 0 && !R.mtk() && !R.baro_due(1) && !R.refill_due(1)) {
     S.ensure_graph(false);
     if (S.blocks_worth()) S.ensure_graph(true);
     if (!timed && S.blocks_worth() && o.steps > Stepper::kBlockSteps) S.ensure_graph(false, true);
@@ -2726,7 +2731,8 @@ void run_batch(const std::vector<Engine*>& es, caps_gpu_state* const* states, co
   // atoms), for 1 to 8 ms more to capture
   long long batch_kernels = 0, graph_nodes = 0;
   bool direct = true;
-  for (size_t r = 0; r < R; ++r) direct = direct && runs[r]->S.direct();
+  for (size_t r = 0; r < R; ++r) direct = direct && runs[r]->S.direct_worth();
+  for (size_t r = 0; r < R; ++r) runs[r]->S.direct = direct;
   bool on_replicas = true;   // the replicas' own streams hold the latest work
   // orders the batch stream after every replica stream, or every replica stream after the batch stream
   auto join_to_batch = [&] {
