@@ -628,22 +628,35 @@ void Engine::set_cell(const double* cell) {
   }
 }
 
-// Entries per work item of the pair list, from the size of the system alone (so that equal systems get equal work items
-// and the mixed path's sums repeat). A work item is one warp's serial work, and the pair kernel has about 20 warps per SM:
-// a small system needs shallow items to occupy them at all, a large one deep items, which share the staging and the
-// force sums of the super-cluster's 64 atoms. Measured pair kernel, us, at 2 / 8 / 16 / 24 entries: 3,900 entries in all
-// 13 / 20 / 29 / 37, 19,400 entries 22 / 22 / 33 / 42, 36,600 entries 33 / 29 / 36 / 47, 246,000 entries 169 / 111 / 108 /
-// 110, 1,800,000 entries 1242 / 686 / 608 / 587. The entries are estimated from the density: half the clusters whose boxes
-// can come within the list radius of a super-cluster's, times 1.5 for the boxes' real shapes and the columns' ends.
+// Entries per work item of the pair list, from the system's size, cell and list radius and the GPU's size, so that equal
+// systems on equal GPUs get equal work items and the mixed path's sums repeat; a cell rescaled across a threshold changes
+// the depth. A work item is one warp's serial work, and the FP32 pair kernel has about 20 warps per SM: a small system
+// needs shallow items to occupy them at all, a large one deep items, which share the staging and the force sums of the
+// super-cluster's 64 atoms. Measured pair kernel, us, at 2 / 4 / 8 / 16 / 24 entries per item, by entries per warp (1.3:
+// 594 atoms, 83: 32,000):
+//         1.3   13 / 15 / 19 / 26 / 33      FP64   17 / 19 / 25 / 36 / 45
+//         2.6   15 / 16 / 20 / 29 / 37             20 / 20 / 25 / 37 / 46
+//         4.1   18 / 17 / 22 / 29 / 36             24 / 23 / 26 / 38 / 45
+//         6.8   23 / 21 / 23 / 31 / 40             32 / 29 / 29 / 40 / 46
+//          12   32 / 28 / 28 / 35 / 41             48 / 40 / 40 / 44 / 55
+//          25   54 / 44 / 41 / 44 / 47             83 / 66 / 61 / 63 / 79
+//          83  168 /125 /109 /105 /108            263 /202 /179 /174 /217
+//         199  370 /267 /222 /203 /200            578 /428 /366 /339 /429
+// (1,800,000 entries in FP32, 608 per warp: 608 us at 16, 587 at 24). The FP64 kernel's staging takes twice the shared
+// memory and at 24 entries leaves room for one block less per SM, so its items stop at 16. The entries are estimated from
+// the density: half the clusters whose boxes can come within the list radius of a super-cluster's, times 1.5 for the
+// boxes' real shapes and the columns' ends.
 int Engine::list_depth(const ListGeom& g) const {
   const double rho = double(n_) / dcell_.vol, R = g.rlist, s = 1.5 * std::cbrt(64.0 / rho);
   const double reach = s * s * s + 6 * s * s * R + 3 * kPi * s * R * R + 4.0 / 3.0 * kPi * R * R * R;
   const double entries = 1.5 * (n_ / 64.0 + 0.5 * g.ncol) * 0.5 * reach * rho / 8.0;
   const double per_warp = entries / (20.0 * dev_sms_);
   // The mixed path sums a work item's i forces in float, so the depth shows in their last bits. In melts of hard beads (no
-  // Coulomb) that grows past 1e-4 of the velocities within two hundred steps: their depth stays what it has been.
+  // Coulomb) that grows past 1e-4 of the velocities within two hundred steps. Their depth is 16 whatever their size, so that
+  // their trajectories stay bit for bit what they were before the depth followed the size; up to 5,000 beads that costs some
+  // 10 us a launch (13 at 2 entries, 23 at 16).
   if (mixed_ && !coul_) return 16;
-  return per_warp < 3 ? 2 : per_warp < 5 ? 4 : per_warp < 20 ? 8 : per_warp < 200 ? 16 : 24;
+  return per_warp < 3 ? 2 : per_warp < 5 ? 4 : per_warp < 20 ? 8 : per_warp < 200 || !mixed_ ? 16 : 24;
 }
 
 void Engine::ensure_list_capacity() {

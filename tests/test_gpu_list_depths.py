@@ -87,3 +87,16 @@ def test_against_direct_sum(name, depth, precision):
     got = out["v"].reshape(-1, 3) * 12.0 / (3 * dt * ACC)
     assert np.abs(got - f).max() <= 10 * max(tol, 1e-8) * np.abs(f).max()
     ev.close()
+
+
+def test_fp64_work_items_stop_at_sixteen_entries():
+    """Deeper ones take a block per SM from the FP64 pair kernel (98,304 atoms: 429 us a launch at 24 entries, 339 at 16)."""
+    m, a = 48, 2.2
+    x = (np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3) + 0.5) * a
+    n = len(x)
+    ff = ForceField(type_index=np.zeros(n, int), charge=np.zeros(n), mass=np.full(n, 12.0), pair_eps=[[0.1]], pair_sigma=[[2.0]],
+                    element=np.full(n, 6))
+    ev = Evaluator(ff, EnergyOptions(cutoff=12.0, skin=2.0, electrostatics="dsf", precision="double"))
+    ev.compute(x, np.concatenate([np.zeros(3), np.diag([m * a] * 3).reshape(-1)]))
+    assert ev.tuning()[0] == 16
+    ev.close()
