@@ -225,10 +225,12 @@ void Engine::pme_run(PmePath<R>& P, const double* d_x, bool ener, bool vir) {
   }
   // enough blocks of the spread for two per SM where atoms are few
   const int pb = std::clamp(n_ / (2 * dev_sms_), 8, kPmeAtoms), nb = blocks_for(size_t(n_), pb);
+  const bool big = grid_needs_64(pk_[0], pk_[1], pk_[2]);
 #define SPREAD(P_)                                                                            \
   do {                                                                                        \
-    if (mixed_) launch_k(k_spread<float, P_>, nb, kPmeThreads, 0, stream_, A, pb, d_grid_.p, d_gridq_.p);      \
-    else launch_k(k_spread<double, P_>, nb, kPmeThreads, 0, stream_, A, pb, d_grid_.p, d_gridq_.p);            \
+    auto* kernel = mixed_ ? (big ? k_spread<float, P_, size_t> : k_spread<float, P_, int>)    \
+                          : (big ? k_spread<double, P_, size_t> : k_spread<double, P_, int>); \
+    launch_k(kernel, nb, kPmeThreads, 0, stream_, A, pb, d_grid_.p, d_gridq_.p);              \
   } while (0)
   switch (order_) {
     case 3: SPREAD(3); break;

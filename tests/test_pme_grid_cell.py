@@ -1,5 +1,5 @@
-"""Where the PME spread writes a grid point (caps_b200/csrc/pme.cuh, grid_cell), compiled for the host: grids up to past 2^31
-points, as long as a line transform can be along one axis."""
+"""Where the PME spread writes a grid point (caps_b200/csrc/pme.cuh, grid_place), compiled for the host: grids up to past 2^31
+points, as long as a line transform can be along one axis, and which of them take places of 64 bits."""
 from __future__ import annotations
 
 import shutil
@@ -15,7 +15,17 @@ SOURCE = """
 #include "pme.cuh"
 int main() {
   int k1, k2, a, b, c;
-  while (std::scanf("%d %d %d %d %d", &k1, &k2, &a, &b, &c) == 5) std::printf("%zu\\n", capsb::grid_cell(a, b * k1, c, k1 * k2));
+  int k3;
+  while (std::scanf("%d %d %d %d %d %d", &k1, &k2, &k3, &a, &b, &c) == 6) {
+    size_t wide = 0;
+    int narrow = 0;
+    const bool needs = capsb::grid_needs_64(k1, k2, k3);
+    const int p[3] = {a, b, c};
+    for (int d = 0; d < 3; ++d) wide += capsb::grid_place<size_t>(p[d], d, k1, k2);
+    if (!needs)
+      for (int d = 0; d < 3; ++d) narrow += capsb::grid_place<int>(p[d], d, k1, k2);
+    std::printf("%d %zu %d\\n", int(needs), wide, narrow);
+  }
 }
 """
 
@@ -26,11 +36,14 @@ def test_grid_cell_past_32_bits(tmp_path):
     subprocess.run([NVCC, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", str(ROOT / "caps_b200" / "csrc"),
                     str(tmp_path / "cell.cu"), "-o", str(tmp_path / "cell")], check=True)
     asked = []
-    for k in [(9, 10, 12), (70, 70, 70), (1280, 1296, 1280), (1296, 1296, 1296), (4800, 700, 800), (27, 9600, 9600)]:
+    for k in [(9, 10, 12), (70, 70, 70), (1280, 1296, 1280), (1296, 1296, 1296), (4800, 700, 800), (27, 9600, 9600), (1024, 1024, 2048),
+              (1024, 1024, 2047), (7, 7, 7 ** 8)]:
         for p in [(0, 0, 0), (k[0] - 1, 0, 0), (0, k[1] - 1, 0), (0, 0, k[2] - 1), tuple(n - 1 for n in k), tuple(n // 2 for n in k)]:
             asked.append((k, p))
-    text = "\n".join(f"{k[0]} {k[1]} {p[0]} {p[1]} {p[2]}" for k, p in asked)
-    got = subprocess.run([str(tmp_path / "cell")], input=text, capture_output=True, text=True, check=True).stdout.split()
-    for (k, p), g in zip(asked, got):
-        assert int(g) == p[0] + k[0] * (p[1] + k[1] * p[2]), (k, p)
-    assert max(int(g) for g in got) > 2 ** 31
+    text = "\n".join(" ".join(map(str, k + p)) for k, p in asked)
+    got = subprocess.run([str(tmp_path / "cell")], input=text, capture_output=True, text=True, check=True).stdout.splitlines()
+    for (k, p), line in zip(asked, got):
+        needs, wide, narrow = map(int, line.split())
+        at = p[0] + k[0] * (p[1] + k[1] * p[2])
+        assert needs == (k[0] * k[1] * k[2] > 2 ** 31 - 1) and wide == at and (needs or narrow == at), (k, p)
+    assert {line[0] for line in got} == {"0", "1"}
