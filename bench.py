@@ -668,7 +668,7 @@ def main():
         line = {
             "metric": METRIC, "value": value, "unit": "ns/day", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "f32 pair/PME spread-gather, int64 fixed-point sums, f64 FFT/bonded/integrator", "data": "synthetic", "config": cfg,
+            "dtype": "f32 pair/PME (FFT included), int64 fixed-point sums, f64 bonded/integrator", "data": "synthetic", "config": cfg,
             "atom_steps_per_s": sps * n * world,
             "list_builds": builds,
             "fp64": {"ns_per_day": nsd64 * world, "ms_per_step": ms64, "steps": k64, "mixed_speedup": ms64 / ms_step},
@@ -690,7 +690,7 @@ def main():
                                       "peak_source": peaks["source"],
                                       "frac": (PAIR_DRAM_BYTES / (pt["avg_ms"] * 1e-3) / 1e9) / peaks["hbm_gbs"] if peaks.get("hbm_gbs") else None}},
             "gpu_launches": launches,
-            "gpu_launches_note": "kernels launched in the timed step loop, counted by the engine: the step graphs' kernel nodes per replayed step (list-build and prune kernels included; they return at once on steps without a build or prune), plus one kinetic-energy kernel per thermo row",
+            "gpu_launches_note": "kernels launched in the timed step loop, counted by the engine: the step graphs' kernel nodes per replayed step (one list kernel among them, whatever the list needs), plus those of each thermo row",
             "clocks": clk.summary(),
             "cpu_baseline": cpu,
             "cpu_baseline_fp64": cpu64,

@@ -521,8 +521,9 @@ __device__ __forceinline__ double pair_f64(const PairArgs& A, const EwaldTab& T,
 // batch of loads into shared memory, a lane's pairs of an entry in one 16-bit word, and both of the lane's j atoms of an
 // entry evaluated side by side, so that two independent chains of FP64 operations fill the pipe's latency. FROZEN: the
 // pairs are those of the frozen set (A.frozen), whatever their distance now (field.cpp:1700).
-// Bound by FP64 issue: 46 double operations per pair (a division and a square root made it 75) on half-rate units, 3 warps
-// per scheduler. GSM: the Ewald table in shared memory (else read through L1, for tables too large for it).
+// Bound by its dependent chains: 46 double operations per pair (a division and a square root made it 75) with three blocks,
+// 11 warps, per SM keep the FP64 pipe 37 % busy and 47 % of the issue slots (32,000 atoms, 176 us); the stalls are fixed-latency
+// waits, shared memory and the work items' loads. GSM: the Ewald table in shared memory (else read through L1, for tables too large for it).
 template <int COUL, bool ENER, bool VIR, bool CAP = false, bool LJ96 = false, bool FROZEN = false, bool GSM = true>
 static __global__ void __launch_bounds__(128, 3) k_pair_f64(PairArgs A) {
   extern __shared__ double4 smem_d4[];
