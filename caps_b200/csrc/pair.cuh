@@ -523,7 +523,9 @@ __device__ __forceinline__ double pair_f64(const PairArgs& A, const EwaldTab& T,
 // pairs are those of the frozen set (A.frozen), whatever their distance now (field.cpp:1700).
 // Bound by its dependent chains: 46 double operations per pair (a division and a square root made it 75) with three blocks,
 // 11 warps, per SM keep the FP64 pipe 37 % busy and 47 % of the issue slots (32,000 atoms, 176 us); the stalls are fixed-latency
-// waits, shared memory and the work items' loads. GSM: the Ewald table in shared memory (else read through L1, for tables too large for it).
+// waits, shared memory and the work items' loads. The rare variants keep the loop over the i clusters rolled: sixteen copies of
+// their pair code missed the instruction cache (a force cap at 32,000 atoms 518 us a launch unrolled, 297 rolled, i forces in
+// local memory and all; frozen pairs 595 and 269). GSM: the Ewald table in shared memory (else read through L1, for tables too large for it).
 template <int COUL, bool ENER, bool VIR, bool CAP = false, bool LJ96 = false, bool FROZEN = false, bool GSM = true>
 static __global__ void __launch_bounds__(128, 3) k_pair_f64(PairArgs A) {
   extern __shared__ double4 smem_d4[];
@@ -613,7 +615,7 @@ static __global__ void __launch_bounds__(128, 3) k_pair_f64(PairArgs A) {
       const double4 a0 = xj_s[8 * el + jq], a1 = xj_s[8 * el + jq + 4];
       const int t0 = tj_s[8 * el + jq], t1 = tj_s[8 * el + jq + 4];
       double f0x = 0, f0y = 0, f0z = 0, f1x = 0, f1y = 0, f1z = 0;
-#pragma unroll
+#pragma unroll(CAP || FROZEN ? 1 : 8)
       for (int c = 0; c < 8; ++c) {
         if (!((imask >> c) & 1u)) continue;
         const double4 xi = xi_s[8 * c + i8];

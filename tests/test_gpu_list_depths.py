@@ -89,6 +89,22 @@ def test_against_direct_sum(name, depth, precision):
     ev.close()
 
 
+@pytest.mark.parametrize("kind", ["a force cap that nothing reaches", "frozen pairs"])
+@pytest.mark.parametrize("name", list(CELLS))
+def test_fp64_rare_variants_against_direct_sum(name, kind):
+    ff, x, edges, vdw, coul, w, f, sizes = _system(name)
+    cell = np.concatenate([np.zeros(3), edges.reshape(-1)])
+    ev = Evaluator(ff, EnergyOptions(cutoff=RC, skin=1.2, electrostatics="dsf", dsf_alpha=ALPHA, tail=False, precision="double",
+                                     force_cap=1e6 if "cap" in kind else 0.0))
+    if kind == "frozen pairs":
+        ev.freeze_pairs(x, cell)
+    t, force = ev.compute(x, cell)
+    ev.close()
+    assert abs(t["vdw"] - vdw) <= 1e-9 * sizes[0] and abs(t["coulomb"] - coul) <= 1e-9 * sizes[1]
+    assert np.abs(np.array(t["w"]) - w).max() <= 1e-9 * sizes[2]
+    assert np.abs(force - f).max() <= 1e-8 * np.abs(f).max()
+
+
 def test_fp64_work_items_stop_at_sixteen_entries():
     """Deeper ones take a block per SM from the FP64 pair kernel (98,304 atoms: 429 us a launch at 24 entries, 339 at 16)."""
     m, a = 48, 2.2
