@@ -615,8 +615,12 @@ static __global__ void __launch_bounds__(128, 3) k_pair_f64(PairArgs A) {
       const double4 a0 = xj_s[8 * el + jq], a1 = xj_s[8 * el + jq + 4];
       const int t0 = tj_s[8 * el + jq], t1 = tj_s[8 * el + jq + 4];
       double f0x = 0, f0y = 0, f0z = 0, f1x = 0, f1y = 0, f1z = 0;
-#pragma unroll(CAP || FROZEN ? 1 : 8)
-      for (int c = 0; c < 8; ++c) {
+      // i clusters in a turn (two loops, not an unroll count on one: with that the plain variants took 177.6 us, not 175.6)
+      constexpr int kTurn = CAP || FROZEN ? 1 : 8;
+#pragma unroll 1
+      for (int c0 = 0; c0 < 8; c0 += kTurn)
+#pragma unroll
+      for (int c = c0; c < c0 + kTurn; ++c) {
         if (!((imask >> c) & 1u)) continue;
         const double4 xi = xi_s[8 * c + i8];
         const int ti = ti_s[8 * c + i8];
